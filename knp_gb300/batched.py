@@ -88,8 +88,8 @@ def uneven_config(seed: int = 8, batch: int = 40, sizes=(96, 128, 64, 10), t_lo:
 
 class BatchedPlan:
     """A batch prepared on the device (knp_gb300_batched_plan_create) and run as one CUDA-graph
-    launch per ``run()``; with ``autotune`` the operand ring depth and the layer ring length are
-    chosen by timing each pair, ``stages`` fixes the depth (0: the deepest that fits)."""
+    launch per ``run()``; with ``autotune`` the operand ring depth is chosen by timing each,
+    ``stages`` fixes it (0: the deepest)."""
 
     def __init__(self, cfg: BatchedConfig, record: bool = False, autotune: bool = False, device: int = 0,
                  segment_steps: int = 0, stages: int = 0):
@@ -136,7 +136,7 @@ class BatchedPlan:
         return int(events.value), float(ms.value)
 
     def info(self):
-        """(operand ring depth, layer ring length, {(depth, ring length): ms of the autotuning run})."""
+        """(operand ring depth, 4, {(depth, 4): ms of the autotuning run}); depths alone are tuned."""
         st = ctypes.c_int(0)
         ring = ctypes.c_int(0)
         t = (ctypes.c_float * 9)()

@@ -6,7 +6,9 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstdint>
+#include <functional>
 #include <memory>
+#include <queue>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -142,7 +144,7 @@ int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, in
 // Batched LIF network (batched / precision form).
 //
 // B independent samples of a feed-forward LIF network (layers of sizes n_0 -> n_1 -> ... -> n_L,
-// all-to-all, delay 1) advance together. Semantics per neuron are the reference LIF
+// all-to-all, delay 1). Semantics per neuron are the reference LIF
 // (knp/backends/cpu/cpu-library/include/knp/backends/cpu-library/impl/populations/lif/lif_impl.h:33-86):
 // outside the refractory period V = V * leak + I, spike iff V > threshold, then V = reset and the
 // counter = period; inside it the counter counts down and input is ignored. Layer l's input at
@@ -150,164 +152,248 @@ int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, in
 // whose spike of source i for sample b at step t is the counter-based Bernoulli draw
 // rand64(key, (t * B + b) * n_0 + i) >> 11 < rate[b][i] * 2^53. Sample b runs steps [0, T_b).
 //
-// Each step of a layer is a BF16 GEMM of the 0/1 spike matrix (exact in BF16) against BF16 weights
-// with FP32 accumulation in tensor memory. A CTA pair (a cluster of two) owns (layer, 128-sample
-// tile, 64-neuron tile): each CTA multiplies one half of the K range against its half of the weight
-// tile (resident in shared memory for the whole run), sends the partner the partial sums of the 32
-// neurons the partner finalises (st.async into the partner's shared memory) and finalises its own
-// 32 neurons, whose LIF state stays in registers.
+// The network is feed-forward, so a layer's input of every step is known once the layer below has
+// run all of its steps: the layers run one after another, and a layer is one matrix product over all
+// (sample, step) columns with the LIF recurrence in its epilogue. The product is taken as
+// D[neuron][column] = W[neuron][k] * S[column][k]: an accumulator row (tensor-memory lane) is one
+// neuron and its columns are consecutive steps of one sample, so the thread that owns the lane runs
+// the recurrence down its row with the membrane state in registers, and no step waits for another
+// CTA. (Stepping all layers together, one step at a time, costs a chain of expansion, product,
+// exchange and hand-over per step: 0.87-0.95 ms for 256 samples of 784-1000-1000-10 and 50-200 steps,
+// the tensor cores idle for most of it; see the kernel for this form's time.)
 //
-// Spikes travel between layers as bitmaps (one 32-bit word per sample and 32 neurons) in a ring of
-// R steps per layer (R tuned, at most kMaxRing). A consumer expands its K half chunk by chunk into BF16 operand chunks in
-// tensor memory (one sample row per lane) while the tensor cores multiply the previous chunk. There
-// is no grid-wide barrier: per (layer, sample tile, ring slot) counters record how
-// many times the layer's CTAs have written the slot (`ready`) and how many times consumer CTAs have
-// read it (`consumed`), so a layer starts step t as soon as every CTA of the layer below has
-// published step t - 1, and overwrites a slot only after every consumer has read it (a layer runs
-// at most R - 2 steps ahead of its consumers). Counting per slot matters: CTAs of one layer are
-// not in lockstep, and a sum over all slots would let a fast CTA stand in for a slow one. Input spikes do not depend on the network, so
-// a separate kernel draws them ahead of the run (layer 0's slots hold every step of a segment; long
-// runs are cut into segments, the LIF state saved and restored between them). Samples are processed
-// sorted by decreasing T, so finished samples leave whole sample tiles idle. Every wait is bounded.
+// Spikes travel between layers as bitmaps: per layer one row of wpad words (bit j of word w = neuron
+// 32 w + j) for every (sample, step) of a segment of steps, a sample's rows consecutive:
+// row_base[s] + j is what the step t0 + j of the layer above reads, i.e. the spikes of step
+// t0 + j - 1. Long runs are cut into segments; LIF state and each sample's last spikes carry over.
 namespace knp_gb300
 {
 namespace
 {
 
-constexpr int kBM = 128, kBN = 32, kBK = 128, kMaxLayers = 4, kMaxItems = 512;
-constexpr int kPairN = 2 * kBN;                 // neurons of a CTA pair's tile; each CTA finalises kBN
+constexpr int kMaxLayers = 4;
+constexpr uint32_t kTileN = 128;      // neurons of a CTA (accumulator rows)
+constexpr uint32_t kStreamCols = 128;  // columns of one stream in a tile (two streams per CTA)
+constexpr uint32_t kCols = 2 * kStreamCols;
+constexpr uint32_t kChunk = 64;                      // K of a staged chunk
+constexpr uint32_t kAChunk = kTileN * kChunk * 2;   // 16 KB of packed weights
+constexpr uint32_t kBChunk = kCols * kChunk * 2;    // 32 KB of expanded spikes
+constexpr uint32_t kLayerStage = kAChunk + kBChunk;
 constexpr int kMinStages = 2, kMaxStages = 4;  // operand ring depths the autotuner tries
-constexpr uint32_t kAccCols = 2 * kPairN;        // tensor-memory columns of the two accumulators
-constexpr uint32_t kStageCols = kBK / 2;         // tensor-memory columns of one 128 x 128 BF16 operand chunk
-constexpr uint32_t kTmemCols = 512;              // the whole tensor memory (one CTA per SM)
-constexpr size_t kMinDynSmem = size_t(120) << 10;  // keeps a second CTA off the SM (it would wait for tensor memory)
-static_assert(kAccCols + kMaxStages * kStageCols <= kTmemCols, "operand stages exceed tensor memory");
-constexpr uint32_t kChunkWords = kBK / 32;       // bitmap words per sample row and chunk
-constexpr uint32_t kMaxHalfChunks = 8;           // chunks of a K half (bounded by shared memory)
-constexpr uint32_t kMaxRing = 16;                // bitmap steps kept per layer at most (counter stride)
-constexpr uint32_t kRingChoices[3] = {4, 8, 16};   // ring lengths the autotuner tries
-constexpr uint32_t kDefaultRing = 8;
-constexpr uint32_t kXchBytes = kBM * kBN * 4;    // one exchange buffer: [kBM][kBN] FP32 partial sums
-constexpr uint32_t kPollLimit = 1u << 22;        // polls of a cross-CTA counter before giving up
-constexpr int kExpandWarps = 4, kEpilogueWarps = 8;  // warps 0-3 expand, 4-11 epilogue, 12 issues
-constexpr int kIssuerWarp = kExpandWarps + kEpilogueWarps;
-constexpr int kExpandThreads = 32 * kExpandWarps, kEpilogueThreads = 32 * kEpilogueWarps;
-constexpr int kBatchThreads = kExpandThreads + kEpilogueThreads + 32;
-constexpr int kEN = 16;                  // neurons per epilogue thread (two threads per sample row)
-constexpr int kStateWords = 3 * kEN;  // V, refractory counter, spike count of an epilogue thread's neurons
-constexpr uint32_t kCntBytes = kBM * kBN * 4;  // last layer's spike counts of a tile, [kBN][kBM] int
-constexpr size_t kInputSlotBudget = size_t(256) << 20;  // bytes of layer 0's slots per segment
+constexpr int kExpandWarps = 8, kScanWarps = 8;
+constexpr int kIssuerWarp = 0, kCopyWarp = 1, kScanWarp0 = 4, kExpandWarp0 = kScanWarp0 + kScanWarps;
+constexpr int kLayerThreads = 32 * (kExpandWarp0 + kExpandWarps);
+constexpr uint32_t kTmemCols = 512;  // two accumulators of kCols columns
+constexpr uint32_t kScanCols = 32;   // columns a scan thread reads from its accumulator at a time
+constexpr uint32_t kPad = 8;         // a sample's columns in a stream are padded to a multiple of this
+constexpr uint32_t kNoRow = 0xFFFFFFFFu;
+constexpr uint32_t kMaxFanIn = 2048;
+constexpr size_t kMinDynSmem = size_t(120) << 10;  // one CTA per SM (a second would wait for tensor memory)
+constexpr size_t kRowBudget = size_t(256) << 20;   // bytes of a layer's rows per segment
+constexpr uint32_t kMaxTiles = 512;  // (layer, 128-sample tile, 64-neuron tile, half) units a plan may have
 
-struct BatchedNet
+// What one launch of a layer needs. A stream is a list of samples whose columns follow one another;
+// CTA (n tile, g) runs streams 2 g and 2 g + 1 side by side, one per half of its columns, so that the
+// scans of two warpgroups share the SM while the next tile's product runs.
+struct LayerArgs
 {
-    int n_layers;
-    uint32_t size[kMaxLayers + 1];
-    uint32_t words[kMaxLayers + 1];   // ceil(size / 32)
-    uint32_t kpad[kMaxLayers + 1];    // kpad[l] = size[l - 1] rounded up to 16 (layer l's K)
-    uint32_t chunks[kMaxLayers + 1];  // chunks[l] = ceil(kpad[l] / 128)
-    uint32_t wpad[kMaxLayers + 1];    // wpad[l] = 4 * chunks[l + 1]: words per sample row of layer l's slots
-    uint32_t n_cta[kMaxLayers + 1];   // CTAs of layer l per sample tile
-    const __nv_bfloat16 *w[kMaxLayers];
-    float leak[kMaxLayers], thr[kMaxLayers], reset[kMaxLayers];
-    uint32_t refract[kMaxLayers];
-    uint32_t batch, m_tiles;
-    const uint32_t *perm;  // slot -> sample
-    const uint32_t *act;   // [t_max]: slots still running at step t (slots sorted by decreasing T)
-    const unsigned long long *rate_thr;  // [batch][size[0]] by sample: rate * 2^53, the draw's threshold
-    // Optional per-sample layer sizes ([batch] by sample, <= size[l]); neurons and inputs beyond a
-    // sample's size do not exist for it (never spike). Null: every sample has the full sizes.
-    const uint32_t *sample_size[kMaxLayers + 1];
-    unsigned long long key;
-    uint32_t t_max;
-    // bits[l]: spikes of layer l as layer l + 1's input, [slot][m tile][kBM][wpad[l]] words (bit j of
-    // word w = neuron 32 w + j, words past words[l] zero). Layer 0: slot j of a segment starting at
-    // step t0 = input drawn at step t0 + j - 1 (nothing before step 0). Layers >= 1: ring slots,
-    // slot (t + 1) % ring written at step t.
-    uint32_t *bits[kMaxLayers];
-    uint32_t ring;           // steps kept per layer ring (3 .. kMaxRing)
-    unsigned int *ready;     // [kMaxLayers + 1][m_tiles][kMaxRing]: writes of layer l's slot by its CTAs
-    unsigned int *consumed;  // [kMaxLayers + 1][m_tiles][kMaxRing]: reads of layer l's slot by layer l + 1's CTAs
-    uint32_t *state;         // [n_items][kEpilogueThreads][kStateWords]: LIF state between segments
-    int *counts;             // [batch][size[L]] by sample
-    uint32_t *record;        // [t_max][sum_l batch * words[l]] by sample, or null
-    unsigned long long rec_off[kMaxLayers + 1];
-    unsigned long long rec_stride;
+    const uint8_t *w;         // packed weights: [n tile][chunk] blocks of kAChunk bytes (pack_weights_kernel)
+    const uint32_t *bits_in;  // rows of the layer below
+    uint32_t wp_in;           // words per row (a multiple of 4)
+    uint32_t *bits_out;       // this layer's rows (null for the last layer)
+    uint32_t wp_out;
+    uint32_t n;               // neurons
+    uint32_t kp;              // fan-in rounded up to 16
+    uint32_t chunks;          // ceil(kp / kChunk)
+    uint32_t n_groups;        // CTAs per neuron tile
+    float leak, thr, reset;
+    uint32_t refract;
+    const uint32_t *st_off;   // [2 n_groups + 1] first entry of each stream
+    const uint32_t *st_len;   // [2 n_groups] columns of each stream (padding included)
+    const uint32_t *st_start;  // per entry: the sample's first column in its stream
+    const uint4 *st_info;     // per entry: sample, its first row, its columns in this segment, its steps in all
+    const uint32_t *own_size, *next_size;  // per-sample sizes of this layer and of the next, or null
+    uint32_t next_n;          // fan-out of a spike (0 for the last layer)
+    uint32_t t0, t1;
+    uint32_t *carry;          // [batch][wp_out] last spikes of a sample that goes on in the next segment
+    uint32_t *state;          // [batch][n][3] its potentials, refractory counters and spike counts
+    int *counts;              // [batch][n], last layer only
+    uint32_t *record;         // or null
+    unsigned long long rec_off, rec_stride;
+    uint32_t wn;              // words of a recorded row
     unsigned long long *events;
-    unsigned int *err;       // bit 0: a wait gave up; bit 1: launched without the 2-CTA cluster shape
-    uint32_t poll_limit;     // polls of a cross-CTA ring counter before a wait gives up
-    uint32_t stall;          // failure test: consumers wait for this many more producer CTAs than exist
-    uint32_t n_items;
-    uint16_t item_layer[kMaxItems];
-    uint16_t item_m[kMaxItems];
-    uint16_t item_n[kMaxItems];  // kPairN-neuron tile index
-    uint8_t item_k[kMaxItems];   // K half = rank in the cluster: items 2i and 2i + 1 are one tile
+    unsigned int *err;        // bit 0: a wait gave up
+    uint32_t poll_limit;
+    uint32_t stall;           // failure test: the issuer waits for this many more expanders than exist
+    uint32_t stages;          // operand ring depth
 };
 
-// Per (sample, input): the 53-bit threshold that the input draw is compared with, rate * 2^53
-// truncated, computed exactly from the FP32 rate's fields (no FP64 on the device): m * 2^(e - 97)
-// for a normal rate in (0, 1) with 24-bit significand m and biased exponent e; 0 for rates <= 0,
-// subnormal or NaN; 2^53 (every draw is below it) for rates >= 1.
-__global__ void rate_threshold_kernel(const float *rates, unsigned long long *thr, size_t n)
+// Position p of a 16-wide K block holds input (p >> 1) + 8 (p & 1) of the block, in the packed
+// weights and in the expanded spikes alike: one word of two BF16 elements then comes from bits i and
+// 8 + i of the block's 16 spike bits, which one shift and one mask isolate.
+__host__ __device__ constexpr uint32_t k_of(uint32_t p) { return (p >> 1) + 8u * (p & 1u); }
+
+// Weights of one layer, BF16 [n][k] row-major (any k), to [n tile][chunk] blocks in the 128-byte
+// swizzled K-major layout of tc::smem_desc_sw128, zero past n and k. One thread per 16 bytes. Repacked
+// in every run (the caller may rewrite the weights between runs): 4 MB, 3 us at 784-1000-1000-10.
+struct PackArgs
 {
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t bits = __float_as_uint(rates[i]);
-    const uint32_t e = (bits >> 23) & 0xFFu;
-    unsigned long long v = 0;
-    if ((bits >> 31) == 0u && e != 0u && e != 0xFFu)
+    const __nv_bfloat16 *w[kMaxLayers];
+    uint8_t *out[kMaxLayers];
+    uint32_t n[kMaxLayers], k[kMaxLayers], chunks[kMaxLayers];
+    unsigned long long first[kMaxLayers + 1];  // first unit of each layer
+    int n_layers;
+};
+
+__global__ void pack_weights_kernel(const __grid_constant__ PackArgs a)
+{
+    const unsigned long long total = a.first[a.n_layers];
+    for (unsigned long long u = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; u < total;
+         u += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
     {
-        const unsigned long long m = (bits & 0x7FFFFFu) | 0x800000u;
-        if (e >= 127u)
-            v = 1ull << 53;
-        else if (e >= 97u)
-            v = m << (e - 97u);
-        else if (97u - e < 64u)
-            v = m >> (97u - e);
+        int l = 0;
+        while (u >= a.first[l + 1]) ++l;
+        const unsigned long long v = u - a.first[l];
+        const uint32_t slot = static_cast<uint32_t>(v & 7u);
+        const uint32_t r = static_cast<uint32_t>((v >> 3) & (kTileN - 1));
+        const unsigned long long blk = v >> 10;  // n tile * chunks + chunk
+        const uint32_t chunk = static_cast<uint32_t>(blk % a.chunks[l]);
+        const uint32_t row = static_cast<uint32_t>(blk / a.chunks[l]) * kTileN + r;
+        __nv_bfloat16 e[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i)
+        {
+            const uint32_t k = chunk * kChunk + (slot >> 1) * 16u + k_of((slot & 1u) * 8u + i);
+            e[i] = (row < a.n[l] && k < a.k[l]) ? a.w[l][static_cast<size_t>(row) * a.k[l] + k] : __float2bfloat16(0.0f);
+        }
+        *reinterpret_cast<uint4 *>(a.out[l] + blk * kAChunk + r * 128u + ((slot ^ (r & 7u)) << 4)) =
+            *reinterpret_cast<uint4 *>(e);
     }
-    else if ((bits >> 31) == 0u && e == 0xFFu && (bits & 0x7FFFFFu) == 0u)
-    {
-        v = 1ull << 53;  // +infinity
-    }
-    thr[i] = v;
 }
 
-// Layer 0's slots of the segment [t0, t1): slot j = the input spikes drawn at step t0 + j - 1, one
-// thread per bitmap word (32 draws). Also writes layer 0's record and adds the synaptic events of
-// each step drawn; the last segment has one extra row of words (j = t1 - t0, the draws of step
-// t_max - 1) that no layer reads.
-__global__ void input_bits_kernel(BatchedNet net, uint32_t t0, uint32_t t1)
+// The 53-bit threshold an input draw is compared with, rate * 2^53 truncated, computed exactly from
+// the FP32 rate's fields (no FP64 on the device): m * 2^(e - 97) for a normal rate in (0, 1) with
+// 24-bit significand m and biased exponent e; 0 for rates <= 0, subnormal or NaN; 2^53 (every draw is
+// below it) for rates >= 1.
+__device__ __forceinline__ unsigned long long rate_threshold(float rate)
 {
-    const uint32_t wp = net.wpad[0], w0 = net.words[0], n_in = net.size[0];
-    const uint32_t span = t1 - t0 + (t1 == net.t_max ? 1u : 0u);
-    const size_t per_slot = static_cast<size_t>(net.m_tiles) * kBM * wp;
-    const size_t total = span * per_slot;
-    unsigned long long ev = 0;
-    for (size_t u = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < total;
-         u += static_cast<size_t>(gridDim.x) * blockDim.x)
+    const uint32_t bits = __float_as_uint(rate);
+    const uint32_t e = (bits >> 23) & 0xFFu;
+    if (bits >> 31) return 0ull;
+    if (e == 0xFFu) return (bits & 0x7FFFFFu) ? 0ull : 1ull << 53;  // NaN, +infinity
+    if (e == 0u) return 0ull;
+    const unsigned long long m = (bits & 0x7FFFFFu) | 0x800000u;
+    if (e >= 127u) return 1ull << 53;
+    if (e >= 97u) return m << (e - 97u);
+    return 97u - e < 64u ? m >> (97u - e) : 0ull;
+}
+
+// Transposes a 32 x 32 bit matrix held one row per lane: afterwards bit j of lane c is what bit c of
+// lane j was.
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, uint32_t lane)
+{
+    uint32_t mask = 0x0000FFFFu;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1)
     {
-        const uint32_t j = static_cast<uint32_t>(u / per_slot);
-        const uint32_t rem = static_cast<uint32_t>(u - static_cast<size_t>(j) * per_slot);
-        const uint32_t row = rem / wp, w = rem - row * wp;  // row = m tile * kBM + slot row
-        const uint32_t t = t0 + j;                           // the step that consumes the draws of t - 1
-        uint32_t word = 0;
-        if (t >= 1 && w < w0 && row < net.act[t - 1])
-        {
-            const uint32_t s = t - 1, smp = net.perm[row];
-            const uint32_t lim = net.sample_size[0] ? min(n_in, net.sample_size[0][smp]) : n_in;
-            const unsigned long long base = (static_cast<unsigned long long>(s) * net.batch + smp) * n_in;
-            const unsigned long long *thr = net.rate_thr + static_cast<size_t>(smp) * n_in;
-            const uint32_t i0 = w * 32;
-            for (uint32_t b = 0; b < 32 && i0 + b < lim; ++b)
-                if ((rand64(net.key, base + i0 + b) >> 11) < thr[i0 + b]) word |= 1u << b;
-            if (net.record)
-                net.record[s * net.rec_stride + net.rec_off[0] + static_cast<size_t>(smp) * w0 + w] = word;
-            ev += static_cast<unsigned long long>(__popc(word)) *
-                  (net.sample_size[1] ? net.sample_size[1][smp] : net.size[1]);
-        }
-        if (j < t1 - t0) net.bits[0][u] = word;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, m);
+        x = (lane & m) ? ((x & ~mask) | ((y & ~mask) >> m)) : ((x & mask) | ((y & mask) << m));
+        mask ^= mask << (m >> 1);
     }
+    return x;
+}
+
+struct DrawArgs
+{
+    const float *rates;  // [batch][n_in]
+    uint32_t n_in, wp, words, batch;
+    const uint32_t *size0, *size1;  // per-sample sizes or null
+    uint32_t n1;
+    const uint4 *rows;  // per sample: first row, columns in this segment
+    uint32_t t0, blocks;  // blocks of 32 rows per sample
+    unsigned long long key;
+    uint32_t *bits;
+    uint32_t *record;
+    unsigned long long rec_stride;
+    unsigned long long *events;
+};
+
+// Layer 0's rows: row j of a sample = the inputs drawn at step t0 + j - 1 (zero before step 0), for j
+// in [0, columns]. A warp takes one word (32 inputs, a lane each, the threshold in a register) of 32
+// consecutive rows, a bit per row, and one transposition across the warp gives the rows' words; a draw is
+// counted and recorded in the segment where it is not row 0. Bound by the draws' integer instructions (two
+// 64-bit products each, half-rate pipes): one lane per input keeps the rate loads coalesced and one
+// threshold serves 32 draws.
+__global__ void __launch_bounds__(256) input_rows_kernel(const __grid_constant__ DrawArgs a)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long items = static_cast<unsigned long long>(a.batch) * a.blocks * a.wp;
+    const unsigned long long warps = static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
+    unsigned long long ev = 0;
+    for (unsigned long long it = blockIdx.x * static_cast<unsigned long long>(blockDim.x >> 5) + (threadIdx.x >> 5);
+         it < items; it += warps)
+    {
+        const uint32_t w = static_cast<uint32_t>(it % a.wp);
+        const unsigned long long sb = it / a.wp;
+        const uint32_t smp = static_cast<uint32_t>(sb / a.blocks), j0 = 32u * static_cast<uint32_t>(sb % a.blocks);
+        const uint4 info = a.rows[smp];
+        const uint32_t cols = info.y;
+        if (cols == 0u || j0 > cols) continue;
+        const uint32_t i = 32u * w + lane;
+        const uint32_t lim = a.size0 ? min(a.n_in, a.size0[smp]) : a.n_in;
+        const unsigned long long thr = i < lim ? rate_threshold(a.rates[static_cast<size_t>(smp) * a.n_in + i]) : 0ull;
+        uint32_t word = 0;  // of row j0 + lane
+        if (w < a.words)
+        {
+            const uint32_t n_rows = min(32u, cols + 1u - j0);
+            // The draw of row j is that of step t0 + j - 1; row 0 of the first segment has none.
+            const uint32_t c0 = a.t0 + j0 == 0u ? 1u : 0u;
+            // rand64(key, ctr) with ctr * G + C carried from step to step by one addition; its first mixing
+            // step y ^ (y >> 30) of y = x ^ key is x ^ (x >> 30) ^ (key ^ (key >> 30)); and (r >> 11) < thr
+            // is r < thr << 11, which the high words decide unless they are equal (2^-32 of the draws), so
+            // the last mixing step's low word is rarely formed.
+            constexpr unsigned long long kG = 0x9E3779B97F4A7C15ull, kC = 0x632BE59BD9B4E019ull;
+            const unsigned long long inc = static_cast<unsigned long long>(a.batch) * a.n_in * kG;
+            const unsigned long long key1 = a.key ^ (a.key >> 30);
+            unsigned long long x =
+                ((static_cast<unsigned long long>(a.t0 + j0 + c0 - 1u) * a.batch + smp) * a.n_in + i) * kG + kC;
+            const bool always = thr >> 53;  // thr << 11 would be 2^64
+            const uint32_t t_hi = always ? 0xFFFFFFFFu : static_cast<uint32_t>(thr >> 21);
+            const uint32_t t_lo = always ? 0xFFFFFFFFu : static_cast<uint32_t>(thr << 11);
+            uint32_t fired = 0;  // bit c: this input fires in row j0 + c
+            auto draw = [&](uint32_t c)
+            {
+                unsigned long long y = (x ^ (x >> 30) ^ key1) * 0xBF58476D1CE4E5B9ull;
+                y = (y ^ (y >> 27)) * 0x94D049BB133111EBull;
+                const uint32_t hi = static_cast<uint32_t>(y >> 32), r_hi = hi ^ (hi >> 31);
+                if (r_hi < t_hi) fired |= 1u << c;
+                if (r_hi == t_hi && (always || static_cast<uint32_t>(y ^ (y >> 31)) < t_lo)) fired |= 1u << c;
+                x += inc;
+            };
+            if (c0 == 0u && n_rows == 32u)
+            {
+#pragma unroll
+                for (uint32_t c = 0; c < 32; ++c) draw(c);
+            }
+            else
+            {
+                for (uint32_t c = c0; c < n_rows; ++c) draw(c);
+            }
+            word = warp_transpose_bits(fired, lane);
+        }
+        const uint32_t j = j0 + lane;
+        if (j > cols) continue;
+        a.bits[(static_cast<size_t>(info.x) + j) * a.wp + w] = word;
+        if (j >= 1u && w < a.words)
+        {
+            if (a.record)
+                a.record[static_cast<size_t>(a.t0 + j - 1u) * a.rec_stride + static_cast<size_t>(smp) * a.words + w] = word;
+            ev += static_cast<unsigned long long>(__popc(word)) * (a.size1 ? a.size1[smp] : a.n1);
+        }
+    }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) ev += __shfl_down_sync(0xffffffffu, ev, o);
-    if ((threadIdx.x & 31) == 0 && ev) atomicAdd(net.events, ev);
+    if (lane == 0 && ev) atomicAdd(a.events, ev);
 }
 
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *mbar, uint32_t bytes)
@@ -317,581 +403,515 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *mbar, uint32_t b
                  : "memory");
 }
 
-// Whether this CTA (its shared failure flag) or any CTA of the launch (the error word) has given up.
-__device__ __forceinline__ bool failed(const volatile int *flag, const unsigned int *gerr)
+// Copies `bytes` (a multiple of 16, both addresses 16-byte aligned) into shared memory, completing
+// them on the mbarrier's transaction count.
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *mbar)
 {
-    return *flag != 0 || *reinterpret_cast<const volatile unsigned int *>(gerr) != 0u;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(tc::smem_u32(mbar))
+                 : "memory");
 }
 
-// Polls (acquire, bounded) until *counter >= target; false after `limit` polls or once a failure has
-// been reported (checked every 64 polls).
-__device__ __forceinline__ bool poll_at_least(const unsigned int *counter, unsigned int target, uint32_t limit,
-                                              const volatile int *flag, const unsigned int *gerr)
+// mbar_wait that also gives up as soon as another role of the CTA has.
+__device__ __forceinline__ bool wait_or_fail(uint64_t *mbar, uint32_t parity, uint32_t limit, const volatile int *fail)
 {
     for (uint32_t i = 0; i < limit; ++i)
     {
-        unsigned int cur;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(counter) : "memory");
-        if (static_cast<int>(cur - target) >= 0) return true;
-        if ((i & 63u) == 63u && failed(flag, gerr)) return false;
-    }
-    return false;
-}
-
-// mbar_wait that also gives up as soon as a failure has been reported (checked after each poll).
-__device__ __forceinline__ bool wait_or_fail(uint64_t *mbar, uint32_t parity, const volatile int *flag,
-                                             const unsigned int *gerr)
-{
-    for (uint32_t i = 0; i < kWaitLimit; ++i)
-    {
         if (tc::mbar_try_wait(mbar, parity)) return true;
-        if (failed(flag, gerr)) return false;
+        if (*fail) return false;
     }
     return false;
 }
 
-__device__ __forceinline__ bool wait_cluster_or_fail(uint64_t *mbar, uint32_t parity, const volatile int *flag,
-                                                     const unsigned int *gerr)
+// wait_or_fail for a whole warp: one lane polls (32 lanes suspended on a barrier cost its other users),
+// every lane gets the outcome. The whole warp calls it.
+__device__ __forceinline__ bool warp_wait(uint64_t *mbar, uint32_t parity, uint32_t limit, const volatile int *fail,
+                                          uint32_t lane)
 {
-    for (uint32_t i = 0; i < kWaitLimit; ++i)
+    int ok = 1;
+    if (lane == 0) ok = wait_or_fail(mbar, parity, limit, fail);
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// The 16 spike bits `h` of a K block as its 16 BF16 elements (8 words): word i = bit i in the low half
+// and bit 8 + i in the high half, as 1.0 (0x3F80 = 127 << 7) or 0.
+__device__ __forceinline__ void expand16(uint32_t h, uint32_t *v)
+{
+    const uint32_t z = __byte_perm(h, 0u, 0x4140);  // byte 0 to the low half, byte 1 to the high half
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = ((z << (7 - i)) & 0x00800080u) * 127u;
+}
+
+__device__ __forceinline__ void st_shared_v4(uint32_t dst, const uint32_t *v)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+
+// One scan warp's share of a layer: 32 neurons of one stream.
+struct ScanTarget
+{
+    uint32_t tmem;      // its lanes and its stream's columns of accumulator 0
+    uint32_t off, len;  // its stream's first entry and its columns
+    uint32_t neuron, wq;  // this thread's neuron, the warp's word in a row
+    uint32_t n_tiles;
+};
+
+// The LIF recurrence of one stream down its accumulator columns (lif_impl.h:33-86: leak and input only
+// outside the refractory period; strict '>'; reset to a value). A thread reads kScanCols columns at a
+// time and collects its spikes as one word, a bit per column; a transposition across the warp turns 32
+// neurons' words into the columns' bitmap words, so a step costs five instructions and no vote. A
+// sample's columns are padded to a multiple of kPad, so that kPad steps at a time need no check
+// for its end. Returns false if a wait gave up.
+template <bool kRefract>
+__device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget &tgt, uint32_t lane, uint64_t *acc_full,
+                                            uint64_t *acc_empty, const volatile int *fail, unsigned long long &events)
+{
+    const float leak = a.leak, thr = a.thr, reset = a.reset;
+    // The sample being scanned (sample, first row, columns, steps in all), its next step (from t0), and
+    // this neuron's state; the next sample's entry is loaded ahead.
+    uint32_t entry = tgt.off, j = 0, fan = 0;
+    uint4 info = make_uint4(0, 0, 0, 0), next = info;
+    bool exists = false;
+    float V = 0.0f;
+    uint32_t RC = 0, count = 0, last_word = 0;
+    uint32_t end = 0;  // the stream column after the sample's last (padded)
+    auto open_sample = [&]()
     {
-        if (tc::mbar_try_wait_cluster(mbar, parity)) return true;
-        if (failed(flag, gerr)) return false;
-    }
-    return false;
-}
-
-// A counter read ahead of need (relaxed: later memory operations do not wait for it). A value
-// found sufficient is followed by fence_acquire() before the data it guards is touched.
-__device__ __forceinline__ unsigned int load_relaxed(const unsigned int *counter)
-{
-    unsigned int v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void fence_acquire() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
-// Whether *counter >= target: from a value read ahead if that suffices, else by polling.
-__device__ __forceinline__ bool reached(const unsigned int *counter, unsigned int target, unsigned int seen,
-                                        uint32_t limit, const volatile int *flag, const unsigned int *gerr)
-{
-    if (static_cast<int>(seen - target) >= 0)
+        info = next;
+        j = 0;
+        end += (info.z + kPad - 1) / kPad * kPad;
+        if (end < tgt.len) next = a.st_info[entry + 1];
+        const uint32_t smp = info.x;
+        exists = tgt.neuron < (a.own_size ? a.own_size[smp] : a.n);
+        fan = a.next_size ? a.next_size[smp] : a.next_n;
+        V = 0.0f;
+        RC = count = 0;
+        if (a.t0 != 0u && tgt.neuron < a.n)
+        {
+            const uint32_t *st = a.state + (static_cast<size_t>(smp) * a.n + tgt.neuron) * 3;
+            V = __uint_as_float(st[0]);
+            RC = st[1];
+            count = st[2];
+        }
+        // The row before the segment's first step: the last spikes of the previous segment.
+        if (a.bits_out && lane == 0)
+            a.bits_out[static_cast<size_t>(info.y) * a.wp_out + tgt.wq] =
+                a.t0 ? a.carry[static_cast<size_t>(smp) * a.wp_out + tgt.wq] : 0u;
+    };
+    auto close_sample = [&]()
     {
-        fence_acquire();
-        return true;
+        const uint32_t smp = info.x;
+        if (info.w <= a.t1)
+        {
+            if (a.counts && tgt.neuron < a.n)
+                a.counts[static_cast<size_t>(smp) * a.n + tgt.neuron] = static_cast<int>(count);
+        }
+        else
+        {
+            if (tgt.neuron < a.n)
+            {
+                uint32_t *st = a.state + (static_cast<size_t>(smp) * a.n + tgt.neuron) * 3;
+                st[0] = __float_as_uint(V);
+                st[1] = RC;
+                st[2] = count;
+            }
+            if (a.bits_out && lane == 0) a.carry[static_cast<size_t>(smp) * a.wp_out + tgt.wq] = last_word;
+        }
+        ++entry;
+    };
+    if (tgt.len)
+    {
+        next = a.st_info[entry];
+        open_sample();
     }
-    return poll_at_least(counter, target, limit, flag, gerr);
+    for (uint32_t tile = 0; tile < tgt.n_tiles; ++tile)
+    {
+        const uint32_t acc = tile & 1u;
+        if (!warp_wait(&acc_full[acc], (tile >> 1) & 1u, a.poll_limit, fail, lane)) return false;
+        tc::fence_after_sync();
+        const uint32_t p0 = tile * kStreamCols;
+        const uint32_t valid = tgt.len > p0 ? min(kStreamCols, tgt.len - p0) : 0u;  // a multiple of kPad
+        for (uint32_t c0 = 0; c0 < kStreamCols; c0 += kScanCols)
+        {
+            const uint32_t here = valid > c0 ? min(kScanCols, valid - c0) : 0u;  // uniform
+            float x[kScanCols];
+            if (here) tc::tmem_ld32(tgt.tmem + acc * kCols + c0, x);
+            if (here < kScanCols || c0 + kScanCols == kStreamCols)
+            {
+                // The last columns of this tile are in registers: the accumulator may be reused.
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&acc_empty[acc]);
+            }
+            if (!here) break;
+            uint32_t bits = 0;  // bit c: this neuron fired at column c0 + c
+            auto step = [&](uint32_t c)
+            {
+                const float v = __fadd_rn(__fmul_rn(V, leak), x[c]);
+                if (kRefract)
+                {
+                    const bool free_ = RC == 0u;
+                    const bool spike = exists && free_ && v > thr;
+                    V = spike ? reset : (free_ ? v : V);
+                    RC = spike ? a.refract : (free_ ? 0u : RC - 1u);
+                    if (spike) bits |= 1u << c;
+                }
+                else
+                {
+                    const bool spike = exists && v > thr;
+                    V = spike ? reset : v;
+                    if (spike) bits |= 1u << c;
+                }
+            };
+            // Columns [from, to) of this block, steps j0 .. of the sample, are done: their bitmap words go
+            // out, one lane each.
+            auto flush = [&](uint32_t from, uint32_t to, uint32_t j0)
+            {
+                const uint32_t span = to - from == 32u ? 0xFFFFFFFFu : ((1u << (to - from)) - 1u) << from;
+                count += __popc(bits & span);
+                const uint32_t word = warp_transpose_bits(bits & span, lane);
+                last_word = __shfl_sync(0xffffffffu, word, static_cast<int>(to - 1u));
+                if (lane >= from && lane < to)
+                {
+                    const uint32_t jj = j0 + (lane - from);
+                    if (a.bits_out)
+                    {
+                        a.bits_out[(static_cast<size_t>(info.y) + jj + 1u) * a.wp_out + tgt.wq] = word;
+                        events += static_cast<unsigned long long>(__popc(word)) * fan;
+                    }
+                    if (a.record && tgt.wq < a.wn)
+                        a.record[static_cast<size_t>(a.t0 + jj) * a.rec_stride + a.rec_off +
+                                 static_cast<size_t>(info.x) * a.wn + tgt.wq] = word;
+                }
+            };
+            uint32_t from = 0, j_from = j;  // first column not flushed, and its step
+#pragma unroll
+            for (uint32_t sb = 0; sb < kScanCols; sb += kPad)
+            {
+                if (sb >= here) break;
+                const uint32_t left = info.z - j;
+                if (left >= kPad)
+                {
+#pragma unroll
+                    for (uint32_t i = 0; i < kPad; ++i) step(sb + i);
+                    j += kPad;
+                }
+                else
+                {
+#pragma unroll
+                    for (uint32_t i = 0; i < kPad; ++i)
+                        if (i < left) step(sb + i);
+                    j += left;
+                }
+                if (j == info.z)
+                {
+                    flush(from, sb + min(left, kPad), j_from);
+                    close_sample();
+                    if (p0 + c0 + sb + kPad < tgt.len) open_sample();
+                    from = sb + kPad;
+                    j_from = 0;
+                }
+            }
+            if (from < here) flush(from, here, j_from);
+            if (here < kScanCols) break;
+        }
+    }
+    return true;
 }
 
-__device__ __forceinline__ void release_add(unsigned int *counter)
-{
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-}
-
-// Roles of the 13 warps: warps 0-3 expand the input bitmaps into the operand ring (one sample row
-// per thread), warps 4-11 run the epilogue (one sample row and 16 of the CTA's 32 neurons per
-// thread), lane 0 of warp 12 issues the MMAs. Two accumulators in tensor memory let the MMAs of
-// step s + 1 run while the epilogue of step s exchanges partial sums and updates the neurons.
-template <int kStages>
-__global__ void __launch_bounds__(kBatchThreads, 1) batched_lif_kernel(BatchedNet net, uint32_t t0, uint32_t t1)
+// One layer over a segment of steps. Roles: warps 0-7 expand spike rows into the BF16 operand, warps
+// 8-15 run the LIF scan (thread = neuron; warps 8-11 the first stream's half of the accumulator, 12-15
+// the second's), warp 16 copies packed weight chunks, warp 17 issues the MMAs (M = 128 neurons, N = 256
+// columns, FP32 accumulator in tensor memory, two of them, so the scan of a tile runs beside the product
+// of the next). Every wait is bounded; a wait that gives up sets bit 0 of *err, stops the roles, lets
+// copies and MMAs in flight land, and frees the tensor memory.
+// kGroups: groups of expander warps that take the chunks in turn. Every stage of the ring belongs to one
+// group (the ring depth is a multiple of kGroups), so that a group waiting for a stage's next release
+// has seen the release before it: a parity wait cannot tell phases two apart.
+template <int kGroups>
+__global__ void __launch_bounds__(kLayerThreads, 1) lif_layer_kernel(const __grid_constant__ LayerArgs a)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t full_w[kMaxStages], full_s[kMaxStages], empty[kMaxStages];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], drain;
     __shared__ uint32_t tmem_slot;
-    __shared__ __align__(8) uint64_t full[kStages];   // operand stage b written (kExpandThreads arrivals)
-    __shared__ __align__(8) uint64_t empty[kStages];  // the MMAs that read stage b have completed (commit)
-    __shared__ __align__(8) uint64_t acc_full[2];     // every MMA into accumulator a has completed (commit)
-    __shared__ __align__(8) uint64_t acc_empty[2];    // the epilogue has read accumulator a (kEpilogueThreads)
-    __shared__ __align__(8) uint64_t xfull[2];        // the partner's partial sums of a step have landed
-    __shared__ __align__(8) uint64_t drain;           // every MMA this CTA issued has completed (teardown)
+    __shared__ int s_fail;
     __shared__ unsigned long long s_events;
-    __shared__ int s_fail;  // some role gave up on a wait (each group reads it through one thread)
-    __shared__ uint32_t s_half[2][2][kBM];  // [step parity][neuron half][row]: epilogue spike masks
-    // Exchange bookkeeping for the teardown: steps whose partial sums this CTA sent to its partner,
-    // exchange phases it received, phases it armed; the partner's sent count (written by the partner).
-    __shared__ uint32_t s_sent, s_recv, s_armed, s_peer_sent;
-    // A launch without the two-CTA cluster shape (every CTA sees the same count) stops here, before
-    // any access to a partner's shared memory.
-    if (tc::cluster_nctarank() != 2u)
-    {
-        if (threadIdx.x == 0) atomicOr(net.err, 2u);
-        return;
-    }
-    const uint32_t item = blockIdx.x;
-    const int layer = net.item_layer[item];  // 1..L
-    const uint32_t m_tile = net.item_m[item];
-    const uint32_t m0 = m_tile * kBM;
-    // The pair's tile is neurons np0 .. np0 + 63 over all K; this CTA multiplies K half kh of it and
-    // finalises neurons n0 .. n0 + 31 (half kh of the tile) after adding the partner's partial sums.
-    const uint32_t kh = net.item_k[item];
-    const uint32_t np0 = net.item_n[item] * kPairN;
-    const uint32_t n0 = np0 + kBN * kh;
-    const uint32_t K = net.size[layer - 1], Kp = net.kpad[layer], N = net.size[layer];
-    const uint32_t wn = net.words[layer];
-    const uint32_t n_chunks_all = net.chunks[layer];
-    const uint32_t c_mid = (n_chunks_all + 1) / 2;
-    const uint32_t c_lo = kh ? c_mid : 0u, c_hi = kh ? n_chunks_all : c_mid;
-    const uint32_t n_chunks = c_hi - c_lo;  // this CTA's chunks (<= kMaxHalfChunks)
-    const uint32_t Kw = c_mid * kBK;        // K extent of the weight tile (the larger half)
-    // Shared memory: weight tile [kPairN x Kw] (K-major core matrices), two exchange buffers, the
-    // last layer's spike counts. Tensor
-    // memory: two accumulators (columns [0, kAccCols)), then kStages operand stages of kStageCols.
-    uint8_t *sW = smem;
-    uint8_t *sX = smem + static_cast<size_t>(kPairN) * Kw * 2;
-    const uint32_t sbo_w = (Kw / 8) * 128;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    // Weight tile rows np0..np0+63 (zero beyond N), inputs c_lo * 128 + [0, Kw) (zero beyond K).
-    for (uint32_t u = threadIdx.x; u < kPairN * (Kw / 8); u += blockDim.x)
-    {
-        const uint32_t r = u / (Kw / 8), g = u % (Kw / 8), n = np0 + r, k = g * 8, kg = c_lo * kBK + k;
-        __nv_bfloat16 tmp[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            tmp[e] = (n < N && kg + e < K) ? net.w[layer - 1][static_cast<size_t>(n) * K + kg + e]
-                                           : __float2bfloat16(0.0f);
-        *reinterpret_cast<uint4 *>(sW + tc::core_offset(r, k, 128, sbo_w)) = *reinterpret_cast<uint4 *>(tmp);
-    }
+    __shared__ uint32_t s_row[2][kCols];  // [tile parity][column]: its row of bits_in, or kNoRow
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t n_tile = blockIdx.x / a.n_groups, group = blockIdx.x - n_tile * a.n_groups;
     if (warp == kIssuerWarp) tc::tmem_alloc(&tmem_slot, kTmemCols);
     if (threadIdx.x == 0)
     {
-        for (int b = 0; b < kStages; ++b)
+        for (int s = 0; s < kMaxStages; ++s)
         {
-            tc::mbar_init(&full[b], kExpandThreads);
-            tc::mbar_init(&empty[b], 1);
+            tc::mbar_init(&full_w[s], 1);
+            tc::mbar_init(&full_s[s], kExpandWarps / kGroups + a.stall);
+            tc::mbar_init(&empty[s], 1);
         }
-        for (int a = 0; a < 2; ++a)
+        for (int i = 0; i < 2; ++i)
         {
-            tc::mbar_init(&acc_full[a], 1);
-            tc::mbar_init(&acc_empty[a], kEpilogueThreads);
-            tc::mbar_init(&xfull[a], 1);
+            tc::mbar_init(&acc_full[i], 1);
+            tc::mbar_init(&acc_empty[i], kScanWarps);
         }
         tc::mbar_init(&drain, 1);
         s_events = 0;
-        // A failure reported by an earlier segment of the run: this launch steps nothing (but keeps
-        // the teardown protocol with its partner).
-        s_fail = *reinterpret_cast<volatile unsigned int *>(net.err) != 0u ? 1 : 0;
-        s_sent = s_recv = s_armed = s_peer_sent = 0;
     }
+    // Everything above overlaps the preceding kernel; from here on its results are read.
+    pdl_begin();
+    if (threadIdx.x == 0) s_fail = *reinterpret_cast<volatile unsigned int *>(a.err) != 0u ? 1 : 0;
     tc::fence_before_sync();
     __syncthreads();
-    tc::cluster_sync();  // the partner's barriers are initialised before any st.async reaches them
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    const uint32_t m_tiles = net.m_tiles;
-    const uint32_t R = net.ring;
-    const size_t ctr_in = (static_cast<size_t>(layer - 1) * m_tiles + m_tile) * kMaxRing;
-    const size_t ctr_out = (static_cast<size_t>(layer) * m_tiles + m_tile) * kMaxRing;
-    const bool producer = layer < net.n_layers;
+    const uint32_t base = (tc::smem_u32(smem) + 1023u) & ~1023u;  // swizzle atoms on 1024-byte boundaries
+    const uint32_t stages = a.stages, chunks = a.chunks;
+    const uint32_t n_tiles =
+        (max(a.st_len[2 * group], a.st_len[2 * group + 1]) + kStreamCols - 1) / kStreamCols;
     unsigned long long my_events = 0;
 
-    if (warp < kExpandWarps)
+    if (warp >= kExpandWarp0)
     {
-        // Expanders: per step, wait until every CTA of layer - 1 (this sample tile) has published
-        // step t - 1, load this row's words of the K half, and write each chunk as BF16 0/1 into a
-        // free operand stage in tensor memory (thread = sample row = tensor-memory lane).
-        const uint32_t xr = threadIdx.x;
-        const uint32_t wp_in = net.wpad[layer - 1];
-        const unsigned int *ready_in = layer > 1 ? net.ready + ctr_in : nullptr;
-        const uint32_t need_in = layer > 1 ? net.n_cta[layer - 1] + net.stall : 0u;
-        const uint32_t x_lane = (32u * warp) << 16;
-        uint32_t seq = 0;
+        // Expanders: thread r looks up the row of column r of a tile; then kGroups groups of warps take
+        // every kGroups-th chunk, a thread expanding kGroups of its 256 rows (a group's wait, expansion
+        // and proxy fence overlap those of the others).
+        constexpr uint32_t kRows = 256 / kGroups;  // threads of a group: rows gr + kRows i
+        static_assert(kRows % 32 == 0 && kExpandWarps == 8, "whole warps");
+        const uint32_t r = threadIdx.x - 32 * kExpandWarp0, stream = 2 * group + (r >> 7);
+        const uint32_t off = a.st_off[stream], entries = a.st_off[stream + 1] - off, len = a.st_len[stream];
+        const uint32_t gr = r & (kRows - 1), sw = gr & 7u;
+        uint32_t c = r / kRows, s = c, ph = 1;  // this group's next chunk, its stage and parity
         bool ok = true;
-        unsigned int ready_seen = 0;  // the next step's counter, read early in this step
-        auto row_words = [&](uint32_t t) -> const uint4 *
+        for (uint32_t tile = 0; tile < n_tiles; ++tile)
         {
-            const uint32_t slot = layer == 1 ? t - t0 : t % R;
-            return reinterpret_cast<const uint4 *>(
-                net.bits[layer - 1] + (static_cast<size_t>(slot) * m_tiles + m_tile) * kBM * wp_in +
-                static_cast<size_t>(xr) * wp_in + c_lo * kChunkWords);
-        };
-        uint4 wv[kMaxHalfChunks];  // this step's words
-        uint4 wn[kMaxHalfChunks];  // the next step's words, when they could be loaded during this step
-        bool have_next = false;
-        for (uint32_t t = t0; t < t1; ++t)
-        {
-            if (m0 >= net.act[t]) break;  // sample tiles finish in order: no steps left
-            bool go = ok;
-            if (threadIdx.x == 0)
-                go = go && !s_fail &&
-                     (have_next || !ready_in || t == 0 ||
-                      reached(ready_in + t % R, need_in * ((t - 1) / R + 1), ready_seen, net.poll_limit, &s_fail,
-                              net.err));
-            if (!tc::named_sync_and(1, kExpandThreads, go))  // the group's decision is uniform
+            const uint32_t p = tile * kStreamCols + (r & (kStreamCols - 1));
+            uint32_t row = kNoRow;
+            if (p < len)
             {
-                s_fail = 1;
-                atomicOr(net.err, 1u);
-                break;
-            }
-            if (have_next)
-            {
-#pragma unroll
-                for (uint32_t c = 0; c < kMaxHalfChunks; ++c) wv[c] = wn[c];
-            }
-            else
-            {
-                const uint4 *rowp = row_words(t);
-#pragma unroll
-                for (uint32_t c = 0; c < kMaxHalfChunks; ++c)
-                    wv[c] = c < n_chunks ? __ldcg(rowp + c) : make_uint4(0, 0, 0, 0);
-            }
-            have_next = false;
-            const bool can_next = t + 1 < t1 && m0 < net.act[t + 1];  // uniform
-            if (threadIdx.x == 0 && ready_in && can_next) ready_seen = load_relaxed(ready_in + (t + 1) % R);
-            // After chunk `c_ask`, the next step's words are loaded (to be used next step) if layer - 1
-            // has already published that step, so their L2 round trip overlaps this step's chunks.
-            const uint32_t c_ask = n_chunks > 1 ? 1u : 0u;
-            // One copy of the chunk body (kept small for the instruction cache); the loaded words
-            // shift down by one chunk per iteration so that every register index stays static.
-#pragma unroll 1
-            for (uint32_t c = 0; c < n_chunks; ++c)
-            {
-                const uint32_t u = seq + c, b = u % kStages;
-                if (ok && u >= kStages && !wait_or_fail(&empty[b], ((u / kStages) - 1u) & 1u, &s_fail, net.err))
+                uint32_t lo = 0, hi = entries;  // the last entry that starts at or before p
+                while (hi - lo > 1)
                 {
-                    // The stage may still be read by MMAs: it is not written, and the failure stops
-                    // the issuer (which waits on this stage) and, at the next step, this group.
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (a.st_start[off + mid] <= p) lo = mid;
+                    else hi = mid;
+                }
+                const uint4 e = a.st_info[off + lo];
+                const uint32_t j = p - a.st_start[off + lo];
+                if (j < e.z) row = e.y + j;
+            }
+            s_row[tile & 1u][r] = row;
+            // The group's decision is uniform; the barrier also publishes the tile's rows (a buffer is
+            // rewritten two tiles later, after every reader has passed the next tile's barrier).
+            if (!tc::named_sync_and(1, 32 * kExpandWarps, ok)) break;
+            const uint32_t *src[kGroups];
+#pragma unroll
+            for (int i = 0; i < kGroups; ++i)
+            {
+                const uint32_t q = s_row[tile & 1u][gr + kRows * i];
+                src[i] = q == kNoRow ? nullptr : a.bits_in + static_cast<size_t>(q) * a.wp_in;
+            }
+            auto load = [&](uint32_t chunk, uint2 (&h)[kGroups])
+            {
+#pragma unroll
+                for (int i = 0; i < kGroups; ++i)
+                    h[i] = src[i] ? __ldcg(reinterpret_cast<const uint2 *>(src[i] + 2 * chunk)) : make_uint2(0, 0);
+            };
+            uint2 h[kGroups];
+            if (c < chunks) load(c, h);
+            while (c < chunks)
+            {
+                uint2 next[kGroups];
+                if (c + kGroups < chunks) load(c + kGroups, next);  // used after this chunk
+                // (the first pass over the ring finds every stage free)
+                if (!warp_wait(&empty[s], ph, a.poll_limit, &s_fail, lane))
+                {
                     ok = false;
+                    break;
+                }
+                const uint32_t dst = base + s * kLayerStage + kAChunk + gr * 128u;
+#pragma unroll
+                for (uint32_t i = 0; i < kGroups; ++i)
+#pragma unroll
+                    for (uint32_t b = 0; b < 4; ++b)
+                    {
+                        uint32_t v[8];
+                        const uint32_t word = b < 2 ? h[i].x : h[i].y;
+                        expand16((b & 1u) ? word >> 16 : word, v);
+                        st_shared_v4(dst + i * (kRows * 128u) + (((2 * b) ^ sw) << 4), v);
+                        st_shared_v4(dst + i * (kRows * 128u) + (((2 * b + 1) ^ sw) << 4), v + 4);
+                    }
+                tc::fence_async_smem();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&full_s[s]);
+#pragma unroll
+                for (int i = 0; i < kGroups; ++i) h[i] = next[i];
+                c += kGroups;
+                s += kGroups;
+                if (s >= stages)
+                {
+                    s -= stages;
+                    ph ^= 1u;
+                }
+            }
+            c -= chunks;  // position in the next tile (wraps only when ok is false)
+        }
+        if (!ok && lane == 0)
+        {
+            s_fail = 1;
+            atomicOr(a.err, 1u);
+        }
+    }
+    else if (warp >= kScanWarp0)
+    {
+        const uint32_t half = (warp - kScanWarp0) >> 2;
+        const uint32_t stream = 2 * group + half;
+        ScanTarget tgt;
+        tgt.tmem = tmem + ((32u * (warp & 3u)) << 16) + half * kStreamCols;
+        tgt.off = a.st_off[stream];
+        tgt.len = a.st_len[stream];
+        tgt.neuron = n_tile * kTileN + 32u * (warp & 3u) + lane;
+        tgt.wq = 4u * n_tile + (warp & 3u);
+        tgt.n_tiles = n_tiles;
+        const bool ok = a.refract ? scan_stream<true>(a, tgt, lane, acc_full, acc_empty, &s_fail, my_events)
+                                  : scan_stream<false>(a, tgt, lane, acc_full, acc_empty, &s_fail, my_events);
+        if (!ok && lane == 0)
+        {
+            s_fail = 1;
+            atomicOr(a.err, 1u);
+        }
+    }
+    else if (warp == kCopyWarp)
+    {
+        if (lane == 0)
+        {
+            const uint8_t *src = a.w + static_cast<size_t>(n_tile) * chunks * kAChunk;
+            const uint32_t total = n_tiles * chunks;
+            uint32_t issued = 0;
+            for (uint32_t u = 0, c = 0, s = 0, ph = 1; u < total; ++u)
+            {
+                if (u >= stages && !wait_or_fail(&empty[s], ph, a.poll_limit, &s_fail))
+                {
                     s_fail = 1;
-                    atomicOr(net.err, 1u);
+                    atomicOr(a.err, 1u);
+                    break;
                 }
-                tc::fence_after_sync();
-                const uint32_t w4[4] = {wv[0].x, wv[0].y, wv[0].z, wv[0].w};
-#pragma unroll
-                for (uint32_t k = 0; k + 1 < kMaxHalfChunks; ++k) wv[k] = wv[k + 1];
-                // tcgen05.st is warp-collective: a warp writes only if all its lanes may.
-                if (__all_sync(0xffffffffu, ok))
+                mbar_arrive_expect_tx(&full_w[s], kAChunk);
+                bulk_copy(base + s * kLayerStage, src + static_cast<size_t>(c) * kAChunk, kAChunk, &full_w[s]);
+                issued = u + 1;
+                if (++c == chunks) c = 0;
+                if (++s == stages)
                 {
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                    {
-                        // Word q holds inputs 32 q .. 32 q + 31 of the chunk: 16 columns of two BF16
-                        // each, bits (2 i, 2 i + 1) -> column i = 1.0 or 0 in its low and high halves.
-                        uint32_t v[16];
-#pragma unroll
-                        for (uint32_t i = 0; i < 16; ++i)
-                            v[i] = (((w4[q] >> (2u * i) & 3u) * 0x8001u) & 0x10001u) * 0x3F80u;
-                        tc::tmem_st16(tmem + x_lane + kAccCols + b * kStageCols + 16u * q, v);
-                    }
-                    tc::tmem_wait_st();
-                    tc::fence_before_sync();
-                    tc::mbar_arrive(&full[b]);
-                }
-                if (c == c_ask && can_next)
-                {
-                    bool nx = true;
-                    if (threadIdx.x == 0 && ready_in)
-                    {
-                        const unsigned int target = need_in * (t / R + 1);
-                        nx = static_cast<int>(ready_seen - target) >= 0;
-                        if (nx) fence_acquire();
-                    }
-                    have_next = tc::named_sync_and(1, kExpandThreads, nx);
-                    if (have_next)
-                    {
-                        const uint4 *rown = row_words(t + 1);
-#pragma unroll
-                        for (uint32_t c2 = 0; c2 < kMaxHalfChunks; ++c2)
-                            wn[c2] = c2 < n_chunks ? __ldcg(rown + c2) : make_uint4(0, 0, 0, 0);
-                    }
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
-            seq += n_chunks;
+            // Copies still in flight after a failed wait land before the CTA leaves (bounded).
+            for (uint32_t u = issued > stages ? issued - stages : 0u; u < issued; ++u)
+                if (!tc::mbar_wait(&full_w[u % stages], (u / stages) & 1u, kWaitLimit)) atomicOr(a.err, 1u);
         }
     }
-    else if (warp < kExpandWarps + kEpilogueWarps)
+    else if (warp == kIssuerWarp && lane == 0)
     {
-        // Epilogue: thread (warp 4 + w, lane) owns sample row er = 32 (w % 4) + lane of the tile and
-        // the CTA's neurons cb .. cb + 15 (cb = 16 (w / 4)), keeping their LIF state in registers;
-        // warp 4 + w reads tensor-memory lanes 32 (w % 4) .. + 31.
-        const uint32_t et = threadIdx.x - kExpandThreads, ew = et >> 5;
-        const uint32_t er = 32u * (ew & 3u) + lane, erow = m0 + er;
-        const uint32_t cb = kEN * (ew >> 2);
-        const uint32_t lane_base = (32u * (warp & 3)) << 16;
-        float V[kEN];
-        uint32_t RC[kEN];
-        uint32_t *saved = net.state + (static_cast<size_t>(item) * kEpilogueThreads + et) * kStateWords;
-#pragma unroll
-        for (int i = 0; i < kEN; ++i)
-        {
-            V[i] = t0 ? __uint_as_float(saved[i]) : 0.f;
-            RC[i] = t0 ? saved[kEN + i] : 0u;
-        }
-        const int li = layer - 1;
-        const float leak = net.leak[li], thr = net.thr[li], rst = net.reset[li];
-        const uint32_t per = net.refract[li];
-        // This row's sample: its own neuron count and its next layer's (the fan-out of its spikes).
-        const uint32_t e_smp = erow < net.batch ? net.perm[erow] : 0u;
-        const uint32_t my_n = (net.sample_size[layer] && erow < net.batch) ? net.sample_size[layer][e_smp] : N;
-        const uint32_t my_fan_out =
-            producer ? ((net.sample_size[layer + 1] && erow < net.batch) ? net.sample_size[layer + 1][e_smp]
-                                                                          : net.size[layer + 1])
-                     : 0u;
-        uint32_t *out_bits = producer ? net.bits[layer] : nullptr;
-        const uint32_t wp_out = producer ? net.wpad[layer] : 0u;
-        unsigned int *ready_out = producer ? net.ready + ctr_out : nullptr;
-        const unsigned int *consumed_out = producer ? net.consumed + ctr_out : nullptr;
-        const uint32_t need_out = producer ? net.n_cta[layer + 1] : 0u;
-        // Last layer: spike counts in shared memory, neuron-major so that a warp's 32 rows hit 32 banks.
-        int *cnt = layer == net.n_layers ? reinterpret_cast<int *>(sX + 2 * kXchBytes) + cb * kBM + er : nullptr;
-        if (cnt)
-#pragma unroll
-            for (int i = 0; i < kEN; ++i) cnt[i * kBM] = t0 ? static_cast<int>(saved[2 * kEN + i]) : 0;
-        const uint32_t peer = tc::cluster_rank() ^ 1u;
-        // Neurons at or past this sample's size do not exist (never updated, never spike).
-        const uint32_t n_here = my_n > n0 + cb ? my_n - n0 - cb : 0u;
-        const uint32_t exists = n_here >= 16u ? 0xFFFFu : (1u << n_here) - 1u;
-        uint32_t s = 0, sent = 0, armed = 0;
-        for (uint32_t t = t0; t < t1; ++t)
-        {
-            const uint32_t b_act = net.act[t];
-            if (m0 >= b_act) break;
-            // Ring slot (t + 1) % R was read at steps t + 1 - R, t + 1 - 2 R, ...: every
-            // consumer must have read it that many times before it is overwritten below (the count
-            // is read now and checked after the update).
-            const bool check_room = et == 0 && producer && t + 1 >= R;
-            const unsigned int room_seen = check_room ? load_relaxed(consumed_out + (t + 1) % R) : 0u;
-            const uint32_t a = s & 1u, ph = (s >> 1) & 1u;
-            // A failed accumulator wait stops the group before it reads tensor memory that MMAs may
-            // still write, and before it sends its partner anything for this step.
-            if (!tc::named_sync_and(2, kEpilogueThreads, wait_or_fail(&acc_full[a], ph, &s_fail, net.err)))
-            {
-                s_fail = 1;
-                atomicOr(net.err, 1u);
-                break;
-            }
-            bool ok = true;
-            tc::fence_after_sync();
-            // Read the accumulator while the tensor cores are idle (the issuer starts the next step's
-            // MMAs once it is released): the partner's columns go straight to the partner (row er,
-            // 16-byte slot q of the row stored at q ^ (er % 8), so that 8 consecutive rows hit
-            // different banks), ours stay in registers. Then our partial + the partner's ((K half 0)
-            // + (K half 1) on both sides) and the LIF update.
-            if (et == 0) mbar_arrive_expect_tx(&xfull[a], kXchBytes);
-            armed = s + 1;
-            const uint32_t row_peer = tc::mapa(tc::smem_u32(sX), peer) + a * kXchBytes + er * (kBN * 4u);
-            const uint32_t xfull_peer = tc::mapa(tc::smem_u32(&xfull[a]), peer);
-            float acc[kEN];
-            if (n_chunks)
-                tc::tmem_ld16(tmem + lane_base + a * kPairN + kBN * (1u - kh) + cb, acc);
-            else
-#pragma unroll
-                for (int i = 0; i < kEN; ++i) acc[i] = 0.0f;
-#pragma unroll
-            for (uint32_t q = 0; q < kEN / 4; ++q)
-                tc::st_async_v4(row_peer + ((((cb >> 2) + q) ^ (er & 7u)) << 4), acc[4 * q], acc[4 * q + 1],
-                                acc[4 * q + 2], acc[4 * q + 3], xfull_peer);
-            sent = s + 1;
-            if (n_chunks)
-                tc::tmem_ld16(tmem + lane_base + a * kPairN + kBN * kh + cb, acc);
-            tc::fence_before_sync();
-            tc::mbar_arrive(&acc_empty[a]);
-            ok = wait_cluster_or_fail(&xfull[a], ph, &s_fail, net.err) && ok;
-            const uint8_t *row_own = sX + a * kXchBytes + er * (kBN * 4u);
-#pragma unroll
-            for (uint32_t q = 0; q < kEN / 4; ++q)
-            {
-                const float4 p4 = *reinterpret_cast<const float4 *>(row_own + ((((cb >> 2) + q) ^ (er & 7u)) << 4));
-                const float pv[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    acc[4 * q + e] = kh ? __fadd_rn(pv[e], acc[4 * q + e]) : __fadd_rn(acc[4 * q + e], pv[e]);
-            }
-            const uint32_t live = (ok && erow < b_act) ? exists : 0u;
-            uint32_t mask = 0;  // this thread's spikes, bit i = neuron cb + i
-#pragma unroll
-            for (int i = 0; i < kEN; ++i)
-            {
-                // lif_impl.h:33-86: leak and input only outside the refractory period; strict '>';
-                // reset to a value. Branch-free: the lanes are different samples.
-                const bool here = (live >> i) & 1u;
-                const bool free_ = RC[i] == 0u;
-                const float v = __fadd_rn(__fmul_rn(V[i], leak), acc[i]);
-                const bool spike = here && free_ && v > thr;
-                V[i] = spike ? rst : ((here && free_) ? v : V[i]);
-                RC[i] = spike ? per : ((here && !free_) ? RC[i] - 1u : RC[i]);
-                mask |= static_cast<uint32_t>(spike) << i;
-            }
-            if (cnt)
-                for (uint32_t m = mask; m; m &= m - 1u) ++cnt[(__ffs(m) - 1) * kBM];
-            s_half[a][ew >> 2][er] = mask;
-            const bool room = !check_room || reached(consumed_out + (t + 1) % R, need_out * ((t + 1 - R) / R + 1),
-                                                     room_seen, net.poll_limit, &s_fail, net.err);
-            const bool go = ok && room && (et != 0 || !s_fail);
-            if (!tc::named_sync_and(2, kEpilogueThreads, go))  // the group's decision is uniform
-            {
-                s_fail = 1;
-                atomicOr(net.err, 1u);
-                if (ok) ++s;  // this step's exchange phase completed in every thread
-                break;
-            }
-            ++s;
-            my_events += static_cast<unsigned long long>(__popc(mask)) * my_fan_out;
-            // The row's word (both halves) is written by the thread of the first half.
-            if (cb == 0 && (n0 >> 5) < wn)  // the second half of a tile may lie past N
-            {
-                const uint32_t word = s_half[a][0][er] | (s_half[a][1][er] << kEN);
-                if (producer)
-                    out_bits[((static_cast<size_t>((t + 1) % R) * m_tiles + m_tile) * kBM + er) * wp_out +
-                             (n0 >> 5)] = word;
-                if (net.record && erow < b_act)
-                    net.record[t * net.rec_stride + net.rec_off[layer] + static_cast<size_t>(e_smp) * wn + (n0 >> 5)] =
-                        word;
-            }
-            if (producer)
-            {
-                tc::named_sync_and(2, kEpilogueThreads, true);
-                if (et == 0) release_add(ready_out + (t + 1) % R);
-            }
-        }
-        if (t1 < net.t_max)
-        {
-#pragma unroll
-            for (int i = 0; i < kEN; ++i)
-            {
-                saved[i] = __float_as_uint(V[i]);
-                saved[kEN + i] = RC[i];
-                if (cnt) saved[2 * kEN + i] = static_cast<uint32_t>(cnt[i * kBM]);
-            }
-        }
-        else if (cnt && erow < net.batch)
-        {
-            // Output spike counts of the last layer: each (sample, neuron) is owned by one thread.
-            for (int i = 0; i < kEN; ++i)
-                if (n0 + cb + i < N) net.counts[static_cast<size_t>(e_smp) * N + n0 + cb + i] = cnt[i * kBM];
-        }
-        if (et == 0)
-        {
-            s_sent = sent;
-            s_recv = s;
-            s_armed = armed;
-        }
-    }
-    else if (lane == 0)
-    {
-        // Issuer: per step, once the epilogue has read the previous step's accumulator, the MMAs of
-        // each expanded stage into accumulator s % 2, then one commit for it. The input slot has been read
-        // once every stage of the step is expanded.
-        constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kPairN);
-        // Matrix descriptor of the weight tile's first K slice; the others follow by adding byte
-        // offsets / 16 to the start-address field. The A operand is read from tensor memory.
-        const uint64_t dW0 = tc::smem_desc(tc::smem_u32(sW), 128, sbo_w);
-        unsigned int *consumed_in = layer > 1 ? net.consumed + ctr_in : nullptr;
-        uint32_t seq = 0, s = 0;
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(kTileN, kCols);
+        const uint64_t d_w = tc::smem_desc_sw128(base, 1024), d_s = tc::smem_desc_sw128(base + kAChunk, 1024);
         bool stop = false;
-        for (uint32_t t = t0; t < t1 && !stop; ++t)
+        uint32_t s = 0, ph = 0;
+        for (uint32_t tile = 0; tile < n_tiles && !stop; ++tile)
         {
-            if (m0 >= net.act[t] || s_fail) break;
-            const uint32_t a = s & 1u;
-            // The epilogue has read the previous step's accumulator (no tensor-memory reads run
-            // beside these MMAs).
-            if (s >= 1 && !wait_or_fail(&acc_empty[(s - 1) & 1u], ((s - 1) >> 1) & 1u, &s_fail, net.err))
+            const uint32_t acc = tile & 1u;
+            if (tile >= 2 && !wait_or_fail(&acc_empty[acc], ((tile >> 1) - 1u) & 1u, a.poll_limit, &s_fail))
             {
                 stop = true;
                 break;
             }
-            tc::fence_after_sync();
-            for (uint32_t c = 0; c < n_chunks; ++c)
+            const uint32_t d_acc = tmem + acc * kCols;
+            for (uint32_t c = 0; c < chunks; ++c)
             {
-                const uint32_t u = seq + c, b = u % kStages;
-                // A stage that was not written is not multiplied: the run stops here.
-                if (!wait_or_fail(&full[b], (u / kStages) & 1u, &s_fail, net.err))
+                if (!wait_or_fail(&full_w[s], ph, a.poll_limit, &s_fail) ||
+                    !wait_or_fail(&full_s[s], ph, a.poll_limit, &s_fail))
                 {
                     stop = true;
                     break;
                 }
                 tc::fence_after_sync();
-                const uint32_t ta = tmem + kAccCols + b * kStageCols;
-                const uint64_t db = dW0 + c * ((kBK / 8 * 128) >> 4);
-                const uint32_t kc = min(static_cast<uint32_t>(kBK), Kp - (c_lo + c) * kBK);
-                for (uint32_t j = 0; j < kc / 16; ++j)
-                    tc::mma_bf16_ta(tmem + a * kPairN, ta + j * 8, db + j * 16, idesc, (c > 0 || j > 0) ? 1u : 0u);
-                tc::commit(&empty[b]);
+                // The stage's descriptors follow from the first one's by their start addresses (in
+                // 16-byte units).
+                const uint64_t dw = d_w + s * (kLayerStage >> 4), ds = d_s + s * (kLayerStage >> 4);
+                const uint32_t blocks = (a.kp - c * kChunk) >> 4;
+                tc::mma_bf16(d_acc, dw, ds, idesc, c ? 1u : 0u);
+                if (blocks >= 4)
+                {
+#pragma unroll
+                    for (uint32_t b = 1; b < 4; ++b) tc::mma_bf16(d_acc, dw + 2 * b, ds + 2 * b, idesc, 1u);
+                }
+                else
+                {
+                    for (uint32_t b = 1; b < blocks; ++b) tc::mma_bf16(d_acc, dw + 2 * b, ds + 2 * b, idesc, 1u);
+                }
+                tc::commit(&empty[s]);
+                if (c + 1 == chunks) tc::commit(&acc_full[acc]);
+                if (++s == stages)
+                {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-            if (stop) break;
-            seq += n_chunks;
-            tc::commit(&acc_full[a]);
-            if (consumed_in) release_add(consumed_in + t % R);
-            ++s;
         }
         if (stop)
         {
             s_fail = 1;
-            atomicOr(net.err, 1u);
+            atomicOr(a.err, 1u);
         }
-        // Every MMA this thread issued completes (bounded wait) before the tensor memory is released;
-        // a drain that does not finish is reported too.
+        // Every issued MMA completes (bounded wait) before the tensor memory is freed.
         tc::commit(&drain);
-        if (!tc::mbar_wait(&drain, 0, kWaitLimit))
-        {
-            s_fail = 1;
-            atomicOr(net.err, 1u);
-        }
+        if (!tc::mbar_wait(&drain, 0, kWaitLimit)) atomicOr(a.err, 1u);
     }
+    __syncwarp();
     if (my_events) atomicAdd(&s_events, my_events);
     tc::fence_before_sync();
     __syncthreads();
-    // Exchange drain: each CTA tells its partner how many steps of partial sums it sent, then waits
-    // (bounded) until every one of them has landed in its own shared memory, so that no store of the
-    // partner is in flight into this CTA when it leaves (after a failure the loops end at different
-    // steps).
-    const bool xthread = threadIdx.x == static_cast<unsigned>(kExpandThreads);  // the first epilogue thread
-    if (xthread) tc::st_cluster_u32(tc::mapa(tc::smem_u32(&s_peer_sent), tc::cluster_rank() ^ 1u), s_sent);
-    tc::cluster_sync();
-    if (xthread)
-    {
-        const uint32_t peer_sent = s_peer_sent;
-        for (uint32_t q = s_recv; q < peer_sent; ++q)
-        {
-            if (q >= s_armed) mbar_arrive_expect_tx(&xfull[q & 1u], kXchBytes);
-            if (!tc::mbar_wait_cluster(&xfull[q & 1u], (q >> 1) & 1u, kWaitLimit))
-            {
-                s_fail = 1;
-                atomicOr(net.err, 1u);
-            }
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        if (s_fail) atomicOr(net.err, 1u);
-        if (s_events) atomicAdd(net.events, s_events);
-    }
-    tc::cluster_sync();  // neither CTA leaves while the other may still write into its shared memory
+    if (threadIdx.x == 0 && s_events) atomicAdd(a.events, s_events);
     if (warp == kIssuerWarp) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
 }  // namespace
 
-// A batch prepared once and run as one CUDA-graph launch: memsets of the run's state, the input
-// threshold kernel, then per segment of steps the input-drawing kernel and the persistent kernel
-// (cluster launch of CTA pairs, every CTA resident). Reusable: every run starts from zero state, so
-// repeated runs of the same plan give identical results.
+// A batch prepared once and run as one CUDA-graph launch: a memset of the run's totals, the weight
+// packing, then per segment of steps the input draws and one kernel per layer. Reusable: every run
+// starts from zero state, so repeated runs of the same plan give identical results.
 struct BatchedPlan
 {
-    BatchedNet net{};
+    struct Segment
+    {
+        DrawArgs draw{};
+        LayerArgs layer[kMaxLayers]{};
+        unsigned grid[kMaxLayers]{};
+    };
+    int n_layers = 0;
+    std::vector<Segment> segs;
+    PackArgs pack{};
     cudaStream_t caller = nullptr;  // the caller's stream: a run starts after its queued work
     cudaStream_t stream = nullptr;  // the plan's own stream (graphs cannot be captured on the legacy stream)
-    cudaEvent_t ready = nullptr;
+    cudaEvent_t ready = nullptr, begin = nullptr, end = nullptr;
     std::vector<void *> allocs;
-    std::vector<std::pair<void *, size_t>> zero;  // cleared at the start of every run
-    const float *rates = nullptr;
-    unsigned long long *d_thr = nullptr;
-    size_t n_thr = 0;
-    size_t w_bytes = 0;  // largest weight tile (shared memory besides the ring and the exchange buffers)
-    uint32_t n_items = 0;
-    uint32_t seg_steps = 0;  // steps per segment
+    unsigned long long *totals = nullptr;       // device: events, then the error word
+    unsigned long long *totals_host = nullptr;  // pinned copy, written by the run
+    uint32_t *record = nullptr;
+    size_t record_bytes = 0;
     cudaGraphExec_t exec = nullptr;
     int stages = 0;
-    bool cooperative = true;  // cluster launch with the cooperative attribute (cleared if refused)
-    float tune_ms[3][kMaxStages + 1] = {};  // [ring choice][operand ring depth] of the autotuning runs
+    float tune_ms[kMaxStages + 1] = {};  // by operand ring depth
 
     ~BatchedPlan()
     {
         if (exec) cudaGraphExecDestroy(exec);
         if (stream) cudaStreamSynchronize(stream);
         for (void *p : allocs) cudaFree(p);
+        if (totals_host) cudaFreeHost(totals_host);
         if (ready) cudaEventDestroy(ready);
+        if (begin) cudaEventDestroy(begin);
+        if (end) cudaEventDestroy(end);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -899,55 +919,13 @@ struct BatchedPlan
 namespace
 {
 
-const void *kernel_for(int stages)
+// A ring of 4 or 2 chunks has a group of expander warps for each; one of 3 has one group for all.
+auto layer_kernel(int stages)
 {
-    switch (stages)
-    {
-        case 2:
-            return reinterpret_cast<const void *>(batched_lif_kernel<2>);
-        case 3:
-            return reinterpret_cast<const void *>(batched_lif_kernel<3>);
-        default:
-            return reinterpret_cast<const void *>(batched_lif_kernel<4>);
-    }
+    return stages == 4 ? lif_layer_kernel<4> : stages == 2 ? lif_layer_kernel<2> : lif_layer_kernel<1>;
 }
 
-size_t smem_bytes(const BatchedPlan &p, int stages)
-{
-    (void)stages;  // operand stages live in tensor memory
-    return std::max(p.w_bytes + 2 * kXchBytes + kCntBytes, kMinDynSmem);
-}
-
-// Whether a ring of `stages` chunks fits (shared memory, every CTA pair resident at once).
-bool variant_fits(const BatchedPlan &p, int stages)
-{
-    int device = 0, smem_max = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    const size_t smem = smem_bytes(p, stages);
-    if (smem + 4096 > static_cast<size_t>(smem_max)) return false;  // 4 KB: the kernel's static shared memory
-    const void *k = kernel_for(stages);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-        return false;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(p.n_items);
-    cfg.blockDim = dim3(kBatchThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess)
-    {
-        cudaGetLastError();
-        return false;
-    }
-    return 2ll * clusters >= p.n_items;
-}
+size_t smem_bytes(int stages) { return std::max(stages * size_t(kLayerStage) + 1024, kMinDynSmem); }
 
 // Captures one run with a ring of `stages` chunks into p.exec.
 cudaError_t capture(BatchedPlan &p, int stages)
@@ -957,38 +935,41 @@ cudaError_t capture(BatchedPlan &p, int stages)
         cudaGraphExecDestroy(p.exec);
         p.exec = nullptr;
     }
-    cudaStream_t s = p.stream;
-    cudaError_t err = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    if (err != cudaSuccess) return err;
-    for (auto &z : p.zero) cudaMemsetAsync(z.first, 0, z.second, s);
-    rate_threshold_kernel<<<static_cast<unsigned>((p.n_thr + 255) / 256), 256, 0, s>>>(p.rates, p.d_thr, p.n_thr);
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const size_t smem = smem_bytes(stages);
+    cudaError_t err =
+        cudaFuncSetAttribute(layer_kernel(stages), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return err;
+    cudaStream_t s = p.stream;
+    err = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+    if (err != cudaSuccess) return err;
     cudaError_t lerr = cudaSuccess;
-    for (uint32_t t0 = 0; t0 < p.net.t_max && lerr == cudaSuccess; t0 += p.seg_steps)
+    auto note = [&](cudaError_t e)
     {
-        uint32_t t1 = std::min(p.net.t_max, t0 + p.seg_steps);
-        const size_t words = (static_cast<size_t>(t1 - t0) + 1) * p.net.m_tiles * kBM * p.net.wpad[0];
-        const unsigned blocks = static_cast<unsigned>(std::min<size_t>((words + 255) / 256, static_cast<size_t>(sms) * 8));
-        input_bits_kernel<<<blocks, 256, 0, s>>>(p.net, t0, t1);
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(p.n_items);
-        cfg.blockDim = dim3(kBatchThreads);
-        cfg.dynamicSmemBytes = smem_bytes(p, stages);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeCooperative;
-        attr[1].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = p.cooperative ? 2 : 1;
-        void *args[] = {&p.net, &t0, &t1};
-        lerr = cudaLaunchKernelExC(&cfg, kernel_for(stages), args);
+        if (lerr == cudaSuccess) lerr = e;
+    };
+    note(cudaMemsetAsync(p.totals, 0, 16, s));
+    if (p.record) note(cudaMemsetAsync(p.record, 0, p.record_bytes, s));
+    const unsigned long long units = p.pack.first[p.pack.n_layers];
+    pack_weights_kernel<<<static_cast<unsigned>(std::min<unsigned long long>((units + 255) / 256, 16ull * sms)), 256, 0,
+                          s>>>(p.pack);
+    note(cudaGetLastError());
+    for (auto &seg : p.segs)
+    {
+        const unsigned long long warps = static_cast<unsigned long long>(seg.draw.batch) * seg.draw.blocks * seg.draw.wp;
+        input_rows_kernel<<<static_cast<unsigned>(std::min<unsigned long long>((warps + 7) / 8, 8ull * sms)), 256, 0, s>>>(
+            seg.draw);
+        note(cudaGetLastError());
+        for (int l = 0; l < p.n_layers; ++l)
+        {
+            LayerArgs a = seg.layer[l];
+            a.stages = static_cast<uint32_t>(stages);
+            note(launch_pdl(layer_kernel(stages), dim3(seg.grid[l]), dim3(kLayerThreads), smem, s, a));
+        }
     }
+    note(cudaMemcpyAsync(p.totals_host, p.totals, 16, cudaMemcpyDeviceToHost, s));
     cudaGraph_t g = nullptr;
     err = cudaStreamEndCapture(s, &g);
     if (lerr != cudaSuccess) err = lerr;
@@ -1000,50 +981,16 @@ cudaError_t capture(BatchedPlan &p, int stages)
 
 cudaError_t launch_timed(BatchedPlan &p, float *ms)
 {
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
     // Order the run after the caller's queued work (weights, rates written on its stream).
-    cudaEventRecord(p.ready, p.caller);
-    cudaStreamWaitEvent(p.stream, p.ready, 0);
-    cudaEventRecord(e0, p.stream);
-    cudaError_t err = cudaGraphLaunch(p.exec, p.stream);
-    cudaEventRecord(e1, p.stream);
-    if (err == cudaSuccess) err = cudaEventSynchronize(e1);
+    cudaError_t err = cudaEventRecord(p.ready, p.caller);
+    if (err == cudaSuccess) err = cudaStreamWaitEvent(p.stream, p.ready, 0);
+    if (err == cudaSuccess) err = cudaEventRecord(p.begin, p.stream);
+    if (err == cudaSuccess) err = cudaGraphLaunch(p.exec, p.stream);
+    if (err == cudaSuccess) err = cudaEventRecord(p.end, p.stream);
+    if (err == cudaSuccess) err = cudaEventSynchronize(p.end);
     float t = 0.f;
-    if (err == cudaSuccess) cudaEventElapsedTime(&t, e0, e1);
+    if (err == cudaSuccess) err = cudaEventElapsedTime(&t, p.begin, p.end);
     if (ms) *ms = t;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return err;
-}
-
-// Whether this process's device accepted a cooperative cluster launch (-1: not tried yet).
-int g_coop_cluster = -1;
-
-// Captures the plan with `stages` and, if `timed` (or to find out whether the cooperative cluster
-// launch is accepted), runs it once. A refused cooperative launch is captured again as a plain
-// cluster launch; co-residency of every CTA pair is still checked by variant_fits.
-cudaError_t prepare(BatchedPlan &p, int stages, bool timed, float *ms)
-{
-    p.cooperative = g_coop_cluster != 0;
-    cudaError_t err = capture(p, stages);
-    if (err == cudaSuccess && (timed || g_coop_cluster < 0)) err = launch_timed(p, ms);
-    if (err == cudaSuccess)
-    {
-        if (p.cooperative) g_coop_cluster = 1;
-        return err;
-    }
-    if (p.cooperative && g_coop_cluster < 0 &&
-        (err == cudaErrorInvalidValue || err == cudaErrorNotSupported || err == cudaErrorInvalidConfiguration ||
-         err == cudaErrorCooperativeLaunchTooLarge))
-    {
-        cudaGetLastError();
-        g_coop_cluster = 0;
-        p.cooperative = false;
-        err = capture(p, stages);
-        if (err == cudaSuccess && timed) err = launch_timed(p, ms);
-    }
     return err;
 }
 
@@ -1052,10 +999,9 @@ cudaError_t prepare(BatchedPlan &p, int stages, bool timed, float *ms)
 // Prepares a batch. Host arrays: sizes[n_layers + 1], leak/threshold/reset/refract[n_layers],
 // steps[batch], sample_sizes[(n_layers + 1) * batch] (layer-major, optional); device arrays:
 // weights[l] (BF16 [sizes[l + 1]][sizes[l]]), rates [batch][sizes[0]], counts [batch][sizes[n_layers]]
-// and record (optional; layouts in knp_gb300.h). With `autotune` > 0, each operand ring depth that
-// fits is run twice and the fastest kept; < 0 uses depth -autotune; 0 the deepest that fits. Every
-// depth computes the same results. `segment_steps` > 0
-// caps the steps per persistent launch (0: as many as layer 0's slot budget allows).
+// and record (optional; layouts in knp_gb300.h). With `autotune` > 0, each operand ring depth is run
+// twice and the fastest kept; < 0 uses depth -autotune; 0 the deepest. Every depth computes the same
+// results. `segment_steps` > 0 caps the steps per segment (0: as many as the row budget allows).
 int batched_plan_create(
     int n_layers, const uint32_t *sizes, const void *const *weights, const float *leak, const float *threshold,
     const float *reset, const uint32_t *refract, uint32_t batch, const uint32_t *steps, const uint32_t *sample_sizes,
@@ -1070,21 +1016,21 @@ int batched_plan_create(
     }
     std::unique_ptr<BatchedPlan> plan(new BatchedPlan());
     BatchedPlan &p = *plan;
-    BatchedNet &net = p.net;
+    p.n_layers = n_layers;
     p.caller = s;
     if (cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&p.ready, cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&p.ready, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreate(&p.begin) != cudaSuccess || cudaEventCreate(&p.end) != cudaSuccess)
     {
         *why = "could not create the plan's stream";
         return -3;
     }
-    // Failure test (KNP_GB300_BATCHED_STALL=1): every consumer layer waits for one producer CTA more
-    // than exists, so its first ring wait runs out (after a short poll limit) and the run ends with
-    // the error word set instead of results.
-    const char *stall = std::getenv("KNP_GB300_BATCHED_STALL");
-    net.stall = (stall && stall[0] == '1') ? 1u : 0u;
-    net.poll_limit = net.stall ? (1u << 16) : kPollLimit;
-    net.n_layers = n_layers;
+    // Failure test (KNP_GB300_BATCHED_STALL=1): the MMA issuer waits for one expander warp more per chunk than
+    // exists, so its first operand wait runs out (after a short poll limit) and the run ends with the
+    // error word set instead of results.
+    const char *stall_env = std::getenv("KNP_GB300_BATCHED_STALL");
+    const uint32_t stall = (stall_env && stall_env[0] == '1') ? 1u : 0u;
+    const uint32_t poll_limit = stall ? (1u << 16) : kWaitLimit;
     for (int l = 0; l <= n_layers; ++l)
     {
         if (sizes[l] == 0 || sizes[l] > 4096)
@@ -1092,18 +1038,10 @@ int batched_plan_create(
             *why = "layer sizes must be in [1, 4096]";
             return -1;
         }
-        net.size[l] = sizes[l];
-        net.words[l] = (sizes[l] + 31) / 32;
-        if (l > 0)
+        if (l < n_layers && sizes[l] > kMaxFanIn)
         {
-            net.kpad[l] = (sizes[l - 1] + 15) / 16 * 16;
-            net.chunks[l] = (net.kpad[l] + kBK - 1) / kBK;
-            net.wpad[l - 1] = net.chunks[l] * kChunkWords;
-            if ((net.chunks[l] + 1) / 2 > kMaxHalfChunks)
-            {
-                *why = "a layer's fan-in exceeds 2048";
-                return -1;
-            }
+            *why = "a layer's fan-in exceeds 2048";
+            return -1;
         }
     }
     for (uint32_t b = 0; b < batch; ++b)
@@ -1121,46 +1059,27 @@ int batched_plan_create(
                     return -1;
                 }
     }
-    // Work items: (layer, 128-sample tile, 64-neuron tile, K half), the two halves of a tile adjacent
-    // (one cluster).
-    const uint32_t m_tiles = (batch + kBM - 1) / kBM;
-    net.m_tiles = m_tiles;
-    for (int l = 1; l <= n_layers; ++l)
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // The batch size a plan takes: (layer, 128-sample tile, 64-neuron tile, half) units, one SM each.
+    unsigned long long units = 0;
+    for (int l = 1; l <= n_layers; ++l) units += 2ull * ((batch + 127) / 128) * ((sizes[l] + 63) / 64);
+    if (units > kMaxTiles)
     {
-        const uint32_t n_tiles = (net.size[l] + kPairN - 1) / kPairN;
-        net.n_cta[l] = 2 * n_tiles;
-        for (uint32_t m = 0; m < m_tiles; ++m)
-            for (uint32_t n = 0; n < n_tiles; ++n)
-                for (uint32_t h = 0; h < 2; ++h)
-                {
-                    if (p.n_items >= kMaxItems)
-                    {
-                        *why = "too many (layer, sample tile, neuron tile) work items";
-                        return -1;
-                    }
-                    net.item_layer[p.n_items] = static_cast<uint16_t>(l);
-                    net.item_m[p.n_items] = static_cast<uint16_t>(m);
-                    net.item_n[p.n_items] = static_cast<uint16_t>(n);
-                    net.item_k[p.n_items] = static_cast<uint8_t>(h);
-                    ++p.n_items;
-                }
-        const uint32_t c_mid = (net.chunks[l] + 1) / 2;
-        p.w_bytes = std::max<size_t>(p.w_bytes, static_cast<size_t>(kPairN) * c_mid * kBK * 2);
-    }
-    net.n_items = p.n_items;
-    int best = 0;
-    for (int st = kMaxStages; st >= kMinStages && !best; --st)
-        if (variant_fits(p, st)) best = st;
-    if (!best)
-    {
-        *why = "the batch does not fit: a layer's weight tile and operand ring exceed one CTA's shared memory "
-               "(fan-in too large) or the CTA pairs exceed the resident clusters";
+        *why = "too many (layer, sample tile, neuron tile) work items";
         return -1;
     }
+    if (units > static_cast<unsigned long long>(sms))
+    {
+        *why = "the batch does not fit: its (layer, sample tile, neuron tile) work items exceed the device";
+        return -1;
+    }
+    int best = kMaxStages;
     if (autotune < 0)
     {
         // A fixed ring depth (-autotune).
-        if (-autotune < kMinStages || -autotune > kMaxStages || !variant_fits(p, -autotune))
+        if (-autotune < kMinStages || -autotune > kMaxStages)
         {
             *why = "the requested operand ring depth is out of range or does not fit";
             return -1;
@@ -1168,28 +1087,6 @@ int batched_plan_create(
         best = -autotune;
         autotune = 0;
     }
-    // Samples sorted by decreasing length.
-    std::vector<uint32_t> perm(batch), st(batch);
-    for (uint32_t b = 0; b < batch; ++b) perm[b] = b;
-    std::stable_sort(perm.begin(), perm.end(), [&](uint32_t a, uint32_t b) { return steps[a] > steps[b]; });
-    for (uint32_t i = 0; i < batch; ++i) st[i] = steps[perm[i]];
-    net.t_max = st[0];
-    net.batch = batch;
-    net.key = key;
-    net.counts = counts;
-    net.record = record;
-    for (int l = 0; l < n_layers; ++l)
-    {
-        net.w[l] = static_cast<const __nv_bfloat16 *>(weights[l]);
-        net.leak[l] = leak ? leak[l] : 1.0f;
-        net.thr[l] = threshold ? threshold[l] : 1.0f;
-        net.reset[l] = reset ? reset[l] : 0.0f;
-        net.refract[l] = refract ? refract[l] : 0u;
-    }
-    // Segments: layer 0's slots of one segment stay within the budget.
-    const size_t slot_bytes = static_cast<size_t>(m_tiles) * kBM * net.wpad[0] * 4;
-    p.seg_steps = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(net.t_max, kInputSlotBudget / slot_bytes)));
-    if (segment_steps) p.seg_steps = std::min(p.seg_steps, segment_steps);
     auto dalloc = [&](size_t bytes) -> void *
     {
         void *q = nullptr;
@@ -1203,88 +1100,211 @@ int batched_plan_create(
         if (q && cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
         return q;
     };
-    // act[t] = slots with T > t (slots are sorted by decreasing T).
-    std::vector<uint32_t> act(net.t_max);
-    for (uint32_t t = 0, a = batch; t < net.t_max; ++t)
+    bool ok = true;
+    const uint32_t t_max = *std::max_element(steps, steps + batch);
+    // Rows of layer l have wp[l] words: whole 128-neuron tiles, 16-byte aligned.
+    uint32_t wp[kMaxLayers + 1], words[kMaxLayers + 1], tiles[kMaxLayers + 1], wp_most = 4;
+    unsigned long long rec_off[kMaxLayers + 1], rec_stride = 0;
+    for (int l = 0; l <= n_layers; ++l)
     {
-        while (a > 0 && st[a - 1] <= t) --a;
-        act[t] = a;
+        tiles[l] = (sizes[l] + kTileN - 1) / kTileN;
+        wp[l] = 4 * tiles[l];
+        words[l] = (sizes[l] + 31) / 32;
+        if (l < n_layers) wp_most = std::max(wp_most, wp[l]);
+        rec_off[l] = rec_stride;
+        rec_stride += static_cast<unsigned long long>(batch) * words[l];
     }
-    bool ok = (net.perm = static_cast<const uint32_t *>(upload(perm.data(), batch * 4))) != nullptr;
-    ok = ok && (net.act = static_cast<const uint32_t *>(upload(act.data(), act.size() * 4))) != nullptr;
+    uint32_t seg_steps = static_cast<uint32_t>(
+        std::max<size_t>(1, std::min<size_t>(t_max, kRowBudget / (static_cast<size_t>(batch) * wp_most * 4))));
+    if (segment_steps) seg_steps = std::min(seg_steps, segment_steps);
+    const uint32_t n_segs = (t_max + seg_steps - 1) / seg_steps;
+
+    // Packed weights.
+    p.pack.n_layers = n_layers;
+    for (int l = 0; l < n_layers; ++l)
+    {
+        const uint32_t kp = (sizes[l] + 15) / 16 * 16, chunks = (kp + kChunk - 1) / kChunk;
+        p.pack.w[l] = static_cast<const __nv_bfloat16 *>(weights[l]);
+        p.pack.n[l] = sizes[l + 1];
+        p.pack.k[l] = sizes[l];
+        p.pack.chunks[l] = chunks;
+        p.pack.first[l + 1] = p.pack.first[l] + static_cast<unsigned long long>(tiles[l + 1]) * chunks * kTileN * 8;
+        ok = ok && (p.pack.out[l] = static_cast<uint8_t *>(dalloc(static_cast<size_t>(tiles[l + 1]) * chunks * kAChunk)));
+    }
+    const uint32_t *d_size[kMaxLayers + 1] = {};
     if (sample_sizes)
         for (int l = 0; l <= n_layers && ok; ++l)
-            ok = (net.sample_size[l] = static_cast<const uint32_t *>(
-                      upload(sample_sizes + static_cast<size_t>(l) * batch, batch * 4))) != nullptr;
-    ok = ok && (net.bits[0] = static_cast<uint32_t *>(dalloc(p.seg_steps * slot_bytes))) != nullptr;
-    for (int l = 1; l < n_layers && ok; ++l)
+            ok = (d_size[l] = static_cast<const uint32_t *>(
+                      upload(sample_sizes + static_cast<size_t>(l) * batch, batch * 4ull))) != nullptr;
+    ok = ok && (p.totals = static_cast<unsigned long long *>(dalloc(16))) != nullptr;
+    ok = ok && cudaHostAlloc(reinterpret_cast<void **>(&p.totals_host), 16, cudaHostAllocDefault) == cudaSuccess;
+    auto *d_err = reinterpret_cast<unsigned int *>(p.totals + 1);
+
+    // Segments: every sample's columns and rows; per layer the streams, samples dealt longest first to
+    // the shortest stream so far.
+    size_t rows_most = 0;
+    std::vector<uint32_t> order(batch);
+    for (uint32_t b = 0; b < batch; ++b) order[b] = b;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return steps[x] > steps[y]; });
+    p.segs.resize(n_segs);
+    for (uint32_t sg = 0; sg < n_segs && ok; ++sg)
     {
-        const size_t bytes = static_cast<size_t>(kMaxRing) * m_tiles * kBM * net.wpad[l] * 4;
-        ok = (net.bits[l] = static_cast<uint32_t *>(dalloc(bytes))) != nullptr;
-        p.zero.emplace_back(net.bits[l], bytes);
+        BatchedPlan::Segment &seg = p.segs[sg];
+        const uint32_t t0 = sg * seg_steps, t1 = std::min(t_max, t0 + seg_steps);
+        std::vector<uint4> rows(batch);
+        size_t at = 0;
+        for (uint32_t b = 0; b < batch; ++b)
+        {
+            const uint32_t cols = steps[b] > t0 ? std::min(steps[b], t1) - t0 : 0u;
+            rows[b] = make_uint4(static_cast<uint32_t>(at), cols, 0, 0);
+            at += cols ? cols + 1 : 0;
+        }
+        rows_most = std::max(rows_most, at);
+        seg.draw.rows = static_cast<const uint4 *>(upload(rows.data(), batch * sizeof(uint4)));
+        ok = ok && seg.draw.rows;
+        seg.draw.t0 = t0;
+        seg.draw.blocks = (t1 - t0 + 1 + 31) / 32;
+        const uint32_t *tab = nullptr;
+        const uint4 *info_d = nullptr;
+        uint32_t groups = 0;
+        for (int l = 0; l < n_layers && ok; ++l)
+        {
+            const uint32_t want = std::max(1u, std::min((batch + 1) / 2, static_cast<uint32_t>(sms) / tiles[l + 1]));
+            if (want != groups)  // layers of equal width share their streams
+            {
+                groups = want;
+                std::vector<std::vector<uint32_t>> streams(2 * groups);
+                std::vector<uint64_t> load(2 * groups, 0);
+                std::priority_queue<std::pair<uint64_t, uint32_t>, std::vector<std::pair<uint64_t, uint32_t>>,
+                                    std::greater<>>
+                    shortest;
+                for (uint32_t q = 0; q < 2 * groups; ++q) shortest.emplace(0, q);
+                for (uint32_t b : order)
+                {
+                    if (!rows[b].y) continue;
+                    const uint32_t q = shortest.top().second;
+                    shortest.pop();
+                    streams[q].push_back(b);
+                    load[q] += (rows[b].y + kPad - 1) / kPad * kPad;
+                    shortest.emplace(load[q], q);
+                }
+                // [off: 2 G + 1][len: 2 G][start: entries]
+                std::vector<uint32_t> t(4 * groups + 1), start;
+                std::vector<uint4> info;
+                for (uint32_t q = 0; q < 2 * groups; ++q)
+                {
+                    t[q] = static_cast<uint32_t>(start.size());
+                    t[2 * groups + 1 + q] = static_cast<uint32_t>(load[q]);
+                    uint32_t pos = 0;
+                    for (uint32_t b : streams[q])
+                    {
+                        start.push_back(pos);
+                        info.push_back(make_uint4(b, rows[b].x, rows[b].y, steps[b]));
+                        pos += (rows[b].y + kPad - 1) / kPad * kPad;
+                    }
+                }
+                t[2 * groups] = static_cast<uint32_t>(start.size());
+                t.insert(t.end(), start.begin(), start.end());
+                tab = static_cast<const uint32_t *>(upload(t.data(), t.size() * 4));
+                info_d = static_cast<const uint4 *>(upload(info.data(), info.size() * sizeof(uint4)));
+                ok = tab && info_d;
+            }
+            LayerArgs &a = seg.layer[l];
+            a.st_off = tab;
+            a.st_len = tab + 2 * groups + 1;
+            a.st_start = tab + 4 * groups + 1;
+            a.st_info = info_d;
+            a.n_groups = groups;
+            a.t0 = t0;
+            a.t1 = t1;
+            seg.grid[l] = tiles[l + 1] * groups;
+        }
     }
-    const size_t n_counters = static_cast<size_t>(kMaxLayers + 1) * m_tiles * kMaxRing;
-    ok = ok && (net.ready = static_cast<unsigned int *>(dalloc(n_counters * 4))) != nullptr;
-    ok = ok && (net.consumed = static_cast<unsigned int *>(dalloc(n_counters * 4))) != nullptr;
-    ok = ok && (net.state = static_cast<uint32_t *>(
-                    dalloc(static_cast<size_t>(p.n_items) * kEpilogueThreads * kStateWords * 4))) != nullptr;
-    p.n_thr = static_cast<size_t>(batch) * sizes[0];
-    ok = ok && (p.d_thr = static_cast<unsigned long long *>(dalloc(p.n_thr * 8))) != nullptr;
-    net.rate_thr = p.d_thr;
-    p.rates = rates;
-    ok = ok && (net.events = static_cast<unsigned long long *>(dalloc(8))) != nullptr;
-    ok = ok && (net.err = static_cast<unsigned int *>(dalloc(4))) != nullptr;
+    uint32_t *bits[kMaxLayers] = {}, *state[kMaxLayers] = {}, *carry[kMaxLayers] = {};
+    for (int l = 0; l < n_layers && ok; ++l)
+    {
+        ok = (bits[l] = static_cast<uint32_t *>(dalloc(rows_most * wp[l] * 4))) != nullptr;
+        if (ok && n_segs > 1)
+        {
+            state[l] = static_cast<uint32_t *>(dalloc(static_cast<size_t>(batch) * sizes[l + 1] * 12));
+            carry[l] = static_cast<uint32_t *>(dalloc(static_cast<size_t>(batch) * wp[l + 1] * 4));
+            ok = state[l] && carry[l];
+        }
+    }
     if (!ok)
     {
         *why = "device allocation failed";
         return -5;
     }
-    p.zero.emplace_back(counts, static_cast<size_t>(batch) * net.size[n_layers] * 4);
-    p.zero.emplace_back(net.events, 8);
-    p.zero.emplace_back(net.err, 4);
-    p.zero.emplace_back(net.ready, n_counters * 4);
-    p.zero.emplace_back(net.consumed, n_counters * 4);
-    unsigned long long off = 0;
-    for (int l = 0; l <= n_layers; ++l)
+    p.record = record;
+    p.record_bytes = static_cast<size_t>(t_max) * rec_stride * 4;
+    for (auto &seg : p.segs)
     {
-        net.rec_off[l] = off;
-        off += static_cast<unsigned long long>(batch) * net.words[l];
+        DrawArgs &d = seg.draw;
+        d.rates = rates;
+        d.n_in = sizes[0];
+        d.wp = wp[0];
+        d.words = words[0];
+        d.batch = batch;
+        d.size0 = d_size[0];
+        d.size1 = d_size[1];
+        d.n1 = sizes[1];
+        d.key = key;
+        d.bits = bits[0];
+        d.record = record;
+        d.rec_stride = rec_stride;
+        d.events = p.totals;
+        for (int l = 0; l < n_layers; ++l)
+        {
+            LayerArgs &a = seg.layer[l];
+            const bool last = l + 1 == n_layers;
+            a.w = p.pack.out[l];
+            a.bits_in = bits[l];
+            a.wp_in = wp[l];
+            a.bits_out = last ? nullptr : bits[l + 1];
+            a.wp_out = wp[l + 1];
+            a.n = sizes[l + 1];
+            a.kp = (sizes[l] + 15) / 16 * 16;
+            a.chunks = p.pack.chunks[l];
+            a.leak = leak ? leak[l] : 1.0f;
+            a.thr = threshold ? threshold[l] : 1.0f;
+            a.reset = reset ? reset[l] : 0.0f;
+            a.refract = refract ? refract[l] : 0u;
+            a.own_size = d_size[l + 1];
+            a.next_size = last ? nullptr : d_size[l + 2];
+            a.next_n = last ? 0u : sizes[l + 2];
+            a.carry = carry[l];
+            a.state = state[l];
+            a.counts = last ? counts : nullptr;
+            a.record = record;
+            a.rec_off = rec_off[l + 1];
+            a.rec_stride = rec_stride;
+            a.wn = words[l + 1];
+            a.events = p.totals;
+            a.err = d_err;
+            a.poll_limit = poll_limit;
+            a.stall = stall;
+        }
     }
-    net.rec_stride = off;
-    if (record) p.zero.emplace_back(record, static_cast<size_t>(net.t_max) * off * 4);
-
     cudaError_t err = cudaSuccess;
-    net.ring = kDefaultRing;
     if (autotune)
     {
-        // Schedule choices that leave every result bit-identical: the operand ring depth and the
-        // length of the layer rings (how far a layer may run ahead of the next).
         float best_ms = 0.f;
-        uint32_t best_ring = kDefaultRing;
-        for (int ri = 0; ri < 3 && err == cudaSuccess; ++ri)
-            for (int stg = kMinStages; stg <= kMaxStages; ++stg)
+        for (int stg = kMinStages; stg <= kMaxStages && err == cudaSuccess; ++stg)
+        {
+            float t = 0.f;
+            err = capture(p, stg);
+            if (err == cudaSuccess) err = launch_timed(p, &t);
+            if (err == cudaSuccess) err = launch_timed(p, &t);
+            p.tune_ms[stg] = t;
+            if (err == cudaSuccess && (!best_ms || t < best_ms))
             {
-                if (!variant_fits(p, stg)) continue;
-                net.ring = kRingChoices[ri];
-                float t = 0.f;
-                err = prepare(p, stg, true, &t);
-                if (err == cudaSuccess) err = launch_timed(p, &t);
-                if (err != cudaSuccess) break;
-                p.tune_ms[ri][stg] = t;
-                if (!best_ms || t < best_ms)
-                {
-                    best_ms = t;
-                    best = stg;
-                    best_ring = kRingChoices[ri];
-                }
+                best_ms = t;
+                best = stg;
             }
-        net.ring = best_ring;
-        if (err == cudaSuccess) err = capture(p, best);
+        }
     }
-    else
-    {
-        err = prepare(p, best, false, nullptr);
-    }
+    if (err == cudaSuccess) err = capture(p, best);
     if (err != cudaSuccess)
     {
         *why = cudaGetErrorString(err);
@@ -1296,34 +1316,31 @@ int batched_plan_create(
 
 int batched_plan_run(BatchedPlan *p, unsigned long long *events_out, float *ms, const char **why)
 {
-    cudaError_t err = launch_timed(*p, ms);
-    unsigned long long ev = 0;
-    unsigned int kerr = 0;
-    if (err == cudaSuccess) err = cudaMemcpy(&ev, p->net.events, 8, cudaMemcpyDeviceToHost);
-    if (err == cudaSuccess) err = cudaMemcpy(&kerr, p->net.err, 4, cudaMemcpyDeviceToHost);
-    if (events_out) *events_out = ev;
+    const cudaError_t err = launch_timed(*p, ms);
     if (err != cudaSuccess)
     {
+        if (events_out) *events_out = 0;
         *why = cudaGetErrorString(err);
         return -3;
     }
-    if (kerr)
+    if (events_out) *events_out = p->totals_host[0];
+    if (static_cast<uint32_t>(p->totals_host[1]))
     {
-        *why = (kerr & 2u) ? "the batched kernel ran without its two-CTA cluster shape"
-                           : "a tensor-core completion wait, the pair exchange or a layer's step counter wait timed out";
+        *why = "a wait of the batched layer kernel (operands, accumulator or tensor-core completion) timed out";
         return -4;
     }
     return 0;
 }
 
+// tune_ms: [3][kMaxStages - kMinStages + 1]; the second and third rows stay 0 (depths alone are tuned).
 void batched_plan_info(const BatchedPlan *p, int *stages, int *ring_steps, float *tune_ms)
 {
     if (stages) *stages = p->stages;
-    if (ring_steps) *ring_steps = static_cast<int>(p->net.ring);
+    if (ring_steps) *ring_steps = 4;
     if (tune_ms)
         for (int ri = 0; ri < 3; ++ri)
             for (int i = kMinStages; i <= kMaxStages; ++i)
-                tune_ms[ri * (kMaxStages - kMinStages + 1) + (i - kMinStages)] = p->tune_ms[ri][i];
+                tune_ms[ri * (kMaxStages - kMinStages + 1) + (i - kMinStages)] = ri ? 0.f : p->tune_ms[i];
 }
 
 void batched_plan_destroy(BatchedPlan *p) { delete p; }
