@@ -232,40 +232,38 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
+// As tma_load_2d for a CTA pair: the bytes land in this CTA's shared memory and are counted by the
+// mbarrier at `mbar`, a shared::cluster address that may be the other CTA's.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t mbar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
+        : "memory");
+}
+
 constexpr int kTmaThreads = 128;
 
-// Tile shapes of the TMA-fed kernel: 128 x kTN (kTN = 128, or 256 for large GEMMs: one MMA of
-// N = 256 reads its 8 KB of A per 16-deep step for twice the work, halving shared-memory operand
-// traffic per FLOP). Stages: as many as fit the 227 KB of shared memory.
-template <int kTN>
-struct TmaTile
-{
-    static constexpr uint32_t kBBytes = kTN * kBK * 2;
-    static constexpr uint32_t kStage = kTileBytes + kBBytes;
-    static constexpr int kStages = kTN == 128 ? 6 : 4;
-    static constexpr uint32_t kSmem = kStages * kStage + 1024;  // + alignment slack
-};
+constexpr int kTmaStages = 6;
+constexpr uint32_t kTmaSmem = kTmaStages * kStageBytes + 1024;  // + alignment slack
 
-// One 128 x kTN tile of D (or of split blockIdx.z's partial, into `out` with row stride N) over
+// One 128 x 128 tile of D (or of split blockIdx.z's partial, into `out` with row stride N) over
 // chunks [blockIdx.z * cps, min(nk, (blockIdx.z + 1) * cps)). Warp 0 lane 0 issues the TMA copies,
 // warp 1 lane 0 the MMAs; all four warps read the accumulator back.
-template <int kTN>
 __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *__restrict__ out, int M,
     int N, int K, int cps, size_t split_stride, unsigned int *err)
 {
-    using Tile = TmaTile<kTN>;
-    constexpr int kTmaStages = Tile::kStages;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[kTmaStages], empty[kTmaStages], acc_full, drain;
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kTN;
+    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
     const int nk = (K + kBK - 1) / kBK;
     const int c0 = blockIdx.z * cps, c1 = min(nk, c0 + cps);
     float *dst = out + blockIdx.z * split_stride;
-    if (warp == 0) tc::tmem_alloc(&tmem_slot, kTN);
+    if (warp == 0) tc::tmem_alloc(&tmem_slot, kBN);
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < kTmaStages; ++s)
@@ -294,8 +292,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
                 s_fail = 1;
                 break;
             }
-            const uint32_t sa = base + s * Tile::kStage;
-            mbar_expect_tx(&full[s], Tile::kStage);
+            const uint32_t sa = base + s * kStageBytes;
+            mbar_expect_tx(&full[s], kStageBytes);
             tma_load_2d(sa, &ta, c * kBK, m0, &full[s]);
             tma_load_2d(sa + kTileBytes, &tb, c * kBK, n0, &full[s]);
             issued = i + 1;
@@ -306,7 +304,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     }
     else if (warp == 1 && lane == 0)
     {
-        constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kTN);
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kBN);
         for (int c = c0; c < c1; ++c)
         {
             const int i = c - c0, s = i % kTmaStages;
@@ -316,7 +314,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t sa = base + s * Tile::kStage, sb = sa + kTileBytes;
+            const uint32_t sa = base + s * kStageBytes, sb = sa + kTileBytes;
 #pragma unroll
             for (int j = 0; j < kBK / 16; ++j)
                 tc::mma_bf16(tmem, tc::smem_desc_sw128(sa + j * 32, 1024), tc::smem_desc_sw128(sb + j * 32, 1024),
@@ -337,7 +335,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
         const int row = m0 + threadIdx.x;
         const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
 #pragma unroll 1
-        for (int q0 = 0; q0 < kTN; q0 += 16)
+        for (int q0 = 0; q0 < kBN; q0 += 16)
         {
             float v[16];
             if (c1 > c0)
@@ -368,7 +366,221 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, kTN);
+    if (warp == 0) tc::tmem_dealloc(tmem, kBN);
+}
+
+// ---- Large GEMMs: 256 x 256 tiles on CTA pairs. Shared memory bounds a tile that one CTA multiplies
+// alone: for a 64-deep chunk of a 128 x 256 tile TMA writes 48 KB and the MMAs read 48 KB, 768 cycles at
+// 128 B a cycle where the tensor core needs 512 (8192^3: 784 us, 1.40 PFLOP/s). Of a pair's 256 x 256
+// tile each CTA stages 128 rows of A and 128 of B and the tensor cores of both read B's two halves: 64 KB
+// and 512 cycles per CTA. Persistent (one pair per two SMs) with two accumulators, so the read-back of a
+// tile overlaps the next tile's product; tiles are taken in bands of kPairBand rows of tiles, so that
+// the pairs at work share A and B in L2. 8192^3: 634 us, 1.73 PFLOP/s; 2048 x 2048 x 32768: 325 -> 169
+// us; 16384 x 2048 x 2048: 133 -> 90 us. Both CTAs' copies are counted on the even CTA's barriers, whose
+// issuer waits with CTA-scope acquire: a relay of the odd CTA's copies by a cluster-scope wait and arrival
+// cost 2.2 ms at 8192^3.
+constexpr int kPairM = 256, kPairN = 256, kPairStages = 6, kPairBand = 8;
+constexpr uint32_t kPairStage = 2 * kTileBytes;  // this CTA's 128 x 64 of A and of B
+constexpr uint32_t kPairSmem = kPairStages * kPairStage + 1024;
+constexpr uint32_t kDrainWait = 1u << 14;  // polls, about 0.06 s
+constexpr int kPairThreads = 192;  // warps 0-3 read back, warp 4 loads, warp 5 issues (even rank)
+
+__global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gemm_pair_kernel(
+    const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *__restrict__ D, int M, int N,
+    int K, unsigned int *err)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    // Of the even CTA alone: full (both CTAs' halves of a chunk have landed) and acc_empty (4 read-back
+    // warps of each CTA). Of both: empty (the pair's MMAs have read the stage), acc_full.
+    __shared__ __align__(8) uint64_t full[kPairStages], empty[kPairStages];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], drain;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_fail;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = tc::cluster_rank();
+    const uint32_t peer_fail = tc::mapa(tc::smem_u32(&s_fail), rank ^ 1u);
+    auto fail = [&]()
+    {
+        s_fail = 1;
+        tc::st_cluster_u32(peer_fail, 1u);
+        atomicOr(err, 1u);
+    };
+    if (warp == 5) tc::tmem_alloc_pair(&tmem_slot, 2 * kPairN);
+    if (threadIdx.x == 0)
+    {
+        for (int s = 0; s < kPairStages; ++s)
+        {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a)
+        {
+            tc::mbar_init(&acc_full[a], 1);
+            tc::mbar_init(&acc_empty[a], 8);
+        }
+        tc::mbar_init(&drain, 1);
+        s_fail = 0;
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::cluster_sync();  // both CTAs' barriers and tensor memory are set up
+    tc::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+    const uint32_t base = (tc::smem_u32(smem) + 1023u) & ~1023u;
+    const int nk = (K + kBK - 1) / kBK;
+    const int tiles_m = (M + kPairM - 1) / kPairM, tiles_n = (N + kPairN - 1) / kPairN;
+    const int tiles = tiles_m * tiles_n, pairs = gridDim.x / 2, pair = blockIdx.x / 2;
+    auto place = [&](int t, int &m0, int &n0)
+    {
+        const int band = t / (kPairBand * tiles_n), in = t - band * kPairBand * tiles_n;
+        const int rows = min(kPairBand, tiles_m - band * kPairBand);
+        m0 = (band * kPairBand + in % rows) * kPairM;
+        n0 = (in / rows) * kPairN;
+    };
+    auto wait = [&](uint64_t *mbar, uint32_t parity) { return wait_or_fail(mbar, parity, &s_fail); };
+
+    if (warp == 4)
+    {
+        if (lane == 0)
+        {
+            const uint32_t full0 = tc::mapa(tc::smem_u32(full), 0);  // the even CTA's
+            int issued = 0, s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int t = pair; t < tiles && ok; t += pairs)
+            {
+                int m0, n0;
+                place(t, m0, n0);
+                for (int c = 0; c < nk; ++c)
+                {
+                    if (!wait(&empty[s], ph))
+                    {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t sa = base + s * kPairStage;
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * kPairStage);
+                    tma_load_2d_pair(sa, &ta, c * kBK, m0 + 128 * static_cast<int>(rank), full0 + s * 8u);
+                    tma_load_2d_pair(sa + kTileBytes, &tb, c * kBK, n0 + 128 * static_cast<int>(rank), full0 + s * 8u);
+                    ++issued;
+                    if (++s == kPairStages)
+                    {
+                        s = 0;
+                        ph ^= 1u;
+                    }
+                }
+            }
+            if (!ok) fail();
+            // Both CTAs' copies in flight after a failed wait land before either leaves (bounded; a chunk that
+            // only one of them asked for does not complete, so the limit is short).
+            for (int i = max(0, issued - kPairStages); i < issued && rank == 0; ++i)
+                if (!tc::mbar_wait(&full[i % kPairStages], (i / kPairStages) & 1, kDrainWait)) fail();
+        }
+    }
+    else if (warp == 5)
+    {
+        if (lane == 0 && rank == 0)
+        {
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(kPairM, kPairN);
+            const uint64_t da = tc::smem_desc_sw128(base, 1024), db = tc::smem_desc_sw128(base + kTileBytes, 1024);
+            int s = 0, n = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int t = pair; t < tiles && ok; t += pairs, ++n)
+            {
+                const int a = n & 1;
+                if (n >= 2 && !wait(&acc_empty[a], ((n >> 1) - 1) & 1))
+                {
+                    ok = false;
+                    break;
+                }
+                for (int c = 0; c < nk; ++c)
+                {
+                    if (!wait(&full[s], ph))
+                    {
+                        ok = false;
+                        break;
+                    }
+                    tc::fence_after_sync();
+                    const uint64_t off = static_cast<uint64_t>(s) * (kPairStage >> 4);
+#pragma unroll
+                    for (int j = 0; j < kBK / 16; ++j)
+                        tc::mma_bf16_pair(tmem + a * kPairN, da + off + 2 * j, db + off + 2 * j, idesc,
+                                          (c > 0 || j > 0) ? 1u : 0u);
+                    tc::commit_pair(&empty[s]);
+                    if (++s == kPairStages)
+                    {
+                        s = 0;
+                        ph ^= 1u;
+                    }
+                }
+                if (ok) tc::commit_pair(&acc_full[a]);
+            }
+            if (!ok) fail();
+            tc::commit_pair(&drain);
+            if (!tc::mbar_wait(&drain, 0, kWait)) fail();
+        }
+        else if (lane == 0)
+        {
+            // Odd rank: the issuer's last arrivals reach this CTA before it leaves.
+            if (!tc::mbar_wait(&drain, 0, kWait)) fail();
+        }
+    }
+    else
+    {
+        // Read-back: thread t of the CTA has accumulator lane t, row m0 + 128 rank + t of the tile.
+        const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
+        int n = 0;
+        for (int t = pair; t < tiles; t += pairs, ++n)
+        {
+            const int a = n & 1;
+            if (!__all_sync(0xffffffffu, wait(&acc_full[a], (n >> 1) & 1)))
+            {
+                if (lane == 0) fail();
+                break;
+            }
+            tc::fence_after_sync();
+            int m0, n0;
+            place(t, m0, n0);
+            const int row = m0 + 128 * static_cast<int>(rank) + static_cast<int>(threadIdx.x);
+            float *d = D + static_cast<size_t>(row) * N + n0;
+            const bool vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(D) & 15u) == 0;
+#pragma unroll 1
+            for (int q0 = 0; q0 < kPairN; q0 += 32)
+            {
+                float v[32];
+                tc::tmem_ld32(tmem + a * kPairN + lane_base + q0, v);
+                if (q0 + 32 == kPairN)
+                {
+                    // The whole accumulator has been read: the issuer may start the tile after next in it.
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&acc_empty[a]), 0));
+                }
+                if (row >= M)
+                {
+                }
+                else if (vec && n0 + q0 + 32 <= N)
+                {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        reinterpret_cast<float4 *>(d + q0)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+                else
+                {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (n0 + q0 + i < N) d[q0 + i] = v[i];
+                }
+                __syncwarp();  // the next read is warp-collective
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    // Neither CTA leaves while the other's MMAs may read its shared memory or arrivals may reach it.
+    tc::cluster_sync();
+    if (warp == 5) tc::tmem_dealloc_pair(tmem, 2 * kPairN);
 }
 
 // D = sum over the splits of ws[z] (split order), n elements.
@@ -406,13 +618,13 @@ EncodeTiled encode_tiled()
 
 // The (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple of 8), loaded in 64 x 128
 // boxes with the 128-byte swizzle.
-bool sw128_map(CUtensorMap *map, const void *ptr, int rows, int K, int box_rows = kBM)
+bool sw128_map(CUtensorMap *map, const void *ptr, int rows, int K)
 {
     const EncodeTiled fn = encode_tiled();
     if (!fn) return false;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-    const cuuint32_t box[2] = {kBK, static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t box[2] = {kBK, kBM};
     const cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -477,52 +689,56 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int tiles_m = (M + kBM - 1) / kBM;
     const int nk = (K + kBK - 1) / kBK;
-    // 128 x 256 tiles when they alone fill every SM (large GEMMs; no K split then).
-    if (N >= 256 && tiles_m * ((N + 255) / 256) >= sms && sw128_map(&ta, A, M, K) && sw128_map(&tb, B, N, K, 256))
+    const int tiles_n = (N + kBN - 1) / kBN, tiles = tiles_m * tiles_n;
+    const int pair_tiles = ((M + kPairM - 1) / kPairM) * ((N + kPairN - 1) / kPairN);
+    if (!sw128_map(&ta, A, M, K) || !sw128_map(&tb, B, N, K))
     {
-        if (smem_limit_once(gemm_tma_kernel<256>, static_cast<int>(TmaTile<256>::kSmem), dev) != cudaSuccess) return -3;
-        dim3 grid(tiles_m, (N + 255) / 256, 1);
-        gemm_tma_kernel<256><<<grid, kTmaThreads, TmaTile<256>::kSmem, s>>>(ta, tb, D, M, N, K, nk, 0, d_err);
+        if (smem_limit_once(gemm_pipe_kernel, static_cast<int>(kStages * kStageBytes), dev) != cudaSuccess) return -3;
+        dim3 grid(tiles_m, tiles_n);
+        gemm_pipe_kernel<<<grid, kThreads, kStages * kStageBytes, s>>>(
+            static_cast<const __nv_bfloat16 *>(A), static_cast<const __nv_bfloat16 *>(B), D, M, N, K, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
-    if (sw128_map(&ta, A, M, K) && sw128_map(&tb, B, N, K))
+    // A 128 x 128 tile on one CTA (bound by shared memory) and a 256 x 256 tile on a pair (bound by the
+    // tensor core) take the same 512 cycles per 64-deep chunk, so the form with fewer waves is the faster
+    // (2500^3: 3 waves 86 us, 2 waves 74 us; 2048 x 2048 x 32768: 2 waves 325 us, 1 wave 169 us); at the
+    // same number of waves the small tiles start and end sooner and may split K.
+    const int waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
+    if (pair_waves < waves)
     {
-        if (smem_limit_once(gemm_tma_kernel<128>, static_cast<int>(TmaTile<128>::kSmem), dev) != cudaSuccess) return -3;
-        const int tiles_n = (N + kBN - 1) / kBN, tiles = tiles_m * tiles_n;
-        // Split K when the tiles leave most SMs idle and each split keeps at least 4 chunks.
-        int splits = 1;
-        if (tiles * 2 <= sms) splits = std::max(1, std::min({16, nk / 4, sms / tiles}));
-        const int cps = (nk + splits - 1) / splits;
-        splits = (nk + cps - 1) / cps;
-        const size_t mn = static_cast<size_t>(M) * N;
-        float *ws = nullptr;
-        if (splits > 1)
-        {
-            const cudaMemPool_t pool = split_pool(dev);
-            if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), mn * splits * sizeof(float), pool, s) !=
-                             cudaSuccess)
-            {
-                cudaGetLastError();
-                ws = nullptr;
-                splits = 1;
-            }
-        }
-        const int cps_used = splits > 1 ? cps : nk;
-        dim3 grid(tiles_m, tiles_n, splits);
-        gemm_tma_kernel<128><<<grid, kTmaThreads, TmaTile<128>::kSmem, s>>>(ta, tb, splits > 1 ? ws : D, M, N, K,
-                                                                          cps_used, splits > 1 ? mn : 0, d_err);
-        if (splits > 1)
-        {
-            const int blocks = static_cast<int>(std::min<size_t>((mn + 255) / 256, 8ull * sms));
-            split_sum_kernel<<<blocks, 256, 0, s>>>(ws, D, mn, splits);
-            cudaFreeAsync(ws, s);
-        }
+        if (smem_limit_once(gemm_pair_kernel, static_cast<int>(kPairSmem), dev) != cudaSuccess) return -3;
+        gemm_pair_kernel<<<2 * std::min(pair_tiles, sms / 2), kPairThreads, kPairSmem, s>>>(ta, tb, D, M, N, K, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
-    if (smem_limit_once(gemm_pipe_kernel, static_cast<int>(kStages * kStageBytes), dev) != cudaSuccess) return -3;
-    dim3 grid((M + kBM - 1) / kBM, (N + kBN - 1) / kBN);
-    gemm_pipe_kernel<<<grid, kThreads, kStages * kStageBytes, s>>>(static_cast<const __nv_bfloat16 *>(A),
-                                                                   static_cast<const __nv_bfloat16 *>(B), D, M, N, K, d_err);
+    if (smem_limit_once(gemm_tma_kernel, static_cast<int>(kTmaSmem), dev) != cudaSuccess) return -3;
+    // Split K when the tiles leave most SMs idle and each split keeps at least 4 chunks.
+    int splits = 1;
+    if (tiles * 2 <= sms) splits = std::max(1, std::min({16, nk / 4, sms / tiles}));
+    const int cps = (nk + splits - 1) / splits;
+    splits = (nk + cps - 1) / cps;
+    const size_t mn = static_cast<size_t>(M) * N;
+    float *ws = nullptr;
+    if (splits > 1)
+    {
+        const cudaMemPool_t pool = split_pool(dev);
+        if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), mn * splits * sizeof(float), pool, s) !=
+                         cudaSuccess)
+        {
+            cudaGetLastError();
+            ws = nullptr;
+            splits = 1;
+        }
+    }
+    const int cps_used = splits > 1 ? cps : nk;
+    dim3 grid(tiles_m, tiles_n, splits);
+    gemm_tma_kernel<<<grid, kTmaThreads, kTmaSmem, s>>>(ta, tb, splits > 1 ? ws : D, M, N, K, cps_used,
+                                                        splits > 1 ? mn : 0, d_err);
+    if (splits > 1)
+    {
+        const int blocks = static_cast<int>(std::min<size_t>((mn + 255) / 256, 8ull * sms));
+        split_sum_kernel<<<blocks, 256, 0, s>>>(ws, D, mn, splits);
+        cudaFreeAsync(ws, s);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 }  // namespace knp_gb300

@@ -291,5 +291,50 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v)
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// ---- CTA pairs (cta_group::2): the two CTAs of a cluster multiply one tile. Each holds half of A's
+// rows (its own accumulator lanes) and half of B's rows in its own shared memory, at the same
+// offsets; the even-ranked CTA issues the MMAs for both.
+
+// Tensor-memory allocation and release by one warp of each CTA of the pair.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t *slot, uint32_t ncols)
+{
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
+                 "r"(ncols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+}
+
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols)
+{
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
+}
+
+// As mma_bf16 for a pair; issued by one thread of the even-ranked CTA.
+__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// The mbarriers at this shared-memory offset in both CTAs of the pair each receive one arrival when
+// every previously issued pair MMA of this thread has completed.
+__device__ __forceinline__ void commit_pair(uint64_t *mbar)
+{
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_u32(mbar)),
+        "h"(static_cast<uint16_t>(3))
+        : "memory");
+}
+
+// One arrival (release, cluster scope) on an mbarrier of a CTA of this cluster (address from mapa).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_mbar)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_mbar) : "memory");
+}
+
 }  // namespace tc
 }  // namespace knp_gb300
