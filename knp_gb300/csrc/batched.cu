@@ -159,8 +159,8 @@ int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, in
 // neuron and its columns are consecutive steps of one sample, so the thread that owns the lane runs
 // the recurrence down its row with the membrane state in registers, and no step waits for another
 // CTA. (Stepping all layers together, one step at a time, costs a chain of expansion, product,
-// exchange and hand-over per step: 0.87-0.95 ms for 256 samples of 784-1000-1000-10 and 50-200 steps,
-// the tensor cores idle for most of it; see the kernel for this form's time.)
+// exchange and hand-over per step: 0.95 ms for 256 samples of 784-1000-1000-10 and 50-200 steps, the
+// tensor cores idle for most of it; this form takes 0.24 ms.)
 //
 // Spikes travel between layers as bitmaps: per layer one row of wpad words (bit j of word w = neuron
 // 32 w + j) for every (sample, step) of a segment of steps, a sample's rows consecutive:
@@ -172,18 +172,27 @@ namespace
 {
 
 constexpr int kMaxLayers = 4;
-constexpr uint32_t kTileN = 128;      // neurons of a CTA (accumulator rows)
-constexpr uint32_t kStreamCols = 128;  // columns of one stream in a tile (two streams per CTA)
+constexpr uint32_t kTileN = 128;  // neurons of a CTA (its accumulator rows); a CTA pair has two tiles
+constexpr uint32_t kStreamCols = 128;  // columns of one stream in a tile (two streams per pair)
 constexpr uint32_t kCols = 2 * kStreamCols;
-constexpr uint32_t kChunk = 64;                      // K of a staged chunk
-constexpr uint32_t kAChunk = kTileN * kChunk * 2;   // 16 KB of packed weights
-constexpr uint32_t kBChunk = kCols * kChunk * 2;    // 32 KB of expanded spikes
-constexpr uint32_t kLayerStage = kAChunk + kBChunk;
+constexpr uint32_t kChunk = 64;                          // K of a staged chunk
+constexpr uint32_t kAChunk = kTileN * kChunk * 2;       // 16 KB of packed weights
+constexpr uint32_t kBChunk = kStreamCols * kChunk * 2;  // 16 KB of expanded spikes, this CTA's stream
+// A stage of the operand ring holds two chunks (weights of both, then spikes of both); the issuer
+// spends as long on a wait and a commit as on two MMAs, so it waits once for eight of them.
+constexpr uint32_t kLayerStage = 2 * (kAChunk + kBChunk);
 constexpr int kMinStages = 2, kMaxStages = 4;  // operand ring depths the autotuner tries
-constexpr int kExpandWarps = 8, kScanWarps = 8;
-constexpr int kIssuerWarp = 0, kCopyWarp = 1, kScanWarp0 = 4, kExpandWarp0 = kScanWarp0 + kScanWarps;
+constexpr int kMaxRing = 3;
+constexpr int ring_stages(int depth) { return depth - 1; }
+constexpr int kExpandWarps = 8, kScanWarps = 8, kRowWarps = 2;
+constexpr int kExpandGroups = 2;  // groups of expander warps, one per chunk of a stage
+constexpr uint32_t kGroupThreads = 32 * kExpandWarps / kExpandGroups;
+constexpr int kIssuerWarp = 0, kCopyWarp = 1, kRowWarp0 = 2, kScanWarp0 = 4, kExpandWarp0 = kScanWarp0 + kScanWarps;
 constexpr int kLayerThreads = 32 * (kExpandWarp0 + kExpandWarps);
-constexpr uint32_t kTmemCols = 512;  // two accumulators of kCols columns
+constexpr uint32_t kRowSlots = 4;  // tiles of row indexes kept ahead of the expanders
+constexpr uint32_t kDrainWait = 1u << 14;  // polls, about 0.06 s
+static_assert(kGroupThreads == kStreamCols, "an expander thread has one row of a chunk");
+constexpr uint32_t kTmemCols = 512;  // two accumulators of kCols columns per CTA
 constexpr uint32_t kScanCols = 32;   // columns a scan thread reads from its accumulator at a time
 constexpr uint32_t kPad = 8;         // a sample's columns in a stream are padded to a multiple of this
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
@@ -193,11 +202,11 @@ constexpr size_t kRowBudget = size_t(256) << 20;   // bytes of a layer's rows pe
 constexpr uint32_t kMaxTiles = 512;  // (layer, 128-sample tile, 64-neuron tile, half) units a plan may have
 
 // What one launch of a layer needs. A stream is a list of samples whose columns follow one another;
-// CTA (n tile, g) runs streams 2 g and 2 g + 1 side by side, one per half of its columns, so that the
-// scans of two warpgroups share the SM while the next tile's product runs.
+// CTA pair (pair of n tiles, g) runs streams 2 g and 2 g + 1 side by side, one per half of its columns:
+// each CTA expands one stream's spikes and scans its own neurons in both.
 struct LayerArgs
 {
-    const uint8_t *w;         // packed weights: [n tile][chunk] blocks of kAChunk bytes (pack_weights_kernel)
+    CUtensorMap w;            // packed weights as rows of kChunk elements: block [n tile][chunk] is 128 rows
     const uint32_t *bits_in;  // rows of the layer below
     uint32_t wp_in;           // words per row (a multiple of 4)
     uint32_t *bits_out;       // this layer's rows (null for the last layer)
@@ -205,7 +214,7 @@ struct LayerArgs
     uint32_t n;               // neurons
     uint32_t kp;              // fan-in rounded up to 16
     uint32_t chunks;          // ceil(kp / kChunk)
-    uint32_t n_groups;        // CTAs per neuron tile
+    uint32_t n_groups;        // CTA pairs per pair of neuron tiles
     float leak, thr, reset;
     uint32_t refract;
     const uint32_t *st_off;   // [2 n_groups + 1] first entry of each stream
@@ -225,7 +234,7 @@ struct LayerArgs
     unsigned int *err;        // bit 0: a wait gave up
     uint32_t poll_limit;
     uint32_t stall;           // failure test: the issuer waits for this many more expanders than exist
-    uint32_t stages;          // operand ring depth
+    uint32_t ring;            // stages of the operand ring
 };
 
 // Position p of a 16-wide K block holds input (p >> 1) + 8 (p & 1) of the block, in the packed
@@ -233,9 +242,10 @@ struct LayerArgs
 // 8 + i of the block's 16 spike bits, which one shift and one mask isolate.
 __host__ __device__ constexpr uint32_t k_of(uint32_t p) { return (p >> 1) + 8u * (p & 1u); }
 
-// Weights of one layer, BF16 [n][k] row-major (any k), to [n tile][chunk] blocks in the 128-byte
-// swizzled K-major layout of tc::smem_desc_sw128, zero past n and k. One thread per 16 bytes. Repacked
-// in every run (the caller may rewrite the weights between runs): 4 MB, 3 us at 784-1000-1000-10.
+// Weights of one layer, BF16 [n][k] row-major (any k), to [n tile][chunk] blocks of 128 rows of 64
+// elements, zero past n and k, which TMA loads with the 128-byte swizzle. One thread per 16 bytes.
+// Repacked in every run (the caller may rewrite the weights between runs): 4 MB, 5 us at
+// 784-1000-1000-10.
 struct PackArgs
 {
     const __nv_bfloat16 *w[kMaxLayers];
@@ -266,7 +276,7 @@ __global__ void pack_weights_kernel(const __grid_constant__ PackArgs a)
             const uint32_t k = chunk * kChunk + (slot >> 1) * 16u + k_of((slot & 1u) * 8u + i);
             e[i] = (row < a.n[l] && k < a.k[l]) ? a.w[l][static_cast<size_t>(row) * a.k[l] + k] : __float2bfloat16(0.0f);
         }
-        *reinterpret_cast<uint4 *>(a.out[l] + blk * kAChunk + r * 128u + ((slot ^ (r & 7u)) << 4)) =
+        *reinterpret_cast<uint4 *>(a.out[l] + blk * kAChunk + r * 128u + (slot << 4)) =
             *reinterpret_cast<uint4 *>(e);
     }
 }
@@ -323,8 +333,8 @@ struct DrawArgs
 // consecutive rows, a bit per row, and one transposition across the warp gives the rows' words; a draw is
 // counted and recorded in the segment where it is not row 0. Bound by the draws' integer instructions (two
 // 64-bit products each, half-rate pipes): one lane per input keeps the rate loads coalesced and one
-// threshold serves 32 draws.
-__global__ void __launch_bounds__(256) input_rows_kernel(const __grid_constant__ DrawArgs a)
+// threshold serves 32 draws. 26 M draws: 49 us (one thread per word of 32 draws: 56 us).
+__global__ void __launch_bounds__(256, 6) input_rows_kernel(const __grid_constant__ DrawArgs a)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long items = static_cast<unsigned long long>(a.batch) * a.blocks * a.wp;
@@ -396,22 +406,6 @@ __global__ void __launch_bounds__(256) input_rows_kernel(const __grid_constant__
     if (lane == 0 && ev) atomicAdd(a.events, ev);
 }
 
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *mbar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(mbar)),
-                 "r"(bytes)
-                 : "memory");
-}
-
-// Copies `bytes` (a multiple of 16, both addresses 16-byte aligned) into shared memory, completing
-// them on the mbarrier's transaction count.
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *mbar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(tc::smem_u32(mbar))
-                 : "memory");
-}
-
 // mbar_wait that also gives up as soon as another role of the CTA has.
 __device__ __forceinline__ bool wait_or_fail(uint64_t *mbar, uint32_t parity, uint32_t limit, const volatile int *fail)
 {
@@ -455,6 +449,7 @@ struct ScanTarget
     uint32_t off, len;  // its stream's first entry and its columns
     uint32_t neuron, wq;  // this thread's neuron, the warp's word in a row
     uint32_t n_tiles;
+    uint32_t acc_empty;  // the even CTA's acc_empty barriers (shared::cluster address)
 };
 
 // The LIF recurrence of one stream down its accumulator columns (lif_impl.h:33-86: leak and input only
@@ -463,9 +458,9 @@ struct ScanTarget
 // neurons' words into the columns' bitmap words, so a step costs five instructions and no vote. A
 // sample's columns are padded to a multiple of kPad, so that kPad steps at a time need no check
 // for its end. Returns false if a wait gave up.
-template <bool kRefract>
+template <bool kRefract, bool kLeak>
 __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget &tgt, uint32_t lane, uint64_t *acc_full,
-                                            uint64_t *acc_empty, const volatile int *fail, unsigned long long &events)
+                                            const volatile int *fail, unsigned long long &events)
 {
     const float leak = a.leak, thr = a.thr, reset = a.reset;
     // The sample being scanned (sample, first row, columns, steps in all), its next step (from t0), and
@@ -474,6 +469,9 @@ __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget
     uint4 info = make_uint4(0, 0, 0, 0), next = info;
     bool exists = false;
     float V = 0.0f;
+    bool spiked = false;
+    const float reset_leak = __fmul_rn(reset, leak);
+    float limit = thr;  // thr, or +infinity for a neuron its sample does not have
     uint32_t RC = 0, count = 0, last_word = 0;
     uint32_t end = 0;  // the stream column after the sample's last (padded)
     auto open_sample = [&]()
@@ -484,6 +482,8 @@ __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget
         if (end < tgt.len) next = a.st_info[entry + 1];
         const uint32_t smp = info.x;
         exists = tgt.neuron < (a.own_size ? a.own_size[smp] : a.n);
+        limit = exists ? thr : __int_as_float(0x7F800000);
+        spiked = false;
         fan = a.next_size ? a.next_size[smp] : a.next_n;
         V = 0.0f;
         RC = count = 0;
@@ -512,7 +512,7 @@ __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget
             if (tgt.neuron < a.n)
             {
                 uint32_t *st = a.state + (static_cast<size_t>(smp) * a.n + tgt.neuron) * 3;
-                st[0] = __float_as_uint(V);
+                st[0] = __float_as_uint(spiked ? reset : V);
                 st[1] = RC;
                 st[2] = count;
             }
@@ -542,15 +542,18 @@ __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget
                 // The last columns of this tile are in registers: the accumulator may be reused.
                 tc::fence_before_sync();
                 __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&acc_empty[acc]);
+                if (lane == 0) tc::mbar_arrive_cluster(tgt.acc_empty + acc * 8u);
             }
             if (!here) break;
             uint32_t bits = 0;  // bit c: this neuron fired at column c0 + c
+            // V is the potential before its reset: `spiked` says whether the last step reset it. The sum
+            // with the reset value is formed beside the sum with the kept one, so the chain from step to
+            // step is a product (leak only; V * 1 is V), a sum and a choice.
             auto step = [&](uint32_t c)
             {
-                const float v = __fadd_rn(__fmul_rn(V, leak), x[c]);
                 if (kRefract)
                 {
+                    const float v = __fadd_rn(__fmul_rn(V, leak), x[c]);
                     const bool free_ = RC == 0u;
                     const bool spike = exists && free_ && v > thr;
                     V = spike ? reset : (free_ ? v : V);
@@ -559,9 +562,11 @@ __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget
                 }
                 else
                 {
-                    const bool spike = exists && v > thr;
-                    V = spike ? reset : v;
-                    if (spike) bits |= 1u << c;
+                    const float kept = __fadd_rn(kLeak ? __fmul_rn(V, leak) : V, x[c]);
+                    const float fresh = __fadd_rn(reset_leak, x[c]);
+                    V = spiked ? fresh : kept;
+                    spiked = V > limit;
+                    if (spiked) bits |= 1u << c;
                 }
             };
             // Columns [from, to) of this block, steps j0 .. of the sample, are done: their bitmap words go
@@ -620,147 +625,153 @@ __device__ __forceinline__ bool scan_stream(const LayerArgs &a, const ScanTarget
     return true;
 }
 
-// One layer over a segment of steps. Roles: warps 0-7 expand spike rows into the BF16 operand, warps
-// 8-15 run the LIF scan (thread = neuron; warps 8-11 the first stream's half of the accumulator, 12-15
-// the second's), warp 16 copies packed weight chunks, warp 17 issues the MMAs (M = 128 neurons, N = 256
-// columns, FP32 accumulator in tensor memory, two of them, so the scan of a tile runs beside the product
-// of the next). Every wait is bounded; a wait that gives up sets bit 0 of *err, stops the roles, lets
-// copies and MMAs in flight land, and frees the tensor memory.
-// kGroups: groups of expander warps that take the chunks in turn. Every stage of the ring belongs to one
-// group (the ring depth is a multiple of kGroups), so that a group waiting for a stage's next release
-// has seen the release before it: a parity wait cannot tell phases two apart.
-template <int kGroups>
-__global__ void __launch_bounds__(kLayerThreads, 1) lif_layer_kernel(const __grid_constant__ LayerArgs a)
+// One layer over a segment of steps, on CTA pairs. Roles in each CTA: warp 0 issues the pair's MMAs (even
+// rank; M = 256 neurons, N = 256 columns, FP32 accumulators in tensor memory, two of them, so the scan of a
+// tile runs beside the product of the next), warp 1 copies packed weight chunks, warps 2-3 look up the
+// columns' spike rows a few tiles ahead, warps 4-11 scan (thread = neuron; 4-7 the first stream's half of
+// the accumulator, 8-11 the second's), warps 12-19 expand this CTA's stream into the BF16 operand. Every wait
+// is bounded; a wait that gives up sets bit 0 of *err and stops the roles of both CTAs, copies and MMAs in
+// flight land, and the tensor memory is freed.
+// A pair rather than one CTA per tile: each CTA expands one stream instead of both, and shared memory
+// carries 128 KB per 128-deep stage instead of 192 KB (1024 cycles of tensor work either way). 256 samples of
+// 784-1000-1000-10, 50-200 steps: the three layers take 66, 73 and 27 us (one CTA per 128 x 256 tile: 93,
+// 112, 33); what is left above the tensor time (about 58 us in all) is a stage's hand-over (wait, eight MMAs
+// and commit take the issuing thread about as long as they run), the scan (about 60 cycles a step beside the
+// expansion) and some 10 us of start and end per launch.
+__global__ void __launch_bounds__(kLayerThreads, 1) __cluster_dims__(2, 1, 1)
+    lif_layer_kernel(const __grid_constant__ LayerArgs a)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t full_w[kMaxStages], full_s[kMaxStages], empty[kMaxStages];
+    // Of the even CTA alone: full (both CTAs' weights and spikes of a stage are in place: its copy warp's
+    // arrival with the bytes of both, and one arrival per expander group) and acc_empty (the scan warps of
+    // both). Of each CTA: empty, acc_full and drain (commits reach both), the row indexes.
+    __shared__ __align__(8) uint64_t full[kMaxRing], empty[kMaxRing];
     __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], drain;
+    __shared__ __align__(8) uint64_t row_full[kRowSlots], row_empty[kRowSlots];
+    __shared__ uint32_t s_row[kRowSlots][kStreamCols];  // a column's row of bits_in, or kNoRow
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
     __shared__ unsigned long long s_events;
-    __shared__ uint32_t s_row[2][kCols];  // [tile parity][column]: its row of bits_in, or kNoRow
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t n_tile = blockIdx.x / a.n_groups, group = blockIdx.x - n_tile * a.n_groups;
-    if (warp == kIssuerWarp) tc::tmem_alloc(&tmem_slot, kTmemCols);
+    const uint32_t rank = tc::cluster_rank();
+    const uint32_t pair = blockIdx.x >> 1;
+    const uint32_t n_pair = pair / a.n_groups, group = pair - n_pair * a.n_groups;
+    const uint32_t n_tile = 2 * n_pair + rank;
+    const uint32_t peer_fail = tc::mapa(tc::smem_u32(&s_fail), rank ^ 1u);
+    auto fail = [&]()
+    {
+        s_fail = 1;
+        tc::st_cluster_u32(peer_fail, 1u);
+        atomicOr(a.err, 1u);
+    };
+    if (warp == kIssuerWarp) tc::tmem_alloc_pair(&tmem_slot, kTmemCols);
     if (threadIdx.x == 0)
     {
-        for (int s = 0; s < kMaxStages; ++s)
+        for (int s = 0; s < kMaxRing; ++s)
         {
-            tc::mbar_init(&full_w[s], 1);
-            tc::mbar_init(&full_s[s], kExpandWarps / kGroups + a.stall);
+            tc::mbar_init(&full[s], 1 + 2 * kExpandGroups + a.stall);
             tc::mbar_init(&empty[s], 1);
         }
         for (int i = 0; i < 2; ++i)
         {
             tc::mbar_init(&acc_full[i], 1);
-            tc::mbar_init(&acc_empty[i], kScanWarps);
+            tc::mbar_init(&acc_empty[i], 2 * kScanWarps);
+        }
+        for (uint32_t i = 0; i < kRowSlots; ++i)
+        {
+            tc::mbar_init(&row_full[i], kRowWarps);
+            tc::mbar_init(&row_empty[i], kExpandWarps);
         }
         tc::mbar_init(&drain, 1);
         s_events = 0;
+        s_fail = 0;
     }
     // Everything above overlaps the preceding kernel; from here on its results are read.
     pdl_begin();
-    if (threadIdx.x == 0) s_fail = *reinterpret_cast<volatile unsigned int *>(a.err) != 0u ? 1 : 0;
-    tc::fence_before_sync();
     __syncthreads();
+    if (threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int *>(a.err) != 0u) s_fail = 1;
+    tc::fence_before_sync();
+    tc::cluster_sync();  // both CTAs' barriers and tensor memory are set up
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
     const uint32_t base = (tc::smem_u32(smem) + 1023u) & ~1023u;  // swizzle atoms on 1024-byte boundaries
-    const uint32_t stages = a.stages, chunks = a.chunks;
+    const uint32_t ring = a.ring, chunks = a.chunks, per_tile = (chunks + 1) / 2;  // stages of a tile
     const uint32_t n_tiles =
         (max(a.st_len[2 * group], a.st_len[2 * group + 1]) + kStreamCols - 1) / kStreamCols;
     unsigned long long my_events = 0;
 
     if (warp >= kExpandWarp0)
     {
-        // Expanders: thread r looks up the row of column r of a tile; then kGroups groups of warps take
-        // every kGroups-th chunk, a thread expanding kGroups of its 256 rows (a group's wait, expansion
-        // and proxy fence overlap those of the others).
-        constexpr uint32_t kRows = 256 / kGroups;  // threads of a group: rows gr + kRows i
-        static_assert(kRows % 32 == 0 && kExpandWarps == 8, "whole warps");
-        const uint32_t r = threadIdx.x - 32 * kExpandWarp0, stream = 2 * group + (r >> 7);
-        const uint32_t off = a.st_off[stream], entries = a.st_off[stream + 1] - off, len = a.st_len[stream];
-        const uint32_t gr = r & (kRows - 1), sw = gr & 7u;
-        uint32_t c = r / kRows, s = c, ph = 1;  // this group's next chunk, its stage and parity
+        // Expanders: group g of four warps expands chunk g of every stage, a thread one of its 128 rows.
+        const uint32_t e = threadIdx.x - 32 * kExpandWarp0, r = e & (kStreamCols - 1), sw = r & 7u;
+        const uint32_t g = e / kGroupThreads;
+        const uint32_t full0 = tc::mapa(tc::smem_u32(full), 0);
+        const uint32_t dst0 = base + 2 * kAChunk + g * kBChunk + r * 128u;
         bool ok = true;
-        for (uint32_t tile = 0; tile < n_tiles; ++tile)
+        // The stage being loaded (tile lt, stage lc of it) runs one ahead of the one being expanded.
+        uint32_t lt = 0, lc = 0;
+        const uint32_t *row = nullptr;
+        auto open_tile = [&]()
         {
-            const uint32_t p = tile * kStreamCols + (r & (kStreamCols - 1));
-            uint32_t row = kNoRow;
-            if (p < len)
+            row = nullptr;
+            if (lt >= n_tiles || !ok) return;
+            const uint32_t slot = lt % kRowSlots;
+            if (!warp_wait(&row_full[slot], (lt / kRowSlots) & 1u, a.poll_limit, &s_fail, lane))
             {
-                uint32_t lo = 0, hi = entries;  // the last entry that starts at or before p
-                while (hi - lo > 1)
-                {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (a.st_start[off + mid] <= p) lo = mid;
-                    else hi = mid;
-                }
-                const uint4 e = a.st_info[off + lo];
-                const uint32_t j = p - a.st_start[off + lo];
-                if (j < e.z) row = e.y + j;
+                ok = false;
+                return;
             }
-            s_row[tile & 1u][r] = row;
-            // The group's decision is uniform; the barrier also publishes the tile's rows (a buffer is
-            // rewritten two tiles later, after every reader has passed the next tile's barrier).
-            if (!tc::named_sync_and(1, 32 * kExpandWarps, ok)) break;
-            const uint32_t *src[kGroups];
-#pragma unroll
-            for (int i = 0; i < kGroups; ++i)
-            {
-                const uint32_t q = s_row[tile & 1u][gr + kRows * i];
-                src[i] = q == kNoRow ? nullptr : a.bits_in + static_cast<size_t>(q) * a.wp_in;
-            }
-            auto load = [&](uint32_t chunk, uint2 (&h)[kGroups])
-            {
-#pragma unroll
-                for (int i = 0; i < kGroups; ++i)
-                    h[i] = src[i] ? __ldcg(reinterpret_cast<const uint2 *>(src[i] + 2 * chunk)) : make_uint2(0, 0);
-            };
-            uint2 h[kGroups];
-            if (c < chunks) load(c, h);
-            while (c < chunks)
-            {
-                uint2 next[kGroups];
-                if (c + kGroups < chunks) load(c + kGroups, next);  // used after this chunk
-                // (the first pass over the ring finds every stage free)
-                if (!warp_wait(&empty[s], ph, a.poll_limit, &s_fail, lane))
-                {
-                    ok = false;
-                    break;
-                }
-                const uint32_t dst = base + s * kLayerStage + kAChunk + gr * 128u;
-#pragma unroll
-                for (uint32_t i = 0; i < kGroups; ++i)
-#pragma unroll
-                    for (uint32_t b = 0; b < 4; ++b)
-                    {
-                        uint32_t v[8];
-                        const uint32_t word = b < 2 ? h[i].x : h[i].y;
-                        expand16((b & 1u) ? word >> 16 : word, v);
-                        st_shared_v4(dst + i * (kRows * 128u) + (((2 * b) ^ sw) << 4), v);
-                        st_shared_v4(dst + i * (kRows * 128u) + (((2 * b + 1) ^ sw) << 4), v + 4);
-                    }
-                tc::fence_async_smem();
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&full_s[s]);
-#pragma unroll
-                for (int i = 0; i < kGroups; ++i) h[i] = next[i];
-                c += kGroups;
-                s += kGroups;
-                if (s >= stages)
-                {
-                    s -= stages;
-                    ph ^= 1u;
-                }
-            }
-            c -= chunks;  // position in the next tile (wraps only when ok is false)
-        }
-        if (!ok && lane == 0)
+            const uint32_t q = s_row[slot][r];
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&row_empty[slot]);
+            if (q != kNoRow) row = a.bits_in + static_cast<size_t>(q) * a.wp_in + 2 * g;
+        };
+        // Rows are padded to whole stages (wp_in is a multiple of 4 words).
+        auto load = [&]() { return row ? __ldcg(reinterpret_cast<const uint2 *>(row + 4 * lc)) : make_uint2(0, 0); };
+        open_tile();
+        uint32_t s = 0, ph = 1;  // the stage and its parity (the first pass finds it free)
+        bool have = n_tiles > 0;
+        uint2 h = have ? load() : make_uint2(0, 0);
+        while (have)
         {
-            s_fail = 1;
-            atomicOr(a.err, 1u);
+            const uint2 now = h;
+            if (++lc == per_tile)
+            {
+                lc = 0;
+                ++lt;
+                open_tile();
+            }
+            have = lt < n_tiles;
+            if (have) h = load();
+            ok = ok && warp_wait(&empty[s], ph, a.poll_limit, &s_fail, lane);
+            if (ok)
+            {
+                const uint32_t dst = dst0 + s * kLayerStage;
+#pragma unroll
+                for (uint32_t b = 0; b < 4; ++b)
+                {
+                    uint32_t v[8];
+                    const uint32_t word = b < 2 ? now.x : now.y;
+                    expand16((b & 1u) ? word >> 16 : word, v);
+                    st_shared_v4(dst + (((2 * b) ^ sw) << 4), v);
+                    st_shared_v4(dst + (((2 * b + 1) ^ sw) << 4), v + 4);
+                }
+            }
+            tc::fence_async_smem();
+            // The group's decision is uniform; one thread tells the issuer.
+            if (!tc::named_sync_and(1 + g, kGroupThreads, ok))
+            {
+                ok = false;
+                break;
+            }
+            if (r == 0) tc::mbar_arrive_cluster(full0 + s * 8u);
+            if (++s == ring)
+            {
+                s = 0;
+                ph ^= 1u;
+            }
         }
+        if (!ok && lane == 0) fail();
     }
     else if (warp >= kScanWarp0)
     {
@@ -769,52 +780,95 @@ __global__ void __launch_bounds__(kLayerThreads, 1) lif_layer_kernel(const __gri
         ScanTarget tgt;
         tgt.tmem = tmem + ((32u * (warp & 3u)) << 16) + half * kStreamCols;
         tgt.off = a.st_off[stream];
-        tgt.len = a.st_len[stream];
         tgt.neuron = n_tile * kTileN + 32u * (warp & 3u) + lane;
         tgt.wq = 4u * n_tile + (warp & 3u);
+        // A tile wholly past the layer (an odd number of tiles): nothing to scan.
+        tgt.len = n_tile * kTileN < a.n ? a.st_len[stream] : 0u;
         tgt.n_tiles = n_tiles;
-        const bool ok = a.refract ? scan_stream<true>(a, tgt, lane, acc_full, acc_empty, &s_fail, my_events)
-                                  : scan_stream<false>(a, tgt, lane, acc_full, acc_empty, &s_fail, my_events);
-        if (!ok && lane == 0)
+        tgt.acc_empty = tc::mapa(tc::smem_u32(acc_empty), 0);
+        const bool ok = a.refract         ? scan_stream<true, true>(a, tgt, lane, acc_full, &s_fail, my_events)
+                        : a.leak == 1.0f ? scan_stream<false, false>(a, tgt, lane, acc_full, &s_fail, my_events)
+                                         : scan_stream<false, true>(a, tgt, lane, acc_full, &s_fail, my_events);
+        if (!ok && lane == 0) fail();
+    }
+    else if (warp >= kRowWarp0)
+    {
+        // Row lookups of this CTA's stream: each thread two columns of a tile.
+        const uint32_t stream = 2 * group + rank;
+        const uint32_t off = a.st_off[stream], entries = a.st_off[stream + 1] - off, len = a.st_len[stream];
+        bool ok = true;
+        for (uint32_t tile = 0; tile < n_tiles && ok; ++tile)
         {
-            s_fail = 1;
-            atomicOr(a.err, 1u);
+            const uint32_t slot = tile % kRowSlots;
+            uint32_t found[2];
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i)
+            {
+                const uint32_t p = tile * kStreamCols + (threadIdx.x - 32 * kRowWarp0) + 64 * i;
+                found[i] = kNoRow;
+                if (p < len)
+                {
+                    uint32_t lo = 0, hi = entries;  // the last entry that starts at or before p
+                    while (hi - lo > 1)
+                    {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if (a.st_start[off + mid] <= p) lo = mid;
+                        else hi = mid;
+                    }
+                    const uint4 info = a.st_info[off + lo];
+                    const uint32_t j = p - a.st_start[off + lo];
+                    if (j < info.z) found[i] = info.y + j;
+                }
+            }
+            ok = warp_wait(&row_empty[slot], ((tile / kRowSlots) & 1u) ^ 1u, a.poll_limit, &s_fail, lane);
+            if (!ok) break;
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) s_row[slot][(threadIdx.x - 32 * kRowWarp0) + 64 * i] = found[i];
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&row_full[slot]);
         }
+        if (!ok && lane == 0) fail();
     }
     else if (warp == kCopyWarp)
     {
         if (lane == 0)
         {
-            const uint8_t *src = a.w + static_cast<size_t>(n_tile) * chunks * kAChunk;
-            const uint32_t total = n_tiles * chunks;
+            const uint32_t full0 = tc::mapa(tc::smem_u32(full), 0);
+            const uint32_t total = n_tiles * per_tile;
+            const int y0 = static_cast<int>(n_tile * chunks * kTileN);  // past the weights: zeros
             uint32_t issued = 0;
             for (uint32_t u = 0, c = 0, s = 0, ph = 1; u < total; ++u)
             {
-                if (u >= stages && !wait_or_fail(&empty[s], ph, a.poll_limit, &s_fail))
+                if (!wait_or_fail(&empty[s], ph, a.poll_limit, &s_fail))
                 {
-                    s_fail = 1;
-                    atomicOr(a.err, 1u);
+                    fail();
                     break;
                 }
-                mbar_arrive_expect_tx(&full_w[s], kAChunk);
-                bulk_copy(base + s * kLayerStage, src + static_cast<size_t>(c) * kAChunk, kAChunk, &full_w[s]);
+                const bool two = c + 1 < chunks;
+                if (rank == 0) tc::mbar_expect_tx(&full[s], two ? 4 * kAChunk : 2 * kAChunk);
+                const uint32_t dst = base + s * kLayerStage;
+                tc::tma_load_2d_pair(dst, &a.w, 0, y0 + static_cast<int>(c * kTileN), full0 + s * 8u);
+                if (two)
+                    tc::tma_load_2d_pair(dst + kAChunk, &a.w, 0, y0 + static_cast<int>((c + 1) * kTileN), full0 + s * 8u);
                 issued = u + 1;
-                if (++c == chunks) c = 0;
-                if (++s == stages)
+                c = c + 2 < chunks ? c + 2 : 0;
+                if (++s == ring)
                 {
                     s = 0;
                     ph ^= 1u;
                 }
             }
-            // Copies still in flight after a failed wait land before the CTA leaves (bounded).
-            for (uint32_t u = issued > stages ? issued - stages : 0u; u < issued; ++u)
-                if (!tc::mbar_wait(&full_w[u % stages], (u / stages) & 1u, kWaitLimit)) atomicOr(a.err, 1u);
+            // After a failure: both CTAs' copies in flight land before either leaves (bounded; a chunk that
+            // not every role reached does not complete, so the limit is short).
+            if (s_fail && rank == 0)
+                for (uint32_t u = issued > ring ? issued - ring : 0u; u < issued; ++u)
+                    tc::mbar_wait(&full[u % ring], (u / ring) & 1u, kDrainWait);
         }
     }
-    else if (warp == kIssuerWarp && lane == 0)
+    else if (lane == 0 && rank == 0)
     {
-        constexpr uint32_t idesc = tc::idesc_bf16_f32(kTileN, kCols);
-        const uint64_t d_w = tc::smem_desc_sw128(base, 1024), d_s = tc::smem_desc_sw128(base + kAChunk, 1024);
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(2 * kTileN, kCols);
+        const uint64_t d_w = tc::smem_desc_sw128(base, 1024), d_s = tc::smem_desc_sw128(base + 2 * kAChunk, 1024);
         bool stop = false;
         uint32_t s = 0, ph = 0;
         for (uint32_t tile = 0; tile < n_tiles && !stop; ++tile)
@@ -826,10 +880,9 @@ __global__ void __launch_bounds__(kLayerThreads, 1) lif_layer_kernel(const __gri
                 break;
             }
             const uint32_t d_acc = tmem + acc * kCols;
-            for (uint32_t c = 0; c < chunks; ++c)
+            for (uint32_t c = 0; c < per_tile; ++c)
             {
-                if (!wait_or_fail(&full_w[s], ph, a.poll_limit, &s_fail) ||
-                    !wait_or_fail(&full_s[s], ph, a.poll_limit, &s_fail))
+                if (!wait_or_fail(&full[s], ph, a.poll_limit, &s_fail))
                 {
                     stop = true;
                     break;
@@ -838,41 +891,48 @@ __global__ void __launch_bounds__(kLayerThreads, 1) lif_layer_kernel(const __gri
                 // The stage's descriptors follow from the first one's by their start addresses (in
                 // 16-byte units).
                 const uint64_t dw = d_w + s * (kLayerStage >> 4), ds = d_s + s * (kLayerStage >> 4);
-                const uint32_t blocks = (a.kp - c * kChunk) >> 4;
-                tc::mma_bf16(d_acc, dw, ds, idesc, c ? 1u : 0u);
-                if (blocks >= 4)
+                const uint32_t blocks = (a.kp - c * 2 * kChunk) >> 4;
+                tc::mma_bf16_pair(d_acc, dw, ds, idesc, c ? 1u : 0u);
+                if (blocks >= 8)
                 {
 #pragma unroll
-                    for (uint32_t b = 1; b < 4; ++b) tc::mma_bf16(d_acc, dw + 2 * b, ds + 2 * b, idesc, 1u);
+                    for (uint32_t b = 1; b < 8; ++b)
+                        tc::mma_bf16_pair(d_acc, dw + (b >> 2) * (kAChunk >> 4) + 2 * (b & 3u),
+                                          ds + (b >> 2) * (kBChunk >> 4) + 2 * (b & 3u), idesc, 1u);
                 }
                 else
                 {
-                    for (uint32_t b = 1; b < blocks; ++b) tc::mma_bf16(d_acc, dw + 2 * b, ds + 2 * b, idesc, 1u);
+                    for (uint32_t b = 1; b < blocks; ++b)
+                        tc::mma_bf16_pair(d_acc, dw + (b >> 2) * (kAChunk >> 4) + 2 * (b & 3u),
+                                          ds + (b >> 2) * (kBChunk >> 4) + 2 * (b & 3u), idesc, 1u);
                 }
-                tc::commit(&empty[s]);
-                if (c + 1 == chunks) tc::commit(&acc_full[acc]);
-                if (++s == stages)
+                tc::commit_pair(&empty[s]);
+                if (c + 1 == per_tile) tc::commit_pair(&acc_full[acc]);
+                if (++s == ring)
                 {
                     s = 0;
                     ph ^= 1u;
                 }
             }
         }
-        if (stop)
-        {
-            s_fail = 1;
-            atomicOr(a.err, 1u);
-        }
+        if (stop) fail();
         // Every issued MMA completes (bounded wait) before the tensor memory is freed.
-        tc::commit(&drain);
-        if (!tc::mbar_wait(&drain, 0, kWaitLimit)) atomicOr(a.err, 1u);
+        tc::commit_pair(&drain);
+        if (!tc::mbar_wait(&drain, 0, kWaitLimit)) fail();
+    }
+    else if (lane == 0)
+    {
+        // Odd rank: the issuer's last arrivals reach this CTA before it leaves.
+        if (!tc::mbar_wait(&drain, 0, kWaitLimit)) fail();
     }
     __syncwarp();
     if (my_events) atomicAdd(&s_events, my_events);
     tc::fence_before_sync();
     __syncthreads();
     if (threadIdx.x == 0 && s_events) atomicAdd(a.events, s_events);
-    if (warp == kIssuerWarp) tc::tmem_dealloc(tmem, kTmemCols);
+    // Neither CTA leaves while the other's MMAs may read its shared memory or arrivals may reach it.
+    tc::cluster_sync();
+    if (warp == kIssuerWarp) tc::tmem_dealloc_pair(tmem, kTmemCols);
 }
 
 }  // namespace
@@ -919,13 +979,7 @@ struct BatchedPlan
 namespace
 {
 
-// A ring of 4 or 2 chunks has a group of expander warps for each; one of 3 has one group for all.
-auto layer_kernel(int stages)
-{
-    return stages == 4 ? lif_layer_kernel<4> : stages == 2 ? lif_layer_kernel<2> : lif_layer_kernel<1>;
-}
-
-size_t smem_bytes(int stages) { return std::max(stages * size_t(kLayerStage) + 1024, kMinDynSmem); }
+size_t smem_bytes(int stages) { return std::max(ring_stages(stages) * size_t(kLayerStage) + 1024, kMinDynSmem); }
 
 // Captures one run with a ring of `stages` chunks into p.exec.
 cudaError_t capture(BatchedPlan &p, int stages)
@@ -940,7 +994,7 @@ cudaError_t capture(BatchedPlan &p, int stages)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const size_t smem = smem_bytes(stages);
     cudaError_t err =
-        cudaFuncSetAttribute(layer_kernel(stages), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cudaFuncSetAttribute(lif_layer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return err;
     cudaStream_t s = p.stream;
     err = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
@@ -959,14 +1013,14 @@ cudaError_t capture(BatchedPlan &p, int stages)
     for (auto &seg : p.segs)
     {
         const unsigned long long warps = static_cast<unsigned long long>(seg.draw.batch) * seg.draw.blocks * seg.draw.wp;
-        input_rows_kernel<<<static_cast<unsigned>(std::min<unsigned long long>((warps + 7) / 8, 8ull * sms)), 256, 0, s>>>(
+        input_rows_kernel<<<static_cast<unsigned>(std::min<unsigned long long>((warps + 7) / 8, 1ull << 20)), 256, 0, s>>>(
             seg.draw);
         note(cudaGetLastError());
         for (int l = 0; l < p.n_layers; ++l)
         {
             LayerArgs a = seg.layer[l];
-            a.stages = static_cast<uint32_t>(stages);
-            note(launch_pdl(layer_kernel(stages), dim3(seg.grid[l]), dim3(kLayerThreads), smem, s, a));
+            a.ring = static_cast<uint32_t>(ring_stages(stages));
+            note(launch_pdl(lif_layer_kernel, dim3(seg.grid[l]), dim3(kLayerThreads), smem, s, a));
         }
     }
     note(cudaMemcpyAsync(p.totals_host, p.totals, 16, cudaMemcpyDeviceToHost, s));
@@ -1025,8 +1079,8 @@ int batched_plan_create(
         *why = "could not create the plan's stream";
         return -3;
     }
-    // Failure test (KNP_GB300_BATCHED_STALL=1): the MMA issuer waits for one expander warp more per chunk than
-    // exists, so its first operand wait runs out (after a short poll limit) and the run ends with the
+    // Failure test (KNP_GB300_BATCHED_STALL=1): the MMA issuer waits for one expander group more per chunk
+    // than exists, so its first operand wait runs out (after a short poll limit) and the run ends with the
     // error word set instead of results.
     const char *stall_env = std::getenv("KNP_GB300_BATCHED_STALL");
     const uint32_t stall = (stall_env && stall_env[0] == '1') ? 1u : 0u;
@@ -1169,7 +1223,8 @@ int batched_plan_create(
         uint32_t groups = 0;
         for (int l = 0; l < n_layers && ok; ++l)
         {
-            const uint32_t want = std::max(1u, std::min((batch + 1) / 2, static_cast<uint32_t>(sms) / tiles[l + 1]));
+            const uint32_t n_pairs = (tiles[l + 1] + 1) / 2;
+            const uint32_t want = std::max(1u, std::min((batch + 1) / 2, static_cast<uint32_t>(sms) / 2 / n_pairs));
             if (want != groups)  // layers of equal width share their streams
             {
                 groups = want;
@@ -1217,7 +1272,7 @@ int batched_plan_create(
             a.n_groups = groups;
             a.t0 = t0;
             a.t1 = t1;
-            seg.grid[l] = tiles[l + 1] * groups;
+            seg.grid[l] = 2 * n_pairs * groups;
         }
     }
     uint32_t *bits[kMaxLayers] = {}, *state[kMaxLayers] = {}, *carry[kMaxLayers] = {};
@@ -1258,7 +1313,11 @@ int batched_plan_create(
         {
             LayerArgs &a = seg.layer[l];
             const bool last = l + 1 == n_layers;
-            a.w = p.pack.out[l];
+            if (!sw128_map(&a.w, p.pack.out[l], static_cast<int>(tiles[l + 1] * p.pack.chunks[l] * kTileN), kChunk))
+            {
+                *why = "could not describe the packed weights to the TMA unit";
+                return -3;
+            }
             a.bits_in = bits[l];
             a.wp_in = wp[l];
             a.bits_out = last ? nullptr : bits[l + 1];

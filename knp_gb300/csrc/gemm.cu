@@ -216,32 +216,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pipe_kernel(
     if (warp == 0) tc::tmem_dealloc(tmem, kBN);
 }
 
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *mbar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(mbar)), "r"(bytes)
-                 : "memory");
-}
-
-// TMA load of the 2-D box at (x, y) of `map` into shared memory at `dst`, completing its bytes on the
-// mbarrier's transaction count.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint64_t *mbar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(tc::smem_u32(mbar))
-        : "memory");
-}
-
-// As tma_load_2d for a CTA pair: the bytes land in this CTA's shared memory and are counted by the
-// mbarrier at `mbar`, a shared::cluster address that may be the other CTA's.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t mbar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
-        : "memory");
-}
-
 constexpr int kTmaThreads = 128;
 
 constexpr int kTmaStages = 6;
@@ -293,9 +267,9 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
                 break;
             }
             const uint32_t sa = base + s * kStageBytes;
-            mbar_expect_tx(&full[s], kStageBytes);
-            tma_load_2d(sa, &ta, c * kBK, m0, &full[s]);
-            tma_load_2d(sa + kTileBytes, &tb, c * kBK, n0, &full[s]);
+            tc::mbar_expect_tx(&full[s], kStageBytes);
+            tc::tma_load_2d(sa, &ta, c * kBK, m0, &full[s]);
+            tc::tma_load_2d(sa + kTileBytes, &tb, c * kBK, n0, &full[s]);
             issued = i + 1;
         }
         // Copies still in flight after a failed wait land before the CTA leaves (bounded).
@@ -459,9 +433,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                         break;
                     }
                     const uint32_t sa = base + s * kPairStage;
-                    if (rank == 0) mbar_expect_tx(&full[s], 2 * kPairStage);
-                    tma_load_2d_pair(sa, &ta, c * kBK, m0 + 128 * static_cast<int>(rank), full0 + s * 8u);
-                    tma_load_2d_pair(sa + kTileBytes, &tb, c * kBK, n0 + 128 * static_cast<int>(rank), full0 + s * 8u);
+                    if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * kPairStage);
+                    tc::tma_load_2d_pair(sa, &ta, c * kBK, m0 + 128 * static_cast<int>(rank), full0 + s * 8u);
+                    tc::tma_load_2d_pair(sa + kTileBytes, &tb, c * kBK, n0 + 128 * static_cast<int>(rank), full0 + s * 8u);
                     ++issued;
                     if (++s == kPairStages)
                     {
@@ -616,21 +590,6 @@ EncodeTiled encode_tiled()
     return fn;
 }
 
-// The (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple of 8), loaded in 64 x 128
-// boxes with the 128-byte swizzle.
-bool sw128_map(CUtensorMap *map, const void *ptr, int rows, int K)
-{
-    const EncodeTiled fn = encode_tiled();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-    const cuuint32_t box[2] = {kBK, kBM};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // The kernel's dynamic shared memory limit raised once per (kernel, device): a per-device setting.
 template <class Kernel>
 cudaError_t smem_limit_once(Kernel kernel, int bytes, int dev)
@@ -674,6 +633,21 @@ cudaMemPool_t split_pool(int dev)
 
 namespace knp_gb300
 {
+// The (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple of 8), loaded in 64 x 128
+// boxes with the 128-byte swizzle.
+bool sw128_map(void *map, const void *ptr, int rows, int K)
+{
+    const EncodeTiled fn = encode_tiled();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
+    const cuuint32_t box[2] = {64, 128};
+    const cuuint32_t estr[2] = {1, 1};
+    return fn(static_cast<CUtensorMap *>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, int K, unsigned int *d_err, cudaStream_t s);
 
 // D = A * B^T (see knp_gb300_bf16_gemm_tn). The pipelined kernel needs 16-byte aligned rows (K a

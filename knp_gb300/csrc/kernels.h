@@ -432,6 +432,10 @@ void launch_apply_impacts(
     const RingView &ring, const uint32_t *post, const float *value, const uint8_t *type, int forcing, uint32_t n,
     uint32_t seq_base, Control *ctl, cudaStream_t s);
 
+// Fills the CUtensorMap at `map` with the (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple
+// of 8, 16-byte aligned), loaded in boxes of 64 x 128 with the 128-byte swizzle (gemm.cu).
+bool sw128_map(void *map, const void *ptr, int rows, int K);
+
 // Network construction on the device.
 cudaError_t build_csr(
     uint64_t n_syn, uint32_t n_rows, const uint32_t *d_row_key, uint32_t *d_perm_out, long long *d_row_ptr,

@@ -6,6 +6,8 @@
 
 #include <cstdint>
 
+#include <cuda.h>
+
 namespace knp_gb300
 {
 namespace tc
@@ -330,10 +332,38 @@ __device__ __forceinline__ void commit_pair(uint64_t *mbar)
         : "memory");
 }
 
-// One arrival (release, cluster scope) on an mbarrier of a CTA of this cluster (address from mapa).
+// One arrival (release) on an mbarrier of a CTA of this cluster (address from mapa). What it orders is
+// tensor-core work and shared memory of this CTA; cluster scope would also wait for the thread's global
+// stores (about 2000 cycles in a kernel that writes results).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_mbar)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_mbar) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_mbar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *mbar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
+                 : "memory");
+}
+
+// TMA load of the 2-D box at (x, y) of `map` into shared memory at `dst`, completing its bytes on the
+// mbarrier's transaction count.
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint64_t *mbar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(mbar))
+        : "memory");
+}
+
+// As tma_load_2d for a CTA pair: the bytes land in this CTA's shared memory and are counted by the
+// mbarrier at `mbar`, a shared::cluster address that may be the other CTA's.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t mbar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
+        : "memory");
 }
 
 }  // namespace tc
