@@ -93,14 +93,14 @@ def bf16_terms(x: torch.Tensor, n: int):
     return terms
 
 
-def gemm_terms(a_terms, b_terms) -> torch.Tensor:
-    """(sum a_i) @ (sum b_j)^T as one GEMM: every pair (a_i, b_j) concatenated along K, each part padded
-    to 16-byte rows."""
+def gemm_terms(a_terms, b_terms, part: int = 8) -> torch.Tensor:
+    """(sum a_i) @ (sum b_j)^T as one GEMM: every pair (a_i, b_j) concatenated along K, each padded to a
+    multiple of ``part`` (8: 16-byte rows)."""
     pairs = [(a, b) for a in a_terms for b in b_terms]
     if len(pairs) == 1:
         return gemm_tn(*pairs[0])
-    return gemm_tn(torch.cat([_pad_k(a.contiguous()) for a, _ in pairs], 1),
-                   torch.cat([_pad_k(b.contiguous()) for _, b in pairs], 1))
+    return gemm_tn(torch.cat([_pad_k(a.contiguous(), part) for a, _ in pairs], 1),
+                   torch.cat([_pad_k(b.contiguous(), part) for _, b in pairs], 1))
 
 
 def _round8(n: int) -> int:
@@ -120,9 +120,10 @@ def operand(x: torch.Tensor, mode: int, transpose: bool, width: int) -> torch.Te
     return out
 
 
-# The hard-threshold path builds its GEMM operands with knp_gb300_bf16_operand (one pass per
-# operand: cast, hi/lo split, transpose, concatenation along K and padding); the relaxed path (three
-# BF16 terms of continuous values) keeps the torch composition of bf16_terms / gemm_terms.
+# The hard-threshold path runs each layer's product and recurrence in one kernel
+# (knp_gb300_lif_layer_forward / _backward) from BF16 copies of the spikes and the weights, and the two
+# gradient products straight from those and from the gradient's BF16 halves. The relaxed path (three BF16
+# terms of continuous values) keeps the torch composition of bf16_terms / gemm_terms and the scan kernels.
 FUSED_OPERANDS = True
 
 
@@ -135,21 +136,23 @@ class LIFLayerFn(torch.autograd.Function):
         n_out = w_master.shape[1]
         s_in = s_in.contiguous()
         fused = FUSED_OPERANDS and not relaxed
+        dev = s_in.device
+        ckpt = torch.empty(((T + checkpoint - 1) // checkpoint, B, n_out), device=dev, dtype=torch.float32)
+        S = torch.empty((T, B, n_out), device=dev, dtype=torch.float32)
         if fused:
-            s2d = s_in.reshape(T * B, n_in)
-            a = operand(s2d, 0, False, _round8(n_in))            # [TB, n_in]: 0/1 spikes, exact in BF16
-            wt = operand(w_master, 0, True, _round8(n_in))       # [n_out, n_in]: W^T
-            I = gemm_tn(a, wt).reshape(T, B, n_out)
-            saved = (w_master, s2d, a, wt)
+            a = operand(s_in.reshape(T * B, n_in), 0, False, _round8(n_in))  # 0/1 spikes, exact in BF16
+            wb = operand(w_master, 0, False, _round8(n_out))                 # [n_in, w2]
+            _capi.check(_capi.lib().knp_gb300_lif_layer_forward(
+                _p(a), _p(wb), _p(S), _p(ckpt), T, B, n_in, a.shape[1], n_out, wb.shape[1], beta, theta, checkpoint,
+                _p(_err_word(dev)), _stream()))
+            saved = (a, wb)
         else:
             wb = w_master.to(torch.bfloat16)  # [n_in, n_out]
             s_terms = bf16_terms(s_in.reshape(T * B, n_in), 3 if relaxed else 1)  # 0/1 spikes are exact
             I = gemm_terms(s_terms, [wb.t().contiguous()]).reshape(T, B, n_out).contiguous()
             saved = (wb, *s_terms)
-        S = torch.empty_like(I)
-        ckpt = torch.empty(((T + checkpoint - 1) // checkpoint, B, n_out), device=I.device, dtype=torch.float32)
-        _capi.check(_capi.lib().knp_gb300_lif_scan_forward(
-            _p(I), _p(S), _p(ckpt), T, B * n_out, beta, theta, checkpoint, int(relaxed), k, _stream()))
+            _capi.check(_capi.lib().knp_gb300_lif_scan_forward(
+                _p(I), _p(S), _p(ckpt), T, B * n_out, beta, theta, checkpoint, int(relaxed), k, _stream()))
         ctx.save_for_backward(ckpt, *saved)
         ctx.cfg = (T, B, beta, theta, checkpoint, relaxed, k, fused, n_in, n_out)
         return S
@@ -158,33 +161,35 @@ class LIFLayerFn(torch.autograd.Function):
     def backward(ctx, dS):
         ckpt, *saved = ctx.saved_tensors
         T, B, beta, theta, checkpoint, relaxed, k, fused, n_in, n_out = ctx.cfg
-        if fused:
-            w_master, s2d, a, wt = saved
-            I = gemm_tn(a, wt).reshape(T, B, n_out)  # recomputed, not stored
-        else:
-            wb, *s_terms = saved
-            I = gemm_terms(s_terms, [wb.t().contiguous()]).reshape(T, B, n_out).contiguous()
         dS = dS.contiguous()
+        ds_in = None
+        if fused:
+            a, wb = saved
+            k8, w2 = a.shape[1], wb.shape[1]
+            dev, err, st, lib = a.device, _p(_err_word(a.device)), _stream(), _capi.lib()
+            # The product is recomputed, not stored; dI comes out as rows of two BF16 halves [hi | lo].
+            dI2 = torch.empty((T * B, 2 * w2), device=dev, dtype=torch.bfloat16)
+            _capi.check(lib.knp_gb300_lif_layer_backward(_p(a), _p(wb), _p(ckpt), _p(dS), _p(dI2), T, B, n_in, k8, n_out,
+                                                         w2, beta, theta, checkpoint, k, err, st))
+            dW = torch.empty((n_in, n_out), device=dev, dtype=torch.float32)
+            _capi.check(lib.knp_gb300_lif_layer_dw(_p(a), _p(dI2), _p(dW), T * B, n_in, k8, n_out, w2, err, st))
+            if ctx.needs_input_grad[0]:
+                ds_in = torch.empty((T, B, n_in), device=dev, dtype=torch.float32)
+                _capi.check(lib.knp_gb300_lif_layer_ds(_p(dI2), _p(wb), _p(ds_in), T * B, n_in, n_out, w2, err, st))
+            return ds_in, dW, None, None, None, None, None
+        wb, *s_terms = saved
+        I = gemm_terms(s_terms, [wb.t().contiguous()]).reshape(T, B, n_out).contiguous()
         dI = torch.empty_like(I)
         _capi.check(_capi.lib().knp_gb300_lif_scan_backward(
             _p(I), _p(ckpt), _p(dS), _p(dI), T, B * n_out, beta, theta, checkpoint, int(relaxed), k, _stream()))
-        ds_in = None
-        if fused:
-            dI2 = dI.reshape(T * B, n_out)
-            tb = _round8(T * B)
-            # dW[n_in, n_out] = S^T (hi + lo): K = 2 T B, [S^T | S^T] against [hi^T | lo^T].
-            dW = gemm_tn(operand(s2d, 1, True, tb), operand(dI2, 2, True, tb))
-            if ctx.needs_input_grad[0]:
-                # ds_in[TB, n_in] = (hi + lo) W^T: K = 2 n_out, [hi | lo] against [W | W].
-                w2 = _round8(n_out)
-                ds_in = gemm_tn(operand(dI2, 2, False, w2), operand(w_master, 1, False, w2)).reshape(T, B, n_in)
-            return ds_in, dW, None, None, None, None, None
         d_terms = bf16_terms(dI.reshape(T * B, n_out), 3 if relaxed else 2)
-        # dW[n_in, n_out] = S^T dI: K = T B per (S term, dI term) pair.
-        dW = gemm_terms([s.t() for s in s_terms], [d.t() for d in d_terms])
+        # dW[n_in, n_out] = S^T dI: K = T B per (S term, dI term) pair; the two-term form pads its parts to the
+        # fused products' chunks of 64, so that both sum in the same order.
+        part = 8 if relaxed else 64
+        dW = gemm_terms([s.t() for s in s_terms], [d.t() for d in d_terms], part)
         if ctx.needs_input_grad[0]:
             # ds_in[TB, n_in] = dI W^T, W as [n_in, n_out]: K = n_out per dI term.
-            ds_in = gemm_terms(d_terms, [wb]).reshape(T, B, n_in)
+            ds_in = gemm_terms(d_terms, [wb], part).reshape(T, B, n_in)
         return ds_in, dW, None, None, None, None, None
 
 

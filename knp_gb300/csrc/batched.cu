@@ -1313,7 +1313,8 @@ int batched_plan_create(
         {
             LayerArgs &a = seg.layer[l];
             const bool last = l + 1 == n_layers;
-            if (!sw128_map(&a.w, p.pack.out[l], static_cast<int>(tiles[l + 1] * p.pack.chunks[l] * kTileN), kChunk))
+            if (!sw128_map(&a.w, p.pack.out[l], static_cast<int>(tiles[l + 1] * p.pack.chunks[l] * kTileN), kChunk,
+                           kTileN))
             {
                 *why = "could not describe the packed weights to the TMA unit";
                 return -3;

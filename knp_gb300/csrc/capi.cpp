@@ -28,6 +28,14 @@ int bernoulli_schedule_noalloc(
 
 namespace knp_gb300
 {
+int lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N, int w2,
+                      float beta, float theta, int seg, unsigned int *err, cudaStream_t s);
+int lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const float *dS, void *dI2, int T, int B, int K,
+                       int k8, int N, int w2, float beta, float theta, int seg, float k, unsigned int *err, cudaStream_t s);
+int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, int n_out, int w2, unsigned int *d_err,
+                cudaStream_t s);
+int lif_dw_gemm(const void *S, const void *dI2, float *dW, int rows, int n_in, int n_in8, int n_out, int w2,
+                unsigned int *d_err, cudaStream_t s);
 int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, unsigned int *d_err, cudaStream_t s);
 int batched_lif_run(
     int n_layers, const uint32_t *sizes, const void *const *weights, const float *leak, const float *threshold,
@@ -464,6 +472,52 @@ int knp_gb300_measure_add_rate(uint64_t n_floats, uint64_t n_adds, double *adds_
     if (knp_gb300::measure_add_rate(n_floats, n_adds, adds_per_s, &why) == 0) return KNP_GB300_OK;
     g_error = why;
     return KNP_GB300_E_CUDA;
+}
+
+// Widths of the layer entry points' BF16 rows: whole 16-byte units that hold the copied extent.
+static bool layer_widths(int K, int k8, int N, int w2) { return K >= 1 && N >= 1 && k8 >= K && w2 >= N && k8 % 8 == 0 && w2 % 8 == 0; }
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+static int layer_status(int rc)
+{
+    if (rc) g_error = rc == -1 ? "bad LIF layer arguments (T, B, N, K >= 1, 1 <= checkpoint interval <= 16)" : "kernel launch failed";
+    return rc == 0 ? KNP_GB300_OK : (rc == -1 ? KNP_GB300_E_INVALID : KNP_GB300_E_CUDA);
+}
+
+int knp_gb300_lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N,
+                                int w2, float beta, float theta, int seg, unsigned int *d_err, void *stream)
+{
+    if (!S_in || !W || !S || !ckpt || !d_err || !layer_widths(K, k8, N, w2) || !aligned16(S_in) || !aligned16(W))
+        return layer_status(-1);
+    return layer_status(knp_gb300::lif_layer_forward(S_in, W, S, ckpt, T, B, K, k8, N, w2, beta, theta, seg, d_err,
+                                                     static_cast<cudaStream_t>(stream)));
+}
+
+int knp_gb300_lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const float *dS, void *dI2, int T,
+                                 int B, int K, int k8, int N, int w2, float beta, float theta, int seg, float k,
+                                 unsigned int *d_err, void *stream)
+{
+    if (!S_in || !W || !ckpt || !dS || !dI2 || !d_err || !layer_widths(K, k8, N, w2) || !aligned16(S_in) || !aligned16(W))
+        return layer_status(-1);
+    return layer_status(knp_gb300::lif_layer_backward(S_in, W, ckpt, dS, dI2, T, B, K, k8, N, w2, beta, theta, seg, k, d_err,
+                                                      static_cast<cudaStream_t>(stream)));
+}
+
+int knp_gb300_lif_layer_ds(const void *dI2, const void *W, float *ds, int rows, int K, int N, int w2, unsigned int *d_err,
+                           void *stream)
+{
+    if (!dI2 || !W || !ds || !d_err || rows < 1 || !layer_widths(K, (K + 7) / 8 * 8, N, w2) || !aligned16(dI2) || !aligned16(W))
+        return layer_status(-1);
+    return layer_status(knp_gb300::lif_ds_gemm(dI2, W, ds, rows, K, N, w2, d_err, static_cast<cudaStream_t>(stream)));
+}
+
+int knp_gb300_lif_layer_dw(const void *S_in, const void *dI2, float *dW, int rows, int K, int k8, int N, int w2,
+                           unsigned int *d_err, void *stream)
+{
+    if (!S_in || !dI2 || !dW || !d_err || rows < 1 || !layer_widths(K, k8, N, w2) || !aligned16(S_in) || !aligned16(dI2))
+        return layer_status(-1);
+    return layer_status(
+        knp_gb300::lif_dw_gemm(S_in, dI2, dW, rows, K, k8, N, w2, d_err, static_cast<cudaStream_t>(stream)));
 }
 
 int knp_gb300_bf16_gemm_tn(

@@ -216,6 +216,54 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pipe_kernel(
     if (warp == 0) tc::tmem_dealloc(tmem, kBN);
 }
 
+// How a GEMM's K is read: nk chunks of 64, in halves of nkh chunks each (one half: nkh = nk); half h of a
+// K-major operand starts h * step elements further along K, of an MN-major one h * step elements further
+// along M or N (an operand that both halves share has step 0).
+struct KPlan
+{
+    int nk, nkh, a_step, b_step;
+};
+
+// Stages chunk c of the 128 rows from r0 of an operand: K-major (row-major [rows][K]) as one 64 x 128 box,
+// MN-major (row-major [K][rows]) as two 64 x 64 boxes, one per 64 rows. Rows and K past the matrix are zeros.
+template <bool kMn, bool kPair>
+__device__ __forceinline__ void load_operand(uint32_t dst, const CUtensorMap *map, int c, int nkh, int step, int r0,
+                                             uint32_t pair_mbar, uint64_t *mbar)
+{
+    const int half = c >= nkh ? 1 : 0, k = (c - half * nkh) * kBK;
+    if (kMn)
+    {
+        const int x = r0 + half * step;
+        if (kPair)
+        {
+            tc::tma_load_2d_pair(dst, map, x, k, pair_mbar);
+            tc::tma_load_2d_pair(dst + kTileBytes / 2, map, x + 64, k, pair_mbar);
+        }
+        else
+        {
+            tc::tma_load_2d(dst, map, x, k, mbar);
+            tc::tma_load_2d(dst + kTileBytes / 2, map, x + 64, k, mbar);
+        }
+    }
+    else if (kPair)
+    {
+        tc::tma_load_2d_pair(dst, map, k + half * step, r0, pair_mbar);
+    }
+    else
+    {
+        tc::tma_load_2d(dst, map, k + half * step, r0, mbar);
+    }
+}
+
+// Descriptor of a staged operand at shared address `a`, and the step of its start address per 16 of K.
+template <bool kMn>
+__device__ __forceinline__ uint64_t operand_desc(uint32_t a)
+{
+    return kMn ? tc::smem_desc_sw128_mn(a, kTileBytes / 2) : tc::smem_desc_sw128(a, 1024);
+}
+template <bool kMn>
+constexpr uint32_t kDescStep = kMn ? 2048 >> 4 : 32 >> 4;
+
 constexpr int kTmaThreads = 128;
 
 constexpr int kTmaStages = 6;
@@ -224,9 +272,10 @@ constexpr uint32_t kTmaSmem = kTmaStages * kStageBytes + 1024;  // + alignment s
 // One 128 x 128 tile of D (or of split blockIdx.z's partial, into `out` with row stride N) over
 // chunks [blockIdx.z * cps, min(nk, (blockIdx.z + 1) * cps)). Warp 0 lane 0 issues the TMA copies,
 // warp 1 lane 0 the MMAs; all four warps read the accumulator back.
+template <bool kMn>
 __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *__restrict__ out, int M,
-    int N, int K, int cps, size_t split_stride, unsigned int *err)
+    int N, KPlan kp, int cps, size_t split_stride, unsigned int *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[kTmaStages], empty[kTmaStages], acc_full, drain;
@@ -234,8 +283,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     __shared__ int s_fail;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
-    const int nk = (K + kBK - 1) / kBK;
-    const int c0 = blockIdx.z * cps, c1 = min(nk, c0 + cps);
+    const int c0 = blockIdx.z * cps, c1 = min(kp.nk, c0 + cps);
     float *dst = out + blockIdx.z * split_stride;
     if (warp == 0) tc::tmem_alloc(&tmem_slot, kBN);
     if (threadIdx.x == 0)
@@ -268,8 +316,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
             }
             const uint32_t sa = base + s * kStageBytes;
             tc::mbar_expect_tx(&full[s], kStageBytes);
-            tc::tma_load_2d(sa, &ta, c * kBK, m0, &full[s]);
-            tc::tma_load_2d(sa + kTileBytes, &tb, c * kBK, n0, &full[s]);
+            load_operand<kMn, false>(sa, &ta, c, kp.nkh, kp.a_step, m0, 0u, &full[s]);
+            load_operand<kMn, false>(sa + kTileBytes, &tb, c, kp.nkh, kp.b_step, n0, 0u, &full[s]);
             issued = i + 1;
         }
         // Copies still in flight after a failed wait land before the CTA leaves (bounded).
@@ -278,7 +326,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     }
     else if (warp == 1 && lane == 0)
     {
-        constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kBN);
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kBN) | (kMn ? tc::kIdescAMn | tc::kIdescBMn : 0u);
         for (int c = c0; c < c1; ++c)
         {
             const int i = c - c0, s = i % kTmaStages;
@@ -291,7 +339,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
             const uint32_t sa = base + s * kStageBytes, sb = sa + kTileBytes;
 #pragma unroll
             for (int j = 0; j < kBK / 16; ++j)
-                tc::mma_bf16(tmem, tc::smem_desc_sw128(sa + j * 32, 1024), tc::smem_desc_sw128(sb + j * 32, 1024),
+                tc::mma_bf16(tmem, operand_desc<kMn>(sa) + j * kDescStep<kMn>, operand_desc<kMn>(sb) + j * kDescStep<kMn>,
                              idesc, (i > 0 || j > 0) ? 1u : 0u);
             tc::commit(&empty[s]);
         }
@@ -359,9 +407,10 @@ constexpr uint32_t kPairSmem = kPairStages * kPairStage + 1024;
 constexpr uint32_t kDrainWait = 1u << 14;  // polls, about 0.06 s
 constexpr int kPairThreads = 192;  // warps 0-3 read back, warp 4 loads, warp 5 issues (even rank)
 
+template <bool kMn>
 __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gemm_pair_kernel(
     const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *__restrict__ D, int M, int N,
-    int K, unsigned int *err)
+    KPlan kp, unsigned int *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     // Of the even CTA alone: full (both CTAs' halves of a chunk have landed) and acc_empty (4 read-back
@@ -401,7 +450,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
     const uint32_t base = (tc::smem_u32(smem) + 1023u) & ~1023u;
-    const int nk = (K + kBK - 1) / kBK;
+    const int nk = kp.nk;
     const int tiles_m = (M + kPairM - 1) / kPairM, tiles_n = (N + kPairN - 1) / kPairN;
     const int tiles = tiles_m * tiles_n, pairs = gridDim.x / 2, pair = blockIdx.x / 2;
     auto place = [&](int t, int &m0, int &n0)
@@ -434,8 +483,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                     }
                     const uint32_t sa = base + s * kPairStage;
                     if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * kPairStage);
-                    tc::tma_load_2d_pair(sa, &ta, c * kBK, m0 + 128 * static_cast<int>(rank), full0 + s * 8u);
-                    tc::tma_load_2d_pair(sa + kTileBytes, &tb, c * kBK, n0 + 128 * static_cast<int>(rank), full0 + s * 8u);
+                    load_operand<kMn, true>(sa, &ta, c, kp.nkh, kp.a_step, m0 + 128 * static_cast<int>(rank),
+                                            full0 + s * 8u, nullptr);
+                    load_operand<kMn, true>(sa + kTileBytes, &tb, c, kp.nkh, kp.b_step,
+                                            n0 + 128 * static_cast<int>(rank), full0 + s * 8u, nullptr);
                     ++issued;
                     if (++s == kPairStages)
                     {
@@ -455,8 +506,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
     {
         if (lane == 0 && rank == 0)
         {
-            constexpr uint32_t idesc = tc::idesc_bf16_f32(kPairM, kPairN);
-            const uint64_t da = tc::smem_desc_sw128(base, 1024), db = tc::smem_desc_sw128(base + kTileBytes, 1024);
+            constexpr uint32_t idesc =
+                tc::idesc_bf16_f32(kPairM, kPairN) | (kMn ? tc::kIdescAMn | tc::kIdescBMn : 0u);
+            const uint64_t da = operand_desc<kMn>(base), db = operand_desc<kMn>(base + kTileBytes);
             int s = 0, n = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -479,8 +531,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                     const uint64_t off = static_cast<uint64_t>(s) * (kPairStage >> 4);
 #pragma unroll
                     for (int j = 0; j < kBK / 16; ++j)
-                        tc::mma_bf16_pair(tmem + a * kPairN, da + off + 2 * j, db + off + 2 * j, idesc,
-                                          (c > 0 || j > 0) ? 1u : 0u);
+                        tc::mma_bf16_pair(tmem + a * kPairN, da + off + j * kDescStep<kMn>, db + off + j * kDescStep<kMn>,
+                                          idesc, (c > 0 || j > 0) ? 1u : 0u);
                     tc::commit_pair(&empty[s]);
                     if (++s == kPairStages)
                     {
@@ -633,46 +685,67 @@ cudaMemPool_t split_pool(int dev)
 
 namespace knp_gb300
 {
-// The (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple of 8), loaded in 64 x 128
-// boxes with the 128-byte swizzle.
-bool sw128_map(void *map, const void *ptr, int rows, int K)
+namespace
+{
+
+// A BF16 tensor of `rank` dimensions (K contiguous), loaded in boxes of 64 x ... with the 128-byte swizzle.
+bool sw128_map_nd(void *map, const void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                  const cuuint32_t *box)
 {
     const EncodeTiled fn = encode_tiled();
     if (!fn) return false;
+    const cuuint32_t estr[3] = {1, 1, 1};
+    auto encode = [&]
+    {
+        return fn(static_cast<CUtensorMap *>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void *>(ptr), dims,
+                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT)
+    {
+        // A thread whose first CUDA call this is (an autograd thread, say) has no current context yet.
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+    }
+    return r == CUDA_SUCCESS;
+}
+
+}  // namespace
+
+// The (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple of 8), in 64 x box_rows boxes.
+bool sw128_map(void *map, const void *ptr, int rows, int K, int box_rows)
+{
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-    const cuuint32_t box[2] = {64, 128};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(static_cast<CUtensorMap *>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
+    return sw128_map_nd(map, ptr, 2, dims, strides, box);
+}
+
+// The (K, t, b) view of the rows t * batch + b of such a matrix, in 64 x box_t x box_b boxes.
+bool sw128_map_3d(void *map, const void *ptr, int T, int batch, int K, int box_t, int box_b)
+{
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(batch)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(batch) * K * 2, static_cast<cuuint64_t>(K) * 2};
+    const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_t), static_cast<cuuint32_t>(box_b)};
+    return sw128_map_nd(map, ptr, 3, dims, strides, box);
 }
 
 int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, int K, unsigned int *d_err, cudaStream_t s);
 
-// D = A * B^T (see knp_gb300_bf16_gemm_tn). The pipelined kernel needs 16-byte aligned rows (K a
-// multiple of 8, 16-byte aligned A and B); other shapes take the single-stage kernel.
-int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, unsigned int *d_err, cudaStream_t s)
+namespace
 {
-    if (M < 1 || N < 1 || K < 1 || !A || !B || !D || !d_err) return -1;
-    const bool aligned = K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
-    if (!aligned) return bf16_gemm_tn_simple(A, B, D, M, N, K, d_err, s);
-    CUtensorMap ta, tb;
+
+// D[M x N] from operands that are both K-major or (kMn) both MN-major.
+template <bool kMn>
+int launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, float *D, int M, int N, KPlan kp, unsigned int *d_err,
+                cudaStream_t s)
+{
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int tiles_m = (M + kBM - 1) / kBM;
-    const int nk = (K + kBK - 1) / kBK;
-    const int tiles_n = (N + kBN - 1) / kBN, tiles = tiles_m * tiles_n;
+    const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + kBN - 1) / kBN, tiles = tiles_m * tiles_n;
     const int pair_tiles = ((M + kPairM - 1) / kPairM) * ((N + kPairN - 1) / kPairN);
-    if (!sw128_map(&ta, A, M, K) || !sw128_map(&tb, B, N, K))
-    {
-        if (smem_limit_once(gemm_pipe_kernel, static_cast<int>(kStages * kStageBytes), dev) != cudaSuccess) return -3;
-        dim3 grid(tiles_m, tiles_n);
-        gemm_pipe_kernel<<<grid, kThreads, kStages * kStageBytes, s>>>(
-            static_cast<const __nv_bfloat16 *>(A), static_cast<const __nv_bfloat16 *>(B), D, M, N, K, d_err);
-        return cudaGetLastError() == cudaSuccess ? 0 : -3;
-    }
     // A 128 x 128 tile on one CTA (bound by shared memory) and a 256 x 256 tile on a pair (bound by the
     // tensor core) take the same 512 cycles per 64-deep chunk, so the form with fewer waves is the faster
     // (2500^3: 3 waves 86 us, 2 waves 74 us; 2048 x 2048 x 32768: 2 waves 325 us, 1 wave 169 us); at the
@@ -680,16 +753,16 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
     const int waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
     if (pair_waves < waves)
     {
-        if (smem_limit_once(gemm_pair_kernel, static_cast<int>(kPairSmem), dev) != cudaSuccess) return -3;
-        gemm_pair_kernel<<<2 * std::min(pair_tiles, sms / 2), kPairThreads, kPairSmem, s>>>(ta, tb, D, M, N, K, d_err);
+        if (smem_limit_once(gemm_pair_kernel<kMn>, static_cast<int>(kPairSmem), dev) != cudaSuccess) return -3;
+        gemm_pair_kernel<kMn><<<2 * std::min(pair_tiles, sms / 2), kPairThreads, kPairSmem, s>>>(ta, tb, D, M, N, kp, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
-    if (smem_limit_once(gemm_tma_kernel, static_cast<int>(kTmaSmem), dev) != cudaSuccess) return -3;
+    if (smem_limit_once(gemm_tma_kernel<kMn>, static_cast<int>(kTmaSmem), dev) != cudaSuccess) return -3;
     // Split K when the tiles leave most SMs idle and each split keeps at least 4 chunks.
     int splits = 1;
-    if (tiles * 2 <= sms) splits = std::max(1, std::min({16, nk / 4, sms / tiles}));
-    const int cps = (nk + splits - 1) / splits;
-    splits = (nk + cps - 1) / cps;
+    if (tiles * 2 <= sms) splits = std::max(1, std::min({16, kp.nk / 4, sms / tiles}));
+    const int cps = (kp.nk + splits - 1) / splits;
+    splits = (kp.nk + cps - 1) / cps;
     const size_t mn = static_cast<size_t>(M) * N;
     float *ws = nullptr;
     if (splits > 1)
@@ -703,9 +776,9 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
             splits = 1;
         }
     }
-    const int cps_used = splits > 1 ? cps : nk;
+    const int cps_used = splits > 1 ? cps : kp.nk;
     dim3 grid(tiles_m, tiles_n, splits);
-    gemm_tma_kernel<<<grid, kTmaThreads, kTmaSmem, s>>>(ta, tb, splits > 1 ? ws : D, M, N, K, cps_used,
+    gemm_tma_kernel<kMn><<<grid, kTmaThreads, kTmaSmem, s>>>(ta, tb, splits > 1 ? ws : D, M, N, kp, cps_used,
                                                         splits > 1 ? mn : 0, d_err);
     if (splits > 1)
     {
@@ -714,5 +787,51 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
         cudaFreeAsync(ws, s);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+}  // namespace
+
+// D = A * B^T (see knp_gb300_bf16_gemm_tn). The TMA-fed kernels need 16-byte aligned rows (K a multiple
+// of 8, 16-byte aligned A and B); other shapes take the single-stage kernel.
+int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, unsigned int *d_err, cudaStream_t s)
+{
+    if (M < 1 || N < 1 || K < 1 || !A || !B || !D || !d_err) return -1;
+    const bool aligned = K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
+    if (!aligned) return bf16_gemm_tn_simple(A, B, D, M, N, K, d_err, s);
+    CUtensorMap ta, tb;
+    const int nk = (K + kBK - 1) / kBK;
+    if (sw128_map(&ta, A, M, K, kBM) && sw128_map(&tb, B, N, K, kBN))
+        return launch_gemm<false>(ta, tb, D, M, N, KPlan{nk, nk, 0, 0}, d_err, s);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (smem_limit_once(gemm_pipe_kernel, static_cast<int>(kStages * kStageBytes), dev) != cudaSuccess) return -3;
+    dim3 grid((M + kBM - 1) / kBM, (N + kBN - 1) / kBN);
+    gemm_pipe_kernel<<<grid, kThreads, kStages * kStageBytes, s>>>(static_cast<const __nv_bfloat16 *>(A),
+                                                                   static_cast<const __nv_bfloat16 *>(B), D, M, N, K, d_err);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// The two products of a LIF layer's backward, with the gradient dI given as rows of two BF16 halves
+// [hi | lo] of width w2 (knp_gb300_lif_layer_backward), summed over hi, then over lo:
+//   ds[rows][n_in] = (hi + lo) W^T   from W as [n_in][w2]: both operands K-major, W shared by the halves;
+//   dW[n_in][n_out] = S^T (hi + lo)  from S as [rows][n_in8]: both operands MN-major, so neither S nor dI is
+// transposed in memory (a transposed copy of each cost 89 us of the 1.03 ms of a 16384-row layer of
+// 2048 x 2048).
+int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, int n_out, int w2, unsigned int *d_err,
+                cudaStream_t s)
+{
+    CUtensorMap ta, tb;
+    const int nkh = (n_out + kBK - 1) / kBK;
+    if (!sw128_map(&ta, dI2, rows, 2 * w2, kBM) || !sw128_map(&tb, W, n_in, w2, kBN)) return -3;
+    return launch_gemm<false>(ta, tb, ds, rows, n_in, KPlan{2 * nkh, nkh, w2, 0}, d_err, s);
+}
+
+int lif_dw_gemm(const void *S, const void *dI2, float *dW, int rows, int n_in, int n_in8, int n_out, int w2,
+                unsigned int *d_err, cudaStream_t s)
+{
+    CUtensorMap ta, tb;
+    const int nkh = (rows + kBK - 1) / kBK;
+    if (!sw128_map(&ta, S, rows, n_in8, kBK) || !sw128_map(&tb, dI2, rows, 2 * w2, kBK)) return -3;
+    return launch_gemm<true>(ta, tb, dW, n_in, n_out, KPlan{2 * nkh, nkh, 0, w2}, d_err, s);
 }
 }  // namespace knp_gb300

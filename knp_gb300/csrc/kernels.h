@@ -433,8 +433,10 @@ void launch_apply_impacts(
     uint32_t seq_base, Control *ctl, cudaStream_t s);
 
 // Fills the CUtensorMap at `map` with the (K, rows) view of a row-major [rows][K] BF16 matrix (K a multiple
-// of 8, 16-byte aligned), loaded in boxes of 64 x 128 with the 128-byte swizzle (gemm.cu).
-bool sw128_map(void *map, const void *ptr, int rows, int K);
+// of 8, 16-byte aligned), loaded in boxes of 64 x box_rows with the 128-byte swizzle (gemm.cu);
+// sw128_map_3d the (K, t, b) view of rows t * batch + b, loaded in boxes of 64 x box_t x box_b.
+bool sw128_map(void *map, const void *ptr, int rows, int K, int box_rows);
+bool sw128_map_3d(void *map, const void *ptr, int T, int batch, int K, int box_t, int box_b);
 
 // Network construction on the device.
 cudaError_t build_csr(

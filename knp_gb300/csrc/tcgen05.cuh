@@ -43,6 +43,20 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t sbo)
     return d;
 }
 
+// Descriptor of an MN-major operand (K rows of contiguous M or N elements) as 64 x 64 TMA boxes with
+// SWIZZLE_128B leave it: a block of 64 elements of M (or N) is 64 K rows of 128 bytes, swizzled as above;
+// blocks are `block` bytes apart along M (or N), 8-row groups of K 1024 bytes. A K step of 16 rows is
+// 2048 bytes of the start address.
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t addr, uint32_t block)
+{
+    uint64_t d = static_cast<uint64_t>((addr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>((block >> 4) & 0x3FFFu) << 16;
+    d |= static_cast<uint64_t>(1024u >> 4) << 32;
+    d |= 1ull << 46;  // descriptor version of tcgen05
+    d |= 2ull << 61;  // 128-byte swizzle
+    return d;
+}
+
 __device__ __forceinline__ uint32_t core_offset(uint32_t r, uint32_t k, uint32_t lbo, uint32_t sbo)
 {
     return (r >> 3) * sbo + (k >> 3) * lbo + (r & 7u) * 16u + (k & 7u) * 2u;
@@ -57,6 +71,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n)
            | (static_cast<uint32_t>(n >> 3) << 17)      // N / 8
            | (static_cast<uint32_t>(m >> 4) << 24);     // M / 16
 }
+
+// Bits of the instruction descriptor that make an operand MN-major.
+constexpr uint32_t kIdescAMn = 1u << 15, kIdescBMn = 1u << 16;
 
 // Allocate `ncols` (power of two, >= 32) tensor-memory columns; one full warp executes it and the
 // base address lands in *slot (shared memory).
@@ -364,6 +381,36 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
         : "memory");
+}
+
+// As tma_load_2d_pair, the 3-D box at (x, y, z).
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, int z,
+                                                 uint32_t mbar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(mbar)
+        : "memory");
+}
+
+// As tmem_ld16, 8 columns, and one column without the wait (tmem_wait_ld).
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v)
+{
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr)
+{
+    uint32_t r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    return __uint_as_float(r);
 }
 
 }  // namespace tc
