@@ -61,3 +61,17 @@ def test_lif_layer_refuses_bad_checkpoint_intervals(seg):
     x, w = torch.zeros(4, 2, 8, device="cuda"), torch.zeros(8, 8, device="cuda")
     with pytest.raises((KnpGb300Error, ZeroDivisionError)):
         bptt.LIFLayerFn.apply(x, w, BETA, THETA, seg, False, K)
+
+
+# Rows whose loads are and are not 16-byte aligned, a width with padding, both halves, an unaligned source.
+@pytest.mark.parametrize("R,C,width,offset", [(3, 8, 8, 0), (5, 12, 16, 0), (4, 7, 8, 0), (33, 333, 336, 0), (6, 16, 24, 1)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_operand_rows_equal_torch(R, C, width, offset, mode):
+    from knp_gb300 import bptt
+
+    g = torch.Generator(device="cuda").manual_seed(R * C)
+    x = torch.randn(R * C + offset, generator=g, device="cuda")[offset:].view(R, C)
+    out = bptt.operand(x, mode, False, width)
+    hi = torch.nn.functional.pad(x.to(torch.bfloat16), (0, width - C))
+    lo = torch.nn.functional.pad((x - x.to(torch.bfloat16).float()).to(torch.bfloat16), (0, width - C))
+    assert torch.equal(out, torch.cat([hi] + ([] if mode == 0 else [hi if mode == 1 else lo]), 1))
