@@ -440,19 +440,21 @@ KNP_GB300_API int knp_gb300_bf16_operand(const void *X, int x_bf16, int64_t R, i
  * Differentiation form: a hard-threshold LIF layer over T steps of B samples, K inputs, N neurons, its
  * input product on the tcgen05 tensor cores with the recurrence of knp_gb300_lif_scan_forward / _backward
  * (relaxed == 0) in the product's epilogue; device memory throughout. S_in: BF16 [T][B][k8] (columns
- * K .. k8 - 1 zero), W: BF16 [K][w2] (columns N .. w2 - 1 zero); k8 and w2 multiples of 8, buffers 16-byte
- * aligned. forward: S [T][B][N] and ckpt [ceil(T / seg)][B][N], FP32. backward: from ckpt and dS [T][B][N],
+ * K .. k8 - 1 zero), W: BF16 [K][wp] (columns N .. w2 - 1 zero, w2 <= wp); k8, w2 and wp multiples of 8,
+ * buffers 16-byte aligned. forward: S [T][B][N] and ckpt [ceil(T / seg)][B][N], FP32. backward: from ckpt and dS [T][B][N],
  * dI as BF16 [T][B][2 w2] (hi = bf16(dI) in columns 0 .. N - 1, lo = bf16(dI - hi) from column w2, the rest
- * zero). ds: [rows = T B][K] = (hi + lo) W^T; dw: [K][N] = S_in^T (hi + lo); FP32, deterministic. 1 <= seg <= 16.
+ * zero). ds: [rows = T B][K] = (hi + lo) W^T, wp = w2 a multiple of 64 (for other
+ * widths knp_gb300_bf16_gemm_tn of dI and W = [W | W], wp = 2 w2); dw: [K][N] = S_in^T (hi + lo); FP32, deterministic. 1 <= seg <= 16.
  * *d_err (device) receives bit 0 if a wait timed out. Launches only.
  */
 KNP_GB300_API int knp_gb300_lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K,
-                                              int k8, int N, int w2, float beta, float theta, int seg,
+                                              int k8, int N, int w2, int wp, float beta, float theta, int seg,
                                               unsigned int *d_err, void *stream);
 KNP_GB300_API int knp_gb300_lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const float *dS,
-                                               void *dI2, int T, int B, int K, int k8, int N, int w2, float beta,
-                                               float theta, int seg, float k, unsigned int *d_err, void *stream);
-KNP_GB300_API int knp_gb300_lif_layer_ds(const void *dI2, const void *W, float *ds, int rows, int K, int N, int w2,
+                                               void *dI2, int T, int B, int K, int k8, int N, int w2, int wp,
+                                               float beta, float theta, int seg, float k, unsigned int *d_err,
+                                               void *stream);
+KNP_GB300_API int knp_gb300_lif_layer_ds(const void *dI2, const void *W, float *ds, int rows, int K, int w2,
                                          unsigned int *d_err, void *stream);
 KNP_GB300_API int knp_gb300_lif_layer_dw(const void *S_in, const void *dI2, float *dW, int rows, int K, int k8, int N,
                                          int w2, unsigned int *d_err, void *stream);

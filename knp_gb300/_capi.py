@@ -90,10 +90,10 @@ def lib():
                                         ctypes.c_float, p], c_int),
         "knp_gb300_lif_scan_backward": ([p, p, p, p, c_int, ctypes.c_int64, ctypes.c_float, ctypes.c_float, c_int,
                                          c_int, ctypes.c_float, p], c_int),
-        "knp_gb300_lif_layer_forward": ([p, p, p, p] + [c_int] * 6 + [ctypes.c_float] * 2 + [c_int, p, p], c_int),
-        "knp_gb300_lif_layer_backward": ([p, p, p, p, p] + [c_int] * 6 + [ctypes.c_float] * 2 +
+        "knp_gb300_lif_layer_forward": ([p, p, p, p] + [c_int] * 7 + [ctypes.c_float] * 2 + [c_int, p, p], c_int),
+        "knp_gb300_lif_layer_backward": ([p, p, p, p, p] + [c_int] * 7 + [ctypes.c_float] * 2 +
                                          [c_int, ctypes.c_float, p, p], c_int),
-        "knp_gb300_lif_layer_ds": ([p, p, p, c_int, c_int, c_int, c_int, p, p], c_int),
+        "knp_gb300_lif_layer_ds": ([p, p, p, c_int, c_int, c_int, p, p], c_int),
         "knp_gb300_lif_layer_dw": ([p, p, p, c_int, c_int, c_int, c_int, c_int, p, p], c_int),
         "knp_gb300_bf16_gemm_tn": ([p, p, p, c_int, c_int, c_int, p, p], c_int),
         "knp_gb300_batched_lif_run": ([c_int, p, p, p, p, p, p, u32, p, p, u64, p, p, ctypes.POINTER(u64),

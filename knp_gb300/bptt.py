@@ -93,14 +93,14 @@ def bf16_terms(x: torch.Tensor, n: int):
     return terms
 
 
-def gemm_terms(a_terms, b_terms, part: int = 8) -> torch.Tensor:
-    """(sum a_i) @ (sum b_j)^T as one GEMM: every pair (a_i, b_j) concatenated along K, each padded to a
-    multiple of ``part`` (8: 16-byte rows)."""
+def gemm_terms(a_terms, b_terms) -> torch.Tensor:
+    """(sum a_i) @ (sum b_j)^T as one GEMM: every pair (a_i, b_j) concatenated along K, each part padded
+    to 16-byte rows."""
     pairs = [(a, b) for a in a_terms for b in b_terms]
     if len(pairs) == 1:
         return gemm_tn(*pairs[0])
-    return gemm_tn(torch.cat([_pad_k(a.contiguous(), part) for a, _ in pairs], 1),
-                   torch.cat([_pad_k(b.contiguous(), part) for _, b in pairs], 1))
+    return gemm_tn(torch.cat([_pad_k(a.contiguous()) for a, _ in pairs], 1),
+                   torch.cat([_pad_k(b.contiguous()) for _, b in pairs], 1))
 
 
 def _round8(n: int) -> int:
@@ -141,10 +141,12 @@ class LIFLayerFn(torch.autograd.Function):
         S = torch.empty((T, B, n_out), device=dev, dtype=torch.float32)
         if fused:
             a = operand(s_in.reshape(T * B, n_in), 0, False, _round8(n_in))  # 0/1 spikes, exact in BF16
-            wb = operand(w_master, 0, False, _round8(n_out))                 # [n_in, w2]
+            # [n_in, w2], or [W | W] where the gradient's halves cannot share W (width not whole chunks of 64).
+            w2 = _round8(n_out)
+            wb = operand(w_master, 0 if w2 % 64 == 0 else 1, False, w2)
             _capi.check(_capi.lib().knp_gb300_lif_layer_forward(
-                _p(a), _p(wb), _p(S), _p(ckpt), T, B, n_in, a.shape[1], n_out, wb.shape[1], beta, theta, checkpoint,
-                _p(_err_word(dev)), _stream()))
+                a.data_ptr(), wb.data_ptr(), S.data_ptr(), ckpt.data_ptr(), T, B, n_in, a.shape[1], n_out, w2, wb.shape[1],
+                beta, theta, checkpoint, _err_word(dev).data_ptr(), _stream()))
             saved = (a, wb)
         else:
             wb = w_master.to(torch.bfloat16)  # [n_in, n_out]
@@ -165,17 +167,23 @@ class LIFLayerFn(torch.autograd.Function):
         ds_in = None
         if fused:
             a, wb = saved
-            k8, w2 = a.shape[1], wb.shape[1]
-            dev, err, st, lib = a.device, _p(_err_word(a.device)), _stream(), _capi.lib()
+            k8, w2, wp = a.shape[1], _round8(n_out), wb.shape[1]
+            dev, err, st, lib = a.device, _err_word(a.device).data_ptr(), _stream(), _capi.lib()
             # The product is recomputed, not stored; dI comes out as rows of two BF16 halves [hi | lo].
             dI2 = torch.empty((T * B, 2 * w2), device=dev, dtype=torch.bfloat16)
-            _capi.check(lib.knp_gb300_lif_layer_backward(_p(a), _p(wb), _p(ckpt), _p(dS), _p(dI2), T, B, n_in, k8, n_out,
-                                                         w2, beta, theta, checkpoint, k, err, st))
+            _capi.check(lib.knp_gb300_lif_layer_backward(a.data_ptr(), wb.data_ptr(), ckpt.data_ptr(), dS.data_ptr(),
+                                                         dI2.data_ptr(), T, B, n_in, k8, n_out, w2, wp, beta, theta,
+                                                         checkpoint, k, err, st))
             dW = torch.empty((n_in, n_out), device=dev, dtype=torch.float32)
-            _capi.check(lib.knp_gb300_lif_layer_dw(_p(a), _p(dI2), _p(dW), T * B, n_in, k8, n_out, w2, err, st))
+            _capi.check(lib.knp_gb300_lif_layer_dw(a.data_ptr(), dI2.data_ptr(), dW.data_ptr(), T * B, n_in, k8, n_out, w2,
+                                                   err, st))
             if ctx.needs_input_grad[0]:
-                ds_in = torch.empty((T, B, n_in), device=dev, dtype=torch.float32)
-                _capi.check(lib.knp_gb300_lif_layer_ds(_p(dI2), _p(wb), _p(ds_in), T * B, n_in, n_out, w2, err, st))
+                if wp == w2:
+                    ds_in = torch.empty((T, B, n_in), device=dev, dtype=torch.float32)
+                    _capi.check(lib.knp_gb300_lif_layer_ds(dI2.data_ptr(), wb.data_ptr(), ds_in.data_ptr(), T * B, n_in,
+                                                           w2, err, st))
+                else:
+                    ds_in = gemm_tn(dI2, wb).reshape(T, B, n_in)
             return ds_in, dW, None, None, None, None, None
         wb, *s_terms = saved
         I = gemm_terms(s_terms, [wb.t().contiguous()]).reshape(T, B, n_out).contiguous()
@@ -183,13 +191,11 @@ class LIFLayerFn(torch.autograd.Function):
         _capi.check(_capi.lib().knp_gb300_lif_scan_backward(
             _p(I), _p(ckpt), _p(dS), _p(dI), T, B * n_out, beta, theta, checkpoint, int(relaxed), k, _stream()))
         d_terms = bf16_terms(dI.reshape(T * B, n_out), 3 if relaxed else 2)
-        # dW[n_in, n_out] = S^T dI: K = T B per (S term, dI term) pair; the two-term form pads its parts to the
-        # fused products' chunks of 64, so that both sum in the same order.
-        part = 8 if relaxed else 64
-        dW = gemm_terms([s.t() for s in s_terms], [d.t() for d in d_terms], part)
+        # dW[n_in, n_out] = S^T dI: K = T B per (S term, dI term) pair.
+        dW = gemm_terms([s.t() for s in s_terms], [d.t() for d in d_terms])
         if ctx.needs_input_grad[0]:
             # ds_in[TB, n_in] = dI W^T, W as [n_in, n_out]: K = n_out per dI term.
-            ds_in = gemm_terms(d_terms, [wb], part).reshape(T, B, n_in)
+            ds_in = gemm_terms(d_terms, [wb]).reshape(T, B, n_in)
         return ds_in, dW, None, None, None, None, None
 
 

@@ -28,11 +28,11 @@ int bernoulli_schedule_noalloc(
 
 namespace knp_gb300
 {
-int lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N, int w2,
+int lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N, int w2, int wp,
                       float beta, float theta, int seg, unsigned int *err, cudaStream_t s);
 int lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const float *dS, void *dI2, int T, int B, int K,
-                       int k8, int N, int w2, float beta, float theta, int seg, float k, unsigned int *err, cudaStream_t s);
-int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, int n_out, int w2, unsigned int *d_err,
+                       int k8, int N, int w2, int wp, float beta, float theta, int seg, float k, unsigned int *err, cudaStream_t s);
+int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, int w2, unsigned int *d_err,
                 cudaStream_t s);
 int lif_dw_gemm(const void *S, const void *dI2, float *dW, int rows, int n_in, int n_in8, int n_out, int w2,
                 unsigned int *d_err, cudaStream_t s);
@@ -485,30 +485,32 @@ static int layer_status(int rc)
 }
 
 int knp_gb300_lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N,
-                                int w2, float beta, float theta, int seg, unsigned int *d_err, void *stream)
+                                int w2, int wp, float beta, float theta, int seg, unsigned int *d_err, void *stream)
 {
-    if (!S_in || !W || !S || !ckpt || !d_err || !layer_widths(K, k8, N, w2) || !aligned16(S_in) || !aligned16(W))
+    if (!S_in || !W || !S || !ckpt || !d_err || !layer_widths(K, k8, N, w2) || wp < w2 || wp % 8 || !aligned16(S_in) ||
+        !aligned16(W))
         return layer_status(-1);
-    return layer_status(knp_gb300::lif_layer_forward(S_in, W, S, ckpt, T, B, K, k8, N, w2, beta, theta, seg, d_err,
+    return layer_status(knp_gb300::lif_layer_forward(S_in, W, S, ckpt, T, B, K, k8, N, w2, wp, beta, theta, seg, d_err,
                                                      static_cast<cudaStream_t>(stream)));
 }
 
 int knp_gb300_lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const float *dS, void *dI2, int T,
-                                 int B, int K, int k8, int N, int w2, float beta, float theta, int seg, float k,
+                                 int B, int K, int k8, int N, int w2, int wp, float beta, float theta, int seg, float k,
                                  unsigned int *d_err, void *stream)
 {
-    if (!S_in || !W || !ckpt || !dS || !dI2 || !d_err || !layer_widths(K, k8, N, w2) || !aligned16(S_in) || !aligned16(W))
+    if (!S_in || !W || !ckpt || !dS || !dI2 || !d_err || !layer_widths(K, k8, N, w2) || wp < w2 || wp % 8 ||
+        !aligned16(S_in) || !aligned16(W))
         return layer_status(-1);
-    return layer_status(knp_gb300::lif_layer_backward(S_in, W, ckpt, dS, dI2, T, B, K, k8, N, w2, beta, theta, seg, k, d_err,
-                                                      static_cast<cudaStream_t>(stream)));
+    return layer_status(knp_gb300::lif_layer_backward(S_in, W, ckpt, dS, dI2, T, B, K, k8, N, w2, wp, beta, theta, seg, k,
+                                                      d_err, static_cast<cudaStream_t>(stream)));
 }
 
-int knp_gb300_lif_layer_ds(const void *dI2, const void *W, float *ds, int rows, int K, int N, int w2, unsigned int *d_err,
+int knp_gb300_lif_layer_ds(const void *dI2, const void *W, float *ds, int rows, int K, int w2, unsigned int *d_err,
                            void *stream)
 {
-    if (!dI2 || !W || !ds || !d_err || rows < 1 || !layer_widths(K, (K + 7) / 8 * 8, N, w2) || !aligned16(dI2) || !aligned16(W))
+    if (!dI2 || !W || !ds || !d_err || rows < 1 || K < 1 || w2 < 1 || w2 % 64 || !aligned16(dI2) || !aligned16(W))
         return layer_status(-1);
-    return layer_status(knp_gb300::lif_ds_gemm(dI2, W, ds, rows, K, N, w2, d_err, static_cast<cudaStream_t>(stream)));
+    return layer_status(knp_gb300::lif_ds_gemm(dI2, W, ds, rows, K, w2, d_err, static_cast<cudaStream_t>(stream)));
 }
 
 int knp_gb300_lif_layer_dw(const void *S_in, const void *dI2, float *dW, int rows, int K, int k8, int N, int w2,

@@ -216,42 +216,60 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pipe_kernel(
     if (warp == 0) tc::tmem_dealloc(tmem, kBN);
 }
 
-// How a GEMM's K is read: nk chunks of 64, in halves of nkh chunks each (one half: nkh = nk); half h of a
-// K-major operand starts h * step elements further along K, of an MN-major one h * step elements further
-// along M or N (an operand that both halves share has step 0).
+// How a GEMM's K is read: nk chunks of 64 positions. Positions from `half` on are the second half of an
+// operand of two: they start over at K 0, in a K-major operand `step` elements further along K, in an
+// MN-major one `step` elements further along M or N (0: both halves share the operand). `half` is a multiple
+// of 64 for K-major operands and of 8 for MN-major ones, or above every position.
 struct KPlan
 {
-    int nk, nkh, a_step, b_step;
+    int nk, half, a_step, b_step;
+};
+constexpr int kOneHalf = 0x7FFFFFFF;
+
+// The operands' tensor maps: 64 x 128 boxes (K-major), or 64 x 64 boxes and 64 x 8 boxes (MN-major).
+struct GemmMaps
+{
+    CUtensorMap a, b, a8, b8;
 };
 
-// Stages chunk c of the 128 rows from r0 of an operand: K-major (row-major [rows][K]) as one 64 x 128 box,
-// MN-major (row-major [K][rows]) as two 64 x 64 boxes, one per 64 rows. Rows and K past the matrix are zeros.
-template <bool kMn, bool kPair>
-__device__ __forceinline__ void load_operand(uint32_t dst, const CUtensorMap *map, int c, int nkh, int step, int r0,
-                                             uint32_t pair_mbar, uint64_t *mbar)
+template <bool kPair>
+__device__ __forceinline__ void load_box(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t pair_mbar,
+                                         uint64_t *mbar)
 {
-    const int half = c >= nkh ? 1 : 0, k = (c - half * nkh) * kBK;
-    if (kMn)
+    if (kPair)
+        tc::tma_load_2d_pair(dst, map, x, y, pair_mbar);
+    else
+        tc::tma_load_2d(dst, map, x, y, mbar);
+}
+
+// Stages chunk c of the 128 rows from r0 of an operand: K-major (row-major [rows][K]) as one 64 x 128 box,
+// MN-major (row-major [K][rows]) as two 64 x 64 boxes, one per 64 rows, or, where the halves meet in the
+// chunk, eight 64 x 8 boxes each. Rows and K past the matrix are zeros.
+template <bool kMn, bool kPair>
+__device__ __forceinline__ void load_operand(uint32_t dst, const CUtensorMap *map, const CUtensorMap *map8, int c, int half,
+                                             int step, int r0, uint32_t pair_mbar, uint64_t *mbar)
+{
+    const int pos = c * kBK;
+    const int second = pos >= half ? 1 : 0;
+    if (!kMn)
     {
-        const int x = r0 + half * step;
-        if (kPair)
-        {
-            tc::tma_load_2d_pair(dst, map, x, k, pair_mbar);
-            tc::tma_load_2d_pair(dst + kTileBytes / 2, map, x + 64, k, pair_mbar);
-        }
-        else
-        {
-            tc::tma_load_2d(dst, map, x, k, mbar);
-            tc::tma_load_2d(dst + kTileBytes / 2, map, x + 64, k, mbar);
-        }
+        load_box<kPair>(dst, map, pos - second * (half - step), r0, pair_mbar, mbar);
     }
-    else if (kPair)
+    else if (second || half - pos >= kBK)
     {
-        tc::tma_load_2d_pair(dst, map, k + half * step, r0, pair_mbar);
+        const int x = r0 + second * step, y = second ? pos - half : pos;
+        load_box<kPair>(dst, map, x, y, pair_mbar, mbar);
+        load_box<kPair>(dst + kTileBytes / 2, map, x + 64, y, pair_mbar, mbar);
     }
     else
     {
-        tc::tma_load_2d(dst, map, k + half * step, r0, mbar);
+        for (int i = 0; i < kBK / 8; ++i)
+        {
+            const bool s = pos + 8 * i >= half;
+            const int x = r0 + (s ? step : 0), y = pos + 8 * i - (s ? half : 0);
+            load_box<kPair>(dst + i * 1024, map8, x, y, pair_mbar, mbar);
+            load_box<kPair>(dst + kTileBytes / 2 + i * 1024, map8, x + 64, y, pair_mbar, mbar);
+        }
     }
 }
 
@@ -274,7 +292,7 @@ constexpr uint32_t kTmaSmem = kTmaStages * kStageBytes + 1024;  // + alignment s
 // warp 1 lane 0 the MMAs; all four warps read the accumulator back.
 template <bool kMn>
 __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
-    const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *__restrict__ out, int M,
+    const __grid_constant__ GemmMaps maps, float *__restrict__ out, int M,
     int N, KPlan kp, int cps, size_t split_stride, unsigned int *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -316,8 +334,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
             }
             const uint32_t sa = base + s * kStageBytes;
             tc::mbar_expect_tx(&full[s], kStageBytes);
-            load_operand<kMn, false>(sa, &ta, c, kp.nkh, kp.a_step, m0, 0u, &full[s]);
-            load_operand<kMn, false>(sa + kTileBytes, &tb, c, kp.nkh, kp.b_step, n0, 0u, &full[s]);
+            load_operand<kMn, false>(sa, &maps.a, &maps.a8, c, kp.half, kp.a_step, m0, 0u, &full[s]);
+            load_operand<kMn, false>(sa + kTileBytes, &maps.b, &maps.b8, c, kp.half, kp.b_step, n0, 0u, &full[s]);
             issued = i + 1;
         }
         // Copies still in flight after a failed wait land before the CTA leaves (bounded).
@@ -405,12 +423,11 @@ constexpr int kPairM = 256, kPairN = 256, kPairStages = 6, kPairBand = 8;
 constexpr uint32_t kPairStage = 2 * kTileBytes;  // this CTA's 128 x 64 of A and of B
 constexpr uint32_t kPairSmem = kPairStages * kPairStage + 1024;
 constexpr uint32_t kDrainWait = 1u << 14;  // polls, about 0.06 s
-constexpr int kPairThreads = 192;  // warps 0-3 read back, warp 4 loads, warp 5 issues (even rank)
+constexpr int kPairThreads = 224;  // warps 0-3 read back, 4 and 6 load A and B, 5 issues (even rank)
 
 template <bool kMn>
 __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gemm_pair_kernel(
-    const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *__restrict__ D, int M, int N,
-    KPlan kp, unsigned int *err)
+    const __grid_constant__ GemmMaps maps, float *__restrict__ D, int M, int N, KPlan kp, unsigned int *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     // Of the even CTA alone: full (both CTAs' halves of a chunk have landed) and acc_empty (4 read-back
@@ -462,10 +479,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
     };
     auto wait = [&](uint64_t *mbar, uint32_t parity) { return wait_or_fail(mbar, parity, &s_fail); };
 
-    if (warp == 4)
+    if (warp == 4 || warp == 6)
     {
         if (lane == 0)
         {
+            // One thread issuing the four boxes of MN-major operands sets the pace (2048 x 2048 x 32768: 197 us
+            // against 173 with a thread for each operand).
+            const bool is_a = warp == 4;
+            const CUtensorMap *map = is_a ? &maps.a : &maps.b, *map8 = is_a ? &maps.a8 : &maps.b8;
+            const int step = is_a ? kp.a_step : kp.b_step;
             const uint32_t full0 = tc::mapa(tc::smem_u32(full), 0);  // the even CTA's
             int issued = 0, s = 0;
             uint32_t ph = 1;
@@ -474,6 +496,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
             {
                 int m0, n0;
                 place(t, m0, n0);
+                const int r0 = (is_a ? m0 : n0) + 128 * static_cast<int>(rank);
                 for (int c = 0; c < nk; ++c)
                 {
                     if (!wait(&empty[s], ph))
@@ -481,12 +504,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                         ok = false;
                         break;
                     }
-                    const uint32_t sa = base + s * kPairStage;
-                    if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * kPairStage);
-                    load_operand<kMn, true>(sa, &ta, c, kp.nkh, kp.a_step, m0 + 128 * static_cast<int>(rank),
+                    if (is_a && rank == 0) tc::mbar_expect_tx(&full[s], 2 * kPairStage);
+                    load_operand<kMn, true>(base + s * kPairStage + (is_a ? 0u : kTileBytes), map, map8, c, kp.half, step, r0,
                                             full0 + s * 8u, nullptr);
-                    load_operand<kMn, true>(sa + kTileBytes, &tb, c, kp.nkh, kp.b_step,
-                                            n0 + 128 * static_cast<int>(rank), full0 + s * 8u, nullptr);
                     ++issued;
                     if (++s == kPairStages)
                     {
@@ -733,13 +753,22 @@ bool sw128_map_3d(void *map, const void *ptr, int T, int batch, int K, int box_t
 
 int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, int K, unsigned int *d_err, cudaStream_t s);
 
+// K is split when the tiles leave most SMs idle and each split keeps at least 4 chunks: the number of
+// splits of nk chunks over `tiles` 128 x 128 tiles, and the chunks of each but the last.
+int gemm_splits(int tiles, int nk, int sms, int &cps)
+{
+    int splits = 1;
+    if (tiles * 2 <= sms) splits = std::max(1, std::min({16, nk / 4, sms / tiles}));
+    cps = (nk + splits - 1) / splits;
+    return (nk + cps - 1) / cps;
+}
+
 namespace
 {
 
 // D[M x N] from operands that are both K-major or (kMn) both MN-major.
 template <bool kMn>
-int launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, float *D, int M, int N, KPlan kp, unsigned int *d_err,
-                cudaStream_t s)
+int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned int *d_err, cudaStream_t s)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -754,15 +783,12 @@ int launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, float *D, int M, i
     if (pair_waves < waves)
     {
         if (smem_limit_once(gemm_pair_kernel<kMn>, static_cast<int>(kPairSmem), dev) != cudaSuccess) return -3;
-        gemm_pair_kernel<kMn><<<2 * std::min(pair_tiles, sms / 2), kPairThreads, kPairSmem, s>>>(ta, tb, D, M, N, kp, d_err);
+        gemm_pair_kernel<kMn><<<2 * std::min(pair_tiles, sms / 2), kPairThreads, kPairSmem, s>>>(maps, D, M, N, kp, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
     if (smem_limit_once(gemm_tma_kernel<kMn>, static_cast<int>(kTmaSmem), dev) != cudaSuccess) return -3;
-    // Split K when the tiles leave most SMs idle and each split keeps at least 4 chunks.
-    int splits = 1;
-    if (tiles * 2 <= sms) splits = std::max(1, std::min({16, kp.nk / 4, sms / tiles}));
-    const int cps = (kp.nk + splits - 1) / splits;
-    splits = (kp.nk + cps - 1) / cps;
+    int cps = 0;
+    int splits = gemm_splits(tiles, kp.nk, sms, cps);
     const size_t mn = static_cast<size_t>(M) * N;
     float *ws = nullptr;
     if (splits > 1)
@@ -778,7 +804,7 @@ int launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, float *D, int M, i
     }
     const int cps_used = splits > 1 ? cps : kp.nk;
     dim3 grid(tiles_m, tiles_n, splits);
-    gemm_tma_kernel<kMn><<<grid, kTmaThreads, kTmaSmem, s>>>(ta, tb, splits > 1 ? ws : D, M, N, kp, cps_used,
+    gemm_tma_kernel<kMn><<<grid, kTmaThreads, kTmaSmem, s>>>(maps, splits > 1 ? ws : D, M, N, kp, cps_used,
                                                         splits > 1 ? mn : 0, d_err);
     if (splits > 1)
     {
@@ -798,10 +824,9 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
     if (M < 1 || N < 1 || K < 1 || !A || !B || !D || !d_err) return -1;
     const bool aligned = K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
     if (!aligned) return bf16_gemm_tn_simple(A, B, D, M, N, K, d_err, s);
-    CUtensorMap ta, tb;
-    const int nk = (K + kBK - 1) / kBK;
-    if (sw128_map(&ta, A, M, K, kBM) && sw128_map(&tb, B, N, K, kBN))
-        return launch_gemm<false>(ta, tb, D, M, N, KPlan{nk, nk, 0, 0}, d_err, s);
+    GemmMaps maps{};
+    if (sw128_map(&maps.a, A, M, K, kBM) && sw128_map(&maps.b, B, N, K, kBN))
+        return launch_gemm<false>(maps, D, M, N, KPlan{(K + kBK - 1) / kBK, kOneHalf, 0, 0}, d_err, s);
     int dev = 0;
     cudaGetDevice(&dev);
     if (smem_limit_once(gemm_pipe_kernel, static_cast<int>(kStages * kStageBytes), dev) != cudaSuccess) return -3;
@@ -813,25 +838,28 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
 
 // The two products of a LIF layer's backward, with the gradient dI given as rows of two BF16 halves
 // [hi | lo] of width w2 (knp_gb300_lif_layer_backward), summed over hi, then over lo:
-//   ds[rows][n_in] = (hi + lo) W^T   from W as [n_in][w2]: both operands K-major, W shared by the halves;
+//   ds[rows][n_in] = (hi + lo) W^T   from W as [n_in][w2] (w2 a multiple of 64: both halves read the same W):
+// both operands K-major;
 //   dW[n_in][n_out] = S^T (hi + lo)  from S as [rows][n_in8]: both operands MN-major, so neither S nor dI is
 // transposed in memory (a transposed copy of each cost 89 us of the 1.03 ms of a 16384-row layer of
-// 2048 x 2048).
-int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, int n_out, int w2, unsigned int *d_err,
-                cudaStream_t s)
+// 2048 x 2048). Positions along K, and so the order of every sum, are those of operands concatenated along K
+// with the rows padded to a multiple of 8.
+int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, int w2, unsigned int *d_err, cudaStream_t s)
 {
-    CUtensorMap ta, tb;
-    const int nkh = (n_out + kBK - 1) / kBK;
-    if (!sw128_map(&ta, dI2, rows, 2 * w2, kBM) || !sw128_map(&tb, W, n_in, w2, kBN)) return -3;
-    return launch_gemm<false>(ta, tb, ds, rows, n_in, KPlan{2 * nkh, nkh, w2, 0}, d_err, s);
+    if (w2 % kBK) return -1;
+    GemmMaps maps{};
+    if (!sw128_map(&maps.a, dI2, rows, 2 * w2, kBM) || !sw128_map(&maps.b, W, n_in, w2, kBN)) return -3;
+    return launch_gemm<false>(maps, ds, rows, n_in, KPlan{2 * w2 / kBK, w2, w2, 0}, d_err, s);
 }
 
 int lif_dw_gemm(const void *S, const void *dI2, float *dW, int rows, int n_in, int n_in8, int n_out, int w2,
                 unsigned int *d_err, cudaStream_t s)
 {
-    CUtensorMap ta, tb;
-    const int nkh = (rows + kBK - 1) / kBK;
-    if (!sw128_map(&ta, S, rows, n_in8, kBK) || !sw128_map(&tb, dI2, rows, 2 * w2, kBK)) return -3;
-    return launch_gemm<true>(ta, tb, dW, n_in, n_out, KPlan{2 * nkh, nkh, 0, w2}, d_err, s);
+    GemmMaps maps{};
+    const int padded = (rows + 7) / 8 * 8;
+    if (!sw128_map(&maps.a, S, rows, n_in8, kBK) || !sw128_map(&maps.b, dI2, rows, 2 * w2, kBK) ||
+        !sw128_map(&maps.a8, S, rows, n_in8, 8) || !sw128_map(&maps.b8, dI2, rows, 2 * w2, 8))
+        return -3;
+    return launch_gemm<true>(maps, dW, n_in, n_out, KPlan{(2 * padded + kBK - 1) / kBK, padded, 0, w2}, d_err, s);
 }
 }  // namespace knp_gb300

@@ -437,6 +437,8 @@ void launch_apply_impacts(
 // sw128_map_3d the (K, t, b) view of rows t * batch + b, loaded in boxes of 64 x box_t x box_b.
 bool sw128_map(void *map, const void *ptr, int rows, int K, int box_rows);
 bool sw128_map_3d(void *map, const void *ptr, int T, int batch, int K, int box_t, int box_b);
+// Splits of the GEMM's K (gemm.cu): their number, and the chunks of 64 of each.
+int gemm_splits(int tiles, int nk, int sms, int &cps);
 
 // Network construction on the device.
 cudaError_t build_csr(

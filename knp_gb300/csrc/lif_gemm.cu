@@ -9,6 +9,10 @@
 //   backward  the same product again, each checkpoint segment's U from its V, then the surrogate-gradient
 //             recurrence from the segment's last step to its first; dI goes out as two BF16 terms
 //             hi = bf16(dI), lo = bf16(dI - hi), the rows that the products for dW and ds_in read.
+// A layer of 2048 x 2048 over 16384 rows: forward 100 us, backward 131 us (tensor time 70 us each), where product
+// and scan took 90 + 79 and 90 + 128 us and the gradient's BF16 rows another 53 + 89. The forward is bound by the
+// product beside the stores of S, the backward by the latency of its scan (an IEEE division and two dependent
+// chains a step), hence two sets of scan warps per half (one: 170 us).
 // Columns: a CTA pair takes a tile of 256 neurons (128 a CTA) and two halves of up to 128 columns, one per
 // CTA's share of the spike operand: whole samples while T fits a half (box_b samples of T steps; a 3-D
 // TMA box brings rows (b, t) in that order from [T][B][K]), else one sample's steps tile by tile, forward in
@@ -35,16 +39,19 @@ constexpr uint32_t kStage = 2 * kOperand;
 constexpr uint32_t kSmem = kStages * kStage + 1024;
 constexpr uint32_t kWait = 1u << 22, kDrainWait = 1u << 14;  // polls
 constexpr int kIssuerWarp = 0, kCopyWarp = 1, kScanWarp0 = 4;
-constexpr int kThreads = 32 * (kScanWarp0 + 8);
+constexpr int kScanWarps = 16;  // two sets of four per half, taking its samples in turn
+constexpr int kThreads = 32 * (kScanWarp0 + kScanWarps);
 constexpr int kMaxSeg = 16;
 
 struct LifGemmArgs
 {
-    CUtensorMap w;  // BF16 W [K][w2], 64 x 64 boxes
+    CUtensorMap w;  // BF16 W [K][wp], 64 x 64 boxes (columns from N on reach no neuron)
     CUtensorMap s;  // BF16 S_in [T][B][K], 64 x box_t x box_b boxes
     int T, B, N, w2;
     int chunks;                 // of K
-    int half_cols;              // columns of a half: 128 or 64
+    int splits, cps;            // K in `splits` runs of cps chunks, each its own accumulator
+    int half_cols;              // columns of a half: 128 .. 16
+    int acc_cols, bufs;         // tensor-memory columns of a tile's accumulators; 2 sets of them if they fit
     int box_t, box_b, t_tiles;  // steps and samples of a half; tiles along time (box_b == 1 if more than one)
     int n_tiles, items;         // pairs of neuron tiles; items = n_tiles * sample groups
     float beta, theta, k;
@@ -75,6 +82,31 @@ struct Lane
     bool real;  // the neuron exists
 };
 
+// kN columns of I from `col`: the runs' sums added in order (as split_sum_kernel of gemm.cu adds them).
+template <int kN, bool kSplit>
+__device__ __forceinline__ void load_cols(const LifGemmArgs &a, uint32_t col, float *x)
+{
+    auto ld = [](uint32_t c, float *v)
+    {
+        if (kN == 16)
+            tc::tmem_ld16(c, v);
+        else if (kN == 8)
+            tc::tmem_ld8(c, v);
+        else
+            v[0] = tc::tmem_ld1(c);
+    };
+    ld(col, x);
+    if (!kSplit) return;
+    for (int p = 1; p < a.splits; ++p)
+    {
+        float y[kN];
+        ld(col + p * 2 * a.half_cols, y);
+#pragma unroll
+        for (int i = 0; i < kN; ++i) x[i] = __fadd_rn(x[i], y[i]);
+    }
+}
+
+template <bool kSplit>
 __device__ __forceinline__ void forward_sample(const LifGemmArgs &a, const Lane &l, int t0, int steps, float &V)
 {
     const size_t stride = static_cast<size_t>(a.B) * a.N;
@@ -101,23 +133,28 @@ __device__ __forceinline__ void forward_sample(const LifGemmArgs &a, const Lane 
     for (; u + 16 <= steps; u += 16)
     {
         float x[16];
-        tc::tmem_ld16(l.col + u, x);
+        load_cols<16, kSplit>(a, l.col + u, x);
 #pragma unroll
         for (int i = 0; i < 16; ++i) step(x[i]);
     }
     if (u + 8 <= steps)
     {
         float x[8];
-        tc::tmem_ld8(l.col + u, x);
+        load_cols<8, kSplit>(a, l.col + u, x);
 #pragma unroll
         for (int i = 0; i < 8; ++i) step(x[i]);
         u += 8;
     }
-    for (; u < steps; ++u) step(tc::tmem_ld1(l.col + u));
+    for (; u < steps; ++u)
+    {
+        float x[1];
+        load_cols<1, kSplit>(a, l.col + u, x);
+        step(x[0]);
+    }
 }
 
 // kSeg: the checkpoint interval when it is 8 (whole segments read as 8 columns), else 0.
-template <int kSeg>
+template <int kSeg, bool kSplit>
 __device__ __forceinline__ void backward_sample(const LifGemmArgs &a, const Lane &l, int t0, int steps, float &dV)
 {
     constexpr int kMost = kSeg ? kSeg : kMaxSeg;
@@ -144,13 +181,13 @@ __device__ __forceinline__ void backward_sample(const LifGemmArgs &a, const Lane
         float U[kMost], g[kMost];
         if (kSeg == 8 && len == 8)
         {
-            tc::tmem_ld8(l.col + c * seg, U);
+            load_cols<8, kSplit>(a, l.col + c * seg, U);
         }
         else
         {
 #pragma unroll
             for (int u = 0; u < kMost; ++u)
-                if (u < len) U[u] = tc::tmem_ld1(l.col + c * seg + u);
+                if (u < len) load_cols<1, kSplit>(a, l.col + c * seg + u, U + u);
         }
         float V = ck;
 #pragma unroll
@@ -191,10 +228,11 @@ __device__ __forceinline__ void backward_sample(const LifGemmArgs &a, const Lane
 }
 
 // Roles in each CTA of a pair: warp 0 issues the pair's MMAs (even rank), warp 1 loads this CTA's operands,
-// warps 4-7 and 8-11 scan the two halves' columns (thread = neuron). Two accumulators: the scan of a tile
+// warps 4-19 scan the two halves' columns (thread = neuron; per half two sets of four warps take its samples
+// in turn: the scans are bound by latency). Two accumulators: the scan of a tile
 // runs beside the product of the next. Persistent over items (a pair of neuron tiles and a group of
 // samples). Waits and their failure are gemm_pair_kernel's (gemm.cu).
-template <bool kBackward, int kSeg>
+template <bool kBackward, int kSeg, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
     lif_gemm_kernel(const __grid_constant__ LifGemmArgs a)
 {
@@ -223,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
         for (int i = 0; i < 2; ++i)
         {
             tc::mbar_init(&acc_full[i], 1);
-            tc::mbar_init(&acc_empty[i], 16);
+            tc::mbar_init(&acc_empty[i], 2 * kScanWarps);
         }
         tc::mbar_init(&drain, 1);
         s_fail = 0;
@@ -294,12 +332,14 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
             for (int it = pair; it < a.items && ok; it += pairs)
                 for (int q = 0; q < a.t_tiles && ok; ++q, ++n)
                 {
-                    const int acc = n & 1;
-                    if (n >= 2 && !wait_or_fail(&acc_empty[acc], ((n >> 1) - 1) & 1, &s_fail))
+                    const int acc = n % a.bufs, use = n / a.bufs;
+                    if (use >= 1 && !wait_or_fail(&acc_empty[acc], (use - 1) & 1, &s_fail))
                     {
                         ok = false;
                         break;
                     }
+                    uint32_t d = tmem + acc * a.acc_cols;
+                    int in_run = 0;  // chunk of the run
                     for (int c = 0; c < a.chunks; ++c)
                     {
                         if (!wait_or_fail(&full[s], ph, &s_fail))
@@ -311,9 +351,14 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
                         const uint64_t off = static_cast<uint64_t>(s) * (kStage >> 4);
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            tc::mma_bf16_pair(tmem + acc * 256, dw + off + j * (2048 >> 4), ds + off + j * (32 >> 4), idesc,
-                                              (c > 0 || j > 0) ? 1u : 0u);
+                            tc::mma_bf16_pair(d, dw + off + j * (2048 >> 4), ds + off + j * (32 >> 4), idesc,
+                                              (in_run > 0 || j > 0) ? 1u : 0u);
                         tc::commit_pair(&empty[s]);
+                        if (++in_run == a.cps)
+                        {
+                            in_run = 0;
+                            d += 2 * a.half_cols;
+                        }
                         if (++s == kStages)
                         {
                             s = 0;
@@ -334,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
     }
     else if (warp >= kScanWarp0)
     {
-        const int half = (warp - kScanWarp0) >> 2;
+        const int half = ((warp - kScanWarp0) >> 2) & 1, set = (warp - kScanWarp0) >> 3;
         const uint32_t lanes = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + half * a.half_cols;
         const uint32_t acc_empty0 = tc::mapa(tc::smem_u32(acc_empty), 0);
         int n = 0;
@@ -348,9 +393,9 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
             float carry = 0.0f;  // V, or dV, from tile to tile of one sample
             for (int q = 0; q < a.t_tiles; ++q, ++n)
             {
-                const int acc = n & 1;
+                const int acc = n % a.bufs;
                 int got = 1;
-                if (lane == 0) got = wait_or_fail(&acc_full[acc], (n >> 1) & 1, &s_fail);
+                if (lane == 0) got = wait_or_fail(&acc_full[acc], (n / a.bufs) & 1, &s_fail);
                 if (!__shfl_sync(0xffffffffu, got, 0))
                 {
                     ok = false;
@@ -358,15 +403,15 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
                 }
                 tc::fence_after_sync();
                 const int t0 = time_tile(q) * a.box_t, steps = min(a.box_t, a.T - t0);
-                for (int i = 0; i < a.box_b && b0 + i < a.B; ++i)
+                for (int i = set; i < a.box_b && b0 + i < a.B; i += 2)
                 {
                     if (a.t_tiles == 1) carry = 0.0f;
                     l.b = b0 + i;
-                    l.col = lanes + acc * 256 + i * a.box_t;
+                    l.col = lanes + acc * a.acc_cols + i * a.box_t;
                     if (kBackward)
-                        backward_sample<kSeg>(a, l, t0, steps, carry);
+                        backward_sample<kSeg, kSplit>(a, l, t0, steps, carry);
                     else
-                        forward_sample(a, l, t0, steps, carry);
+                        forward_sample<kSplit>(a, l, t0, steps, carry);
                 }
                 tc::fence_before_sync();
                 __syncwarp();
@@ -383,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
     if (warp == kIssuerWarp) tc::tmem_dealloc_pair(tmem, 512);
 }
 
-int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, bool backward, cudaStream_t s)
+int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, int wp, bool backward, cudaStream_t s)
 {
     if (a.T < 1 || a.B < 1 || a.N < 1 || K < 1 || a.seg < 1 || a.seg > kMaxSeg) return -1;
     int dev = 0, sms = 0;
@@ -391,10 +436,16 @@ int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, bool 
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int pairs = std::max(1, sms / 2);
     a.chunks = (K + 63) / 64;
+    // The product alone would split K here when its 128 x 128 tiles leave most SMs idle; the runs are kept
+    // apart and added in the same order, so that I has the same bits.
+    const long long tiles = ((static_cast<long long>(a.T) * a.B + 127) / 128) * ((a.N + 127) / 128);
+    a.splits = gemm_splits(static_cast<int>(std::min<long long>(tiles, 1 << 20)), a.chunks, sms, a.cps);
     a.n_tiles = (a.N + 255) / 256;
     auto plan = [&](int cols)
     {
         a.half_cols = cols;
+        a.acc_cols = 2 * cols * a.splits;
+        a.bufs = 2 * a.acc_cols <= 512 ? 2 : 1;
         // Tiles along time start on a checkpoint.
         a.box_t = a.T <= cols ? a.T : cols / a.seg * a.seg;
         a.box_b = a.T <= cols ? std::min(cols / a.T, a.B) : 1;
@@ -402,12 +453,21 @@ int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, bool 
         a.items = a.n_tiles * ((a.B + 2 * a.box_b - 1) / (2 * a.box_b));
         return (a.items + pairs - 1) / pairs;
     };
-    // Halves of 64 columns when they spread the samples over more of the device: a tile of them takes about
-    // half as long, so they win while they need fewer than twice the waves.
-    const int waves = plan(128);
-    if (a.T > 64 || plan(64) >= 2 * waves) plan(128);
-    if (!sw128_map(&a.w, W, K, a.w2, 64) || !sw128_map_3d(&a.s, S_in, a.T, a.B, k8, a.box_t, a.box_b)) return -3;
-    auto kernel = !backward ? lif_gemm_kernel<false, 0> : a.seg == 8 ? lif_gemm_kernel<true, 8> : lif_gemm_kernel<true, 0>;
+    if (a.splits > 1)
+    {
+        plan(a.splits <= 4 ? 64 : a.splits <= 8 ? 32 : 16);  // at most 16 runs: 512 columns
+    }
+    else
+    {
+        // Halves of 64 columns when they spread the samples over more of the device: a tile of them takes
+        // about half as long, so they win while they need fewer than twice the waves.
+        const int waves = plan(128);
+        if (a.T > 64 || plan(64) >= 2 * waves) plan(128);
+    }
+    if (!sw128_map(&a.w, W, K, wp, 64) || !sw128_map_3d(&a.s, S_in, a.T, a.B, k8, a.box_t, a.box_b)) return -3;
+    auto kernel = !backward   ? (a.splits > 1 ? lif_gemm_kernel<false, 0, true> : lif_gemm_kernel<false, 0, false>)
+                  : a.seg == 8 ? (a.splits > 1 ? lif_gemm_kernel<true, 8, true> : lif_gemm_kernel<true, 8, false>)
+                               : (a.splits > 1 ? lif_gemm_kernel<true, 0, true> : lif_gemm_kernel<true, 0, false>);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -3;
     kernel<<<2 * std::min(a.items, pairs), kThreads, kSmem, s>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
@@ -415,8 +475,9 @@ int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, bool 
 
 }  // namespace
 
-// S_in: BF16 [T B][k8], W: BF16 [K][w2] (rows of whole 16-byte units).
-int lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N, int w2,
+// S_in: BF16 [T B][k8], W: BF16 [K][wp] with the weights in columns 0 .. N - 1 and zeros up to w2 (rows of
+// whole 16-byte units).
+int lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, int T, int B, int K, int k8, int N, int w2, int wp,
                       float beta, float theta, int seg, unsigned int *err, cudaStream_t s)
 {
     LifGemmArgs a{};
@@ -430,11 +491,11 @@ int lif_layer_forward(const void *S_in, const void *W, float *S, float *ckpt, in
     a.S = S;
     a.ckpt = ckpt;
     a.err = err;
-    return launch(a, S_in, W, K, k8, false, s);
+    return launch(a, S_in, W, K, k8, wp, false, s);
 }
 
 int lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const float *dS, void *dI2, int T, int B, int K,
-                       int k8, int N, int w2, float beta, float theta, int seg, float k, unsigned int *err, cudaStream_t s)
+                       int k8, int N, int w2, int wp, float beta, float theta, int seg, float k, unsigned int *err, cudaStream_t s)
 {
     LifGemmArgs a{};
     a.T = T;
@@ -449,7 +510,7 @@ int lif_layer_backward(const void *S_in, const void *W, const float *ckpt, const
     a.dS = dS;
     a.dI2 = static_cast<__nv_bfloat16 *>(dI2);
     a.err = err;
-    return launch(a, S_in, W, K, k8, true, s);
+    return launch(a, S_in, W, K, k8, wp, true, s);
 }
 
 }  // namespace knp_gb300
