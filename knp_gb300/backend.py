@@ -29,7 +29,9 @@ SUPPORTED_SYNAPSES = ["DeltaSynapse", "AdditiveSTDPDeltaSynapse"]
 
 
 def _ptr(a):
-    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
+    """Address of an array's data for a c_void_p argument (cheaper than ``a.ctypes``, which a step's calls would
+    make several times)."""
+    return None if a is None else a.__array_interface__["data"][0]
 
 
 class GB300Backend:
@@ -43,6 +45,7 @@ class GB300Backend:
         self._pops: dict = {}
         self._projs: dict = {}
         self._recorded: set = set()
+        self._uids: dict = {}  # uid -> its C struct, for the calls of every step
         self._initialized = False
         self._started = False
         self._stop = False
@@ -67,6 +70,12 @@ class GB300Backend:
 
     def _chk(self, rc):
         _capi.check(rc)
+
+    def _uid(self, uid: bytes):
+        c = self._uids.get(uid)
+        if c is None:
+            c = self._uids[uid] = T.to_c_uid(uid)
+        return c
 
     # ------------------------------------------------------------------ interface queries (backend.h:103-127)
     def plasticity_supported(self) -> bool:
@@ -273,7 +282,7 @@ class GB300Backend:
     def send_spikes(self, sender: bytes, indexes, send_time: int | None = None):
         idx = np.ascontiguousarray(indexes, np.uint32)
         t = self.get_step() if send_time is None else send_time
-        self._chk(self._lib.knp_gb300_send_spikes(self._h, T.to_c_uid(sender), t, idx.size, _ptr(idx)))
+        self._chk(self._lib.knp_gb300_send_spikes(self._h, self._uid(sender), t, idx.size, _ptr(idx)))
 
     def send_impacts(self, sender: bytes, pop: bytes, post_idx, values, out_type=None, is_forcing: bool = True):
         post_idx = np.ascontiguousarray(post_idx, np.uint32)
@@ -299,11 +308,11 @@ class GB300Backend:
         if out is None or out.dtype != np.uint32 or not out.flags.c_contiguous or out.size < max(n, 1):
             out = np.empty(max(n, 1), np.uint32)
         cnt = ctypes.c_uint32(0)
-        self._chk(self._lib.knp_gb300_read_spikes(self._h, T.to_c_uid(pop), step, out.size, _ptr(out),
+        self._chk(self._lib.knp_gb300_read_spikes(self._h, self._uid(pop), step, out.size, _ptr(out),
                                                   ctypes.byref(cnt)))
         if cnt.value > out.size:
             out = np.empty(cnt.value, np.uint32)
-            self._chk(self._lib.knp_gb300_read_spikes(self._h, T.to_c_uid(pop), step, out.size, _ptr(out),
+            self._chk(self._lib.knp_gb300_read_spikes(self._h, self._uid(pop), step, out.size, _ptr(out),
                                                       ctypes.byref(cnt)))
         return out[: cnt.value]
 
@@ -311,7 +320,7 @@ class GB300Backend:
         """Writes at most ``out.size`` ascending spike indexes of ``pop`` at ``step`` into ``out``
         (uint32) and returns the step's full spike count."""
         cnt = ctypes.c_uint32(0)
-        self._chk(self._lib.knp_gb300_read_spikes(self._h, T.to_c_uid(pop), step, out.size, _ptr(out),
+        self._chk(self._lib.knp_gb300_read_spikes(self._h, self._uid(pop), step, out.size, _ptr(out),
                                                   ctypes.byref(cnt)))
         return int(cnt.value)
 

@@ -34,7 +34,7 @@ def _p(t: torch.Tensor):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch.cuda.current_stream().cuda_stream
 
 
 def bf16_values(w: torch.Tensor) -> torch.Tensor:
@@ -47,15 +47,18 @@ _ERR = {}
 
 def _err_word(device) -> torch.Tensor:
     """Device error word of the GEMMs on `device` (bit 0: a tensor-core completion wait timed out)."""
-    key = str(device)
-    if key not in _ERR:
-        _ERR[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _ERR[key]
+    e = _ERR.get(device)
+    if e is None:
+        e = _ERR[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return e
 
 
 def check_gemm_errors(device="cuda"):
     """Raises if a GEMM of this module reported a timeout on `device` (one device-to-host read)."""
-    e = _err_word(torch.device(device))
+    device = torch.device(device)
+    if device.index is None:
+        device = torch.device(device.type, torch.cuda.current_device())
+    e = _err_word(device)
     if int(e.item()) != 0:
         e.zero_()
         raise RuntimeError("a tcgen05 GEMM completion wait timed out")

@@ -84,9 +84,10 @@ constexpr size_t kExpandBlockWords = 4096;
 
 struct RecordedStep
 {
-    std::vector<uint32_t> bits;  // bit i of word i / 32: neuron i fired
+    bool is_list = false;        // data holds the step's ascending indexes, else its bitmap
+    std::vector<uint32_t> data;  // bitmap: bit i of word i / 32: neuron i fired
     uint32_t count = 0;
-    std::vector<uint32_t> block_prefix;  // spikes before each block of kExpandBlockWords words
+    std::vector<uint32_t> block_prefix;  // bitmap: spikes before each block of kExpandBlockWords words
 };
 
 // Host worker threads for large bitmap expansions: run(n, fn) calls fn(0 .. n - 1) on the workers
@@ -200,11 +201,21 @@ struct ProjectionSlot
     uint64_t res_offset = 0;
 };
 
+// What a host-sent message of a step puts on the device: the channel's descriptor with the offsets and the
+// indexes it points to behind it, one copy. Longer messages use the channel's own arrays.
+struct ChannelMessage
+{
+    static constexpr uint32_t kMost = 2048;
+    ChannelDev desc;
+    long long offsets[2];
+    uint32_t idx[kMost];
+};
+
 struct Channel
 {
     Uid uid;
     ChannelDev host{};
-    ChannelDev *dev = nullptr;  // device descriptor read by kernels
+    ChannelDev *dev = nullptr;  // device descriptor read by kernels, with room for a message (ChannelMessage)
     // device data
     long long *offsets = nullptr;
     uint32_t *idx = nullptr;
@@ -331,6 +342,8 @@ private:
     // pinned host buffer that recorded bitmaps are drained through
     uint32_t *rec_host_ = nullptr;
     size_t rec_host_words_ = 0;
+    uint32_t *rec_counts_ = nullptr, *rec_counts_host_ = nullptr;  // segment counts of a drain (readback.cu)
+    size_t rec_counts_n_ = 0;
     uint64_t neurons_total_ = 0;
     uint64_t updates_before_init_ = 0;
     cudaGraphExec_t graph1_ = nullptr, graphK_ = nullptr;

@@ -440,6 +440,15 @@ bool sw128_map_3d(void *map, const void *ptr, int T, int batch, int K, int box_t
 // Splits of the GEMM's K (gemm.cu): their number, and the chunks of 64 of each.
 int gemm_splits(int tiles, int nk, int sms, int &cps);
 
+// Read-back of recorded steps (readback.cu): the spikes of steps first .. first + n_steps - 1 (n_steps at most
+// 65535) of a recording ring of `slots` bitmaps of W words. counts (device) and counts_host receive the
+// spikes per segment of kReadbackSegWords words, [n_steps][readback_segments(W)]; lists_host (pinned,
+// [n_steps][W]) each step's ascending indexes, unless it has more than W.
+constexpr uint32_t kReadbackSegWords = 1024;
+uint32_t readback_segments(uint32_t W);
+cudaError_t launch_spike_lists(const uint32_t *bits, uint32_t W, uint32_t slots, uint64_t first, uint32_t n_steps,
+                               uint32_t *counts, uint32_t *counts_host, uint32_t *lists_host, cudaStream_t s);
+
 // Network construction on the device.
 cudaError_t build_csr(
     uint64_t n_syn, uint32_t n_rows, const uint32_t *d_row_key, uint32_t *d_perm_out, long long *d_row_ptr,
