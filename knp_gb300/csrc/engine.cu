@@ -1013,6 +1013,7 @@ void Backend::build_projection(ProjectionSlot &p)
     ProjectionDev &d = p.dev;
     d.row_ptr = p.row_ptr;
     d.n_rows = p.n_rows;
+    d.short_rows = p.n_syn <= 2 * static_cast<uint64_t>(p.n_rows) ? 1 : 0;
     d.col = p.col;
     d.w = p.w;
     d.delay = p.delay_d;
@@ -1245,6 +1246,7 @@ void Backend::build_pull(ProjectionSlot &p)
     g.max_delay = p.max_delay;
     g.hist_slots = p.max_delay + 1;
     g.n_windows = (post->n + kPullWindow - 1) / kPullWindow;
+    g.n_bm = 1;
     const int grid = static_cast<int>(std::max<uint32_t>(1, std::min<uint32_t>(g.n_windows, sm_count_)));
     const size_t smem = gather_smem_bytes(g, grid);
     int smem_max = 0;
@@ -1263,6 +1265,15 @@ void Backend::build_pull(ProjectionSlot &p)
     g.threshold = static_cast<uint32_t>(std::max(1.0, std::ceil(p.pull_fraction * p.n_rows)));
     // 32 copies of the weight dictionary (one per bank) when shared memory has room for them.
     if (g.wtab && smem + static_cast<size_t>(g.n_tab) * 32 * 4 + 2048 <= static_cast<size_t>(smem_max)) g.tab_rep = 1;
+    // Shares cut between delays, then as many bitmaps at a time as fit beside the kernels' static shared memory.
+    g.split_delays = static_cast<uint64_t>(g.n_windows) * g.max_delay < 0xFFFFFFFFull ? 1 : 0;
+    if (g.split_delays && gather_smem_bytes(g, grid) + 8192 > static_cast<size_t>(smem_max)) g.split_delays = 0;
+    for (uint32_t k = 2; k <= std::min(kGatherBitmaps, g.max_delay); ++k)
+    {
+        PullDev more = g;
+        more.n_bm = k;
+        if (gather_smem_bytes(more, grid) + 8192 <= static_cast<size_t>(smem_max)) g.n_bm = k;
+    }
     KNP_CUDA(set_gather_smem(std::max<size_t>(gather_smem_bytes(g, grid), 48 * 1024)));
     p.dev.pull = g;
     p.pull = true;

@@ -143,19 +143,24 @@ __device__ __forceinline__ unsigned long long project(const ProjectionDev &p, un
             else
             {
                 uint32_t *bm = p.pull.bitmap + static_cast<size_t>(sl) * p.pull.words;
-                for (uint32_t j = gthread; j < total; j += n_threads)
+                for (uint32_t j0 = gthread - lane; j0 < total; j0 += n_threads)
                 {
-                    uint32_t jj = j;
-                    int k = 0;
-                    while (jj >= cnt[k])
+                    uint32_t jj = j0 + lane, pre = kNoSpike;
+                    if (jj < total)
                     {
-                        jj -= cnt[k];
-                        ++k;
+                        int k = 0;
+                        while (jj >= cnt[k])
+                        {
+                            jj -= cnt[k];
+                            ++k;
+                        }
+                        pre = idx[k][jj];
+                        if (pre < p.n_rows)
+                            ev += static_cast<unsigned long long>(p.row_ptr[pre + 1] - p.row_ptr[pre]);
+                        else
+                            pre = kNoSpike;
                     }
-                    const uint32_t pre = idx[k][jj];
-                    if (pre >= p.n_rows) continue;
-                    atomicOr(bm + (pre >> 5), 1u << (pre & 31));
-                    ev += static_cast<unsigned long long>(p.row_ptr[pre + 1] - p.row_ptr[pre]);
+                    mark_spikes(bm, pre, lane);
                 }
             }
 #pragma unroll
@@ -205,7 +210,9 @@ __device__ __forceinline__ bool grid_stdp_rules(const SmallStdp *rules, uint32_t
 
 __device__ __forceinline__ void grid_gather(const ProjectionDev &p, unsigned long long tn, uint4 *smem)
 {
-    if (p.pull.wtab)
+    if (p.pull.wtab && p.pull.tab_rep)
+        gather_block<kDictRep>(p, tn, blockIdx.x, gridDim.x, smem);
+    else if (p.pull.wtab)
         gather_block<kDict>(p, tn, blockIdx.x, gridDim.x, smem);
     else if (p.pull.w16)
         gather_block<kHalf>(p, tn, blockIdx.x, gridDim.x, smem);

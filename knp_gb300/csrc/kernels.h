@@ -267,6 +267,7 @@ struct SpikeSource
 constexpr int kPullWindow = 256;
 constexpr int kPullSlice = 32;
 constexpr int kPullSlicesPerWindow = kPullWindow / kPullSlice;
+constexpr uint32_t kGatherBitmaps = 8;
 
 struct PullDev
 {
@@ -285,6 +286,8 @@ struct PullDev
     const float *wtab;           // [256] weight dictionary (entry 0 is +0.0), used when the projection has at
                                  // most 256 distinct weights and fewer than 2^24 presynaptic neurons; else null
     uint32_t n_tab;              // dictionary entries in use
+    uint32_t n_bm;               // steps' bitmaps a gather block holds at a time (1 .. kGatherBitmaps)
+    uint32_t split_delays;       // 1: the gather is cut over blocks in units of (window, delay), 0: whole windows
     uint32_t tab_rep;            // 1: the gather keeps 32 copies of the dictionary in shared memory (entry
                                  // i of lane l at 32 i + l: conflict-free lookups); 0: one copy
     const float *w;              // FP32 weights (negated for inhibitory current), or null
@@ -305,6 +308,7 @@ struct ProjectionDev
     PullDev pull;  // pull.bitmap == nullptr: scatter only
     const long long *row_ptr;
     uint32_t n_rows;
+    uint32_t short_rows;  // rows hold two synapses on average at most: scattered a lane per row
     const int32_t *col;
     float *w;
     const uint8_t *delay;

@@ -55,19 +55,24 @@ __global__ void __launch_bounds__(256) projection_kernel(ProjectionDev p, Contro
         {
             uint32_t *bm = p.pull.bitmap + static_cast<size_t>(sl) * p.pull.words;
             const uint32_t stride = gridDim.x * blockDim.x;
-            for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += stride)
+            for (uint32_t j0 = blockIdx.x * blockDim.x + threadIdx.x - lane; j0 < total; j0 += stride)
             {
-                uint32_t jj = j;
-                int k = 0;
-                while (jj >= cnt[k])
+                uint32_t jj = j0 + lane, pre = kNoSpike;
+                if (jj < total)
                 {
-                    jj -= cnt[k];
-                    ++k;
+                    int k = 0;
+                    while (jj >= cnt[k])
+                    {
+                        jj -= cnt[k];
+                        ++k;
+                    }
+                    pre = idx[k][jj];
+                    if (pre < p.n_rows)
+                        events += static_cast<unsigned long long>(p.row_ptr[pre + 1] - p.row_ptr[pre]);
+                    else
+                        pre = kNoSpike;
                 }
-                const uint32_t pre = idx[k][jj];
-                if (pre >= p.n_rows) continue;
-                atomicOr(bm + (pre >> 5), 1u << (pre & 31));
-                events += static_cast<unsigned long long>(p.row_ptr[pre + 1] - p.row_ptr[pre]);
+                mark_spikes(bm, pre, lane);
             }
             // Per-thread counts: reduce over the warp, then the block.
 #pragma unroll

@@ -122,6 +122,17 @@ __device__ __forceinline__ uint32_t resolve_sources(
     return total;
 }
 
+// Records a warp's spikes (`pre`, or kNoSpike) in a bitmap: neighbouring spikes of an ascending list share
+// words, so the lanes of a word send one atomic. The whole warp calls it.
+constexpr uint32_t kNoSpike = 0xFFFFFFFFu;
+__device__ __forceinline__ void mark_spikes(uint32_t *bm, uint32_t pre, int lane)
+{
+    const uint32_t word = pre >> 5;
+    const uint32_t peers = __match_any_sync(0xffffffffu, word);
+    const uint32_t bits = __reduce_or_sync(peers, pre == kNoSpike ? 0u : 1u << (pre & 31));
+    if (pre != kNoSpike && lane == __ffs(peers) - 1) atomicOr(bm + word, bits);
+}
+
 // Scatters the rows of this step's `total` spikes over warps: this is warp `warp` of `n_warps`.
 // Returns the events (synapses of the rows) this warp started, the same value in every lane.
 template <bool kFixed, bool kUniformExc>
@@ -130,6 +141,53 @@ __device__ __forceinline__ unsigned long long scatter_rows(
     const uint32_t (&cnt)[kMaxSources], uint32_t total, uint32_t warp, uint32_t n_warps, int lane)
 {
     unsigned long long events = 0;
+    if (p.short_rows)
+    {
+        // Rows of a synapse or two (one-to-one drive): a lane per row, so that a warp has 32 rows' chains of
+        // loads in flight instead of one (200k neurons, 60k spikes a step: 41 -> 16 us for the phase with
+        // the bitmap below). A longer row among them is taken by the whole warp.
+        for (uint32_t j0 = 32u * warp; j0 < total; j0 += 32u * n_warps)
+        {
+            uint32_t jj = j0 + lane;
+            int64_t a = 0, b = 0;
+            if (jj < total)
+            {
+                int k = 0;
+                while (jj >= cnt[k])
+                {
+                    jj -= cnt[k];
+                    ++k;
+                }
+                const uint32_t pre = idx[k][jj];
+                if (pre < p.n_rows)
+                {
+                    a = p.row_ptr[pre];
+                    b = p.row_ptr[pre + 1];
+                }
+            }
+            events += static_cast<unsigned long long>(b - a);
+            const bool is_long = b - a > 8;
+            if (!is_long)
+                for (int64_t e = a; e < b; ++e)
+                {
+                    const int ty = kUniformExc ? 0 : (p.type ? __ldg(p.type + e) : p.uniform_type);
+                    deliver<kFixed, kUniformExc>(p, slot_base, e, __ldg(p.col + e), p.w[e], __ldg(p.delay + e), ty);
+                }
+            for (uint32_t m = __ballot_sync(0xffffffffu, is_long); m; m &= m - 1u)
+            {
+                const int src = __ffs(m) - 1;
+                const int64_t la = __shfl_sync(0xffffffffu, a, src), lb = __shfl_sync(0xffffffffu, b, src);
+                for (int64_t e = la + lane; e < lb; e += 32)
+                {
+                    const int ty = kUniformExc ? 0 : (p.type ? __ldg(p.type + e) : p.uniform_type);
+                    deliver<kFixed, kUniformExc>(p, slot_base, e, __ldg(p.col + e), p.w[e], __ldg(p.delay + e), ty);
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) events += __shfl_xor_sync(0xffffffffu, events, o);
+        return events;
+    }
     // Each row is split over F warps (warp f of a row takes its 128-synapse rounds f, f + F, ...), so
     // that one long row does not serialise the step and the rows' parts spread evenly over the warps:
     // about four parts per warp (with whole rows, 1.25 rows per warp would leave a quarter of the warps

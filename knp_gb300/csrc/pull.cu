@@ -202,7 +202,9 @@ size_t gather_smem_bytes(const PullDev &p, int grid) { return gather_smem_for(p,
 void launch_gather(const ProjectionDev &p, Control *ctl, int grid, cudaStream_t s)
 {
     const size_t smem = gather_smem_bytes(p.pull, grid);
-    if (p.pull.wtab)
+    if (p.pull.wtab && p.pull.tab_rep)
+        launch_pdl(gather_kernel<kDictRep>, dim3(grid), dim3(kGatherThreads), smem, s, p, ctl);
+    else if (p.pull.wtab)
         launch_pdl(gather_kernel<kDict>, dim3(grid), dim3(kGatherThreads), smem, s, p, ctl);
     else if (p.pull.w16)
         launch_pdl(gather_kernel<kHalf>, dim3(grid), dim3(kGatherThreads), smem, s, p, ctl);
@@ -214,6 +216,8 @@ cudaError_t set_gather_smem(size_t bytes)
 {
     const int b = static_cast<int>(bytes);
     cudaError_t err = cudaFuncSetAttribute(gather_kernel<kDict>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (err == cudaSuccess)
+        err = cudaFuncSetAttribute(gather_kernel<kDictRep>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (err == cudaSuccess)
         err = cudaFuncSetAttribute(gather_kernel<kHalf>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (err == cudaSuccess)

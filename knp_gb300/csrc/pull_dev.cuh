@@ -39,18 +39,46 @@ constexpr uint32_t kPrefetchAhead = 16;
 
 enum WeightForm
 {
-    kDict = 0,  // 8-bit dictionary index in the top bits of the packed entry
-    kHalf = 1,  // FP16
-    kFull = 2,  // FP32
+    kDict = 0,     // 8-bit dictionary index in the top bits of the packed entry
+    kHalf = 1,     // FP16
+    kFull = 2,     // FP32
+    kDictRep = 3,  // as kDict, with 32 copies of the dictionary in shared memory (PullDev::tab_rep)
 };
 
 
-// Shared memory of one gather block: the step's spike bitmap, the accumulators of the block's
+// The gather's work is cut over G blocks in units of (window, delay), window-major: block `block` takes units
+// [u0, u1), so that the blocks' shares are equal to within one unit, and for each delay a run of windows that
+// differs by one at either end at most. (Without split_delays: whole windows.) A window cut between two
+// blocks is summed by both.
+struct GatherShare
+{
+    uint32_t D, u0, u1;
+    __host__ __device__ GatherShare(const PullDev &p, uint32_t block, uint32_t G)
+        : D(p.split_delays ? p.max_delay : 1u),
+          u0(static_cast<uint32_t>(static_cast<uint64_t>(block) * p.n_windows * D / G)),
+          u1(static_cast<uint32_t>(static_cast<uint64_t>(block + 1) * p.n_windows * D / G))
+    {
+    }
+    // First window of delay d (1 ..) at or after unit u.
+    __device__ uint32_t window_at(uint32_t u, uint32_t d) const
+    {
+        const uint32_t r = D > 1u ? d - 1u : 0u;
+        return u > r ? (u - r + D - 1u) / D : 0u;
+    }
+    __device__ uint32_t first_window() const { return u0 / D; }
+};
+
+// Largest number of windows that a block's share touches.
+__host__ __device__ inline uint32_t gather_windows(const PullDev &p, uint32_t G)
+{
+    return (p.n_windows + G - 1) / G + (p.split_delays ? 1u : 0u);
+}
+
+// Shared memory of one gather block: the spike bitmaps of n_bm steps, the accumulators of the block's
 // windows and (dictionary weights) 32 replicas of the dictionary.
 __host__ __device__ inline size_t gather_smem_for(const PullDev &p, uint32_t G)
 {
-    const uint64_t windows_per_block = (p.n_windows + G - 1) / G;
-    return static_cast<size_t>(p.words) * 4 + windows_per_block * kPullWindow * 4 +
+    return static_cast<size_t>(p.n_bm) * p.words * 4 + static_cast<size_t>(gather_windows(p, G)) * kPullWindow * 4 +
            (p.tab_rep ? static_cast<size_t>(p.n_tab) * 32 * 4 : 0);
 }
 
@@ -76,84 +104,126 @@ __device__ __forceinline__ void clear_bitmap_slot(const PullDev &g, unsigned lon
 // Block `block` of G gather blocks completes the input of step tn (every thread of the block calls
 // it; it contains block barriers), and clears its share of the bitmap slot that step tn's spikes
 // will be recorded in. smem_u4: gather_smem_for(p.pull, G) bytes of dynamic shared memory.
+//
+// The delays are walked in groups of n_bm, whose bitmaps are in shared memory together: the slices of a group
+// are handed out from one pool, so that the block's 32 warps wait for one another once per group. (One
+// delay at a time, a block of 200k neurons' gather had 48 slices a delay for 32 warps, half a round of idle
+// warps at each of 20 barriers, and 5 or 6 whole windows a block: 271 us a step at a third of the neurons
+// firing, against 218 us. Loading the next round's entries during the current one gave 226 us at 8 entries
+// a round and 253 at 16, 64 registers being too few for both.)
 template <int kForm>
 __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned long long tn, uint32_t block, uint32_t G,
                                              uint4 *smem_u4)
 {
-    __shared__ uint32_t s_next;  // next slice of the current delay to hand out
+    __shared__ uint32_t s_next;  // next slice of the current group to hand out
     __shared__ float s_tab[256];
     __shared__ uint8_t s_pflag[256];  // pulled flag of step tn - d, d = 1 .. max_delay (max_delay <= 255)
+    // The group's delays, its slices before each, and the first window of each.
+    __shared__ uint32_t s_delay[kGatherBitmaps], s_before[kGatherBitmaps + 1], s_window[kGatherBitmaps];
     const PullDev &g = p.pull;
-    uint32_t *bm = reinterpret_cast<uint32_t *>(smem_u4);
-    float *acc = reinterpret_cast<float *>(bm + g.words);
-    float *rep = acc + static_cast<size_t>((g.n_windows + G - 1) / G) * kPullWindow;  // after the largest acc
+    uint32_t *bm0 = reinterpret_cast<uint32_t *>(smem_u4);
+    float *acc = reinterpret_cast<float *>(bm0 + static_cast<size_t>(g.n_bm) * g.words);
+    float *rep = acc + static_cast<size_t>(gather_windows(g, G)) * kPullWindow;  // after the largest acc
+    if (kForm == kDictRep)
+        for (uint32_t i = threadIdx.x; i < g.n_tab * 32u; i += blockDim.x) rep[i] = g.wtab[i >> 5];
     if (kForm == kDict)
-    {
-        if (g.tab_rep)
-            for (uint32_t i = threadIdx.x; i < g.n_tab * 32u; i += blockDim.x) rep[i] = g.wtab[i >> 5];
-        else
-            for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab[i] = g.wtab[i];
-    }
-    const uint32_t w0 = static_cast<uint32_t>(static_cast<uint64_t>(block) * g.n_windows / G);
-    const uint32_t w1 = static_cast<uint32_t>(static_cast<uint64_t>(block + 1) * g.n_windows / G);
-    const uint32_t n_acc = (w1 - w0) * kPullWindow;
+        for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab[i] = g.wtab[i];
+    const GatherShare share(g, block, G);
+    const uint32_t w0 = share.first_window(), w_end = (share.u1 + share.D - 1) / share.D;
+    const uint32_t n_acc = share.u1 > share.u0 ? (w_end - w0) * kPullWindow : 0u;
     const int lane = threadIdx.x & 31;
     for (uint32_t d = 1 + threadIdx.x; d <= g.max_delay; d += blockDim.x)
         s_pflag[d] = d <= tn ? static_cast<uint8_t>(g.pulled[static_cast<uint32_t>((tn - d) % g.hist_slots)]) : 0;
+    for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x) acc[i] = 0.0f;
     __syncthreads();
 
     bool any = false;
-    for (uint32_t d = 1; d <= g.max_delay && d <= tn; ++d)
+    uint32_t d_next = 1;  // the first delay not yet in a group; the same in every thread
+    while (n_acc)
     {
-        const unsigned long long s = tn - d;
-        const uint32_t sl = static_cast<uint32_t>(s % g.hist_slots);
-        const uint32_t pflag = s_pflag[d];
-        if (!pflag) continue;
-        const bool all = pflag == 2u;  // every presynaptic neuron fired at step s: no bitmap needed
-        if (!any)
+        // The next n_bm delays whose step was pulled.
+        uint32_t n_in = 0, delays[kGatherBitmaps];
+#pragma unroll
+        for (uint32_t k = 0; k < kGatherBitmaps; ++k)
         {
-            for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x) acc[i] = 0.0f;
-            any = true;
+            if (k >= g.n_bm) break;
+            while (d_next <= g.max_delay && !s_pflag[d_next]) ++d_next;
+            if (d_next > g.max_delay) break;
+            delays[k] = d_next++;
+            n_in = k + 1;
         }
-        __syncthreads();  // the previous bitmap is no longer read
-        if (!all)
+        if (!n_in) break;
+        any = true;
+        __syncthreads();  // the previous group's bitmaps and tables are no longer read
+        if (threadIdx.x == 0)
         {
+            s_next = 0;
+            uint32_t before = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kGatherBitmaps; ++k)
+            {
+                if (k >= n_in) break;
+                const uint32_t wa = share.window_at(share.u0, delays[k]), wb = share.window_at(share.u1, delays[k]);
+                s_delay[k] = delays[k];
+                s_window[k] = wa;
+                s_before[k] = before;
+                before += (wb - wa) * kPullSlicesPerWindow;
+            }
+            s_before[n_in] = before;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kGatherBitmaps; ++k)
+        {
+            if (k >= n_in) break;
+            if (s_pflag[delays[k]] == 2u) continue;  // every presynaptic neuron fired: no bitmap needed
+            const uint32_t sl = static_cast<uint32_t>((tn - delays[k]) % g.hist_slots);
             const uint4 *src = reinterpret_cast<const uint4 *>(g.bitmap + static_cast<size_t>(sl) * g.words);
-            for (uint32_t i = threadIdx.x; i < g.words / 4; i += blockDim.x) smem_u4[i] = src[i];
+            uint4 *dst = smem_u4 + static_cast<size_t>(k) * (g.words / 4);
+            for (uint32_t i = threadIdx.x; i < g.words / 4; i += blockDim.x) dst[i] = src[i];
         }
-        if (threadIdx.x == 0) s_next = 0;
         __syncthreads();
-        const size_t q0 = (static_cast<size_t>(d - 1) * g.n_windows + w0) * kPullSlicesPerWindow;
-        const uint32_t n_q = (w1 - w0) * kPullSlicesPerWindow;
+        const uint32_t n_q = s_before[n_in];
+        // Index in the layout of slice qi of the group, which is one of its k-th delay's.
+        auto slice_at = [&](uint32_t qi, uint32_t k) -> size_t
+        {
+            return (static_cast<size_t>(s_delay[k] - 1) * g.n_windows + s_window[k]) * kPullSlicesPerWindow +
+                   (qi - s_before[k]);
+        };
+        uint32_t in_group = 0;  // the delay of this warp's slice: slices are handed out in order
         // Slices are handed out one at a time (lists differ in length: longest first within a window).
         for (;;)
         {
             uint32_t qi = 0;
             if (lane == 0) qi = atomicAdd(&s_next, 1u);
             qi = __shfl_sync(0xffffffffu, qi, 0);
-            if (qi >= n_q)
+            if (qi >= n_q) break;
+            while (qi >= s_before[in_group + 1]) ++in_group;
+            const size_t q = slice_at(qi, in_group);
+            if (lane == 0)
             {
-                // The first kPrefetchAhead warps to run out prefetch the first slices of the next
-                // delay (those no earlier slice's prefetch covered).
-                const uint32_t r = qi - n_q;
-                if (lane == 0 && r < kPrefetchAhead && r < n_q && d < g.max_delay && d < tn &&
-                    g.pulled[static_cast<uint32_t>((tn - d - 1) % g.hist_slots)])
+                // Ask L2 for the slice kPrefetchAhead further on; at the end of the group, for the first
+                // ones of the next pulled delay.
+                const uint32_t ahead = qi + kPrefetchAhead;
+                size_t qa = q + kPrefetchAhead;
+                bool ask = ahead < s_before[in_group + 1];
+                if (!ask)
                 {
-                    const size_t qa = (static_cast<size_t>(d) * g.n_windows + w0) * kPullSlicesPerWindow + r;
-                    const uint32_t la = g.slice_len[qa];
-                    if (la)
+                    if (ahead < n_q)
                     {
-                        prefetch_l2(g.packed + g.slice_ptr[qa], la * kPullSlice * 4u);
-                        if (kForm == kHalf) prefetch_l2(g.w16 + g.slice_ptr[qa], la * kPullSlice * 2u);
-                        if (kForm == kFull) prefetch_l2(g.w + g.slice_ptr[qa], la * kPullSlice * 4u);
+                        uint32_t k = in_group + 1;
+                        while (ahead >= s_before[k + 1]) ++k;
+                        qa = slice_at(ahead, k);
+                        ask = true;
+                    }
+                    else if (d_next <= g.max_delay && s_pflag[d_next])
+                    {
+                        const uint32_t r = ahead - n_q;
+                        const uint32_t wa = share.window_at(share.u0, d_next), wb = share.window_at(share.u1, d_next);
+                        qa = (static_cast<size_t>(d_next - 1) * g.n_windows + wa) * kPullSlicesPerWindow + r;
+                        ask = r < (wb - wa) * kPullSlicesPerWindow;
                     }
                 }
-                break;
-            }
-            if (lane == 0 && qi + kPrefetchAhead < n_q)
-            {
-                const size_t qa = q0 + qi + kPrefetchAhead;
-                const uint32_t la = g.slice_len[qa];
+                const uint32_t la = ask ? g.slice_len[qa] : 0u;
                 if (la)
                 {
                     // Slices start on 32-entry boundaries; one slice is len x 32 entries.
@@ -162,33 +232,35 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
                     if (kForm == kFull) prefetch_l2(g.w + g.slice_ptr[qa], la * kPullSlice * 4u);
                 }
             }
-            const size_t q = q0 + qi;
+            const bool all = s_pflag[s_delay[in_group]] == 2u;
+            const uint32_t *bm = bm0 + static_cast<size_t>(in_group) * g.words;
+            const uint32_t window = s_window[in_group] + (qi - s_before[in_group]) / kPullSlicesPerWindow;
             const uint32_t len = g.slice_len[q];
             if (len == 0) continue;
             // Entry k of this lane's list is at slice_ptr + 32 k + lane (a warp load reads 128
-            // consecutive bytes). Full rounds of kDepth entries run without bounds checks; an absent
-            // spike adds +0.0, which leaves the sum unchanged (the sum is never -0.0: it starts at
-            // +0.0 and a round-to-nearest sum is -0.0 only if both terms are).
+            // consecutive bytes).
             const long long off = g.slice_ptr[q] + lane;
             const uint32_t *pk = g.packed + off;
             const uint16_t *ph = kForm == kHalf ? g.w16 + off : nullptr;
             const float *pf = kForm == kFull ? g.w + off : nullptr;
+            const float *rep_lane = rep + lane;
             // Two copies of the walk: with the bit test, and without it for a step in which every
             // presynaptic neuron fired (the test would always pass).
             auto walk = [&](auto all_tag) -> float
             {
                 constexpr bool kAll = decltype(all_tag)::value;
-                auto value = [&](uint32_t pn, float wi) -> float
-                {
-                    if (kForm == kDict)
-                    {
-                        wi = g.tab_rep ? rep[((pn >> 24) << 5) + lane] : s_tab[pn >> 24];
-                        pn &= 0xFFFFFFu;
-                    }
-                    if (kAll) return wi;
-                    return ((bm[pn >> 5] >> (pn & 31)) & 1u) ? wi : 0.0f;
-                };
                 float sum = 0.0f;
+                // One entry: its weight, and (the shift takes its amount modulo 32) its presynaptic bit.
+                auto take = [&](uint32_t pn, float wi)
+                {
+                    if (kForm == kDictRep) wi = rep_lane[(pn >> 24) * 32u];
+                    if (kForm == kDict) wi = s_tab[pn >> 24];
+                    if (kAll)
+                        sum = __fadd_rn(sum, wi);
+                    else if (__funnelshift_r(bm[(pn >> 5) & 0x7FFFFu], 0u, pn) & 1u)
+                        sum = __fadd_rn(sum, wi);
+                };
+                // Rounds of kDepth entries, the rest in rounds of 4 (len is the same in every lane).
                 uint32_t k0 = 0;
                 for (; k0 + kDepth <= len; k0 += kDepth)
                 {
@@ -204,15 +276,15 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
                         if (kForm == kFull) w[i] = __ldcs(pf + o + i * kPullSlice);
                     }
 #pragma unroll
-                    for (int i = 0; i < kDepth; ++i) sum = __fadd_rn(sum, value(pre[i], w[i]));
+                    for (int i = 0; i < kDepth; ++i) take(pre[i], w[i]);
                 }
-                if (k0 < len)
+                for (; k0 < len; k0 += 4)
                 {
                     const size_t o = static_cast<size_t>(k0) * kPullSlice;
-                    uint32_t pre[kDepth];
-                    float w[kDepth];
+                    uint32_t pre[4];
+                    float w[4];
 #pragma unroll
-                    for (int i = 0; i < kDepth; ++i)
+                    for (int i = 0; i < 4; ++i)
                     {
                         pre[i] = 0u;
                         w[i] = 0.0f;
@@ -224,15 +296,16 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < kDepth; ++i)
-                        if (k0 + i < len) sum = __fadd_rn(sum, value(pre[i], w[i]));
+                    for (int i = 0; i < 4; ++i)
+                        if (k0 + i < len) take(pre[i], w[i]);
                 }
                 return sum;
             };
             const float sum = all ? walk(std::true_type{}) : walk(std::false_type{});
-            // This lane's target: one owner per (delay, target), so a plain add.
+            // This lane's target. Another warp may hold it for another delay of the group: an atomic add (the
+            // sums are exact in any order).
             const uint32_t t = g.perm[q * kPullSlice + lane];
-            if (sum != 0.0f) acc[(qi / kPullSlicesPerWindow) * kPullWindow + t] += sum;
+            if (sum != 0.0f) atomicAdd(&acc[(window - w0) * kPullWindow + t], sum);
         }
     }
     __syncthreads();
@@ -243,7 +316,7 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
         for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x)
         {
             const uint32_t j = w0 * kPullWindow + i;
-            if (j < g.n_post && acc[i] != 0.0f) ring[j] = __fadd_rn(ring[j], acc[i]);
+            if (j < g.n_post && acc[i] != 0.0f) atomicAdd(ring + j, acc[i]);  // a window may be another block's too
         }
     }
     clear_bitmap_slot(g, tn, block, G);
