@@ -1251,7 +1251,7 @@ void Backend::build_pull(ProjectionSlot &p)
     const size_t smem = gather_smem_bytes(g, grid);
     int smem_max = 0;
     KNP_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-    if (smem > static_cast<size_t>(smem_max)) return;
+    if (smem + kGatherStaticSmem > static_cast<size_t>(smem_max)) return;
     size_t free_b = 0, total_b = 0;
     KNP_CUDA(cudaMemGetInfo(&free_b, &total_b));
     if (free_b < p.n_syn * 36 + static_cast<size_t>(p.max_delay) * post->n * 16 + (1ull << 30)) return;
@@ -1264,7 +1264,7 @@ void Backend::build_pull(ProjectionSlot &p)
     g.pulled = arena_.make<uint32_t>(g.hist_slots);
     g.threshold = static_cast<uint32_t>(std::max(1.0, std::ceil(p.pull_fraction * p.n_rows)));
     // 32 copies of the weight dictionary (one per bank) when shared memory has room for them.
-    if (g.wtab && smem + static_cast<size_t>(g.n_tab) * 32 * 4 + 2048 <= static_cast<size_t>(smem_max)) g.tab_rep = 1;
+    if (g.wtab && smem + static_cast<size_t>(g.n_tab) * 32 * 4 + kGatherStaticSmem <= static_cast<size_t>(smem_max)) g.tab_rep = 1;
     // Shares cut between delays, then as many bitmaps at a time as fit beside the kernels' static shared memory.
     g.split_delays = static_cast<uint64_t>(g.n_windows) * g.max_delay < 0xFFFFFFFFull ? 1 : 0;
     if (g.split_delays && gather_smem_bytes(g, grid) + 8192 > static_cast<size_t>(smem_max)) g.split_delays = 0;

@@ -268,6 +268,7 @@ constexpr int kPullWindow = 256;
 constexpr int kPullSlice = 32;
 constexpr int kPullSlicesPerWindow = kPullWindow / kPullSlice;
 constexpr uint32_t kGatherBitmaps = 8;
+constexpr uint32_t kGatherStaticSmem = 2048;  // bytes beside gather_smem_for's, at most
 
 struct PullDev
 {

@@ -52,20 +52,23 @@ enum WeightForm
 // blocks is summed by both.
 struct GatherShare
 {
-    uint32_t D, u0, u1;
+    uint32_t u0, u1, q0, r0, q1, r1;  // u = q D + r
+    GatherShare() = default;
     __host__ __device__ GatherShare(const PullDev &p, uint32_t block, uint32_t G)
-        : D(p.split_delays ? p.max_delay : 1u),
-          u0(static_cast<uint32_t>(static_cast<uint64_t>(block) * p.n_windows * D / G)),
-          u1(static_cast<uint32_t>(static_cast<uint64_t>(block + 1) * p.n_windows * D / G))
     {
+        const uint32_t D = p.split_delays ? p.max_delay : 1u;
+        u0 = static_cast<uint32_t>(static_cast<uint64_t>(block) * p.n_windows * D / G);
+        u1 = static_cast<uint32_t>(static_cast<uint64_t>(block + 1) * p.n_windows * D / G);
+        q0 = u0 / D;
+        r0 = u0 % D;
+        q1 = u1 / D;
+        r1 = u1 % D;
     }
-    // First window of delay d (1 ..) at or after unit u.
-    __device__ uint32_t window_at(uint32_t u, uint32_t d) const
-    {
-        const uint32_t r = D > 1u ? d - 1u : 0u;
-        return u > r ? (u - r + D - 1u) / D : 0u;
-    }
-    __device__ uint32_t first_window() const { return u0 / D; }
+    // The block's windows of delay d (1 ..): [first(d), last(d)); unit (w, d) is w D + d - 1. Whole windows have
+    // r = 0. Of all delays: [q0, end()).
+    __device__ uint32_t first(uint32_t d) const { return q0 + (r0 >= d ? 1u : 0u); }
+    __device__ uint32_t last(uint32_t d) const { return q1 + (r1 >= d ? 1u : 0u); }
+    __device__ uint32_t end() const { return q1 + (r1 ? 1u : 0u); }
 };
 
 // Largest number of windows that a block's share touches.
@@ -101,6 +104,31 @@ __device__ __forceinline__ void clear_bitmap_slot(const PullDev &g, unsigned lon
     for (uint32_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) dst[i] = 0u;
 }
 
+// Static shared memory of a gather block (one copy, whichever weight form runs).
+struct GatherTables
+{
+    // The descriptor: the gather's loops write memory, so the compiler reads the fields they use again for every
+    // slice. (From a descriptor in global memory, as the whole-step kernel has it, 226 us a step against 218 for
+    // 200k neurons of which a third fire, and 710 against 699 for 10^6 that all fire.)
+    alignas(16) uint32_t desc[sizeof(PullDev) / 4];
+    GatherShare share;
+    uint8_t pflag[256];  // pulled flag of step tn - d, d = 1 .. max_delay (max_delay <= 255)
+    // The group's delays, its slices before each, and the first window of each; their number; the first pulled
+    // delay after them, its first slice of this block in the layout (of the delay) and its number of them. (One thread's work: in every thread's registers it made the slices' loop spill, 237 us
+    // against 218 and 720 against 676.)
+    uint32_t delay[kGatherBitmaps], before[kGatherBitmaps + 1], window[kGatherBitmaps];
+    uint32_t n_group, delay_next, q_next, slices_next;
+    uint32_t next;  // next slice of the current group to hand out
+};
+static_assert(sizeof(GatherTables) + 256 * sizeof(float) <= kGatherStaticSmem, "reserved beside the dynamic part");
+static_assert(sizeof(PullDev) % 4 == 0, "copied by words");
+
+__device__ __forceinline__ GatherTables &gather_tables()
+{
+    __shared__ GatherTables tables;
+    return tables;
+}
+
 // Block `block` of G gather blocks completes the input of step tn (every thread of the block calls
 // it; it contains block barriers), and clears its share of the bitmap slot that step tn's spikes
 // will be recorded in. smem_u4: gather_smem_for(p.pull, G) bytes of dynamic shared memory.
@@ -115,112 +143,126 @@ template <int kForm>
 __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned long long tn, uint32_t block, uint32_t G,
                                              uint4 *smem_u4)
 {
-    __shared__ uint32_t s_next;  // next slice of the current group to hand out
-    __shared__ float s_tab[256];
-    __shared__ uint8_t s_pflag[256];  // pulled flag of step tn - d, d = 1 .. max_delay (max_delay <= 255)
-    // The group's delays, its slices before each, and the first window of each.
-    __shared__ uint32_t s_delay[kGatherBitmaps], s_before[kGatherBitmaps + 1], s_window[kGatherBitmaps];
-    const PullDev &g = p.pull;
+    __shared__ float s_dict[256];  // kDict only
+    GatherTables &tab = gather_tables();
+    for (uint32_t i = threadIdx.x; i < sizeof(PullDev) / 4; i += blockDim.x)
+        tab.desc[i] = reinterpret_cast<const uint32_t *>(&p.pull)[i];
+    __syncthreads();
+    const PullDev &g = *reinterpret_cast<const PullDev *>(tab.desc);
     uint32_t *bm0 = reinterpret_cast<uint32_t *>(smem_u4);
     float *acc = reinterpret_cast<float *>(bm0 + static_cast<size_t>(g.n_bm) * g.words);
     float *rep = acc + static_cast<size_t>(gather_windows(g, G)) * kPullWindow;  // after the largest acc
     if (kForm == kDictRep)
         for (uint32_t i = threadIdx.x; i < g.n_tab * 32u; i += blockDim.x) rep[i] = g.wtab[i >> 5];
     if (kForm == kDict)
-        for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab[i] = g.wtab[i];
-    const GatherShare share(g, block, G);
-    const uint32_t w0 = share.first_window(), w_end = (share.u1 + share.D - 1) / share.D;
-    const uint32_t n_acc = share.u1 > share.u0 ? (w_end - w0) * kPullWindow : 0u;
+        for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_dict[i] = g.wtab[i];
+    if (threadIdx.x == 0)
+    {
+        tab.share = GatherShare(g, block, G);
+        tab.delay_next = 1;
+    }
     const int lane = threadIdx.x & 31;
     for (uint32_t d = 1 + threadIdx.x; d <= g.max_delay; d += blockDim.x)
-        s_pflag[d] = d <= tn ? static_cast<uint8_t>(g.pulled[static_cast<uint32_t>((tn - d) % g.hist_slots)]) : 0;
-    for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x) acc[i] = 0.0f;
+        tab.pflag[d] = d <= tn ? static_cast<uint8_t>(g.pulled[static_cast<uint32_t>((tn - d) % g.hist_slots)]) : 0;
     __syncthreads();
+    const uint32_t w0 = tab.share.q0;
+    const uint32_t n_acc = tab.share.u1 > tab.share.u0 ? (tab.share.end() - w0) * kPullWindow : 0u;
+    for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x) acc[i] = 0.0f;
 
     bool any = false;
-    uint32_t d_next = 1;  // the first delay not yet in a group; the same in every thread
     while (n_acc)
     {
-        // The next n_bm delays whose step was pulled.
-        uint32_t n_in = 0, delays[kGatherBitmaps];
-#pragma unroll
-        for (uint32_t k = 0; k < kGatherBitmaps; ++k)
-        {
-            if (k >= g.n_bm) break;
-            while (d_next <= g.max_delay && !s_pflag[d_next]) ++d_next;
-            if (d_next > g.max_delay) break;
-            delays[k] = d_next++;
-            n_in = k + 1;
-        }
-        if (!n_in) break;
-        any = true;
         __syncthreads();  // the previous group's bitmaps and tables are no longer read
         if (threadIdx.x == 0)
         {
-            s_next = 0;
-            uint32_t before = 0;
-#pragma unroll
-            for (uint32_t k = 0; k < kGatherBitmaps; ++k)
+            // The next n_bm delays whose step was pulled.
+            const GatherShare share = tab.share;
+            uint32_t n = 0, before = 0, d = tab.delay_next;
+            for (; d <= g.max_delay && n < g.n_bm; ++d)
             {
-                if (k >= n_in) break;
-                const uint32_t wa = share.window_at(share.u0, delays[k]), wb = share.window_at(share.u1, delays[k]);
-                s_delay[k] = delays[k];
-                s_window[k] = wa;
-                s_before[k] = before;
-                before += (wb - wa) * kPullSlicesPerWindow;
+                if (!tab.pflag[d]) continue;
+                tab.delay[n] = d;
+                tab.window[n] = share.first(d);
+                tab.before[n] = before;
+                before += (share.last(d) - share.first(d)) * kPullSlicesPerWindow;
+                ++n;
             }
-            s_before[n_in] = before;
+            tab.before[n] = before;
+            while (d <= g.max_delay && !tab.pflag[d]) ++d;
+            tab.delay_next = d;
+            tab.q_next = share.first(d) * kPullSlicesPerWindow;
+            tab.slices_next = d <= g.max_delay ? (share.last(d) - share.first(d)) * kPullSlicesPerWindow : 0u;
+            tab.n_group = n;
+            tab.next = 0;
         }
-#pragma unroll
-        for (uint32_t k = 0; k < kGatherBitmaps; ++k)
+        __syncthreads();
+        const uint32_t n_in = tab.n_group;
+        if (!n_in) break;
+        any = true;
+        for (uint32_t k = 0; k < n_in; ++k)
         {
-            if (k >= n_in) break;
-            if (s_pflag[delays[k]] == 2u) continue;  // every presynaptic neuron fired: no bitmap needed
-            const uint32_t sl = static_cast<uint32_t>((tn - delays[k]) % g.hist_slots);
+            const uint32_t d = tab.delay[k];
+            if (tab.pflag[d] == 2u) continue;  // every presynaptic neuron fired: no bitmap needed
+            const uint32_t sl = static_cast<uint32_t>((tn - d) % g.hist_slots);
             const uint4 *src = reinterpret_cast<const uint4 *>(g.bitmap + static_cast<size_t>(sl) * g.words);
             uint4 *dst = smem_u4 + static_cast<size_t>(k) * (g.words / 4);
             for (uint32_t i = threadIdx.x; i < g.words / 4; i += blockDim.x) dst[i] = src[i];
         }
         __syncthreads();
-        const uint32_t n_q = s_before[n_in];
+        const uint32_t n_q = tab.before[n_in];
         // Index in the layout of slice qi of the group, which is one of its k-th delay's.
         auto slice_at = [&](uint32_t qi, uint32_t k) -> size_t
         {
-            return (static_cast<size_t>(s_delay[k] - 1) * g.n_windows + s_window[k]) * kPullSlicesPerWindow +
-                   (qi - s_before[k]);
+            return (static_cast<size_t>(tab.delay[k] - 1) * g.n_windows + tab.window[k]) * kPullSlicesPerWindow +
+                   (qi - tab.before[k]);
         };
-        uint32_t in_group = 0;  // the delay of this warp's slice: slices are handed out in order
+        // The delay of this warp's slice (slices are handed out in order), kept in registers until it changes:
+        // its place in the group, its slices in the pool, its first slice in the layout, its first window's
+        // accumulators and its bitmap.
+        uint32_t in_group = 0, before = 0, end = 0;
+        size_t q_first = 0;
+        float *acc_first = acc;
+        const uint32_t *bm = bm0;
+        bool all = false;
         // Slices are handed out one at a time (lists differ in length: longest first within a window).
         for (;;)
         {
             uint32_t qi = 0;
-            if (lane == 0) qi = atomicAdd(&s_next, 1u);
+            if (lane == 0) qi = atomicAdd(&tab.next, 1u);
             qi = __shfl_sync(0xffffffffu, qi, 0);
             if (qi >= n_q) break;
-            while (qi >= s_before[in_group + 1]) ++in_group;
-            const size_t q = slice_at(qi, in_group);
+            if (qi >= end)
+            {
+                while (qi >= tab.before[in_group + 1]) ++in_group;
+                before = tab.before[in_group];
+                end = tab.before[in_group + 1];
+                q_first = slice_at(before, in_group);
+                acc_first = acc + static_cast<size_t>(tab.window[in_group] - w0) * kPullWindow;
+                bm = bm0 + static_cast<size_t>(in_group) * g.words;
+                all = tab.pflag[tab.delay[in_group]] == 2u;
+            }
+            const size_t q = q_first + (qi - before);
             if (lane == 0)
             {
                 // Ask L2 for the slice kPrefetchAhead further on; at the end of the group, for the first
                 // ones of the next pulled delay.
                 const uint32_t ahead = qi + kPrefetchAhead;
                 size_t qa = q + kPrefetchAhead;
-                bool ask = ahead < s_before[in_group + 1];
+                bool ask = ahead < end;
                 if (!ask)
                 {
                     if (ahead < n_q)
                     {
                         uint32_t k = in_group + 1;
-                        while (ahead >= s_before[k + 1]) ++k;
+                        while (ahead >= tab.before[k + 1]) ++k;
                         qa = slice_at(ahead, k);
                         ask = true;
                     }
-                    else if (d_next <= g.max_delay && s_pflag[d_next])
+                    else if (ahead - n_q < tab.slices_next)
                     {
-                        const uint32_t r = ahead - n_q;
-                        const uint32_t wa = share.window_at(share.u0, d_next), wb = share.window_at(share.u1, d_next);
-                        qa = (static_cast<size_t>(d_next - 1) * g.n_windows + wa) * kPullSlicesPerWindow + r;
-                        ask = r < (wb - wa) * kPullSlicesPerWindow;
+                        qa = static_cast<size_t>(tab.delay_next - 1) * g.n_windows * kPullSlicesPerWindow + tab.q_next +
+                             (ahead - n_q);
+                        ask = true;
                     }
                 }
                 const uint32_t la = ask ? g.slice_len[qa] : 0u;
@@ -232,9 +274,6 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
                     if (kForm == kFull) prefetch_l2(g.w + g.slice_ptr[qa], la * kPullSlice * 4u);
                 }
             }
-            const bool all = s_pflag[s_delay[in_group]] == 2u;
-            const uint32_t *bm = bm0 + static_cast<size_t>(in_group) * g.words;
-            const uint32_t window = s_window[in_group] + (qi - s_before[in_group]) / kPullSlicesPerWindow;
             const uint32_t len = g.slice_len[q];
             if (len == 0) continue;
             // Entry k of this lane's list is at slice_ptr + 32 k + lane (a warp load reads 128
@@ -244,6 +283,10 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
             const uint16_t *ph = kForm == kHalf ? g.w16 + off : nullptr;
             const float *pf = kForm == kFull ? g.w + off : nullptr;
             const float *rep_lane = rep + lane;
+            // This lane's target, read before the walk (after it, one more trip to memory in turn: 748 us for 10^6
+            // that all fire, against 699). Where the group has several delays, another warp may hold it for another of
+            // them (the sums are exact in any order).
+            float *mine = acc_first + (qi - before) / kPullSlicesPerWindow * kPullWindow + g.perm[q * kPullSlice + lane];
             // Two copies of the walk: with the bit test, and without it for a step in which every
             // presynaptic neuron fired (the test would always pass).
             auto walk = [&](auto all_tag) -> float
@@ -254,58 +297,56 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
                 auto take = [&](uint32_t pn, float wi)
                 {
                     if (kForm == kDictRep) wi = rep_lane[(pn >> 24) * 32u];
-                    if (kForm == kDict) wi = s_tab[pn >> 24];
+                    if (kForm == kDict) wi = s_dict[pn >> 24];
                     if (kAll)
                         sum = __fadd_rn(sum, wi);
                     else if (__funnelshift_r(bm[(pn >> 5) & 0x7FFFFu], 0u, pn) & 1u)
                         sum = __fadd_rn(sum, wi);
                 };
-                // Rounds of kDepth entries, the rest in rounds of 4 (len is the same in every lane).
-                uint32_t k0 = 0;
-                for (; k0 + kDepth <= len; k0 += kDepth)
+                // Entries k0 .. k0 + kN - 1 in one round of loads; kTail leaves out those past the list's end.
+                auto round = [&](auto n_tag, auto tail_tag, uint32_t k0)
                 {
+                    constexpr int kN = decltype(n_tag)::value;
+                    constexpr bool kTail = decltype(tail_tag)::value;
                     const size_t o = static_cast<size_t>(k0) * kPullSlice;
-                    uint32_t pre[kDepth];
-                    float w[kDepth];
+                    uint32_t pre[kN];
+                    float w[kN];
 #pragma unroll
-                    for (int i = 0; i < kDepth; ++i)
+                    for (int i = 0; i < kN; ++i)
                     {
-                        pre[i] = __ldcs(pk + o + i * kPullSlice);
+                        pre[i] = 0u;
                         w[i] = 0.0f;
+                        if (kTail && k0 + i >= len) continue;
+                        pre[i] = __ldcs(pk + o + i * kPullSlice);
                         if (kForm == kHalf) w[i] = __half2float(__ushort_as_half(__ldcs(ph + o + i * kPullSlice)));
                         if (kForm == kFull) w[i] = __ldcs(pf + o + i * kPullSlice);
                     }
 #pragma unroll
-                    for (int i = 0; i < kDepth; ++i) take(pre[i], w[i]);
-                }
-                for (; k0 < len; k0 += 4)
-                {
-                    const size_t o = static_cast<size_t>(k0) * kPullSlice;
-                    uint32_t pre[4];
-                    float w[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                    {
-                        pre[i] = 0u;
-                        w[i] = 0.0f;
-                        if (k0 + i < len)
-                        {
-                            pre[i] = __ldcs(pk + o + i * kPullSlice);
-                            if (kForm == kHalf) w[i] = __half2float(__ushort_as_half(__ldcs(ph + o + i * kPullSlice)));
-                            if (kForm == kFull) w[i] = __ldcs(pf + o + i * kPullSlice);
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (k0 + i < len) take(pre[i], w[i]);
-                }
+                    for (int i = 0; i < kN; ++i)
+                        if (!kTail || k0 + i < len) take(pre[i], w[i]);
+                };
+                // Rounds of kDepth, then the rest in one more round of about its size (len is the same in every
+                // lane): lists of about 10 are one trip to memory, and 50 pay for 2 entries at the end, not 16.
+                uint32_t k0 = 0;
+                for (; k0 + kDepth <= len; k0 += kDepth)
+                    round(std::integral_constant<int, kDepth>{}, std::false_type{}, k0);
+                const uint32_t rest = len - k0;
+                if (rest > 8u)
+                    round(std::integral_constant<int, kDepth>{}, std::true_type{}, k0);
+                else if (rest > 4u)
+                    round(std::integral_constant<int, 8>{}, std::true_type{}, k0);
+                else if (rest)
+                    round(std::integral_constant<int, 4>{}, std::true_type{}, k0);
                 return sum;
             };
             const float sum = all ? walk(std::true_type{}) : walk(std::false_type{});
-            // This lane's target. Another warp may hold it for another delay of the group: an atomic add (the
-            // sums are exact in any order).
-            const uint32_t t = g.perm[q * kPullSlice + lane];
-            if (sum != 0.0f) atomicAdd(&acc[(window - w0) * kPullWindow + t], sum);
+            if (sum != 0.0f)
+            {
+                if (g.n_bm == 1u)
+                    *mine += sum;
+                else
+                    atomicAdd(mine, sum);
+            }
         }
     }
     __syncthreads();
@@ -316,7 +357,11 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
         for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x)
         {
             const uint32_t j = w0 * kPullWindow + i;
-            if (j < g.n_post && acc[i] != 0.0f) atomicAdd(ring + j, acc[i]);  // a window may be another block's too
+            if (j >= g.n_post || acc[i] == 0.0f) continue;
+            if (g.split_delays)
+                atomicAdd(ring + j, acc[i]);  // the window may be another block's too
+            else
+                ring[j] = __fadd_rn(ring[j], acc[i]);
         }
     }
     clear_bitmap_slot(g, tn, block, G);
