@@ -1427,7 +1427,7 @@ void Backend::set_step_mode(int mode)
     step_mode_ = mode;
 }
 
-// The fused kernel is one cluster of at most 8 CTAs: it pays off while a step is a few microseconds
+// The fused kernel is one cluster of at most 16 CTAs: it pays off while a step is a few microseconds
 // of work, and it has no gather form (in AUTO mode a projection with a gather layout keeps the per-phase kernels; the
 // FUSED mode builds no gather layout).
 bool Backend::small_net_eligible(std::string &why) const
@@ -1613,6 +1613,7 @@ void Backend::build_small_net()
         }
         std::vector<ProjectionDev> projs;
         std::vector<SmallStdp> rules;
+        std::vector<SmallSource> sources;
         small_pull_.clear();
         for (auto &p : projs_)
         {
@@ -1624,6 +1625,7 @@ void Backend::build_small_net()
                 {
                     d.src[k].count = cnt(d.src[k].count);
                     d.src[k].idx = list(d.src[k].idx);
+                    sources.push_back({static_cast<uint32_t>(projs.size()), d.src[k]});
                 }
                 projs.push_back(d);
             }
@@ -1648,14 +1650,20 @@ void Backend::build_small_net()
             small_.n_pops = static_cast<uint32_t>(pops.size());
             small_.n_projs = static_cast<uint32_t>(projs.size());
             small_.n_stdp = static_cast<uint32_t>(rules.size());
+            small_.n_sources = static_cast<uint32_t>(sources.size());
+            uint64_t words = 0;
+            for (auto &q : pops_) words += (static_cast<uint64_t>(q->n) + 3) / 4 * 4;
+            small_.list_words = static_cast<uint32_t>(std::min<uint64_t>(words, 0xFFFFFFFFu));
             SmallPop *dp = arena_.make<SmallPop>(2 * std::max<size_t>(pops.size(), 1));
             ProjectionDev *dj = arena_.make<ProjectionDev>(2 * std::max<size_t>(projs.size(), 1));
             SmallStdp *ds = arena_.make<SmallStdp>(2 * std::max<size_t>(rules.size(), 1));
+            SmallSource *dq = arena_.make<SmallSource>(2 * std::max<size_t>(sources.size(), 1));
             for (int k = 0; k < 2; ++k)
             {
                 small_.pops[k] = dp + k * std::max<size_t>(pops.size(), 1);
                 small_.projs[k] = dj + k * std::max<size_t>(projs.size(), 1);
                 small_.stdp[k] = ds + k * std::max<size_t>(rules.size(), 1);
+                small_.sources[k] = dq + k * std::max<size_t>(sources.size(), 1);
             }
         }
         small_.end[set] = StepEnd{base, n_counters_, n_spike_counters_};
@@ -1665,6 +1673,8 @@ void Backend::build_small_net()
                             projs.size() * sizeof(ProjectionDev), cudaMemcpyHostToDevice));
         KNP_CUDA(cudaMemcpy(const_cast<SmallStdp *>(small_.stdp[set]), rules.data(), rules.size() * sizeof(SmallStdp),
                             cudaMemcpyHostToDevice));
+        KNP_CUDA(cudaMemcpy(const_cast<SmallSource *>(small_.sources[set]), sources.data(),
+                            sources.size() * sizeof(SmallSource), cudaMemcpyHostToDevice));
     }
 }
 

@@ -368,6 +368,12 @@ struct SmallStdp
     SpikeSource src[kMaxSources];
     int both[kMaxSources];  // the source fills both histories (STDPAndSpike)
 };
+// One spike source of a projection with sources.
+struct SmallSource
+{
+    uint32_t proj;  // index into SmallNet::projs
+    SpikeSource src;
+};
 // Two descriptor sets that differ only in their per-step counters (spike counts, STDP touched
 // counts) and population spike lists: step t uses set t & 1, so step t - 1's STDP rules can read its
 // spikes, and its counters can be zeroed, while step t runs; a step needs no end-of-step phase. Set 0
@@ -377,7 +383,9 @@ struct SmallNet
     const SmallPop *pops[2];
     const ProjectionDev *projs[2];
     const SmallStdp *stdp[2];
-    uint32_t n_pops, n_projs, n_stdp;
+    const SmallSource *sources[2];  // of all projections, in their order
+    uint32_t n_pops, n_projs, n_stdp, n_sources;
+    uint32_t list_words;  // of all populations' spike lists, each padded to 4
     StepEnd end[2];
 };
 
@@ -410,7 +418,7 @@ void launch_stdp_append(const StdpDev &d, SpikeSource src, int both_lists, Contr
 void launch_stdp_modify(const StdpDev &d, Control *ctl, cudaStream_t s);
 void launch_step_end(const StepEnd &e, Control *ctl, cudaStream_t s);
 // Runs n_steps whole steps of a small network in one launch of one cluster of `cluster` CTAs
-// (advances Control::step). small_net_cluster() is the largest cluster size (8, 4, 2 or 1) the
+// (advances Control::step). small_net_cluster() is the largest cluster size (16, 8, 4, 2 or 1) the
 // device can schedule for it.
 int small_net_cluster();
 cudaError_t launch_small_net(const SmallNet &net, Control *ctl, uint32_t n_steps, int cluster, cudaStream_t s);

@@ -25,12 +25,29 @@ namespace
 __device__ __forceinline__ float pf(const ParamF &p, uint32_t i) { return p.a ? p.a[i] : p.u; }
 __device__ __forceinline__ uint32_t pu(const ParamU &p, uint32_t i) { return p.a ? p.a[i] : p.u; }
 
-__device__ __forceinline__ float4 ld4(const float *p, uint32_t i) { return *reinterpret_cast<const float4 *>(p + i); }
-__device__ __forceinline__ void st4(float *p, uint32_t i, float4 v) { *reinterpret_cast<float4 *>(p + i) = v; }
-__device__ __forceinline__ uint4 ld4u(const uint32_t *p, uint32_t i) { return *reinterpret_cast<const uint4 *>(p + i); }
-__device__ __forceinline__ void st4u(uint32_t *p, uint32_t i, uint4 v) { *reinterpret_cast<uint4 *>(p + i) = v; }
-__device__ __forceinline__ float &at(float4 &v, int k) { return reinterpret_cast<float *>(&v)[k]; }
-__device__ __forceinline__ uint32_t &at(uint4 &v, int k) { return reinterpret_cast<uint32_t *>(&v)[k]; }
+// State of a thread's kN consecutive neurons (4, or 1 in small networks), moved as one 4 kN-byte word.
+template <int kN>
+struct alignas(4 * kN) FloatN
+{
+    float v[kN];
+};
+template <int kN>
+struct alignas(4 * kN) UintN
+{
+    uint32_t v[kN];
+};
+template <int kN>
+__device__ __forceinline__ FloatN<kN> ldf(const float *p, size_t i) { return *reinterpret_cast<const FloatN<kN> *>(p + i); }
+template <int kN>
+__device__ __forceinline__ void stf(float *p, size_t i, FloatN<kN> v) { *reinterpret_cast<FloatN<kN> *>(p + i) = v; }
+template <int kN>
+__device__ __forceinline__ UintN<kN> ldu(const uint32_t *p, size_t i) { return *reinterpret_cast<const UintN<kN> *>(p + i); }
+template <int kN>
+__device__ __forceinline__ void stu(uint32_t *p, size_t i, UintN<kN> v) { *reinterpret_cast<UintN<kN> *>(p + i) = v; }
+template <int kN>
+__device__ __forceinline__ float &at(FloatN<kN> &v, int k) { return v.v[k]; }
+template <int kN>
+__device__ __forceinline__ uint32_t &at(UintN<kN> &v, int k) { return v.v[k]; }
 
 // Append this thread's spikes (bit k of mask = neuron i0 + k) to list[*count ...] with one atomic
 // per block; indexes stay ascending within a block. With a recording slot `rec` (rec_words words),
@@ -87,10 +104,16 @@ __device__ __forceinline__ void emit_spikes(
         if (mask & (1u << k)) list[pos++] = i0 + k;
 }
 
+// t % slots (the 64-bit remainder is a call of a hundred instructions and more).
+__device__ __forceinline__ uint32_t step_slot(unsigned long long t, uint32_t slots)
+{
+    return t >> 32 ? static_cast<uint32_t>(t % slots) : static_cast<uint32_t>(t) % slots;
+}
+
 __device__ __forceinline__ uint32_t *record_slot(uint32_t *rec_bits, uint32_t rec_words, uint32_t rec_slots,
                                                  unsigned long long t)
 {
-    return rec_bits ? rec_bits + static_cast<size_t>(t % rec_slots) * rec_words : nullptr;
+    return rec_bits ? rec_bits + static_cast<size_t>(step_slot(t, rec_slots)) * rec_words : nullptr;
 }
 
 struct NeuronState
@@ -342,60 +365,68 @@ __device__ __forceinline__ void resource_mark(const BlifatDev &p, uint32_t i, un
     if (need) p.syn.work[atomicAdd(p.syn.work_count, 1u)] = i;
 }
 
-// Steps neurons i0 .. i0 + 3 of a BLIFAT population (those below n) at step t and returns their spike
+// Steps neurons i0 .. i0 + kN - 1 of a BLIFAT population (those below n) at step t and returns their spike
 // mask (bit k = neuron i0 + k fired).
-template <bool kFixed, bool kRS = false>
+template <bool kFixed, bool kRS = false, int kN = 4>
 __device__ __forceinline__ uint32_t blifat_quad(const BlifatDev &p, unsigned long long t, uint32_t i0)
 {
+    static_assert(kN == 4 || !kRS, "the non-finite impacts' bytes are cleared a word at a time");
     const uint32_t f = p.flags;
     uint32_t mask = 0;
     if (i0 < p.n)
     {
         const RingView &rg = p.ring;
-        const uint32_t slot = static_cast<uint32_t>(t % rg.slots);
+        const uint32_t slot = step_slot(t, rg.slots);
         const size_t ro = static_cast<size_t>(slot) * rg.pitch + i0;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        long long acc_hi[4] = {0, 0, 0, 0}, acc_lo[4] = {0, 0, 0, 0};
-        if (kFixed)
+        FloatN<kN> acc = FloatN<kN>{};
+        long long acc_hi[kN] = {}, acc_lo[kN] = {};
+        if (kFixed && kN == 1)
+        {
+            acc_hi[0] = rg.v64[ro];
+            acc_lo[0] = rg.v64lo[ro];
+            rg.v64[ro] = rg.v64lo[ro] = 0;
+        }
+        else if (kFixed)
         {
             longlong2 *a = reinterpret_cast<longlong2 *>(rg.v64 + ro);
             longlong2 *b = reinterpret_cast<longlong2 *>(rg.v64lo + ro);
             const longlong2 x = a[0], y = a[1], xl = b[0], yl = b[1];
             acc_hi[0] = x.x;
-            acc_hi[1] = x.y;
-            acc_hi[2] = y.x;
-            acc_hi[3] = y.y;
+            acc_hi[1 % kN] = x.y;
+            acc_hi[2 % kN] = y.x;
+            acc_hi[3 % kN] = y.y;
             acc_lo[0] = xl.x;
-            acc_lo[1] = xl.y;
-            acc_lo[2] = yl.x;
-            acc_lo[3] = yl.y;
+            acc_lo[1 % kN] = xl.y;
+            acc_lo[2 % kN] = yl.x;
+            acc_lo[3 % kN] = yl.y;
             a[0] = a[1] = b[0] = b[1] = make_longlong2(0, 0);
         }
         else
         {
-            acc = ld4(rg.v32, ro);
-            st4(rg.v32, ro, make_float4(0.f, 0.f, 0.f, 0.f));
+            acc = ldf<kN>(rg.v32, ro);
+            stf<kN>(rg.v32, ro, FloatN<kN>{});
         }
-        float4 gin = make_float4(0.f, 0.f, 0.f, 0.f), din = gin;
+        FloatN<kN> gin = FloatN<kN>{}, din = gin;
         if (rg.g)
         {
-            gin = ld4(rg.g, ro);
-            st4(rg.g, ro, make_float4(0.f, 0.f, 0.f, 0.f));
+            gin = ldf<kN>(rg.g, ro);
+            stf<kN>(rg.g, ro, FloatN<kN>{});
         }
         if (rg.dopa)
         {
-            din = ld4(rg.dopa, ro);
-            st4(rg.dopa, ro, make_float4(0.f, 0.f, 0.f, 0.f));
+            din = ldf<kN>(rg.dopa, ro);
+            stf<kN>(rg.dopa, ro, FloatN<kN>{});
         }
         uint32_t forced_bits = 0;
         if (rg.forced)
         {
             uint32_t *wp = rg.forced + static_cast<size_t>(slot) * rg.words + (i0 >> 5);
-            forced_bits = (*wp >> (i0 & 31)) & 0xFu;
-            if (forced_bits) atomicAnd(wp, ~(0xFu << (i0 & 31)));
+            constexpr uint32_t kMask = (1u << kN) - 1;
+            forced_bits = (*wp >> (i0 & 31)) & kMask;
+            if (forced_bits) atomicAnd(wp, ~(kMask << (i0 & 31)));
         }
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 V = (kRS || (f & kLiveVRead)) ? ld4(p.V, i0) : z;
+        const FloatN<kN> z = FloatN<kN>{};
+        FloatN<kN> V = (kRS || (f & kLiveVRead)) ? ldf<kN>(p.V, i0) : z;
         uint32_t nf_bits = 0;  // kRS: the four neurons' non-finite impact bytes
         if (kRS && rg.nf)
         {
@@ -403,18 +434,18 @@ __device__ __forceinline__ uint32_t blifat_quad(const BlifatDev &p, unsigned lon
             nf_bits = *wp;
             if (nf_bits) *wp = 0u;
         }
-        float4 thr_dyn = (f & kLiveThrDyn) ? ld4(p.thr_dyn, i0) : z;
-        float4 trace = (f & kLiveTrace) ? ld4(p.trace, i0) : z;
-        float4 g = (f & kLiveG) ? ld4(p.g, i0) : z;
-        float4 dopa = ((f & kLiveDopa) && !(f & kResource)) ? ld4(p.dopa, i0) : z;
-        float4 add_thr = (f & kLiveAddThr) ? ld4(p.add_thr, i0) : z;
-        uint4 ns = (f & kLiveRefract) ? ld4u(p.n_since, i0) : make_uint4(0, 0, 0, 0);
-        uint4 phase = (f & kLiveBurst) ? ld4u(p.burst_phase, i0) : make_uint4(0, 0, 0, 0);
-        float4 vpre;
-        const uint4 ns_old = ns;
+        FloatN<kN> thr_dyn = (f & kLiveThrDyn) ? ldf<kN>(p.thr_dyn, i0) : z;
+        FloatN<kN> trace = (f & kLiveTrace) ? ldf<kN>(p.trace, i0) : z;
+        FloatN<kN> g = (f & kLiveG) ? ldf<kN>(p.g, i0) : z;
+        FloatN<kN> dopa = ((f & kLiveDopa) && !(f & kResource)) ? ldf<kN>(p.dopa, i0) : z;
+        FloatN<kN> add_thr = (f & kLiveAddThr) ? ldf<kN>(p.add_thr, i0) : z;
+        UintN<kN> ns = (f & kLiveRefract) ? ldu<kN>(p.n_since, i0) : UintN<kN>{};
+        UintN<kN> phase = (f & kLiveBurst) ? ldu<kN>(p.burst_phase, i0) : UintN<kN>{};
+        FloatN<kN> vpre;
+        const UintN<kN> ns_old = ns;
         uint32_t dopamine_due = 0;  // neurons whose dopamine stability change follows the loop
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < kN; ++k)
         {
             const uint32_t i = i0 + k;
             if (i >= p.n) break;
@@ -461,24 +492,24 @@ __device__ __forceinline__ uint32_t blifat_quad(const BlifatDev &p, unsigned lon
             if (f & kLiveBlock) p.blocking[i] = s.block;
         }
         // Padding lanes beyond n write their (unused) slots too; the arrays are padded to n_pad.
-        st4(p.V, i0, V);
-        if (f & kLiveVPre) st4(p.V_pre, i0, vpre);
-        if (f & kLiveThrDyn) st4(p.thr_dyn, i0, thr_dyn);
-        if (f & kLiveTrace) st4(p.trace, i0, trace);
-        if (f & kLiveG) st4(p.g, i0, g);
-        if ((f & kLiveDopa) || (f & kResource)) st4(p.dopa, i0, dopa);
-        if ((f & kLiveAddThr) || (f & kResource)) st4(p.add_thr, i0, add_thr);
+        stf<kN>(p.V, i0, V);
+        if (f & kLiveVPre) stf<kN>(p.V_pre, i0, vpre);
+        if (f & kLiveThrDyn) stf<kN>(p.thr_dyn, i0, thr_dyn);
+        if (f & kLiveTrace) stf<kN>(p.trace, i0, trace);
+        if (f & kLiveG) stf<kN>(p.g, i0, g);
+        if ((f & kLiveDopa) || (f & kResource)) stf<kN>(p.dopa, i0, dopa);
+        if ((f & kLiveAddThr) || (f & kResource)) stf<kN>(p.add_thr, i0, add_thr);
         if (f & kLiveRefract)
-            st4u(p.n_since, i0, ns);
+            stu<kN>(p.n_since, i0, ns);
         else if (mask)
         {
             // Lazy refractory tracking: record the step of the last spike.
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < kN; ++k)
                 if (mask & (1u << k)) p.n_since[i0 + k] = at(ns, k);
         }
         (void)ns_old;
-        if (f & kLiveBurst) st4u(p.burst_phase, i0, phase);
+        if (f & kLiveBurst) stu<kN>(p.burst_phase, i0, phase);
         for (; dopamine_due; dopamine_due &= dopamine_due - 1)
         {
             const uint32_t k = __ffs(dopamine_due) - 1, i = i0 + k;
@@ -497,19 +528,20 @@ __device__ __forceinline__ uint32_t blifat_quad(const BlifatDev &p, unsigned lon
 // FP32 input ring. blifat_step then reduces to: the potential is +0 plus this step's input sum, a
 // spike iff the step is not step 0 and the potential reaches the threshold, the reset, and the
 // min-potential clamp; the same operations in the same order, so results are identical.
+template <int kN = 4>
 __device__ __forceinline__ uint32_t blifat_quad_lean(const BlifatDev &p, unsigned long long t, uint32_t i0)
 {
     uint32_t mask = 0;
     if (i0 < p.n)
     {
         const RingView &rg = p.ring;
-        const uint32_t slot = static_cast<uint32_t>(t % rg.slots);
+        const uint32_t slot = step_slot(t, rg.slots);
         const size_t ro = static_cast<size_t>(slot) * rg.pitch + i0;
-        float4 acc = ld4(rg.v32, ro);
-        st4(rg.v32, ro, make_float4(0.f, 0.f, 0.f, 0.f));
-        float4 V = make_float4(0.f, 0.f, 0.f, 0.f);
+        FloatN<kN> acc = ldf<kN>(rg.v32, ro);
+        stf<kN>(rg.v32, ro, FloatN<kN>{});
+        FloatN<kN> V = FloatN<kN>{};
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < kN; ++k)
         {
             const uint32_t i = i0 + k;
             if (i >= p.n) break;
@@ -525,18 +557,19 @@ __device__ __forceinline__ uint32_t blifat_quad_lean(const BlifatDev &p, unsigne
             if (v < vmin) v = vmin;
             at(V, k) = v;
         }
-        st4(p.V, i0, V);
+        stf<kN>(p.V, i0, V);
     }
     return mask;
 }
 
 // The BLIFAT quad step of any plain population (no resource-STDP synapses) for the fused and grid
 // kernels.
+template <int kN = 4>
 __device__ __forceinline__ uint32_t blifat_quad_any(const BlifatDev &p, unsigned long long t, uint32_t i0)
 {
-    if (p.ring.fixed) return blifat_quad<true>(p, t, i0);
-    if (p.flags == 0u) return blifat_quad_lean(p, t, i0);
-    return blifat_quad<false>(p, t, i0);
+    if (p.ring.fixed) return blifat_quad<true, false, kN>(p, t, i0);
+    if (p.flags == 0u) return blifat_quad_lean<kN>(p, t, i0);
+    return blifat_quad<false, false, kN>(p, t, i0);
 }
 
 // AltAI-LIF neurons i0 .. i0 + 3 (altai_impl.h:33-168) at step t; returns their spike mask. The
@@ -551,7 +584,7 @@ __device__ __forceinline__ uint32_t altai_quad(const AltaiDev &p, unsigned long 
     uint32_t mask = 0;
     if (i0 >= p.n) return 0;
     const RingView &rg = p.ring;
-    const uint32_t slot = static_cast<uint32_t>(t % rg.slots);
+    const uint32_t slot = step_slot(t, rg.slots);
     const size_t ro = static_cast<size_t>(slot) * rg.pitch + i0;
     uint32_t forced_bits = 0;
     if (rg.forced)
@@ -681,20 +714,21 @@ __device__ __forceinline__ uint32_t altai_quad(const AltaiDev &p, unsigned long 
     return mask;
 }
 
+template <int kN = 4>
 __device__ __forceinline__ uint32_t lif_quad(const LifDev &p, unsigned long long t, uint32_t i0)
 {
     uint32_t mask = 0;
     if (i0 < p.n)
     {
         const RingView &rg = p.ring;
-        const uint32_t slot = static_cast<uint32_t>(t % rg.slots);
+        const uint32_t slot = step_slot(t, rg.slots);
         const size_t ro = static_cast<size_t>(slot) * rg.pitch + i0;
-        float4 acc = ld4(rg.v32, ro);
-        st4(rg.v32, ro, make_float4(0.f, 0.f, 0.f, 0.f));
-        float4 V = ld4(p.V, i0);
-        uint4 rc = ld4u(p.refract, i0);
+        FloatN<kN> acc = ldf<kN>(rg.v32, ro);
+        stf<kN>(rg.v32, ro, FloatN<kN>{});
+        FloatN<kN> V = ldf<kN>(p.V, i0);
+        UintN<kN> rc = ldu<kN>(p.refract, i0);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < kN; ++k)
         {
             const uint32_t i = i0 + k;
             if (i >= p.n) break;
@@ -719,8 +753,8 @@ __device__ __forceinline__ uint32_t lif_quad(const LifDev &p, unsigned long long
             at(V, k) = v;
             at(rc, k) = r;
         }
-        st4(p.V, i0, V);
-        st4u(p.refract, i0, rc);
+        stf<kN>(p.V, i0, V);
+        stu<kN>(p.refract, i0, rc);
     }
     return mask;
 }
