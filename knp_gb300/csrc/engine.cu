@@ -1680,6 +1680,17 @@ void Backend::build_small_net()
 
 // ------------------------------------------------------------------------------------ stepping
 
+uint32_t Backend::train_blocks(const PopulationSlot &q) const
+{
+    return static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((q.n + 7) / 8, 4ull * sm_count_)));
+}
+
+TrainView Backend::train_view(const PopulationSlot &q)
+{
+    if (q.is_altai()) return {q.adev.res, q.adev.syn, q.adev.dopa, q.adev.spikes, q.adev.spike_count};
+    return {q.bdev.res, q.bdev.syn, q.bdev.dopa, q.bdev.spikes, q.bdev.spike_count};
+}
+
 // One population's step: its kernel, then (resource-STDP populations with resource-STDP synapses)
 // the training that ends the population's step in the reference (populations_old.h:207-209).
 void Backend::launch_population(const PopulationSlot &q)
@@ -1695,38 +1706,78 @@ void Backend::launch_population(const PopulationSlot &q)
         launch_altai(q.adev, ctl_, stream_);
         if (q.adev.flags & kResource)
         {
-            const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((q.n + 7) / 8, 4ull * sm_count_));
-            const TrainView v{q.adev.res, q.adev.syn, q.adev.dopa, q.adev.spikes, q.adev.spike_count};
-            launch_resource_train(v, static_cast<int>(blocks), ctl_, stream_);
+            launch_resource_train(train_view(q), static_cast<int>(train_blocks(q)), ctl_, stream_);
         }
         return;
     }
     launch_blifat(q.bdev, ctl_, stream_);
     if (q.bdev.flags & kResSyn)
+        launch_resource_train(train_view(q), static_cast<int>(train_blocks(q)), ctl_, stream_);
+}
+
+// The populations' steps. A BLIFAT population of no more than a block's neurons for every SM leaves the device
+// mostly idle and its launch is its time: such ones share a launch, and so does their training after it. (The
+// populations of a step do not read one another.)
+void Backend::launch_populations()
+{
+    const uint32_t small = 256u * static_cast<uint32_t>(sm_count_);
+    BlifatBatch steps{};
+    TrainBatch trains{};
+    auto flush = [&]
     {
-        const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((q.n + 7) / 8, 4ull * sm_count_));
-        const TrainView v{q.bdev.res, q.bdev.syn, q.bdev.dopa, q.bdev.spikes, q.bdev.spike_count};
-        launch_resource_train(v, static_cast<int>(blocks), ctl_, stream_);
+        if (steps.n) launch_blifat_batch(steps, ctl_, stream_);
+        if (trains.n) launch_train_batch(trains, ctl_, stream_);
+        steps = {};
+        trains = {};
+    };
+    for (auto &q : pops_)
+    {
+        if (q->kind == KNP_NEURON_LIF || q->is_altai() || q->n > small || q->n == 0)
+        {
+            launch_population(*q);
+            continue;
+        }
+        steps.add(q->bdev, blifat_batch_blocks(q->n));
+        if (q->bdev.flags & kResSyn) trains.add(train_view(*q), train_blocks(*q));
+        if (steps.n == BlifatBatch::kCapacity) flush();
     }
+    flush();
+}
+
+// The projections' steps, and the gathers. Projections of few rows share launches, as populations do.
+void Backend::launch_projections()
+{
+    ProjectionBatch few{};
+    auto flush = [&]
+    {
+        if (few.n == 1)
+            launch_projection(few.item[0], ctl_, static_cast<int>(few.blocks()), stream_);
+        else if (few.n)
+            launch_projection_batch(few, ctl_, stream_);
+        few = {};
+    };
+    for (auto &p : projs_)
+    {
+        if (p->dev.n_src == 0) continue;
+        const uint64_t bound = static_cast<uint64_t>(p->dev.n_src) * p->n_rows;
+        const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((bound + 7) / 8, 8ull * sm_count_));
+        if (blocks > 2ull * sm_count_)
+        {
+            launch_projection(p->dev, ctl_, static_cast<int>(blocks), stream_);
+            continue;
+        }
+        few.add(p->dev, static_cast<uint32_t>(blocks));
+        if (few.n == ProjectionBatch::kCapacity) flush();
+    }
+    flush();
+    for (auto &p : projs_)
+        if (p->pull) launch_gather(p->dev, ctl_, gather_grid(*p), stream_);
 }
 
 void Backend::enqueue_step()
 {
-    for (auto &q : pops_) launch_population(*q);
-    for (auto &p : projs_)
-    {
-        if (p->dev.n_src == 0) continue;
-        uint64_t bound = 0;
-        for (int k = 0; k < p->dev.n_src; ++k)
-        {
-            const SpikeSource &s = p->dev.src[k];
-            bound += s.channel ? p->n_rows : p->n_rows;
-        }
-        const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((bound + 7) / 8, 8ull * sm_count_));
-        launch_projection(p->dev, ctl_, static_cast<int>(blocks), stream_);
-    }
-    for (auto &p : projs_)
-        if (p->pull) launch_gather(p->dev, ctl_, gather_grid(*p), stream_);
+    launch_populations();
+    launch_projections();
     for (auto &p : projs_)
     {
         if (p->kind != KNP_SYNAPSE_ADDITIVE_STDP_DELTA || p->n_syn == 0 || p->stdp_sources.empty()) continue;
@@ -2003,17 +2054,9 @@ void Backend::profile_phases(uint64_t n, float *ms)
     {
         if (any_recording_ && steps_before_drain() == 0) drain_recordings();
         KNP_CUDA(cudaEventRecord(ev[0], stream_));
-        for (auto &q : pops_) launch_population(*q);
+        launch_populations();
         KNP_CUDA(cudaEventRecord(ev[1], stream_));
-        for (auto &p : projs_)
-        {
-            if (p->dev.n_src == 0) continue;
-            const uint64_t bound = static_cast<uint64_t>(p->dev.n_src) * p->n_rows;
-            const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((bound + 7) / 8, 8ull * sm_count_));
-            launch_projection(p->dev, ctl_, static_cast<int>(blocks), stream_);
-        }
-        for (auto &p : projs_)
-            if (p->pull) launch_gather(p->dev, ctl_, gather_grid(*p), stream_);
+        launch_projections();
         KNP_CUDA(cudaEventRecord(ev[2], stream_));
         for (auto &p : projs_)
         {

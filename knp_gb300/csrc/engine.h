@@ -311,6 +311,10 @@ private:
     void wire();
     void enqueue_step();
     void launch_population(const PopulationSlot &q);
+    void launch_populations();
+    void launch_projections();
+    uint32_t train_blocks(const PopulationSlot &q) const;
+    static TrainView train_view(const PopulationSlot &q);
     bool small_net_eligible(std::string &why) const;
     bool grid_net_eligible(std::string &why);
     void build_small_net();

@@ -404,8 +404,41 @@ struct GridNet
     uint32_t pull[kMaxGridPull];
 };
 
+// Descriptors that one launch takes, each for blocks of its own.
+template <typename T, int kMax>
+struct Batch
+{
+    static constexpr int kCapacity = kMax;
+    T item[kMax];
+    uint32_t first[kMax + 1];  // item k has the blocks first[k] .. first[k + 1] - 1
+    uint32_t n;
+    void add(const T &t, uint32_t blocks)
+    {
+        if (n == 0) first[0] = 0;
+        item[n] = t;
+        first[n + 1] = first[n] + blocks;
+        ++n;
+    }
+    uint32_t blocks() const { return n ? first[n] : 0; }
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t of_block(uint32_t block) const
+    {
+        uint32_t k = 0;
+        while (k + 1 < n && block >= first[k + 1]) ++k;
+        return k;
+    }
+#endif
+};
+using ProjectionBatch = Batch<ProjectionDev, 8>;
+using BlifatBatch = Batch<BlifatDev, 4>;
+using TrainBatch = Batch<TrainView, 4>;
+
 // ---------------------------------------------------------------- launchers (stream-ordered)
 void launch_blifat(const BlifatDev &p, Control *ctl, cudaStream_t s);
+uint32_t blifat_batch_blocks(uint32_t n);  // blocks of a population of n in a batch
+void launch_blifat_batch(const BlifatBatch &b, Control *ctl, cudaStream_t s);
+void launch_train_batch(const TrainBatch &b, Control *ctl, cudaStream_t s);
+void launch_projection_batch(const ProjectionBatch &b, Control *ctl, cudaStream_t s);
 void launch_resource_train(const TrainView &p, int blocks, Control *ctl, cudaStream_t s);
 void launch_altai(const AltaiDev &p, Control *ctl, cudaStream_t s);
 void launch_altai_blocking(const AltaiDev &p, Control *ctl, cudaStream_t s);

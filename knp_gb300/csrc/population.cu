@@ -25,6 +25,19 @@ __global__ void __launch_bounds__(kBlock, 3) blifat_kernel(BlifatDev p, Control 
                         p.rec_words);
 }
 
+// Several small populations in one launch, a neuron a thread (the chain of a neuron's operations is what their
+// step takes; four in turn take twice as long and more).
+__global__ void __launch_bounds__(kBlock, 3) blifat_batch_kernel(const __grid_constant__ BlifatBatch b, Control *ctl)
+{
+    pdl_begin();
+    const unsigned long long t = ctl->step;
+    const uint32_t k = b.of_block(blockIdx.x);
+    const BlifatDev &p = b.item[k];
+    const uint32_t i = (blockIdx.x - b.first[k]) * kBlock + threadIdx.x;
+    const uint32_t mask = p.flags & kResSyn ? blifat_quad<true, true, 1>(p, t, i) : blifat_quad_any<1>(p, t, i);
+    emit_warp(mask, i, p.spikes, p.spike_count, record_slot(p.rec_bits, p.rec_words, p.rec_slots, t), p.rec_words);
+}
+
 __global__ void __launch_bounds__(kBlock) lif_kernel(LifDev p, Control *ctl)
 {
     pdl_begin();
@@ -186,6 +199,13 @@ void launch_blifat(const BlifatDev &p, Control *ctl, cudaStream_t s)
         launch_pdl(blifat_kernel<true, false>, dim3(grid), dim3(kBlock), 0, s, p, ctl);
     else
         launch_pdl(blifat_kernel<false, false>, dim3(grid), dim3(kBlock), 0, s, p, ctl);
+}
+
+uint32_t blifat_batch_blocks(uint32_t n) { return (n + kBlock - 1) / kBlock; }
+
+void launch_blifat_batch(const BlifatBatch &b, Control *ctl, cudaStream_t s)
+{
+    launch_pdl(blifat_batch_kernel, dim3(b.blocks()), dim3(kBlock), 0, s, b, ctl);
 }
 
 void launch_altai(const AltaiDev &p, Control *ctl, cudaStream_t s)

@@ -116,6 +116,21 @@ __device__ __forceinline__ uint32_t *record_slot(uint32_t *rec_bits, uint32_t re
     return rec_bits ? rec_bits + static_cast<size_t>(step_slot(t, rec_slots)) * rec_words : nullptr;
 }
 
+// emit_spikes for a thread a neuron (i0 = 32 k + lane): a warp's spikes are one word of the bitmap, and one atomic
+// reserves their place in the list; the whole warp calls it.
+__device__ __forceinline__ void emit_warp(uint32_t mask, uint32_t i0, uint32_t *list, uint32_t *count, uint32_t *rec,
+                                          uint32_t rec_words)
+{
+    const uint32_t lane = threadIdx.x & 31, word = i0 >> 5;
+    const uint32_t fired = __ballot_sync(0xffffffffu, mask != 0);
+    if (rec && lane == 0 && word < rec_words) rec[word] = fired;
+    if (!fired) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, static_cast<uint32_t>(__popc(fired)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (mask) list[base + __popc(fired & ((1u << lane) - 1u))] = i0;
+}
+
 struct NeuronState
 {
     float V, V_pre, thr_dyn, trace, g, dopa, add_thr;
@@ -370,7 +385,6 @@ __device__ __forceinline__ void resource_mark(const BlifatDev &p, uint32_t i, un
 template <bool kFixed, bool kRS = false, int kN = 4>
 __device__ __forceinline__ uint32_t blifat_quad(const BlifatDev &p, unsigned long long t, uint32_t i0)
 {
-    static_assert(kN == 4 || !kRS, "the non-finite impacts' bytes are cleared a word at a time");
     const uint32_t f = p.flags;
     uint32_t mask = 0;
     if (i0 < p.n)
@@ -427,8 +441,14 @@ __device__ __forceinline__ uint32_t blifat_quad(const BlifatDev &p, unsigned lon
         }
         const FloatN<kN> z = FloatN<kN>{};
         FloatN<kN> V = (kRS || (f & kLiveVRead)) ? ldf<kN>(p.V, i0) : z;
-        uint32_t nf_bits = 0;  // kRS: the four neurons' non-finite impact bytes
-        if (kRS && rg.nf)
+        uint32_t nf_bits = 0;  // kRS: the neurons' non-finite impact bytes
+        if (kRS && rg.nf && kN == 1)
+        {
+            uint8_t *bp = reinterpret_cast<uint8_t *>(rg.nf) + ro;
+            nf_bits = *bp;
+            if (nf_bits) *bp = 0u;
+        }
+        else if (kRS && rg.nf)
         {
             uint32_t *wp = rg.nf + (ro >> 2);
             nf_bits = *wp;

@@ -199,14 +199,12 @@ __device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long 
     }
 }
 
-__global__ void __launch_bounds__(kTrainThreads) resource_train_kernel(TrainView p, Control *ctl)
+__device__ __forceinline__ void train_block(const TrainView &p, unsigned long long t, uint32_t block, uint32_t n_blocks)
 {
-    pdl_begin();
-    const unsigned long long t = ctl->step;
     const uint32_t n_spk = *p.spike_count, n_work = *p.syn.work_count;
     const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t warp = (block * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t n_warps = (n_blocks * blockDim.x) >> 5;
     for (uint32_t j = warp; j < n_spk + n_work; j += n_warps)
     {
         const bool spiked = j < n_spk;
@@ -214,11 +212,30 @@ __global__ void __launch_bounds__(kTrainThreads) resource_train_kernel(TrainView
     }
 }
 
+__global__ void __launch_bounds__(kTrainThreads) resource_train_kernel(TrainView p, Control *ctl)
+{
+    pdl_begin();
+    train_block(p, ctl->step, blockIdx.x, gridDim.x);
+}
+
+// Several populations' training in one launch.
+__global__ void __launch_bounds__(kTrainThreads) train_batch_kernel(const __grid_constant__ TrainBatch b, Control *ctl)
+{
+    pdl_begin();
+    const uint32_t k = b.of_block(blockIdx.x);
+    train_block(b.item[k], ctl->step, blockIdx.x - b.first[k], b.first[k + 1] - b.first[k]);
+}
+
 }  // namespace
 
 void launch_resource_train(const TrainView &p, int blocks, Control *ctl, cudaStream_t s)
 {
     launch_pdl(resource_train_kernel, dim3(blocks > 0 ? blocks : 1), dim3(kTrainThreads), 0, s, p, ctl);
+}
+
+void launch_train_batch(const TrainBatch &b, Control *ctl, cudaStream_t s)
+{
+    launch_pdl(train_batch_kernel, dim3(b.blocks()), dim3(kTrainThreads), 0, s, b, ctl);
 }
 
 }  // namespace knp_gb300

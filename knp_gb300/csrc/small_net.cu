@@ -260,18 +260,9 @@ __device__ __forceinline__ void emit(const Pop &p, uint32_t mask, uint32_t i0, u
 {
     uint32_t *rec = record_slot(p.rec_bits, p.rec_words, p.rec_slots, t);
     if (kN == 4)
-    {
         emit_spikes<kSmallThreads>(mask, i0, p.spikes, p.spike_count, rec, p.rec_words);
-        return;
-    }
-    const uint32_t lane = threadIdx.x & 31, word = i0 >> 5;
-    const uint32_t fired = __ballot_sync(0xffffffffu, mask != 0);
-    if (rec && lane == 0 && word < p.rec_words) rec[word] = fired;
-    if (!fired) return;
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(p.spike_count, static_cast<uint32_t>(__popc(fired)));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (mask) p.spikes[base + __popc(fired & ((1u << lane) - 1u))] = i0;
+    else
+        emit_warp(mask, i0, p.spikes, p.spike_count, rec, p.rec_words);
 }
 
 // One population's step t, kN neurons a thread: 1 while the cluster has a thread for every neuron (the chain of
