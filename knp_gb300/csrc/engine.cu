@@ -1265,14 +1265,18 @@ void Backend::build_pull(ProjectionSlot &p)
     g.threshold = static_cast<uint32_t>(std::max(1.0, std::ceil(p.pull_fraction * p.n_rows)));
     // 32 copies of the weight dictionary (one per bank) when shared memory has room for them.
     if (g.wtab && smem + static_cast<size_t>(g.n_tab) * 32 * 4 + kGatherStaticSmem <= static_cast<size_t>(smem_max)) g.tab_rep = 1;
-    // Shares cut between delays, then as many bitmaps at a time as fit beside the kernels' static shared memory.
+    // Shares cut between delays, then as many bitmaps at a time as leave the scatter, which the same kernel runs, an
+    // L1 cache to keep its loads in flight: 200k neurons' gather takes 264, 218, 204, 196, 193 and 193 us a step at
+    // 1, 2, 3, 4, 5 and 8 of them (a third firing), their scatter at half a per cent firing 19.4 us up to 5 and
+    // 30.3 at 8; 400k neurons' 28 us up to 2, 32 at 3, 50 at 4.
+    constexpr size_t kGatherSmemGoal = 160 * 1024;
     g.split_delays = static_cast<uint64_t>(g.n_windows) * g.max_delay < 0xFFFFFFFFull ? 1 : 0;
     if (g.split_delays && gather_smem_bytes(g, grid) + 8192 > static_cast<size_t>(smem_max)) g.split_delays = 0;
     for (uint32_t k = 2; k <= std::min(kGatherBitmaps, g.max_delay); ++k)
     {
         PullDev more = g;
         more.n_bm = k;
-        if (gather_smem_bytes(more, grid) + 8192 <= static_cast<size_t>(smem_max)) g.n_bm = k;
+        if (gather_smem_bytes(more, grid) + kGatherStaticSmem <= std::min<size_t>(kGatherSmemGoal, smem_max)) g.n_bm = k;
     }
     KNP_CUDA(set_gather_smem(std::max<size_t>(gather_smem_bytes(g, grid), 48 * 1024)));
     p.dev.pull = g;
@@ -1485,7 +1489,7 @@ bool Backend::grid_net_eligible(std::string &why)
         why = "the device does not take cooperative launches";
         return false;
     }
-    size_t smem = 0;
+    size_t smem = grid_net_min_smem();
     uint32_t n_pull = 0;
     for (auto &q : pops_)
         if (q->is_altai())

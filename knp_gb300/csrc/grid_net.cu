@@ -34,6 +34,7 @@
 #include "population_dev.cuh"
 #include "projection_dev.cuh"
 #include "pull_dev.cuh"
+#include "scatter_list.cuh"
 #include "stdp_dev.cuh"
 
 namespace knp_gb300
@@ -42,7 +43,7 @@ namespace
 {
 
 constexpr int kGridThreads = kGatherThreads;  // the gather phase is tuned for 32 warps per SM
-constexpr uint32_t kGridWarps = kGridThreads / 32;
+constexpr int kInFlight = 2;  // synapses of the scatter's list a thread loads at a time (64 registers)
 // Longest wait at a barrier: above the longest phase a legitimate step can have (a saturated
 // scatter-only step of 10^9 events takes a few seconds).
 constexpr unsigned long long kBarrierNs = 30000000000ull;  // 30 s
@@ -116,60 +117,53 @@ __device__ __forceinline__ bool pull_window_active(const ProjectionDev &p, unsig
     return need;
 }
 
-// One projection's work of step t over the whole grid: the pull decision and bitmap (gather form),
-// or the scatter of its spike rows. Returns the synaptic events this warp accounted for (the same
-// value in every lane).
-template <bool kFixed, bool kUniformExc>
-__device__ __forceinline__ unsigned long long project(const ProjectionDev &p, unsigned long long t, uint32_t gthread,
-                                                      uint32_t n_threads, uint32_t gwarp, uint32_t n_warps, int lane)
+// A step at or above the threshold of a projection with a gather form is only recorded (as projection_kernel,
+// projection.cu, does; such a projection has one source, a population): its pulled flag, and its spikes' bitmap.
+// Returns the synaptic events this warp accounted for (the same value in every lane).
+__device__ __forceinline__ unsigned long long record_pulled(const ProjectionDev &p, unsigned long long t, uint32_t gthread,
+                                                            uint32_t n_threads, int lane)
 {
-    const uint32_t *idx[kMaxSources];
-    uint32_t cnt[kMaxSources];
-    const uint32_t total = resolve_sources(p, t, idx, cnt);
-    if (p.pull.bitmap)
+    const uint32_t *idx = p.src[0].idx;
+    const uint32_t total = *p.src[0].count;
+    const bool pull = total >= p.pull.threshold;
+    const bool full = pull && p.src[0].n && total >= p.src[0].n;
+    const uint32_t sl = static_cast<uint32_t>(t % p.pull.hist_slots);
+    if (gthread == 0) p.pull.pulled[sl] = pull ? (full ? 2u : 1u) : 0u;
+    if (!pull) return 0;
+    unsigned long long ev = 0;
+    if (full)
     {
-        // As projection_kernel (projection.cu): a step at or above the threshold is only recorded.
-        const bool pull = total >= p.pull.threshold;
-        const bool full = pull && p.n_src == 1 && !p.src[0].channel && p.src[0].n && total >= p.src[0].n;
-        const uint32_t sl = static_cast<uint32_t>(t % p.pull.hist_slots);
-        if (gthread == 0) p.pull.pulled[sl] = pull ? (full ? 2u : 1u) : 0u;
-        if (pull)
+        if (gthread == 0) ev = static_cast<unsigned long long>(p.row_ptr[p.n_rows] - p.row_ptr[0]);
+    }
+    else
+    {
+        uint32_t *bm = p.pull.bitmap + static_cast<size_t>(sl) * p.pull.words;
+        for (uint32_t j0 = gthread - lane; j0 < total; j0 += n_threads)
         {
-            unsigned long long ev = 0;
-            if (full)
-            {
-                if (gthread == 0) ev = static_cast<unsigned long long>(p.row_ptr[p.n_rows] - p.row_ptr[0]);
-            }
+            uint32_t pre = kNoSpike;
+            if (j0 + lane < total) pre = idx[j0 + lane];
+            if (pre < p.n_rows)
+                ev += static_cast<unsigned long long>(p.row_ptr[pre + 1] - p.row_ptr[pre]);
             else
-            {
-                uint32_t *bm = p.pull.bitmap + static_cast<size_t>(sl) * p.pull.words;
-                for (uint32_t j0 = gthread - lane; j0 < total; j0 += n_threads)
-                {
-                    uint32_t jj = j0 + lane, pre = kNoSpike;
-                    if (jj < total)
-                    {
-                        int k = 0;
-                        while (jj >= cnt[k])
-                        {
-                            jj -= cnt[k];
-                            ++k;
-                        }
-                        pre = idx[k][jj];
-                        if (pre < p.n_rows)
-                            ev += static_cast<unsigned long long>(p.row_ptr[pre + 1] - p.row_ptr[pre]);
-                        else
-                            pre = kNoSpike;
-                    }
-                    mark_spikes(bm, pre, lane);
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ev += __shfl_xor_sync(0xffffffffu, ev, o);
-            return ev;
+                pre = kNoSpike;
+            mark_spikes(bm, pre, lane);
         }
     }
-    const uint32_t slot_base = static_cast<uint32_t>(t % p.ring.slots);
-    return scatter_rows<kFixed, kUniformExc>(p, slot_base, idx, cnt, total, gwarp, n_warps, lane);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ev += __shfl_xor_sync(0xffffffffu, ev, o);
+    return ev;
+}
+
+// The projections of step t that are not recorded for a gather. (Within 64 registers: more synapses in flight, or
+// more of a projection's fields in registers, made the gather's loops beside it spill, 703 and 748 us a step for
+// 10^6 neurons that all fire against 690.)
+__device__ __forceinline__ unsigned long long grid_scatter(const ProjectionDev *projs, const SmallSource *sources,
+                                                        uint32_t n_sources, unsigned long long t, uint32_t rank, uint32_t G)
+{
+    extern __shared__ uint4 grid_smem[];
+    return project_rows<kGridThreads, kInFlight, false>(
+        projs, sources, n_sources, t, rank, G, *reinterpret_cast<ScatterTables<kGridThreads> *>(grid_smem),
+        [](const ProjectionDev &p, uint32_t count) { return p.pull.bitmap && count >= p.pull.threshold ? 0u : count; });
 }
 
 __device__ __forceinline__ void retire(const StepEnd &e, uint32_t gthread, uint32_t n_threads, unsigned long long *spikes)
@@ -223,13 +217,18 @@ __device__ __forceinline__ void grid_gather(const ProjectionDev &p, unsigned lon
 
 __global__ void __launch_bounds__(kGridThreads, 1) grid_net_kernel(GridNet g, Control *ctl, uint32_t n_steps)
 {
-    extern __shared__ uint4 grid_smem[];
+    extern __shared__ uint4 grid_smem[];  // the gathers', or the scatter's tables
+    auto &tab = *reinterpret_cast<ScatterTables<kGridThreads> *>(grid_smem);
     __shared__ unsigned long long s_spikes;
     const SmallNet &net = g.net;
     const int lane = threadIdx.x & 31;
     const uint32_t G = gridDim.x;
-    const uint32_t gthread = blockIdx.x * kGridThreads + threadIdx.x, n_threads = G * kGridThreads;
-    const uint32_t gwarp = gthread >> 5, n_warps = G * kGridWarps;
+    // Warps are dealt to the CTAs in turn: what takes some of them (10^4 spikes of a projection of short rows are
+    // 313 warps' work, 2 10^5 neurons 1563's) is then on all SMs. (With a CTA's warps in a row the first CTAs had
+    // all of it: a third of the neurons of 2 10^5 firing, the projections took 16 us, now 13.7; at half a per cent of
+    // 10^6, the first CTA was 14 us behind the others.)
+    const uint32_t n_threads = G * kGridThreads;
+    const uint32_t gwarp = (threadIdx.x >> 5) * G + blockIdx.x, gthread = 32 * gwarp + lane;
     const uint32_t sthread = (gthread + n_threads / 2) % n_threads;
     if (threadIdx.x == 0) s_spikes = 0;
     unsigned long long t = ctl->step;
@@ -255,6 +254,12 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_net_kernel(GridNet g, Co
         const bool odd = t & 1u;
         const SmallPop *pops = odd ? net.pops[1] : net.pops[0];
         const ProjectionDev *projs = odd ? net.projs[1] : net.projs[0];
+        // What the channels send at step t is known already.
+        if (threadIdx.x >= kGridThreads - 32 && lane < static_cast<int>(min(net.n_sources, kSourcesAtATime)))
+        {
+            const SpikeSource &src = (odd ? net.sources[1] : net.sources[0])[lane].src;
+            if (src.channel) resolve_source(src, t, tab.idx[lane], tab.count[lane]);
+        }
         // ---- phase A: populations of step t (a pass covers 4 * n_threads neurons; each CTA compacts
         // its own spikes into the list), STDP rules of step t - 1.
         for (uint32_t k = 0; k < net.n_pops; ++k)
@@ -304,22 +309,11 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_net_kernel(GridNet g, Co
         }
         // ---- phase B: step t - 1's counters are no longer read; projections of step t.
         retire(odd ? net.end[0] : net.end[1], gthread, n_threads, &s_spikes);
-        for (uint32_t k = 0; k < net.n_projs; ++k)
-        {
-            const ProjectionDev &p = projs[k];
-            if (p.n_src == 0) continue;
-            const bool uexc = !p.type && p.uniform_type == 0;
-            if (p.ring.fixed)
-                events += uexc ? project<true, true>(p, t, gthread, n_threads, gwarp, n_warps, lane)
-                               : project<true, false>(p, t, gthread, n_threads, gwarp, n_warps, lane);
-            else
-                events += uexc ? project<false, true>(p, t, gthread, n_threads, gwarp, n_warps, lane)
-                               : project<false, false>(p, t, gthread, n_threads, gwarp, n_warps, lane);
-        }
         // Gathers complete step t + 1's input when a step of their delay window was pulled: every CTA
         // takes the same decision from this step's spike counts (the pulled flag of step t is being
         // written in this phase) and the flags of earlier steps. The bitmap slot step t + 1 fills
         // holds step t - max_delay, which the last gathers (of step t - 1) have read.
+        // (Before the projections: after them these few loads would queue behind their adds.)
         bool need = false;
         for (uint32_t k = 0; k < g.n_pull; ++k)
         {
@@ -328,6 +322,10 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_net_kernel(GridNet g, Co
             need = need || pull_window_active(p, t);
         }
         need = __syncthreads_or(need) != 0;
+        for (uint32_t k = 0; k < g.n_pull; ++k) events += record_pulled(projs[g.pull[k]], t, gthread, n_threads, lane);
+        const unsigned long long ev =
+            grid_scatter(projs, odd ? net.sources[1] : net.sources[0], net.n_sources, t, blockIdx.x, G);
+        if (threadIdx.x == 0) events += ev;
         // The scatter's writes (slots t + 1 .. t + D) are complete before step t + 1's populations
         // read slot t + 1, and the step's bitmaps before the gathers read them.
         target += G;
@@ -404,6 +402,7 @@ int grid_net_ctas(size_t smem)
 }
 
 size_t grid_net_smem(const PullDev &p, int ctas) { return gather_smem_for(p, static_cast<uint32_t>(ctas)); }
+size_t grid_net_min_smem() { return sizeof(ScatterTables<kGridThreads>); }
 
 cudaError_t launch_grid_net(const GridNet &g, Control *ctl, uint32_t n_steps, int ctas, size_t smem,
                             const cudaAccessPolicyWindow *window, cudaStream_t s)

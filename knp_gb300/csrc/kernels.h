@@ -461,6 +461,7 @@ cudaError_t launch_small_net(const SmallNet &net, Control *ctl, uint32_t n_steps
 // needs in it. `window` (may be null): L2 access policy of the launch (persisting input ring).
 int grid_net_ctas(size_t smem);
 size_t grid_net_smem(const PullDev &p, int ctas);
+size_t grid_net_min_smem();  // what its scatter needs
 cudaError_t launch_grid_net(const GridNet &g, Control *ctl, uint32_t n_steps, int ctas, size_t smem,
                             const cudaAccessPolicyWindow *window, cudaStream_t s);
 void launch_gather(const ProjectionDev &p, Control *ctl, int grid, cudaStream_t s);

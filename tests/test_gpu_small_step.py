@@ -1,6 +1,6 @@
-"""The fused step kernel at the edges of its shares: populations around the number of the cluster's threads, more
+"""The fused and the grid step kernel at the edges of their shares: populations around the number of the cluster's threads, more
 rows than the tables hold, more sources than one look resolves, more descriptors than shared memory takes, rows
-too long for the list. Its results are the per-phase kernels', bit for bit: sums are exact in any order (dyadic
+too long for the list. Their results are the per-phase kernels', bit for bit: sums are exact in any order (dyadic
 weights, or the fixed-point ring)."""
 import numpy as np
 import pytest
@@ -17,16 +17,19 @@ def _run(net, sched, steps, mode):
     return got
 
 
-def _same(net, sched, steps):
+def _same(net, sched, steps, modes=None):
     from knp_gb300 import types as T
 
-    (spikes, weights, counts), (ref, ref_w, ref_c) = (_run(net, sched, steps, m) for m in (T.STEP_FUSED, T.STEP_PHASES))
-    assert counts == ref_c and ref_c[1] > 0
-    for a, b in zip(spikes, ref):
-        for t in range(steps):
-            np.testing.assert_array_equal(a[t], b[t])
-    for a, b in zip(weights, ref_w):
-        np.testing.assert_array_equal(a, b)
+    ref, ref_w, ref_c = _run(net, sched, steps, T.STEP_PHASES)
+    assert ref_c[1] > 0
+    for mode in modes or (T.STEP_FUSED, T.STEP_GRID):
+        spikes, weights, counts = _run(net, sched, steps, mode)
+        assert counts == ref_c
+        for a, b in zip(spikes, ref):
+            for t in range(steps):
+                np.testing.assert_array_equal(a[t], b[t])
+        for a, b in zip(weights, ref_w):
+            np.testing.assert_array_equal(a, b)
 
 
 def _schedule(N, chan, trains):
@@ -89,7 +92,7 @@ def test_a_row_longer_than_the_list():
     from knp_gb300 import types as T
 
     rng = np.random.default_rng(1)
-    n, n_in, long_row = 300, 40, (1 << 20) + 77
+    n, n_in, long_row = 300, 700, (1 << 20) + 77
     per_row = np.full(n_in, 9, np.int64)
     per_row[[7, 31]] = long_row, 1 << 20  # one above the length that is walked by itself, one at it
     m = int(per_row.sum())
@@ -98,5 +101,41 @@ def test_a_row_longer_than_the_list():
                       rng.integers(0, n, m).astype(np.uint32), (rng.integers(-3, 4, m) / 256.0).astype(np.float32),
                       rng.integers(1, 4, m).astype(np.uint32))
     net = N.Network([N.Population(pop, T.BLIFAT, T.blifat_defaults(n))], [pr], [(inp, chan)])
-    trains = [np.array(x) for x in ([7], [3, 7, 31], [31], list(range(n_in)))]
-    _same(net, [_schedule(N, chan, trains)], 8)
+    # A few rows are cut into parts; 100 are not on 16 CTAs, 700 not on any number.
+    trains = [np.array(x) for x in ([7], [3, 7, 31], [31], list(range(100)), list(range(n_in)))]
+    _same(net, [_schedule(N, chan, trains)], 10)
+
+
+# Rows on either side of every cut of a 16- and a 152-CTA kernel (64 and 608 rows, halved six times), of odd lengths.
+@pytest.mark.parametrize("n_spikes", [1, 2, 9, 10, 19, 33, 64, 65, 152, 153, 304, 608, 609])
+def test_rows_cut_into_parts(n_spikes):
+    from knp_gb300 import network as N
+    from knp_gb300 import types as T
+
+    rng = np.random.default_rng(n_spikes)
+    n, n_in = 400, 620
+    per_row = rng.integers(0, 140, n_in)
+    per_row[:5] = [0, 1, 31, 63, 65]
+    m = int(per_row.sum())
+    pop, inp, chan = (T.uid_from_int(5850 + i) for i in range(3))
+    pr = N.Projection(inp, T.DELTA, T.NULL_UID, pop, np.repeat(np.arange(n_in, dtype=np.uint32), per_row),
+                      rng.integers(0, n, m).astype(np.uint32), (rng.integers(20, 100, m) / 64.0).astype(np.float32),
+                      rng.integers(1, 4, m).astype(np.uint32))
+    net = N.Network([N.Population(pop, T.BLIFAT, T.blifat_defaults(n))], [pr], [(inp, chan)])
+    trains = [np.sort(rng.choice(n_in, n_spikes, replace=False)) for _ in range(5)] + [np.arange(n_in)[:n_spikes]]
+    _same(net, [_schedule(N, chan, trains)], 10)
+
+
+def test_more_rows_than_the_grid_kernel_tables_hold():
+    from knp_gb300 import network as N
+    from knp_gb300 import types as T
+
+    rng = np.random.default_rng(3)
+    n = 160000  # 1024 rows a CTA are 155648
+    pop, inp, rec, chan = (T.uid_from_int(5870 + i) for i in range(4))
+    ids = np.arange(n, dtype=np.uint32)
+    drive = N.Projection(inp, T.DELTA, T.NULL_UID, pop, ids, ids, np.ones(n, np.float32), np.ones(n, np.uint32))
+    back = N.Projection(rec, T.DELTA, pop, pop, rng.integers(0, n, 3 * n).astype(np.uint32), np.repeat(ids, 3),
+                        (rng.integers(-96, 97, 3 * n) / 256).astype(np.float32), rng.integers(1, 6, 3 * n).astype(np.uint32))
+    net = N.Network([N.Population(pop, T.BLIFAT, T.blifat_defaults(n))], [drive, back], [(inp, chan)])
+    _same(net, [_schedule(N, chan, [ids, ids[::2], ids])], 6, [T.STEP_GRID])
