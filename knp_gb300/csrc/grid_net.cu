@@ -161,7 +161,7 @@ __device__ __forceinline__ unsigned long long grid_scatter(const ProjectionDev *
                                                         uint32_t n_sources, unsigned long long t, uint32_t rank, uint32_t G)
 {
     extern __shared__ uint4 grid_smem[];
-    return project_rows<kGridThreads, kInFlight, false>(
+    return project_rows<kGridThreads, kInFlight, false, true>(
         projs, sources, n_sources, t, rank, G, *reinterpret_cast<ScatterTables<kGridThreads> *>(grid_smem),
         [](const ProjectionDev &p, uint32_t count) { return p.pull.bitmap && count >= p.pull.threshold ? 0u : count; });
 }

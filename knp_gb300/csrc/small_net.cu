@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_net_kernel(SmallNet ne
         // ---- phase B
         // Step t - 1's counters are no longer read by anyone. (Beside the first warp's look at the sources.)
         if (rank == 0 && warp == kSmallWarps - 1) retire_counters(odd ? net.end[0] : net.end[1], lane, &s_spikes);
-        events += project_rows<kSmallThreads, kInFlight, true>(projs, sources, net.n_sources, t, rank, C, tab,
+        events += project_rows<kSmallThreads, kInFlight, true, false>(projs, sources, net.n_sources, t, rank, C, tab,
                                                          [](const ProjectionDev &, uint32_t count) { return count; });
         tc::cluster_sync();
     }

@@ -139,3 +139,36 @@ def test_more_rows_than_the_grid_kernel_tables_hold():
                         (rng.integers(-96, 97, 3 * n) / 256).astype(np.float32), rng.integers(1, 6, 3 * n).astype(np.uint32))
     net = N.Network([N.Population(pop, T.BLIFAT, T.blifat_defaults(n))], [drive, back], [(inp, chan)])
     _same(net, [_schedule(N, chan, [ids, ids[::2], ids])], 6, [T.STEP_GRID])
+
+
+# 10^7 synapses and more a step are 65536 a CTA: rows of 20011 of every third source, so that runs of 128 cross them.
+@pytest.mark.parametrize("fixed", [False, True])
+def test_long_lists(fixed):
+    from knp_gb300 import GB300Backend
+    from knp_gb300 import network as N
+    from knp_gb300 import types as T
+
+    n, n_in, steps = 20011, 1600, 6
+    pop, inp, rec, chan = (T.uid_from_int(5880 + i) for i in range(4))
+    got = []
+    for mode in (T.STEP_PHASES, T.STEP_GRID):
+        with GB300Backend() as b:
+            b.load_populations([N.Population(pop, T.BLIFAT, T.blifat_defaults(n))])
+            b.generate_projection(inp, T.NULL_UID, pop, T.GEN_ALL_TO_ALL, n_in, n, -8, 9, 1, 4, 7, 10)
+            b.generate_fixed_fan_in_projection(rec, pop, pop, n, n, 37, -32, 32, 1, 3, 8, 20)
+            b.subscribe(inp, [chan])
+            b.record_spikes(pop)
+            if fixed:
+                b.set_accumulator(pop, T.ACC_FIXED64)
+            b.set_pull_threshold(rec, -1.0)
+            b.set_step_mode(mode)
+            b._init()
+            trains = [np.arange(k % 3, n_in, 3) if k % 2 else np.arange(n_in) for k in range(steps)]
+            offs = np.concatenate([[0], np.cumsum([t.size for t in trains])]).astype(np.int64)
+            b.load_spike_schedule(N.SpikeSchedule(chan, offs, np.concatenate(trains).astype(np.uint32)), 0)
+            b.step(steps)
+            got.append(([b.spikes(pop, t) for t in range(steps)], b.counters()))
+    (ref, ref_c), (spikes, counts) = got
+    assert counts == ref_c and ref_c[1] > 0
+    for a, c in zip(spikes, ref):
+        np.testing.assert_array_equal(a, c)
