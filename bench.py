@@ -315,7 +315,7 @@ def batched_dense_measure(device: int, reps: int = 5, warmup: int = 3):
     flops = 2.0 * float(sum(int(cfg.steps.sum()) * a * c for a, c in zip(cfg.sizes[:-1], cfg.sizes[1:])))
     return {
         "workload": "batched_dense: 256 LIF samples 784-1000-1000-10, T in [50,200], inputs rate U[0,0.2], "
-                    "weights N(0,1/fan_in) as BF16, FP32 accumulation, one persistent launch",
+                    "weights N(0,1/fan_in) as BF16, FP32 accumulation, one product per layer with the LIF recurrence in its epilogue",
         "value": events / (ms_b / 1e3), "unit": UNIT, "ms_per_run": ms_b, "events_per_run": events,
         "plain_fp32_path": {"value": ev_p / (ms_p / 1e3), "unit": UNIT, "ms_per_run": ms_p, "events_per_run": ev_p,
                             "build_s": t_build, "mismatch_vs_fp64_oracle": mp64 / max(tp64, 1)},
@@ -326,8 +326,8 @@ def batched_dense_measure(device: int, reps: int = 5, warmup: int = 3):
                        "sample's own steps; pinned to the reference-header oracle on a smaller batch",
         "tensor": {"dense_flops_per_run": flops, "achieved_tflops": flops / (ms_b / 1e3) / 1e12},
         "dtype": "bf16 x bf16 -> fp32", "l2": "flushed (256 MB write) before each timed run",
-        "launch": "one CUDA graph per batch (state memsets, input thresholds, input spike bitmaps drawn ahead, "
-                  "persistent kernel of CTA-pair clusters)",
+        "launch": "one CUDA graph per batch (state memsets, weights packed, input thresholds, input spike rows drawn "
+                  "ahead, one kernel of CTA-pair clusters per layer)",
         "autotuned_ring_depth": stages, "autotuned_layer_ring_steps": ring,
         "autotune_ms": {f"depth{d}_ring{r}": v for (d, r), v in tuned.items()},
     }
@@ -461,8 +461,8 @@ def bptt_measure(device: int, iters: int = 10, warmup: int = 3):
             "execution": "one CUDA graph per iteration (forward, backward, SGD step)", "ms_per_iter_eager": ms_eager,
             "gemm_flops_per_iter": flops, "achieved_tflops": flops / (ms / 1e3) / 1e12,
             "tensor_flops_executed_per_iter": executed,
-            "gemm": "tcgen05 BF16 (knp_gb300_bf16_gemm_tn: TMA-fed 128x128 tiles, 128-byte swizzle, split K "
-                    "when tiles are few), FP32 accumulation; gradients as BF16 hi + lo",
+            "gemm": "tcgen05 BF16 (TMA-fed tiles, 128-byte swizzle, split K when tiles are few; a layer's product "
+                    "and LIF recurrence in one kernel), FP32 accumulation; gradients as BF16 hi + lo",
             "loss": loss}
 
 

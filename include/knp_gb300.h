@@ -226,7 +226,7 @@ KNP_GB300_API int knp_gb300_set_pull_threshold(knp_gb300_backend *b, knp_uid pro
 
 /**
  * Step execution mode (before init). The fused mode runs every phase of a step, and many steps per
- * launch, in one thread-block cluster (up to 8 CTAs) with cluster barriers between the phases; it
+ * launch, in one thread-block cluster (up to 16 CTAs) with cluster barriers between the phases; it
  * takes networks of at most 16384 neurons and 2^22 synapses whose projections have no gather form
  * and at most 8 STDP populations each. The grid mode runs every phase of a step, and many steps per
  * launch, in one cooperative launch of one 1024-thread CTA per SM with bounded grid barriers
@@ -473,10 +473,10 @@ KNP_GB300_API int knp_gb300_bf16_gemm_tn(
  * `batch` independent samples of a feed-forward LIF network with n_layers all-to-all delay-1
  * layers (sizes[0] inputs -> sizes[1] -> ... -> sizes[n_layers], each <= 4096, fan-in <= 2048; reference LIF
  * semantics lif_impl.h:33-86 with per-layer leak / threshold / reset / refractory period, NULL =
- * reference defaults 1, 1, 0, 0) run in a persistent kernel of CTA pairs on the tcgen05 tensor cores:
- * every step each layer's input is the previous layer's 0/1 spike matrix (BF16, exact) times its BF16
- * weights (device, d_weights[l] = [sizes[l + 1]][sizes[l]] row-major) with FP32 accumulation in tensor
- * memory. Sample b runs steps[b] (host array) steps; its input i spikes at step t iff
+ * reference defaults 1, 1, 0, 0) run layer by layer on the tcgen05 tensor cores (CTA pairs): a layer's
+ * input of all steps is the layer below's 0/1 spikes (BF16, exact) times its BF16 weights (device,
+ * d_weights[l] = [sizes[l + 1]][sizes[l]] row-major) with FP32 accumulation in tensor memory, the LIF
+ * recurrence in the product's epilogue. Sample b runs steps[b] (host array) steps; its input i spikes at step t iff
  * rand64(stream_key(seed, 5), (t * batch + b) * sizes[0] + i) >> 11 < d_rates[b][i] * 2^53 (the
  * generator of knp_gb300/network.py; a rate below 0 or NaN never fires, 1 or above always). Outputs: d_counts[batch][sizes[n_layers]] (device, int32) output
  * spike counts; optional d_record (device, uint32) with every layer's spike bitmap of every step,
@@ -495,17 +495,15 @@ KNP_GB300_API int knp_gb300_batched_lif_run(
  *                 l (<= sizes[l]); inputs and neurons beyond it do not exist for that sample (never
  *                 spike, carry no events). NULL: every sample has the full sizes (uneven network
  *                 instances over shared weights, or inputs of uneven width).
- *   autotune      > 0: each operand ring depth that fits (2..4 chunks of 32 KB) with each layer
- *                 ring length (4, 8, 16 steps) is run twice at creation and the fastest pair kept;
- *                 < 0: depth -autotune (layer rings of 8); 0: the deepest that fits. Neither choice
- *                 changes any result.
- *   segment_steps non-zero: at most this many steps per persistent launch (0: as many as a 256 MB
- *                 buffer of pre-drawn input spike bitmaps holds); segments do not change any result.
+ *   autotune      > 0: each operand ring depth (2..4) is run twice at creation and the fastest kept;
+ *                 < 0: depth -autotune; 0: the deepest. The depth changes no result.
+ *   segment_steps non-zero: at most this many steps per segment (0: as many as 256 MB of a layer's spike
+ *                 rows hold); segments do not change any result.
  * The device buffers (weights, rates, counts, record) must stay valid for the plan's life; their
  * contents are read / written by every knp_gb300_batched_plan_run, so rates and weights may be
- * rewritten between runs. One run: memsets of the run's state, the input-threshold kernel and, per
- * segment of steps, the input-drawing kernel and the persistent kernel (cluster launch of CTA pairs),
- * launched as one graph on `stream`; synchronous. Runs of one plan must not overlap (they share the
+ * rewritten between runs. One run: memsets of the run's state, the weights' packing, the input-threshold
+ * kernel and, per segment of steps, the input-drawing kernel and one kernel per layer (cluster launches
+ * of CTA pairs), launched as one graph on `stream`; synchronous. Runs of one plan must not overlap (they share the
  * plan's device state).
  */
 typedef struct knp_gb300_batched_plan knp_gb300_batched_plan;
@@ -520,10 +518,9 @@ KNP_GB300_API int knp_gb300_batched_plan_create(
 KNP_GB300_API int knp_gb300_batched_plan_run(knp_gb300_batched_plan *plan, uint64_t *events, float *ms);
 
 /**
- * The operand ring depth and the layer ring length (steps a layer may hold; it runs at most that
- * many minus 2 steps ahead of the next layer) in use, and, after autotuning, the time of each pair
- * tried: tune_ms[9], index 3 * r + (depth - 2) for layer rings of 4, 8, 16 steps (r = 0, 1, 2) and
- * depths 2, 3, 4; 0 = not tried.
+ * The operand ring depth in use and, after autotuning, the time of each depth tried: tune_ms[9], index
+ * depth - 2 for depths 2, 3, 4; 0 = not tried, as entries 3 .. 8 are (*ring_steps, 4, and they are of a
+ * layer ring that is no longer there).
  */
 KNP_GB300_API int knp_gb300_batched_plan_info(const knp_gb300_batched_plan *plan, int *stages, int *ring_steps,
                                               float *tune_ms);

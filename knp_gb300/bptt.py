@@ -3,8 +3,9 @@
 A feed-forward LIF network (all-to-all layers, membrane decay beta, threshold theta, reset by
 subtraction) is trained on spike counts. Per layer the synaptic input of all T steps is one GEMM of
 the previous layer's spikes with the layer's weights (BF16 values of the FP32 master weights,
-products exact in FP32, FP32 accumulation); the LIF recurrence over T and its backward are the
-hand-written kernels of knp_gb300/csrc/bptt.cu behind ``LIFLayerFn`` (torch.autograd.Function).
+products exact in FP32, FP32 accumulation), with the LIF recurrence over T, and its backward, in the
+same kernel (knp_gb300/csrc/lif_gemm.cu) behind ``LIFLayerFn`` (torch.autograd.Function); the relaxed
+forward and long checkpoint intervals take product and scan apart (knp_gb300/csrc/bptt.cu).
 The forward keeps the membrane state only every ``checkpoint`` steps; the backward recomputes each
 segment. The reference has no gradient-based training; this form has no counterpart there.
 
