@@ -1686,13 +1686,16 @@ void Backend::build_small_net()
 
 uint32_t Backend::train_blocks(const PopulationSlot &q) const
 {
-    return static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((q.n + 7) / 8, 4ull * sm_count_)));
+    return static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(q.n, 4ull * sm_count_)));
 }
 
 TrainView Backend::train_view(const PopulationSlot &q)
 {
-    if (q.is_altai()) return {q.adev.res, q.adev.syn, q.adev.dopa, q.adev.spikes, q.adev.spike_count};
-    return {q.bdev.res, q.bdev.syn, q.bdev.dopa, q.bdev.spikes, q.bdev.spike_count};
+    uint64_t synapses = 0;
+    for (const ProjectionSlot *p : q.res_projs) synapses += p->n_syn;
+    const uint32_t per = static_cast<uint32_t>(std::min<uint64_t>(synapses / std::max<uint64_t>(q.n, 1), 0xFFFFFFFFu));
+    if (q.is_altai()) return {q.adev.res, q.adev.syn, q.adev.dopa, q.adev.spikes, q.adev.spike_count, per};
+    return {q.bdev.res, q.bdev.syn, q.bdev.dopa, q.bdev.spikes, q.bdev.spike_count, per};
 }
 
 // One population's step: its kernel, then (resource-STDP populations with resource-STDP synapses)

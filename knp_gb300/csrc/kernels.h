@@ -233,6 +233,7 @@ struct TrainView
     const float *dopa;
     const uint32_t *spikes;
     const uint32_t *spike_count;
+    uint32_t per_neuron;  // synapses of a neuron, on average
 };
 
 // External spike schedule of one sender channel (device-resident window).

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) projection_kernel(ProjectionDev p, Contro
 }
 
 // Several projections of a few rows each in one launch: a step of a network with seven of them (784 inputs, 200
-// neurons, resource STDP) took 48 us, launch after launch that each leave most of the device idle, and takes 26 this way, its
+// neurons, resource STDP) took 48 us, launch after launch that each leave most of the device idle, and took 26 this way, its
 // populations and their training batched too.
 __global__ void __launch_bounds__(256) projection_batch_kernel(const __grid_constant__ ProjectionBatch b, Control *ctl)
 {

@@ -7,14 +7,15 @@
 //   do_dopamine_plasticity_impl (:106-155) and renormalize_resource (impl/populations/training/
 //     stdp.h:152-186) for every neuron, with recalculate_synapse_weights (training/stdp.h:40-52).
 //
-// Neurons are independent (a neuron's synapses are the ones into it), so one warp trains one neuron
-// through all three stages in the reference's order. The work list is this step's spike list
+// Neurons are independent (a neuron's synapses are the ones into it), so one warp, or one block, trains one
+// neuron through all three stages in the reference's order. The work list is this step's spike list
 // followed by the non-spiking neurons the population kernel found with dopamine or renormalisation
 // work; every other neuron would be left unchanged. A neuron's synapses are its entries of the
 // column index, in get_all_connected_synapses order (projection load order, then synapse index),
-// skipping locked projections. Per-synapse updates run on the warp's lanes; the two quantities the
+// skipping locked projections. Per-synapse updates run on its threads; the two quantities the
 // reference accumulates across synapses (the FP64 additional threshold and the FP32 free
-// resource) are accumulated in synapse order, so every rounding is the reference's.
+// resource) are accumulated in synapse order, so every rounding is the reference's (or in another
+// order where none rounds).
 #include <cstdint>
 
 #include "kernels.h"
@@ -67,10 +68,84 @@ __device__ __forceinline__ bool working_synapse(const ResSynDev &y, long long e,
     return y.locked[ent >> kResSlotShift] == 0u;
 }
 
-__device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long t, bool spiked, int lane)
+constexpr int kPer = 4;  // synapses of a thread in a tile
+
+// Exponents that bound the additional threshold's FP64 sum: every term is a multiple of 2^lo and less than 2^hi.
+struct SumRange
+{
+    int lo = 1 << 20, hi = -(1 << 20);
+    __device__ void add(float x)
+    {
+        const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
+        if (!u) return;
+        const int e = static_cast<int>(u >> 23);
+        if (e == 0xFF)  // infinite or NaN: no order is free
+        {
+            hi = 1 << 20;
+            return;
+        }
+        const uint32_t m = e ? (u & 0x7FFFFFu) | 0x800000u : u;
+        const int ulp = (e ? e : 1) - 150;
+        lo = min(lo, ulp + __ffs(static_cast<int>(m)) - 1);
+        hi = max(hi, ulp + 24);
+    }
+    __device__ void join(int l, int h)
+    {
+        lo = min(lo, l);
+        hi = max(hi, h);
+    }
+    // Whether sums of up to n such terms are exact in FP64, in whatever order.
+    __device__ bool exact(unsigned long long n) const { return hi + 64 - __clzll(static_cast<long long>(n)) - lo <= 53; }
+};
+
+// Shared memory of the kT threads that train a neuron together.
+template <int kT>
+struct TrainShared
+{
+    float x[kT * kPer], du[kT * kPer];  // a tile's terms of the additional threshold and changes of the resource
+    uint32_t ok[kT * kPer / 32], hebb[kT * kPer / 32];
+    double part[kT / 32];
+    int lo[kT / 32], hi[kT / 32];
+    uint32_t count[kT / 32];
+    float f, g;  // values that one thread makes for all
+};
+
+template <int kT>
+__device__ __forceinline__ void group_sync()
+{
+    if (kT == 32)
+        __syncwarp();
+    else
+        __syncthreads();
+}
+
+// Sum of v over the group, in every thread.
+template <int kT>
+__device__ __forceinline__ uint32_t group_sum(TrainShared<kT> &sh, uint32_t v, int tid)
+{
+    v = __reduce_add_sync(kFull, v);
+    if (kT == 32) return v;
+    if ((tid & 31) == 0) sh.count[tid >> 5] = v;
+    __syncthreads();
+    uint32_t all = 0;
+#pragma unroll
+    for (int k = 0; k < kT / 32; ++k) all += sh.count[k];
+    __syncthreads();
+    return all;
+}
+
+// Trains neuron i with kT threads (this is thread tid of them): a warp for neurons of few synapses, a block for ones
+// of many, whose per-synapse work is then one round of loads instead of one per 32. What has to be taken in synapse
+// order is done by the first warp from shared memory: the free resource (FP32, a chain of adds), and the additional
+// threshold where its FP64 sum would round (else it is the same in any order, and FP64 is a slow unit). A label step
+// of 200 neurons with 784 synapses each took 182 us by warps that shuffled every synapse's terms to all lanes, and
+// takes 19.
+template <int kT>
+__device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long t, bool spiked, int tid, TrainShared<kT> &sh)
 {
     const ResourceDev &r = p.res;
     const ResSynDev &y = p.syn;
+    const int lane = tid & 31, warp = tid >> 5;
     int32_t status = r.isi_status[i];
     const bool forced = r.is_forced[i] != 0;
     const float dopa = p.dopa[i];
@@ -87,53 +162,113 @@ __device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long 
         last_spike = t;
         status = update_isi(status, forced, dopa, isi_max, t, last_step, first);
         if (status == 1) stab = __fsub_rn(stab, pf(r.stability_change_at_isi, i));
-        const float d_h = __fmul_rn(pf(r.d_h, i), resource_factor(stab));
+        if (tid == 0) sh.g = __fmul_rn(pf(r.d_h, i), resource_factor(stab));
+        group_sync<kT>();
+        const float d_h = sh.g;
         double add = 0.0;
-        for (long long base = a; base < b; base += 32)
+        SumRange range;
+        for (long long base = a; base < b; base += kT * kPer)
         {
-            unsigned long long pos = 0;
-            const bool ok = working_synapse(y, base + lane, b, pos);
-            float x = 0.0f, du = 0.0f;
-            bool hebb = false;
-            if (ok)
+            double part = 0.0;
+            SumRange mine;
+#pragma unroll
+            for (int u = 0; u < kPer; ++u)
             {
-                const float w = y.w[pos];
-                x = __fmul_rn(w, w > 0.0f ? 1.0f : 0.0f);
-                const bool had_spike = in_interval(t - y.period[pos], t, y.last_spike[pos] + y.delay[pos] - 1ull);
-                uint32_t fl = y.flags[pos];
-                if (status != 2 || had_spike) fl = had_spike ? (fl | 2u) : (fl & ~2u);
-                if (status != 2) fl &= ~1u;
-                float res = y.resource[pos];
-                if (status != 0)
+                const int q = u * kT + tid;
+                unsigned long long pos = 0;
+                const bool ok = working_synapse(y, base + q, b, pos);
+                float x = 0.0f, du = 0.0f;
+                bool hebb = false;
+                if (ok)
                 {
-                    du = y.d_u[pos];
-                    res = __fsub_rn(res, du);
-                    if ((fl & 2u) && !(fl & 1u))
+                    const float w = y.w[pos];
+                    x = __fmul_rn(w, w > 0.0f ? 1.0f : 0.0f);
+                    const bool had_spike = in_interval(t - y.period[pos], t, y.last_spike[pos] + y.delay[pos] - 1ull);
+                    uint32_t fl = y.flags[pos];
+                    if (status != 2 || had_spike) fl = had_spike ? (fl | 2u) : (fl & ~2u);
+                    if (status != 2) fl &= ~1u;
+                    float res = y.resource[pos];
+                    if (status != 0)
                     {
-                        res = __fadd_rn(res, d_h);
-                        fl |= 1u;
-                        hebb = true;
+                        du = y.d_u[pos];
+                        res = __fsub_rn(res, du);
+                        if ((fl & 2u) && !(fl & 1u))
+                        {
+                            res = __fadd_rn(res, d_h);
+                            fl |= 1u;
+                            hebb = true;
+                        }
+                    }
+                    y.resource[pos] = res;
+                    y.flags[pos] = static_cast<uint8_t>(fl);
+                    y.w[pos] = synapse_weight(res, y.w_min[pos], y.w_max[pos]);
+                    mine.add(x);
+                    part = __dadd_rn(part, static_cast<double>(x));
+                }
+                sh.x[q] = x;
+                sh.du[q] = du;
+                const unsigned okm = __ballot_sync(kFull, ok), hm = __ballot_sync(kFull, hebb);
+                if (lane == 0)
+                {
+                    sh.ok[q >> 5] = okm;
+                    sh.hebb[q >> 5] = hm;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) part = __dadd_rn(part, __shfl_xor_sync(kFull, part, o));
+            const int lo = __reduce_min_sync(kFull, mine.lo), hi = __reduce_max_sync(kFull, mine.hi);
+            if (lane == 0)
+            {
+                sh.part[warp] = part;
+                sh.lo[warp] = lo;
+                sh.hi[warp] = hi;
+            }
+            group_sync<kT>();
+            if (warp == 0)
+            {
+                const long long left = b - base;
+                const int n = left < kT * kPer ? static_cast<int>(left) : kT * kPer;
+#pragma unroll
+                for (int k = 0; k < kT / 32; ++k) range.join(sh.lo[k], sh.hi[k]);
+                if (range.exact(static_cast<unsigned long long>(base - a) + n + 1))
+                {
+#pragma unroll
+                    for (int k = 0; k < kT / 32; ++k) add = __dadd_rn(add, sh.part[k]);
+                }
+                else
+                {
+                    for (int q = 0; q < n; ++q)
+                        if ((sh.ok[q >> 5] >> (q & 31)) & 1u) add = __dadd_rn(add, static_cast<double>(sh.x[q]));
+                }
+                for (int w = 0; status != 0 && w * 32 < n; ++w)
+                {
+                    const uint32_t okm = sh.ok[w], hm = sh.hebb[w];
+                    const float *du = sh.du + 32 * w;
+                    if (okm == kFull && hm == 0u)
+                    {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) fr = __fadd_rn(fr, du[q]);
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q)
+                        {
+                            if ((okm >> q) & 1u) fr = __fadd_rn(fr, du[q]);
+                            if ((hm >> q) & 1u) fr = __fsub_rn(fr, d_h);
+                        }
                     }
                 }
-                y.resource[pos] = res;
-                y.flags[pos] = static_cast<uint8_t>(fl);
-                y.w[pos] = synapse_weight(res, y.w_min[pos], y.w_max[pos]);
             }
-            const unsigned okm = __ballot_sync(kFull, ok), hm = __ballot_sync(kFull, hebb);
-            for (int q = 0; q < 32; ++q)
-            {
-                const float xq = __shfl_sync(kFull, x, q), dq = __shfl_sync(kFull, du, q);
-                if (!((okm >> q) & 1u)) continue;
-                add = __dadd_rn(add, static_cast<double>(xq));
-                if (status != 0)
-                {
-                    fr = __fadd_rn(fr, dq);
-                    if ((hm >> q) & 1u) fr = __fsub_rn(fr, d_h);
-                }
-            }
+            group_sync<kT>();  // the tile is used again
         }
-        add = __dmul_rn(add, static_cast<double>(pf(r.add_thr_coef, i)));
-        if (lane == 0) y.add_thr[i] = add;
+        if (tid == 0)
+        {
+            y.add_thr[i] = __dmul_rn(add, static_cast<double>(pf(r.add_thr_coef, i)));
+            sh.f = fr;
+        }
+        group_sync<kT>();
+        fr = sh.f;
     }
 
     if (dopa > 0.0f || (dopa < 0.0f && status != 0))
@@ -141,44 +276,48 @@ __device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long 
         // do_dopamine_plasticity_impl: resource change of contributing synapses while the last spike
         // is recent, stability change, new weights of every synapse.
         const bool recent = t - last_spike <= pu(r.dopamine_time, i);
-        const float change = __fmul_rn(dopa, resource_factor(stab));
-        for (long long base = a; base < b; base += 32)
+        group_sync<kT>();  // sh.g and sh.f have been read
+        if (tid == 0) sh.g = __fmul_rn(dopa, resource_factor(stab));
+        group_sync<kT>();
+        const float change = sh.g;
+        uint32_t n_app = 0;
+#pragma unroll 4
+        for (long long e = a + tid; e < b; e += kT)
         {
             unsigned long long pos = 0;
-            const bool ok = working_synapse(y, base + lane, b, pos);
-            bool app = false;
-            if (ok)
+            if (working_synapse(y, e, b, pos))
             {
                 float res = y.resource[pos];
                 if (recent && (y.flags[pos] & 2u))
                 {
                     res = __fadd_rn(res, change);
                     y.resource[pos] = res;
-                    app = true;
+                    ++n_app;
                 }
                 y.w[pos] = synapse_weight(res, y.w_min[pos], y.w_max[pos]);
             }
-            const unsigned am = __ballot_sync(kFull, app);
-            for (int q = 0; q < 32; ++q)
-                if ((am >> q) & 1u) fr = __fsub_rn(fr, change);
         }
-        stab = dopamine_stability(stab, dopa, pf(r.stability_change_param, i), forced, t, first, isi_max);
+        n_app = group_sum<kT>(sh, n_app, tid);
+        for (uint32_t k = 0; k < n_app; ++k) fr = __fsub_rn(fr, change);
+        if (tid == 0) stab = dopamine_stability(stab, dopa, pf(r.stability_change_param, i), forced, t, first, isi_max);
     }
 
     if (!(t - last_step <= isi_max && status != 0) && !(fabsf(fr) < pf(r.resource_threshold, i)))
     {
         // renormalize_resource: the free resource divided over the working synapses and the drain.
-        unsigned long long n_syn = 0;
-        for (long long base = a; base < b; base += 32)
+        uint32_t mine = 0;
+        for (long long e = a + tid; e < b; e += kT)
         {
             unsigned long long pos = 0;
-            n_syn += __popc(__ballot_sync(kFull, working_synapse(y, base + lane, b, pos)));
+            mine += working_synapse(y, e, b, pos) ? 1u : 0u;
         }
+        const unsigned long long n_syn = group_sum<kT>(sh, mine, tid);
         const float add_v = __fdiv_rn(fr, __ull2float_rn(n_syn + pu(r.drain, i)));
-        for (long long base = a; base < b; base += 32)
+#pragma unroll 4
+        for (long long e = a + tid; e < b; e += kT)
         {
             unsigned long long pos = 0;
-            if (working_synapse(y, base + lane, b, pos))
+            if (working_synapse(y, e, b, pos))
             {
                 const float res = __fadd_rn(y.resource[pos], add_v);
                 y.resource[pos] = res;
@@ -188,7 +327,7 @@ __device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long 
         fr = 0.0f;
     }
 
-    if (lane == 0)
+    if (tid == 0)
     {
         r.isi_status[i] = status;
         r.last_step[i] = last_step;
@@ -197,19 +336,38 @@ __device__ void train_neuron(const TrainView &p, uint32_t i, unsigned long long 
         r.stability[i] = stab;
         r.free_resource[i] = fr;
     }
+    group_sync<kT>();  // the shared memory is the next neuron's
 }
 
-__device__ __forceinline__ void train_block(const TrainView &p, unsigned long long t, uint32_t block, uint32_t n_blocks)
+template <int kT>
+__device__ __forceinline__ void train_groups(const TrainView &p, unsigned long long t, uint32_t block, uint32_t n_blocks,
+                                             TrainShared<kT> *shared)
 {
+    constexpr uint32_t kGroups = kTrainThreads / kT;
     const uint32_t n_spk = *p.spike_count, n_work = *p.syn.work_count;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = (block * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (n_blocks * blockDim.x) >> 5;
-    for (uint32_t j = warp; j < n_spk + n_work; j += n_warps)
+    const uint32_t group = threadIdx.x / kT;
+    for (uint32_t j = block * kGroups + group; j < n_spk + n_work; j += n_blocks * kGroups)
     {
         const bool spiked = j < n_spk;
-        train_neuron(p, spiked ? p.spikes[j] : p.syn.work[j - n_spk], t, spiked, lane);
+        train_neuron<kT>(p, spiked ? p.spikes[j] : p.syn.work[j - n_spk], t, spiked, static_cast<int>(threadIdx.x % kT),
+                         shared[group]);
     }
+}
+
+// A neuron of kBlockSynapses synapses or more on average is a block's work, else a warp's.
+constexpr uint32_t kBlockSynapses = 128;
+__device__ __forceinline__ void train_block(const TrainView &p, unsigned long long t, uint32_t block, uint32_t n_blocks)
+{
+    __shared__ union Shared
+    {
+        TrainShared<kTrainThreads> block;
+        TrainShared<32> warp[kTrainThreads / 32];
+        __device__ Shared() {}
+    } shared;
+    if (p.per_neuron >= kBlockSynapses)
+        train_groups<kTrainThreads>(p, t, block, n_blocks, &shared.block);
+    else
+        train_groups<32>(p, t, block, n_blocks, shared.warp);
 }
 
 __global__ void __launch_bounds__(kTrainThreads) resource_train_kernel(TrainView p, Control *ctl)
