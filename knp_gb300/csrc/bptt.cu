@@ -18,6 +18,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "kernels.h"
+
 namespace knp_gb300
 {
 namespace
@@ -161,6 +163,7 @@ template <bool kVec>
 __global__ void operand_rows8_kernel(const float *__restrict__ X, long long R, long long C, int mode, long long P,
                                      __nv_bfloat16 *__restrict__ out)
 {
+    pdl_begin();
     const long long units = R * (P / 8), H = mode == 0 ? 1 : 2;
     for (long long u = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; u < units;
          u += static_cast<long long>(gridDim.x) * blockDim.x)
@@ -233,8 +236,8 @@ int bf16_operand(const void *X, int x_bf16, long long R, long long C, int mode, 
         {
             const long long blocks = std::min<long long>((R * (P / 8) + 255) / 256, 1ll << 20);
             const bool vec = C % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
-            (vec ? operand_rows8_kernel<true> : operand_rows8_kernel<false>)<<<static_cast<unsigned>(blocks), 256, 0, s>>>(
-                static_cast<const float *>(X), R, C, mode, P, o);
+            launch_pdl(vec ? operand_rows8_kernel<true> : operand_rows8_kernel<false>, dim3(static_cast<unsigned>(blocks)),
+                       dim3(256), 0, s, static_cast<const float *>(X), R, C, mode, P, o);
             return cudaGetLastError() == cudaSuccess ? 0 : -3;
         }
         const long long gx = (P / 2 + 255) / 256;

@@ -315,6 +315,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
         tc::mbar_init(&drain, 1);
         s_fail = 0;
     }
+    // What is above overlaps the end of the kernel before (programmatic dependent launch); nothing below does.
+    pdl_begin();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -461,6 +463,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
         tc::mbar_init(&drain, 1);
         s_fail = 0;
     }
+    pdl_begin();
     tc::fence_before_sync();
     __syncthreads();
     tc::cluster_sync();  // both CTAs' barriers and tensor memory are set up
@@ -632,6 +635,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
 // D = sum over the splits of ws[z] (split order), n elements.
 __global__ void split_sum_kernel(const float *__restrict__ ws, float *__restrict__ D, size_t n, int splits)
 {
+    pdl_begin();
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<size_t>(gridDim.x) * blockDim.x)
     {
@@ -783,7 +787,8 @@ int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned
     if (pair_waves < waves)
     {
         if (smem_limit_once(gemm_pair_kernel<kMn>, static_cast<int>(kPairSmem), dev) != cudaSuccess) return -3;
-        gemm_pair_kernel<kMn><<<2 * std::min(pair_tiles, sms / 2), kPairThreads, kPairSmem, s>>>(maps, D, M, N, kp, d_err);
+        launch_pdl(gemm_pair_kernel<kMn>, dim3(2 * std::min(pair_tiles, sms / 2)), dim3(kPairThreads), kPairSmem, s, maps, D, M, N,
+                   kp, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
     if (smem_limit_once(gemm_tma_kernel<kMn>, static_cast<int>(kTmaSmem), dev) != cudaSuccess) return -3;
@@ -804,12 +809,12 @@ int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned
     }
     const int cps_used = splits > 1 ? cps : kp.nk;
     dim3 grid(tiles_m, tiles_n, splits);
-    gemm_tma_kernel<kMn><<<grid, kTmaThreads, kTmaSmem, s>>>(maps, splits > 1 ? ws : D, M, N, kp, cps_used,
-                                                        splits > 1 ? mn : 0, d_err);
+    launch_pdl(gemm_tma_kernel<kMn>, grid, dim3(kTmaThreads), kTmaSmem, s, maps, splits > 1 ? ws : D, M, N, kp, cps_used,
+               splits > 1 ? mn : 0, d_err);
     if (splits > 1)
     {
         const int blocks = static_cast<int>(std::min<size_t>((mn + 255) / 256, 8ull * sms));
-        split_sum_kernel<<<blocks, 256, 0, s>>>(ws, D, mn, splits);
+        launch_pdl(split_sum_kernel, dim3(blocks), dim3(256), 0, s, static_cast<const float *>(ws), D, mn, splits);
         cudaFreeAsync(ws, s);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
