@@ -326,7 +326,7 @@ def batched_dense_measure(device: int, reps: int = 5, warmup: int = 3):
                        "sample's own steps; pinned to the reference-header oracle on a smaller batch",
         "tensor": {"dense_flops_per_run": flops, "achieved_tflops": flops / (ms_b / 1e3) / 1e12},
         "dtype": "bf16 x bf16 -> fp32", "l2": "flushed (256 MB write) before each timed run",
-        "launch": "one CUDA graph per batch (state memsets, weights packed, input thresholds, input spike rows drawn "
+        "launch": "one CUDA graph per batch (state memsets, weights packed, input spike rows drawn "
                   "ahead, one kernel of CTA-pair clusters per layer)",
         "autotuned_ring_depth": stages, "autotuned_layer_ring_steps": ring,
         "autotune_ms": {f"depth{d}_ring{r}": v for (d, r), v in tuned.items()},

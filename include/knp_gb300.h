@@ -501,9 +501,9 @@ KNP_GB300_API int knp_gb300_batched_lif_run(
  *                 rows hold); segments do not change any result.
  * The device buffers (weights, rates, counts, record) must stay valid for the plan's life; their
  * contents are read / written by every knp_gb300_batched_plan_run, so rates and weights may be
- * rewritten between runs. One run: memsets of the run's state, the weights' packing, the input-threshold
- * kernel and, per segment of steps, the input-drawing kernel and one kernel per layer (cluster launches
- * of CTA pairs), launched as one graph on `stream`; synchronous. Runs of one plan must not overlap (they share the
+ * rewritten between runs. One run: memsets of the run's state, the weights' packing and, per segment
+ * of steps, the input-drawing kernel and one kernel per layer (cluster launches of CTA pairs), launched
+ * as one graph on `stream`; synchronous. Runs of one plan must not overlap (they share the
  * plan's device state).
  */
 typedef struct knp_gb300_batched_plan knp_gb300_batched_plan;
