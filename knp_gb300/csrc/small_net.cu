@@ -291,28 +291,26 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_net_kernel(SmallNet ne
 
 int small_net_cluster()
 {
-    static int c = [] {
-        cudaLaunchConfig_t cfg{};
-        cfg.blockDim = dim3(kSmallThreads);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        // 16 CTAs are more than every device schedules; the query below says.
-        cudaFuncSetAttribute(small_net_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        for (int size = 16; size > 1; size /= 2)
-        {
-            cfg.gridDim = dim3(size);
-            attr[0].val.clusterDim.x = size;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, small_net_kernel, &cfg) == cudaSuccess && n > 0) return size;
-            cudaGetLastError();
-        }
-        return 1;
-    }();
-    return c;
+    // 16 CTAs are more than the portable size: allowed per device, so asked for and set for the current one.
+    if (cudaFuncSetAttribute(small_net_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kSmallThreads);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    for (int size = 16; size > 1; size /= 2)
+    {
+        cfg.gridDim = dim3(size);
+        attr[0].val.clusterDim.x = size;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, small_net_kernel, &cfg) == cudaSuccess && n > 0) return size;
+        cudaGetLastError();
+    }
+    return 1;
 }
 
 cudaError_t launch_small_net(const SmallNet &net, Control *ctl, uint32_t n_steps, int cluster, cudaStream_t s)
