@@ -100,21 +100,17 @@ __device__ __forceinline__ bool grid_sync(unsigned long long *bar, Control *ctl,
 }
 
 // Whether a step of the gather's delay window for step t + 1 (t + 1 - d, d = 1 .. max_delay) was
-// pulled: step t from its spike count (the rule of project()), earlier steps from their flags.
+// pulled: step t from its spike count (the rule of record_pulled()), earlier steps from their flags.
 // Every thread of the CTA may call it; threads share the flag reads.
 __device__ __forceinline__ bool pull_window_active(const ProjectionDev &p, unsigned long long t)
 {
     const PullDev &g = p.pull;
-    if (threadIdx.x == 0 && p.n_src != 0)
-    {
-        const uint32_t *idx[kMaxSources];
-        uint32_t cnt[kMaxSources];
-        if (resolve_sources(p, t, idx, cnt) >= g.threshold) return true;
-    }
-    bool need = false;
+    // No branch on what is loaded: the caller needs the answer only after the scatter.
+    uint32_t need = 0;
+    if (threadIdx.x == 0) need = *p.src[0].count >= g.threshold ? 1u : 0u;
     for (uint32_t d = 2 + threadIdx.x; d <= g.max_delay && d <= t + 1; d += blockDim.x)
-        need = need || g.pulled[static_cast<uint32_t>((t + 1 - d) % g.hist_slots)] != 0u;
-    return need;
+        need |= g.pulled[step_slot(t + 1 - d, g.hist_slots)];
+    return need != 0u;
 }
 
 // A step at or above the threshold of a projection with a gather form is only recorded (as projection_kernel,
@@ -319,13 +315,13 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_net_kernel(GridNet g, Co
         {
             const ProjectionDev &p = projs[g.pull[k]];
             clear_bitmap_slot(p.pull, t + 1, blockIdx.x, G);
-            need = need || pull_window_active(p, t);
+            need |= pull_window_active(p, t);
         }
-        need = __syncthreads_or(need) != 0;
         for (uint32_t k = 0; k < g.n_pull; ++k) events += record_pulled(projs[g.pull[k]], t, gthread, n_threads, lane);
         const unsigned long long ev =
             grid_scatter(projs, odd ? net.sources[1] : net.sources[0], net.n_sources, t, blockIdx.x, G);
         if (threadIdx.x == 0) events += ev;
+        need = __syncthreads_or(need) != 0;
         // The scatter's writes (slots t + 1 .. t + D) are complete before step t + 1's populations
         // read slot t + 1, and the step's bitmaps before the gathers read them.
         target += G;
