@@ -993,8 +993,7 @@ cudaError_t capture(BatchedPlan &p, int stages)
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const size_t smem = smem_bytes(stages);
-    cudaError_t err =
-        cudaFuncSetAttribute(lif_layer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t err = allow_dynamic_smem(lif_layer_kernel);
     if (err != cudaSuccess) return err;
     cudaStream_t s = p.stream;
     err = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);

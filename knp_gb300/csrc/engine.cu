@@ -1220,7 +1220,7 @@ void Backend::build_resource_synapses(PopulationSlot &q)
     }
 }
 
-cudaError_t set_gather_smem(size_t bytes);
+cudaError_t allow_gather_smem();
 
 int Backend::gather_grid(const ProjectionSlot &p) const
 {
@@ -1278,7 +1278,7 @@ void Backend::build_pull(ProjectionSlot &p)
         more.n_bm = k;
         if (gather_smem_bytes(more, grid) + kGatherStaticSmem <= std::min<size_t>(kGatherSmemGoal, smem_max)) g.n_bm = k;
     }
-    KNP_CUDA(set_gather_smem(std::max<size_t>(gather_smem_bytes(g, grid), 48 * 1024)));
+    KNP_CUDA(allow_gather_smem());
     p.dev.pull = g;
     p.pull = true;
 }

@@ -666,19 +666,6 @@ EncodeTiled encode_tiled()
     return fn;
 }
 
-// The kernel's dynamic shared memory limit raised once per (kernel, device): a per-device setting.
-template <class Kernel>
-cudaError_t smem_limit_once(Kernel kernel, int bytes, int dev)
-{
-    static std::mutex mu;
-    static std::map<std::pair<const void *, int>, cudaError_t> done;
-    std::lock_guard<std::mutex> lock(mu);
-    const std::pair<const void *, int> key{reinterpret_cast<const void *>(kernel), dev};
-    const auto it = done.find(key);
-    if (it != done.end()) return it->second;
-    return done[key] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 // Stream-ordered pool of the split-K workspaces of device `dev` (memory kept by the pool between
 // calls). Allocating on the call's stream keeps concurrent streams apart and lets a call be captured
 // in a CUDA graph (the allocation becomes a graph memory node).
@@ -786,12 +773,12 @@ int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned
     const int waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
     if (pair_waves < waves)
     {
-        if (smem_limit_once(gemm_pair_kernel<kMn>, static_cast<int>(kPairSmem), dev) != cudaSuccess) return -3;
+        if (allow_dynamic_smem(gemm_pair_kernel<kMn>) != cudaSuccess) return -3;
         launch_pdl(gemm_pair_kernel<kMn>, dim3(2 * std::min(pair_tiles, sms / 2)), dim3(kPairThreads), kPairSmem, s, maps, D, M, N,
                    kp, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
-    if (smem_limit_once(gemm_tma_kernel<kMn>, static_cast<int>(kTmaSmem), dev) != cudaSuccess) return -3;
+    if (allow_dynamic_smem(gemm_tma_kernel<kMn>) != cudaSuccess) return -3;
     int cps = 0;
     int splits = gemm_splits(tiles, kp.nk, sms, cps);
     const size_t mn = static_cast<size_t>(M) * N;
@@ -832,9 +819,7 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
     GemmMaps maps{};
     if (sw128_map(&maps.a, A, M, K, kBM) && sw128_map(&maps.b, B, N, K, kBN))
         return launch_gemm<false>(maps, D, M, N, KPlan{(K + kBK - 1) / kBK, kOneHalf, 0, 0}, d_err, s);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (smem_limit_once(gemm_pipe_kernel, static_cast<int>(kStages * kStageBytes), dev) != cudaSuccess) return -3;
+    if (allow_dynamic_smem(gemm_pipe_kernel) != cudaSuccess) return -3;
     dim3 grid((M + kBM - 1) / kBM, (N + kBN - 1) / kBN);
     gemm_pipe_kernel<<<grid, kThreads, kStages * kStageBytes, s>>>(static_cast<const __nv_bfloat16 *>(A),
                                                                    static_cast<const __nv_bfloat16 *>(B), D, M, N, K, d_err);

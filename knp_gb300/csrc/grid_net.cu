@@ -382,9 +382,7 @@ int grid_net_ctas(size_t smem)
     int device = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(grid_net_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-            cudaSuccess)
+    if (allow_dynamic_smem(grid_net_kernel) != cudaSuccess)
     {
         cudaGetLastError();
         return 0;

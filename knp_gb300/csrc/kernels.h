@@ -20,6 +20,8 @@
 #include <cstdint>
 
 #include <cuda_runtime.h>
+#include <map>
+#include <mutex>
 #include <utility>
 
 namespace knp_gb300
@@ -808,6 +810,29 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// Lets a kernel be launched with as much dynamic shared memory as a block of the current device has beside the
+// kernel's own. The limit is one value per kernel and device, whoever launches it: a caller that set it to its own
+// need would take away what an earlier one (another backend, another plan) still launches with.
+template <typename... KArgs>
+inline cudaError_t allow_dynamic_smem(void (*kernel)(KArgs...))
+{
+    static std::mutex mu;
+    static std::map<std::pair<const void *, int>, bool> done;
+    int dev = 0, most = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    const void *f = reinterpret_cast<const void *>(kernel);
+    std::lock_guard<std::mutex> lock(mu);
+    if (done[{f, dev}]) return cudaSuccess;
+    cudaFuncAttributes attr{};
+    err = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (err == cudaSuccess) err = cudaFuncGetAttributes(&attr, f);
+    if (err == cudaSuccess)
+        err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most - static_cast<int>(attr.sharedSizeBytes));
+    done[{f, dev}] = err == cudaSuccess;
+    return err;
 }
 #endif
 

@@ -212,16 +212,12 @@ void launch_gather(const ProjectionDev &p, Control *ctl, int grid, cudaStream_t 
         launch_pdl(gather_kernel<kFull>, dim3(grid), dim3(kGatherThreads), smem, s, p, ctl);
 }
 
-cudaError_t set_gather_smem(size_t bytes)
+cudaError_t allow_gather_smem()
 {
-    const int b = static_cast<int>(bytes);
-    cudaError_t err = cudaFuncSetAttribute(gather_kernel<kDict>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(gather_kernel<kDictRep>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(gather_kernel<kHalf>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(gather_kernel<kFull>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    cudaError_t err = allow_dynamic_smem(gather_kernel<kDict>);
+    if (err == cudaSuccess) err = allow_dynamic_smem(gather_kernel<kDictRep>);
+    if (err == cudaSuccess) err = allow_dynamic_smem(gather_kernel<kHalf>);
+    if (err == cudaSuccess) err = allow_dynamic_smem(gather_kernel<kFull>);
     return err;
 }
 
