@@ -1816,10 +1816,17 @@ void Backend::capture_graphs()
     for (int which = 0; which < 2; ++which)
     {
         cudaGraph_t g = nullptr;
+        cudaGetLastError();
         KNP_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
         const uint64_t k = which ? kGraphSteps : 1;
         for (uint64_t i = 0; i < k; ++i) enqueue_step();
-        KNP_CUDA(cudaStreamEndCapture(stream_, &g));
+        // A refused launch would be missing from the graph; the capture is ended either way.
+        const cudaError_t launched = cudaGetLastError();
+        const cudaError_t ended = cudaStreamEndCapture(stream_, &g);
+        if (launched != cudaSuccess && g) cudaGraphDestroy(g);
+        cudaGetLastError();
+        KNP_CUDA(launched);
+        KNP_CUDA(ended);
         cudaGraphExec_t ex = nullptr;
         KNP_CUDA(cudaGraphInstantiate(&ex, g, 0));
         cudaGraphDestroy(g);
@@ -2074,6 +2081,7 @@ void Backend::profile_phases(uint64_t n, float *ms)
         KNP_CUDA(cudaEventRecord(ev[3], stream_));
         StepEnd e{counters_, n_counters_, n_spike_counters_};
         launch_step_end(e, ctl_, stream_);
+        KNP_CUDA(cudaGetLastError());
         KNP_CUDA(cudaEventRecord(ev[4], stream_));
         KNP_CUDA(cudaEventSynchronize(ev[4]));
         for (int k = 0; k < 4; ++k)
