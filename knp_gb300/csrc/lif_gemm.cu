@@ -443,7 +443,8 @@ int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, int w
     // apart and added in the same order, so that I has the same bits.
     const long long tiles = ((static_cast<long long>(a.T) * a.B + 127) / 128) * ((a.N + 127) / 128);
     a.splits = gemm_splits(static_cast<int>(std::min<long long>(tiles, 1 << 20)), a.chunks, sms, a.cps);
-    a.n_tiles = (a.N + 255) / 256;
+    // The backward writes its rows up to their width, which a caller may have chosen above the neurons' last tile.
+    a.n_tiles = ((backward ? std::max(a.N, a.w2) : a.N) + 255) / 256;
     auto plan = [&](int cols)
     {
         a.half_cols = cols;
