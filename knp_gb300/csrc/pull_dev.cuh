@@ -357,11 +357,9 @@ __device__ __forceinline__ void gather_block(const ProjectionDev &p, unsigned lo
         for (uint32_t i = threadIdx.x; i < n_acc; i += blockDim.x)
         {
             const uint32_t j = w0 * kPullWindow + i;
-            if (j >= g.n_post || acc[i] == 0.0f) continue;
-            if (g.split_delays)
-                atomicAdd(ring + j, acc[i]);  // the window may be another block's too
-            else
-                ring[j] = __fadd_rn(ring[j], acc[i]);
+            // The window may be another block's too: of this projection where delays are split, or of another
+            // projection into the same population, whose gather the grid kernel runs without waiting for this one.
+            if (j < g.n_post && acc[i] != 0.0f) atomicAdd(ring + j, acc[i]);
         }
     }
     clear_bitmap_slot(g, tn, block, G);
