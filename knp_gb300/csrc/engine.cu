@@ -1579,7 +1579,6 @@ void Backend::setup_ring_window()
 // counter array and a second spike list per population.
 void Backend::build_small_net()
 {
-    small_cluster_ = small_net_cluster();
     if (!counters_alt_)
     {
         counters_alt_ = arena_.make<uint32_t>(std::max<uint32_t>(n_counters_, 1));
@@ -1680,6 +1679,7 @@ void Backend::build_small_net()
         KNP_CUDA(cudaMemcpy(const_cast<SmallSource *>(small_.sources[set]), sources.data(),
                             sources.size() * sizeof(SmallSource), cudaMemcpyHostToDevice));
     }
+    if (fused_) small_cluster_ = small_net_cluster(small_);
 }
 
 // ------------------------------------------------------------------------------------ stepping

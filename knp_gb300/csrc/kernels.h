@@ -455,8 +455,8 @@ void launch_stdp_modify(const StdpDev &d, Control *ctl, cudaStream_t s);
 void launch_step_end(const StepEnd &e, Control *ctl, cudaStream_t s);
 // Runs n_steps whole steps of a small network in one launch of one cluster of `cluster` CTAs
 // (advances Control::step). small_net_cluster() is the largest cluster size (16, 8, 4, 2 or 1) the
-// device can schedule for it.
-int small_net_cluster();
+// device can schedule with the shared memory that the network's launches take.
+int small_net_cluster(const SmallNet &net);
 cudaError_t launch_small_net(const SmallNet &net, Control *ctl, uint32_t n_steps, int cluster, cudaStream_t s);
 // Runs n_steps whole steps of a network in one cooperative launch of `ctas` CTAs (advances
 // Control::step). grid_net_ctas(smem) is the CTA count (one per SM) when the kernel fits with `smem`

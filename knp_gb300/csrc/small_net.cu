@@ -289,23 +289,49 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_net_kernel(SmallNet ne
 
 }  // namespace
 
-int small_net_cluster()
+namespace
 {
-    // 16 CTAs are more than the portable size: allowed per device, so asked for and set for the current one.
-    if (cudaFuncSetAttribute(small_net_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        cudaGetLastError();
+
+// Shared memory of a launch beside the kernel's own: the copies, as far as they fit.
+struct SmallSmem
+{
+    size_t desc, lists;
+    explicit SmallSmem(const SmallNet &net) : desc(desc_copy_bytes(net)), lists(2 * static_cast<size_t>(net.list_words) * 4)
+    {
+        if (desc > kDescCopyMax) desc = 0;
+        if (!desc || lists > kListMax) lists = 0;
+    }
+};
+
+cudaLaunchConfig_t small_net_config(const SmallSmem &smem, int cluster, cudaStream_t s, cudaLaunchAttribute *attr)
+{
     cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster);
     cfg.blockDim = dim3(kSmallThreads);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
+    cfg.dynamicSmemBytes = smem.desc + smem.lists;
+    cfg.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = cluster;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    return cfg;
+}
+
+}  // namespace
+
+int small_net_cluster(const SmallNet &net)
+{
+    // 16 CTAs are more than the portable size: allowed per device, so asked for and set for the current one.
+    if (cudaFuncSetAttribute(small_net_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        allow_dynamic_smem(small_net_kernel) != cudaSuccess)
+        cudaGetLastError();
+    const SmallSmem smem(net);
     for (int size = 16; size > 1; size /= 2)
     {
-        cfg.gridDim = dim3(size);
-        attr[0].val.clusterDim.x = size;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = small_net_config(smem, size, nullptr, &attr);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, small_net_kernel, &cfg) == cudaSuccess && n > 0) return size;
         cudaGetLastError();
@@ -316,29 +342,11 @@ int small_net_cluster()
 cudaError_t launch_small_net(const SmallNet &net, Control *ctl, uint32_t n_steps, int cluster, cudaStream_t s)
 {
     if (!n_steps) return cudaSuccess;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(cluster);
-    cfg.blockDim = dim3(kSmallThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    size_t desc = desc_copy_bytes(net), lists = 2 * static_cast<size_t>(net.list_words) * 4;
-    if (desc > kDescCopyMax) desc = 0;
-    if (!desc || lists > kListMax) lists = 0;
-    cfg.dynamicSmemBytes = desc + lists;
-    if (cfg.dynamicSmemBytes > 32 * 1024)
-    {
-        const cudaError_t err = cudaFuncSetAttribute(small_net_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(kDescCopyMax + kListMax));
-        if (err != cudaSuccess) return err;
-    }
-    return cudaLaunchKernelEx(&cfg, small_net_kernel, net, ctl, n_steps, static_cast<uint32_t>(desc),
-                              static_cast<uint32_t>(lists));
+    const SmallSmem smem(net);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = small_net_config(smem, cluster, s, &attr);
+    return cudaLaunchKernelEx(&cfg, small_net_kernel, net, ctl, n_steps, static_cast<uint32_t>(smem.desc),
+                              static_cast<uint32_t>(smem.lists));
 }
 
 }  // namespace knp_gb300
