@@ -151,7 +151,8 @@ class LIFLayerFn(torch.autograd.Function):
             _capi.check(_capi.lib().knp_gb300_lif_layer_forward(
                 a.data_ptr(), wb.data_ptr(), S.data_ptr(), ckpt.data_ptr(), T, B, n_in, a.shape[1], n_out, w2, wb.shape[1],
                 beta, theta, checkpoint, _err_word(dev).data_ptr(), _stream()))
-            saved = (a, wb)
+            # The last two are not read: autograd refuses the backward if either was changed in place since.
+            saved = (a, wb, w_master, s_in)
         else:
             wb = w_master.to(torch.bfloat16)  # [n_in, n_out]
             s_terms = bf16_terms(s_in.reshape(T * B, n_in), 3 if relaxed else 1)  # 0/1 spikes are exact
@@ -170,7 +171,7 @@ class LIFLayerFn(torch.autograd.Function):
         dS = dS.contiguous()
         ds_in = None
         if fused:
-            a, wb = saved
+            a, wb = saved[:2]
             k8, w2, wp = a.shape[1], _round8(n_out), wb.shape[1]
             dev, err, st, lib = a.device, _err_word(a.device).data_ptr(), _stream(), _capi.lib()
             # The product is recomputed, not stored; dI comes out as rows of two BF16 halves [hi | lo].
