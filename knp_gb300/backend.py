@@ -72,6 +72,8 @@ class GB300Backend:
         _capi.check(rc)
 
     def _uid(self, uid: bytes):
+        if type(uid) is not bytes:  # a buffer's contents may change from call to call
+            return T.to_c_uid(uid)
         c = self._uids.get(uid)
         if c is None:
             c = self._uids[uid] = T.to_c_uid(uid)
