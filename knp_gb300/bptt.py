@@ -57,8 +57,8 @@ def _err_word(device) -> torch.Tensor:
 def check_gemm_errors(device="cuda"):
     """Raises if a GEMM of this module reported a timeout on `device` (one device-to-host read)."""
     device = torch.device(device)
-    if device.index is None:
-        device = torch.device(device.type, torch.cuda.current_device())
+    if device.type == "cuda" and device.index is None:
+        device = torch.device("cuda", torch.cuda.current_device())
     e = _err_word(device)
     if int(e.item()) != 0:
         e.zero_()

@@ -28,3 +28,9 @@ def test_a_uid_in_a_buffer_is_read_at_every_call():
     assert bytes(b._uid(buf).bytes) == bytes(range(16))
     buf[0] = 200
     assert bytes(b._uid(buf).bytes)[0] == 200
+
+
+def test_gemm_errors_are_checked_without_a_gpu():
+    from knp_gb300 import bptt
+
+    bptt.check_gemm_errors("cpu")  # nothing ran there
