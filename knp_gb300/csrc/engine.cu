@@ -1870,6 +1870,18 @@ void Backend::stage_host_inputs()
     {
         if (!c->has_pending) continue;
         const uint64_t n = c->pending.size();
+        if (c->scheduled || c->owns_generated)
+        {
+            // The message takes the schedule's place.
+            KNP_CUDA(cudaStreamSynchronize(stream_));
+            if (c->idx && c->owns_generated) cudaFree(c->idx);
+            else if (c->idx) arena_.release(c->idx);
+            if (c->offsets) arena_.release(c->offsets);
+            c->idx = nullptr;
+            c->offsets = nullptr;
+            c->cap_idx = c->cap_steps = 0;
+            c->scheduled = c->owns_generated = false;
+        }
         if (n <= ChannelMessage::kMost)
         {
             // Descriptor, offsets and indexes in one copy (three small copies cost a step several microseconds).
@@ -1881,26 +1893,22 @@ void Backend::stage_host_inputs()
             std::copy(c->pending.begin(), c->pending.end(), m.idx);
             const size_t bytes = offsetof(ChannelMessage, idx) + n * 4;
             KNP_CUDA(cudaMemcpyAsync(d, stage(&m, bytes), bytes, cudaMemcpyHostToDevice, stream_));
-            c->scheduled = false;
             c->pending.clear();
             c->has_pending = false;
             continue;
         }
-        if (n > c->cap_idx || c->cap_steps < 1 || c->scheduled || c->owns_generated)
+        if (n > c->cap_idx || c->cap_steps < 1)
         {
             KNP_CUDA(cudaStreamSynchronize(stream_));
-            if (c->idx && !c->owns_generated) arena_.release(c->idx);
-            if (c->idx && c->owns_generated) cudaFree(c->idx);
+            if (c->idx) arena_.release(c->idx);
             if (c->offsets) arena_.release(c->offsets);
             c->cap_idx = std::max<uint64_t>(n * 2, 1024);
             c->cap_steps = 1;
             c->idx = arena_.make<uint32_t>(c->cap_idx, false);
             c->offsets = arena_.make<long long>(2);
-            c->owns_generated = false;
         }
         const long long offs[2] = {0, static_cast<long long>(n)};
         c->host = ChannelDev{step_, 1, c->offsets, c->idx};
-        c->scheduled = false;
         char *a = stage(offs, sizeof(offs));
         KNP_CUDA(cudaMemcpyAsync(c->offsets, a, sizeof(offs), cudaMemcpyHostToDevice, stream_));
         if (n)
