@@ -2149,7 +2149,17 @@ void Backend::drain_recordings(uint64_t upto)
     const uint64_t steps = upto - drained_to_;
     cudaStream_t cs = by_event ? copy_stream_ : stream_;
     if (by_event) KNP_CUDA(cudaStreamWaitEvent(copy_stream_, step_ev_[ev], 0));
-    auto as_lists = [&](const PopulationSlot &q) { return !by_event && q.rec_words >= kReadbackSegWords && steps <= 65535; };
+    // Two kernels and their wait (12 us) against 5 ns a word for copying and scanning: 30 us and 17 for one step of
+    // 40000 neurons, equal at 200000, 31 and 98 at 10^6. Steps of more spikes than words, which the kernels give
+    // up after counting, are copied one by one (500000 neurons of which a tenth fire: 195 us a step against 184),
+    // unless there are enough words for the count to pay (four steps of 10^6: 347 us against 375).
+    constexpr uint64_t kListWords = 8192, kCountWords = 65536;
+    auto as_lists = [&](const PopulationSlot &q)
+    {
+        const uint64_t words = steps * q.rec_words;
+        return !by_event && q.rec_words >= kReadbackSegWords && steps <= 65535 &&
+               words >= (q.rec_dense ? kCountWords : kListWords) && (!q.rec_dense || q.rec_words >= kCountWords / 4);
+    };
     // Every recorded population's steps go to their own span of the pinned buffer, then the control
     // block; one wait for all of them.
     size_t need = 0, segs = 0;
@@ -2245,6 +2255,7 @@ void Backend::drain_recordings(uint64_t upto)
         const size_t W = q->rec_words;
         const bool lists = as_lists(*q);
         const uint32_t S = lists ? readback_segments(q->rec_words) : 0u;
+        uint64_t dense = 0;
         for (uint64_t k = 0; k < steps; ++k, coff += S)
         {
             const uint64_t step = drained_to_ + k;
@@ -2265,6 +2276,7 @@ void Backend::drain_recordings(uint64_t upto)
                     if (i % (kExpandBlockWords / kReadbackSegWords) == 0) r.block_prefix.push_back(c);
                     c += rec_counts_host_[coff + i];
                 }
+                ++dense;
                 continue;
             }
             r.data.assign(bits, bits + W);
@@ -2283,7 +2295,9 @@ void Backend::drain_recordings(uint64_t upto)
                 if (w % kExpandBlockWords == 0) r.block_prefix[w / kExpandBlockWords] = r.count;
                 r.count += static_cast<uint32_t>(__builtin_popcount(bits[w]));
             }
+            dense += r.count > W ? 1 : 0;
         }
+        q->rec_dense = 2 * dense > steps;
         off += static_cast<size_t>(steps) * W;
     }
     drained_to_ = upto;

@@ -146,6 +146,7 @@ struct PopulationSlot
     // recorded spikes drained to the host: per step, the spike bitmap and its count
     std::map<uint64_t, RecordedStep> recorded;
     uint64_t record_from = 0;
+    bool rec_dense = false;  // most steps of the last read-back had more spikes than bitmap words
     // SynapticResourceSTDPDeltaSynapse projections into this population (load order) and their
     // concatenated synapse arrays; the training runs for resource-STDP BLIFAT populations.
     std::vector<ProjectionSlot *> res_projs;
