@@ -2130,12 +2130,24 @@ void Backend::record_step_event(uint64_t last_step)
     step_ev_of_[slot] = last_step + 1;
 }
 
+// Steps that one read brings over at most, its own among them. A window's steps are mostly read in their order, and
+// together they take one wait; a read of an early step alone pays for the rest, 0.1 us a step of 1000 neurons, 0.3 of
+// 40000, 0.7 of 10^6. So 4 MB of bitmaps, a step counted as 16 KB at least: some 60 us at most (a whole
+// recording ring of 40000 neurons took 1.3 ms).
+uint64_t Backend::read_ahead() const
+{
+    uint64_t step_bytes = 16 << 10;
+    for (auto &q : pops_)
+        if (q->record && q->rec_bits) step_bytes += q->rec_words * 4ull;
+    return std::max<uint64_t>(1, (4 << 20) / step_bytes);
+}
+
 // Brings the recorded steps [drained_to_, upto) to the host: read_spikes hands out a step's ascending
 // indexes, the order of the reference's SpikeMessage (populations_old.h:104-118).
 //
 // Steps queued after step upto - 1 keep running: when that step's completion event is at hand, the
 // bitmaps are copied (by the copy engine, on copy_stream_) once it has fired, and the host expands them.
-// Otherwise the stream is waited for, so everything recorded is brought over at once, and for large
+// Otherwise the stream is waited for, so the steps after it are brought over with it (read_ahead), and for large
 // populations the device turns the bitmaps into index lists first (readback.cu): the step kernels leave
 // no room for that while they run. 20 steps of 10^6 neurons, 5300 spikes each: 2.9 ms with bitmaps copied
 // step by step and counted and scanned on the host; with lists a window and its reads take 1.95 ms instead of 3.85.
@@ -2145,7 +2157,7 @@ void Backend::drain_recordings(uint64_t upto)
     if (upto <= drained_to_) return;
     const uint64_t ev = (upto - 1) % kStepEvents;
     const bool by_event = upto < step_ && step_ev_of_[ev] == upto;
-    if (!by_event) upto = step_;
+    if (!by_event) upto = std::min(step_, std::max(upto, drained_to_ + read_ahead()));
     const uint64_t steps = upto - drained_to_;
     cudaStream_t cs = by_event ? copy_stream_ : stream_;
     if (by_event) KNP_CUDA(cudaStreamWaitEvent(copy_stream_, step_ev_[ev], 0));

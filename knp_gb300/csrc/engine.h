@@ -324,6 +324,7 @@ private:
     void stage_host_inputs();
     void drain_recordings() { drain_recordings(step_); }
     void drain_recordings(uint64_t upto);
+    uint64_t read_ahead() const;
     void check_device_error();
     void alloc_recording(PopulationSlot &p);
     uint64_t steps_before_drain() const;

@@ -63,3 +63,29 @@ def test_one_step_of_few_words_does_not_pay_for_lists():
         times.append(np.median(took[20:]))
         b.close()
     assert times[1] < 1.4 * times[0], times
+
+
+def test_a_read_of_an_early_step_leaves_most_of_a_long_window_for_later():
+    """600 steps of 200000 neurons (15 MB of bitmaps): the first step's read takes less than what is left then."""
+    n, steps = 200000, 600
+    b, pop, chan = _backend(n)
+    out = np.zeros(n, np.uint32)
+    first, rest = [], []
+    for w in range(3):
+        t = b.get_step()
+        b.generate_bernoulli_schedule(chan, n, 0.005, t, steps, 3 + w)
+        b.step(steps)
+        b.synchronize()
+        t0 = time.perf_counter()
+        n_first = b.spikes_capped(pop, t + 1, out)
+        t1 = time.perf_counter()
+        b.spikes_capped(pop, t + steps - 1, out)
+        t2 = time.perf_counter()
+        first.append(t1 - t0)
+        rest.append(t2 - t1)
+        assert 0 < n_first < 0.01 * n
+        for k in (2, 90, 99, 100, 101, 102, 103, 300, steps - 1):  # either side of what the first read brought
+            assert 0 < b.spikes_capped(pop, t + k, out) < 0.01 * n
+        b.discard_spikes(t + steps)
+    assert min(first) < min(rest), (first, rest)
+    b.close()
