@@ -1013,7 +1013,9 @@ void Backend::build_projection(ProjectionSlot &p)
     ProjectionDev &d = p.dev;
     d.row_ptr = p.row_ptr;
     d.n_rows = p.n_rows;
-    d.short_rows = p.n_syn <= 2 * static_cast<uint64_t>(p.n_rows) ? 1 : 0;
+    uint32_t longest = 0;
+    if (p.n_syn <= 2 * static_cast<uint64_t>(p.n_rows)) KNP_CUDA(longest_row(p.row_ptr, p.n_rows, &longest, stream_));
+    d.short_rows = p.n_syn <= 2 * static_cast<uint64_t>(p.n_rows) && longest <= kShortRow ? 1 : 0;
     d.col = p.col;
     d.w = p.w;
     d.delay = p.delay_d;

@@ -136,6 +136,16 @@ __global__ void __launch_bounds__(256) projection_batch_kernel(const __grid_cons
         project_block<false, false>(p, ctl, block, n_blocks, block_events);
 }
 
+__global__ void longest_row_kernel(const long long *row_ptr, uint32_t n_rows, unsigned int *longest)
+{
+    unsigned int most = 0;
+    for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r < n_rows;
+         r += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+        most = max(most, static_cast<unsigned int>(min(row_ptr[r + 1] - row_ptr[r], 0xFFFFFFFFll)));
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most) atomicMax(longest, most);
+}
+
 // Random FP32 adds of 1/256 into buf[0, n), n < 2^32: thread g's i-th add goes to position
 // floor(h * n / 2^32) of the 32-bit hash h = mix64(seed, g, i) (a multiply, not a division).
 __global__ void add_rate_kernel(float *buf, uint32_t n, uint32_t per, unsigned long long seed)
@@ -215,6 +225,24 @@ void launch_projection(const ProjectionDev &p, Control *ctl, int grid, cudaStrea
 void launch_projection_batch(const ProjectionBatch &b, Control *ctl, cudaStream_t s)
 {
     launch_pdl(projection_batch_kernel, dim3(b.blocks()), dim3(256), 0, s, b, ctl);
+}
+
+cudaError_t longest_row(const long long *row_ptr, uint32_t n_rows, uint32_t *longest, cudaStream_t s)
+{
+    unsigned int *d = nullptr;
+    cudaError_t err = cudaMallocAsync(reinterpret_cast<void **>(&d), sizeof(*d), s);
+    if (err != cudaSuccess) return err;
+    err = cudaMemsetAsync(d, 0, sizeof(*d), s);
+    if (err == cudaSuccess)
+    {
+        const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((n_rows + 255ull) / 256, 1024));
+        longest_row_kernel<<<std::max(blocks, 1u), 256, 0, s>>>(row_ptr, n_rows, d);
+        err = cudaGetLastError();
+    }
+    if (err == cudaSuccess) err = cudaMemcpyAsync(longest, d, sizeof(*d), cudaMemcpyDeviceToHost, s);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+    cudaFreeAsync(d, s);
+    return err;
 }
 
 }  // namespace knp_gb300

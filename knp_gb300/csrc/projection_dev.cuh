@@ -145,45 +145,27 @@ __device__ __forceinline__ unsigned long long scatter_rows(
     {
         // Rows of a synapse or two (one-to-one drive): a lane per row, so that a warp has 32 rows' chains of
         // loads in flight instead of one (200k neurons, 60k spikes a step: 41 -> 16 us for the phase with
-        // the bitmap below). A longer row among them is taken by the whole warp.
-        for (uint32_t j0 = 32u * warp; j0 < total; j0 += 32u * n_warps)
+        // the bitmap below).
+        for (uint32_t j = 32u * warp + lane; j < total; j += 32u * n_warps)
         {
-            uint32_t jj = j0 + lane;
-            int64_t a = 0, b = 0;
-            if (jj < total)
+            uint32_t jj = j;
+            int k = 0;
+            while (jj >= cnt[k])
             {
-                int k = 0;
-                while (jj >= cnt[k])
-                {
-                    jj -= cnt[k];
-                    ++k;
-                }
-                const uint32_t pre = idx[k][jj];
-                if (pre < p.n_rows)
-                {
-                    a = p.row_ptr[pre];
-                    b = p.row_ptr[pre + 1];
-                }
+                jj -= cnt[k];
+                ++k;
             }
+            const uint32_t pre = idx[k][jj];
+            if (pre >= p.n_rows) continue;
+            const int64_t a = p.row_ptr[pre], b = p.row_ptr[pre + 1];
             events += static_cast<unsigned long long>(b - a);
-            const bool is_long = b - a > 8;
-            if (!is_long)
-                for (int64_t e = a; e < b; ++e)
-                {
-                    const int ty = kUniformExc ? 0 : (p.type ? __ldg(p.type + e) : p.uniform_type);
-                    deliver<kFixed, kUniformExc>(p, slot_base, e, __ldg(p.col + e), p.w[e], __ldg(p.delay + e), ty);
-                }
-            for (uint32_t m = __ballot_sync(0xffffffffu, is_long); m; m &= m - 1u)
+            for (int64_t e = a; e < b; ++e)
             {
-                const int src = __ffs(m) - 1;
-                const int64_t la = __shfl_sync(0xffffffffu, a, src), lb = __shfl_sync(0xffffffffu, b, src);
-                for (int64_t e = la + lane; e < lb; e += 32)
-                {
-                    const int ty = kUniformExc ? 0 : (p.type ? __ldg(p.type + e) : p.uniform_type);
-                    deliver<kFixed, kUniformExc>(p, slot_base, e, __ldg(p.col + e), p.w[e], __ldg(p.delay + e), ty);
-                }
+                const int ty = kUniformExc ? 0 : (p.type ? __ldg(p.type + e) : p.uniform_type);
+                deliver<kFixed, kUniformExc>(p, slot_base, e, __ldg(p.col + e), p.w[e], __ldg(p.delay + e), ty);
             }
         }
+        __syncwarp();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) events += __shfl_xor_sync(0xffffffffu, events, o);
         return events;
