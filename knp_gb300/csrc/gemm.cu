@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
 // cost 2.2 ms at 8192^3.
 constexpr int kPairM = 256, kPairN = 256, kPairStages = 6, kPairBand = 8;
 constexpr uint32_t kPairStage = 2 * kTileBytes;  // this CTA's 128 x 64 of A and of B
-constexpr uint32_t kPairSmem = kPairStages * kPairStage + 1024;
+constexpr uint32_t kTurn = 32 * 33 * 4;  // a read-back warp's 32 x 32 of the accumulator, rows 33 words apart
+constexpr uint32_t kPairSmem = kPairStages * kPairStage + 1024 + 4 * kTurn;
 constexpr uint32_t kDrainWait = 1u << 14;  // polls, about 0.06 s
 constexpr int kPairThreads = 224;  // warps 0-3 read back, 4 and 6 load A and B, 5 issues (even rank)
 
@@ -577,8 +578,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
     }
     else
     {
-        // Read-back: thread t of the CTA has accumulator lane t, row m0 + 128 rank + t of the tile.
+        // Read-back: thread t of the CTA has accumulator lane t, row m0 + 128 rank + t of the tile. Where D's rows are
+        // whole 16-byte units a thread stores its row; else a warp turns its 32 x 32 values in shared memory and
+        // stores row after row, 128 bytes at a time: a thread's 4-byte stores touch 32 rows at a time (8192 x 8190 x 64:
+        // 410 us that way, 76 so; 8192 x 8190 x 8192: 768 and 628). Turned, whole rows are no better where the product
+        // carries the time (2500^3: 83 us against 79; 16384 x 2048 x 2048: 91.5 against 89.7).
         const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
+        float *turn = reinterpret_cast<float *>(smem + (base - tc::smem_u32(smem)) + kPairStages * kPairStage + warp * kTurn);
         int n = 0;
         for (int t = pair; t < tiles; t += pairs, ++n)
         {
@@ -606,22 +612,24 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&acc_empty[a]), 0));
                 }
-                if (row >= M)
+                if (vec && n0 + q0 + 32 <= N)
                 {
-                }
-                else if (vec && n0 + q0 + 32 <= N)
-                {
+                    if (row < M)
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        reinterpret_cast<float4 *>(d + q0)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                        for (int q = 0; q < 8; ++q)
+                            reinterpret_cast<float4 *>(d + q0)[q] =
+                                make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    __syncwarp();  // the next read is warp-collective
+                    continue;
                 }
-                else
-                {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (n0 + q0 + i < N) d[q0 + i] = v[i];
-                }
-                __syncwarp();  // the next read is warp-collective
+                for (int i = 0; i < 32; ++i) turn[lane * 33 + i] = v[i];
+                __syncwarp();
+                const int col = n0 + q0 + lane, rows = min(32, M - (row - lane));
+                float *out = D + static_cast<size_t>(row - lane) * N + col;
+                if (col < N)
+                    for (int r = 0; r < rows; ++r) out[static_cast<size_t>(r) * N] = turn[r * 33 + lane];
+                __syncwarp();
             }
         }
     }
