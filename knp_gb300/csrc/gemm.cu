@@ -290,7 +290,7 @@ constexpr uint32_t kTmaSmem = kTmaStages * kStageBytes + 1024;  // + alignment s
 // One 128 x 128 tile of D (or of split blockIdx.z's partial, into `out` with row stride N) over
 // chunks [blockIdx.z * cps, min(nk, (blockIdx.z + 1) * cps)). Warp 0 lane 0 issues the TMA copies,
 // warp 1 lane 0 the MMAs; all four warps read the accumulator back.
-template <bool kMn>
+template <bool kAMn, bool kBMn>
 __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     const __grid_constant__ GemmMaps maps, float *__restrict__ out, int M,
     int N, KPlan kp, int cps, size_t split_stride, unsigned int *err)
@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
             }
             const uint32_t sa = base + s * kStageBytes;
             tc::mbar_expect_tx(&full[s], kStageBytes);
-            load_operand<kMn, false>(sa, &maps.a, &maps.a8, c, kp.half, kp.a_step, m0, 0u, &full[s]);
-            load_operand<kMn, false>(sa + kTileBytes, &maps.b, &maps.b8, c, kp.half, kp.b_step, n0, 0u, &full[s]);
+            load_operand<kAMn, false>(sa, &maps.a, &maps.a8, c, kp.half, kp.a_step, m0, 0u, &full[s]);
+            load_operand<kBMn, false>(sa + kTileBytes, &maps.b, &maps.b8, c, kp.half, kp.b_step, n0, 0u, &full[s]);
             issued = i + 1;
         }
         // Copies still in flight after a failed wait land before the CTA leaves (bounded).
@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
     }
     else if (warp == 1 && lane == 0)
     {
-        constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kBN) | (kMn ? tc::kIdescAMn | tc::kIdescBMn : 0u);
+        constexpr uint32_t idesc =
+            tc::idesc_bf16_f32(kBM, kBN) | (kAMn ? tc::kIdescAMn : 0u) | (kBMn ? tc::kIdescBMn : 0u);
         for (int c = c0; c < c1; ++c)
         {
             const int i = c - c0, s = i % kTmaStages;
@@ -359,8 +360,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
             const uint32_t sa = base + s * kStageBytes, sb = sa + kTileBytes;
 #pragma unroll
             for (int j = 0; j < kBK / 16; ++j)
-                tc::mma_bf16(tmem, operand_desc<kMn>(sa) + j * kDescStep<kMn>, operand_desc<kMn>(sb) + j * kDescStep<kMn>,
-                             idesc, (i > 0 || j > 0) ? 1u : 0u);
+                tc::mma_bf16(tmem, operand_desc<kAMn>(sa) + j * kDescStep<kAMn>,
+                             operand_desc<kBMn>(sb) + j * kDescStep<kBMn>, idesc, (i > 0 || j > 0) ? 1u : 0u);
             tc::commit(&empty[s]);
         }
         tc::commit(&acc_full);
@@ -428,7 +429,7 @@ constexpr uint32_t kPairSmem = kPairStages * kPairStage + 1024 + 4 * kTurn;
 constexpr uint32_t kDrainWait = 1u << 14;  // polls, about 0.06 s
 constexpr int kPairThreads = 224;  // warps 0-3 read back, 4 and 6 load A and B, 5 issues (even rank)
 
-template <bool kMn>
+template <bool kAMn, bool kBMn>
 __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gemm_pair_kernel(
     const __grid_constant__ GemmMaps maps, float *__restrict__ D, int M, int N, KPlan kp, unsigned int *err)
 {
@@ -509,8 +510,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                         break;
                     }
                     if (is_a && rank == 0) tc::mbar_expect_tx(&full[s], 2 * kPairStage);
-                    load_operand<kMn, true>(base + s * kPairStage + (is_a ? 0u : kTileBytes), map, map8, c, kp.half, step, r0,
-                                            full0 + s * 8u, nullptr);
+                    const uint32_t dst = base + s * kPairStage + (is_a ? 0u : kTileBytes);
+                    if (is_a ? kAMn : kBMn)
+                        load_operand<true, true>(dst, map, map8, c, kp.half, step, r0, full0 + s * 8u, nullptr);
+                    else
+                        load_operand<false, true>(dst, map, map8, c, kp.half, step, r0, full0 + s * 8u, nullptr);
                     ++issued;
                     if (++s == kPairStages)
                     {
@@ -531,8 +535,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
         if (lane == 0 && rank == 0)
         {
             constexpr uint32_t idesc =
-                tc::idesc_bf16_f32(kPairM, kPairN) | (kMn ? tc::kIdescAMn | tc::kIdescBMn : 0u);
-            const uint64_t da = operand_desc<kMn>(base), db = operand_desc<kMn>(base + kTileBytes);
+                tc::idesc_bf16_f32(kPairM, kPairN) | (kAMn ? tc::kIdescAMn : 0u) | (kBMn ? tc::kIdescBMn : 0u);
+            const uint64_t da = operand_desc<kAMn>(base), db = operand_desc<kBMn>(base + kTileBytes);
             int s = 0, n = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -555,7 +559,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1) gem
                     const uint64_t off = static_cast<uint64_t>(s) * (kPairStage >> 4);
 #pragma unroll
                     for (int j = 0; j < kBK / 16; ++j)
-                        tc::mma_bf16_pair(tmem + a * kPairN, da + off + j * kDescStep<kMn>, db + off + j * kDescStep<kMn>,
+                        tc::mma_bf16_pair(tmem + a * kPairN, da + off + j * kDescStep<kAMn>, db + off + j * kDescStep<kBMn>,
                                           idesc, (c > 0 || j > 0) ? 1u : 0u);
                     tc::commit_pair(&empty[s]);
                     if (++s == kPairStages)
@@ -765,8 +769,8 @@ int gemm_splits(int tiles, int nk, int sms, int &cps)
 namespace
 {
 
-// D[M x N] from operands that are both K-major or (kMn) both MN-major.
-template <bool kMn>
+// D[M x N] from operands that are K-major or (kAMn, kBMn) MN-major.
+template <bool kAMn, bool kBMn>
 int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned int *d_err, cudaStream_t s)
 {
     int dev = 0, sms = 0;
@@ -781,12 +785,12 @@ int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned
     const int waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
     if (pair_waves < waves)
     {
-        if (allow_dynamic_smem(gemm_pair_kernel<kMn>) != cudaSuccess) return -3;
-        launch_pdl(gemm_pair_kernel<kMn>, dim3(2 * std::min(pair_tiles, sms / 2)), dim3(kPairThreads), kPairSmem, s, maps, D, M, N,
+        if (allow_dynamic_smem(gemm_pair_kernel<kAMn, kBMn>) != cudaSuccess) return -3;
+        launch_pdl(gemm_pair_kernel<kAMn, kBMn>, dim3(2 * std::min(pair_tiles, sms / 2)), dim3(kPairThreads), kPairSmem, s, maps, D, M, N,
                    kp, d_err);
         return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
-    if (allow_dynamic_smem(gemm_tma_kernel<kMn>) != cudaSuccess) return -3;
+    if (allow_dynamic_smem(gemm_tma_kernel<kAMn, kBMn>) != cudaSuccess) return -3;
     int cps = 0;
     int splits = gemm_splits(tiles, kp.nk, sms, cps);
     const size_t mn = static_cast<size_t>(M) * N;
@@ -804,7 +808,7 @@ int launch_gemm(const GemmMaps &maps, float *D, int M, int N, KPlan kp, unsigned
     }
     const int cps_used = splits > 1 ? cps : kp.nk;
     dim3 grid(tiles_m, tiles_n, splits);
-    launch_pdl(gemm_tma_kernel<kMn>, grid, dim3(kTmaThreads), kTmaSmem, s, maps, splits > 1 ? ws : D, M, N, kp, cps_used,
+    launch_pdl(gemm_tma_kernel<kAMn, kBMn>, grid, dim3(kTmaThreads), kTmaSmem, s, maps, splits > 1 ? ws : D, M, N, kp, cps_used,
                splits > 1 ? mn : 0, d_err);
     if (splits > 1)
     {
@@ -826,7 +830,7 @@ int bf16_gemm_tn(const void *A, const void *B, float *D, int M, int N, int K, un
     if (!aligned) return bf16_gemm_tn_simple(A, B, D, M, N, K, d_err, s);
     GemmMaps maps{};
     if (sw128_map(&maps.a, A, M, K, kBM) && sw128_map(&maps.b, B, N, K, kBN))
-        return launch_gemm<false>(maps, D, M, N, KPlan{(K + kBK - 1) / kBK, kOneHalf, 0, 0}, d_err, s);
+        return launch_gemm<false, false>(maps, D, M, N, KPlan{(K + kBK - 1) / kBK, kOneHalf, 0, 0}, d_err, s);
     if (allow_dynamic_smem(gemm_pipe_kernel) != cudaSuccess) return -3;
     dim3 grid((M + kBM - 1) / kBM, (N + kBN - 1) / kBN);
     gemm_pipe_kernel<<<grid, kThreads, kStages * kStageBytes, s>>>(static_cast<const __nv_bfloat16 *>(A),
@@ -847,7 +851,7 @@ int lif_ds_gemm(const void *dI2, const void *W, float *ds, int rows, int n_in, i
     if (w2 % kBK) return -1;
     GemmMaps maps{};
     if (!sw128_map(&maps.a, dI2, rows, 2 * w2, kBM) || !sw128_map(&maps.b, W, n_in, w2, kBN)) return -3;
-    return launch_gemm<false>(maps, ds, rows, n_in, KPlan{2 * w2 / kBK, w2, w2, 0}, d_err, s);
+    return launch_gemm<false, false>(maps, ds, rows, n_in, KPlan{2 * w2 / kBK, w2, w2, 0}, d_err, s);
 }
 
 int lif_dw_gemm(const void *S, const void *dI2, float *dW, int rows, int n_in, int n_in8, int n_out, int w2,
@@ -858,6 +862,23 @@ int lif_dw_gemm(const void *S, const void *dI2, float *dW, int rows, int n_in, i
     if (!sw128_map(&maps.a, S, rows, n_in8, kBK) || !sw128_map(&maps.b, dI2, rows, 2 * w2, kBK) ||
         !sw128_map(&maps.a8, S, rows, n_in8, 8) || !sw128_map(&maps.b8, dI2, rows, 2 * w2, 8))
         return -3;
-    return launch_gemm<true>(maps, dW, n_in, n_out, KPlan{(2 * padded + kBK - 1) / kBK, padded, 0, w2}, d_err, s);
+    return launch_gemm<true, true>(maps, dW, n_in, n_out, KPlan{(2 * padded + kBK - 1) / kBK, padded, 0, w2}, d_err, s);
+}
+
+// I[rows][N] = S W from S as [rows][k8] (K-major) and W as [K][wp] (MN-major, columns from N on unused).
+int lif_input_gemm(const void *S, const void *W, float *I, int rows, int K, int k8, int N, int wp, unsigned int *d_err,
+                   cudaStream_t s)
+{
+    GemmMaps maps{};
+    if (!sw128_map(&maps.a, S, rows, k8, kBM) || !sw128_map(&maps.b, W, K, wp, kBK)) return -3;
+    return launch_gemm<false, true>(maps, I, rows, N, KPlan{(K + kBK - 1) / kBK, kOneHalf, 0, 0}, d_err, s);
+}
+
+cudaError_t workspace_alloc(void **p, size_t bytes, cudaStream_t s)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const cudaMemPool_t pool = split_pool(dev);
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaErrorMemoryAllocation;
 }
 }  // namespace knp_gb300

@@ -492,6 +492,18 @@ void launch_apply_impacts(
 // sw128_map_3d the (K, t, b) view of rows t * batch + b, loaded in boxes of 64 x box_t x box_b.
 bool sw128_map(void *map, const void *ptr, int rows, int K, int box_rows);
 bool sw128_map_3d(void *map, const void *ptr, int T, int batch, int K, int box_t, int box_b);
+// I[rows][N] (FP32) = S W, S BF16 [rows][k8], W BF16 [K][wp] (gemm.cu); a stream-ordered workspace from the pool of
+// its split sums, given back with cudaFreeAsync.
+int lif_input_gemm(const void *S, const void *W, float *I, int rows, int K, int k8, int N, int wp, unsigned int *d_err,
+                   cudaStream_t s);
+cudaError_t workspace_alloc(void **p, size_t bytes, cudaStream_t s);
+// The LIF recurrence over given inputs, and the BF16 rows of a matrix (bptt.cu).
+int lif_scan_forward(const float *I, float *S, float *ckpt, int T, long long BN, float beta, float theta, int K, int relaxed,
+                     float k, cudaStream_t s);
+int lif_scan_backward(const float *I, const float *ckpt, const float *dS, float *dI, int T, long long BN, float beta,
+                      float theta, int K, int relaxed, float k, cudaStream_t s);
+int bf16_operand(const void *X, int x_bf16, long long R, long long C, int mode, int transpose, long long P, void *out,
+                 cudaStream_t s);
 // Splits of the GEMM's K (gemm.cu): their number, and the chunks of 64 of each.
 int gemm_splits(int tiles, int nk, int sms, int &cps);
 

@@ -13,6 +13,7 @@
 // and scan took 90 + 79 and 90 + 128 us and the gradient's BF16 rows another 53 + 89. The forward is bound by the
 // product beside the stores of S, the backward by the latency of its scan (an IEEE division and two dependent
 // chains a step), hence two sets of scan warps per half (one: 170 us).
+// Layers whose product fills few tiles and has many inputs take product and scan apart instead (apart_is_faster).
 // Columns: a CTA pair takes a tile of 256 neurons (128 a CTA) and two halves of up to 128 columns, one per
 // CTA's share of the spike operand: whole samples while T fits a half (box_b samples of T steps; a 3-D
 // TMA box brings rows (b, t) in that order from [T][B][K]), else one sample's steps tile by tile, forward in
@@ -431,6 +432,49 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
     if (warp == kIssuerWarp) tc::tmem_dealloc_pair(tmem, 512);
 }
 
+// The layer as a product, the scan of bptt.cu and (backward) the gradient's BF16 rows: the same bits.
+int launch_apart(const LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, int wp, bool backward, cudaStream_t s)
+{
+    const int rows = a.T * a.B;
+    const size_t n = (static_cast<size_t>(rows) * a.N + 3) / 4 * 4;
+    const long long BN = static_cast<long long>(a.B) * a.N;
+    float *I = nullptr;
+    if (workspace_alloc(reinterpret_cast<void **>(&I), (backward ? 2 : 1) * n * sizeof(float), s) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return -3;
+    }
+    int rc = lif_input_gemm(S_in, W, I, rows, K, k8, a.N, wp, a.err, s);
+    if (rc == 0 && !backward) rc = lif_scan_forward(I, a.S, a.ckpt, a.T, BN, a.beta, a.theta, a.seg, 0, 0.0f, s);
+    if (rc == 0 && backward)
+    {
+        rc = lif_scan_backward(I, a.ckpt, a.dS, I + n, a.T, BN, a.beta, a.theta, a.seg, 0, a.k, s);
+        if (rc == 0) rc = bf16_operand(I + n, 0, rows, a.N, 2, 0, a.w2, a.dI2, s);
+    }
+    cudaFreeAsync(I, s);
+    return rc;
+}
+
+// Where the product alone would split K over CTAs, a pair here takes the runs one after another, and a time tile after
+// another, while most of the device idles; the product apart takes a run in parallel with the others, and then the scan
+// takes a segment after another on threads that have little else to hide its loads. What either does in sequence, in
+// units of a chunk of a pair's product (0.37 us): fitted to 400 layers of 1..1000 steps, 1..300 samples, 200..8000
+// inputs, 4..2000 neurons and intervals of 1..16 (50 x 2, 5000 -> 300: forward 135 us here, 27 apart; 64 x 8, 2048 -> 10: 37
+// and 22; 27 x 12, 526 -> 1585: 12 and 25; 559 x 1, 561 -> 173, interval 1: 44 and 460). The form taken was the slower one by 8 % or
+// more in one of 20.
+bool apart_is_faster(const LifGemmArgs &a, int waves, bool backward)
+{
+    const long long tiles = static_cast<long long>(waves) * a.t_tiles;
+    const long long samples = tiles * ((a.box_b + 1) / 2);  // that a set of scan warps takes, tile by tile
+    const int t = a.box_t, n_seg = (a.T + a.seg - 1) / a.seg;
+    const int reads = a.splits * (backward ? (a.seg == 8 ? t / 8 + t % 8 : t) : t / 16 + t % 16 / 8 + t % 8);
+    const double here = static_cast<double>(tiles) * a.chunks +
+                        static_cast<double>(samples) * (backward ? reads / 6.0 + 3.0 * ((t + a.seg - 1) / a.seg)
+                                                                 : reads / 7.0 + t / 23.0);
+    const double apart = backward ? 4 + 2.0 * a.cps + 2.5 * n_seg + a.T / 4.0 : 7 + 1.7 * a.cps + 2.0 * n_seg + a.T / 12.0;
+    return here > apart;
+}
+
 int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, int wp, bool backward, cudaStream_t s)
 {
     if (a.T < 1 || a.B < 1 || a.N < 1 || K < 1 || a.seg < 1 || a.seg > kMaxSeg) return -1;
@@ -457,17 +501,24 @@ int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, int w
         a.items = a.n_tiles * ((a.B + 2 * a.box_b - 1) / (2 * a.box_b));
         return (a.items + pairs - 1) / pairs;
     };
+    int waves;
     if (a.splits > 1)
     {
-        plan(a.splits <= 4 ? 64 : a.splits <= 8 ? 32 : 16);  // at most 16 runs: 512 columns
+        waves = plan(a.splits <= 4 ? 64 : a.splits <= 8 ? 32 : 16);  // at most 16 runs: 512 columns
     }
     else
     {
         // Halves of 64 columns when they spread the samples over more of the device: a tile of them takes
         // about half as long, so they win while they need fewer than twice the waves.
-        const int waves = plan(128);
-        if (a.T > 64 || plan(64) >= 2 * waves) plan(128);
+        waves = plan(128);
+        const int narrow = a.T > 64 ? 2 * waves : plan(64);
+        if (narrow < 2 * waves)
+            waves = narrow;
+        else
+            plan(128);
     }
+    // (A product of one wave: its time is one tile's.)
+    if (tiles <= sms && apart_is_faster(a, waves, backward)) return launch_apart(a, S_in, W, K, k8, wp, backward, s);
     if (!sw128_map(&a.w, W, K, wp, 64) || !sw128_map_3d(&a.s, S_in, a.T, a.B, k8, a.box_t, a.box_b)) return -3;
     auto kernel = !backward   ? (a.splits > 1 ? lif_gemm_kernel<false, 0, true> : lif_gemm_kernel<false, 0, false>)
                   : a.seg == 8 ? (a.splits > 1 ? lif_gemm_kernel<true, 8, true> : lif_gemm_kernel<true, 8, false>)
