@@ -517,8 +517,8 @@ int launch(LifGemmArgs &a, const void *S_in, const void *W, int K, int k8, int w
         else
             plan(128);
     }
-    // (A product of one wave: its time is one tile's.)
-    if (tiles <= sms && apart_is_faster(a, waves, backward)) return launch_apart(a, S_in, W, K, k8, wp, backward, s);
+    // (A product of one wave: its time is one tile's. The gradient's rows are stored 16 bytes at a time then.)
+    if (tiles <= sms && (reinterpret_cast<uintptr_t>(a.dI2) & 15u) == 0 && apart_is_faster(a, waves, backward)) return launch_apart(a, S_in, W, K, k8, wp, backward, s);
     if (!sw128_map(&a.w, W, K, wp, 64) || !sw128_map_3d(&a.s, S_in, a.T, a.B, k8, a.box_t, a.box_b)) return -3;
     auto kernel = !backward   ? (a.splits > 1 ? lif_gemm_kernel<false, 0, true> : lif_gemm_kernel<false, 0, false>)
                   : a.seg == 8 ? (a.splits > 1 ? lif_gemm_kernel<true, 8, true> : lif_gemm_kernel<true, 8, false>)

@@ -87,3 +87,33 @@ def test_eight_times_the_inputs_do_not_take_several_times_as_long(T, B, n_out):
                 bptt.LIFLayerFn.apply(x, w, BETA, THETA, 8, False, K)
         took.append(_graph_us(f))
     assert took[1] < 2.5 * took[0], took
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+def test_gradient_rows_at_any_alignment(offset):
+    """The C entry point with rows of dI that start off a 16-byte boundary: the same bits, nothing outside them."""
+    import ctypes
+
+    from knp_gb300 import _capi
+
+    T, B, n_in, N, w2 = 50, 2, 5000, 20, 24
+    g = torch.Generator(device="cuda").manual_seed(1)
+    s_in = (torch.rand(T * B, n_in, generator=g, device="cuda") < 0.01).to(torch.bfloat16)
+    w = torch.zeros(n_in, w2, device="cuda", dtype=torch.bfloat16)
+    w[:, :N] = torch.randn(n_in, N, generator=g, device="cuda") * 0.3
+    S = torch.empty(T, B, N, device="cuda")
+    ckpt = torch.empty(7, B, N, device="cuda")
+    dS = torch.randn(T, B, N, generator=g, device="cuda")
+    err = torch.zeros(1, device="cuda", dtype=torch.int32)
+    lib, st, f = _capi.lib(), torch.cuda.current_stream().cuda_stream, ctypes.c_float
+    _capi.check(lib.knp_gb300_lif_layer_forward(s_in.data_ptr(), w.data_ptr(), S.data_ptr(), ckpt.data_ptr(), T, B, n_in,
+                                                n_in, N, w2, w2, f(0.9), f(1.0), 8, err.data_ptr(), st))
+    rows = []
+    for at in (0, offset):
+        buf = torch.full((T * B * 2 * w2 + 16,), 7.0, device="cuda", dtype=torch.bfloat16)
+        _capi.check(lib.knp_gb300_lif_layer_backward(s_in.data_ptr(), w.data_ptr(), ckpt.data_ptr(), dS.data_ptr(),
+                                                     buf[8 + at:].data_ptr(), T, B, n_in, n_in, N, w2, w2, f(0.9), f(1.0), 8,
+                                                     f(25.0), err.data_ptr(), st))
+        rows.append(buf[8 + at:8 + at + T * B * 2 * w2].clone())
+        assert (buf[:8 + at] == 7.0).all() and (buf[8 + at + T * B * 2 * w2:] == 7.0).all()
+    assert torch.equal(rows[0], rows[1]) and rows[0].any() and int(err.item()) == 0
