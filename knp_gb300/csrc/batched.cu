@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <queue>
 #include <vector>
 
@@ -935,6 +936,49 @@ __global__ void __launch_bounds__(kLayerThreads, 1) __cluster_dims__(2, 1, 1)
     if (warp == kIssuerWarp) tc::tmem_dealloc_pair(tmem, kTmemCols);
 }
 
+// Pinned words that runs leave their totals in: one page of them for the process, handed out two words a plan (pinning
+// a plan's own costs 130 us and unpinning it 160, as much as the rest of a small plan's life); plans past its 256 have
+// their own.
+class PinnedTotals
+{
+public:
+    unsigned long long *take()
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (!page_)
+        {
+            if (cudaHostAlloc(reinterpret_cast<void **>(&page_), kSlots * 16, cudaHostAllocPortable) != cudaSuccess)
+                return page_ = nullptr;
+            for (int i = kSlots; i-- > 0;) free_.push_back(page_ + 2 * i);
+        }
+        unsigned long long *p = nullptr;
+        if (free_.empty())
+            return cudaHostAlloc(reinterpret_cast<void **>(&p), 16, cudaHostAllocPortable) == cudaSuccess ? p : nullptr;
+        p = free_.back();
+        free_.pop_back();
+        return p;
+    }
+    void give_back(unsigned long long *p)
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (p >= page_ && p < page_ + 2 * kSlots)
+            free_.push_back(p);
+        else
+            cudaFreeHost(p);
+    }
+
+private:
+    static constexpr int kSlots = 256;
+    std::mutex mu_;
+    unsigned long long *page_ = nullptr;
+    std::vector<unsigned long long *> free_;
+};
+PinnedTotals &pinned_totals()
+{
+    static PinnedTotals *t = new PinnedTotals();  // outlives every plan
+    return *t;
+}
+
 }  // namespace
 
 // A batch prepared once and run as one CUDA-graph launch: a memset of the run's totals, the weight
@@ -954,7 +998,7 @@ struct BatchedPlan
     cudaStream_t caller = nullptr;  // the caller's stream: a run starts after its queued work
     cudaStream_t stream = nullptr;  // the plan's own stream (graphs cannot be captured on the legacy stream)
     cudaEvent_t ready = nullptr, begin = nullptr, end = nullptr;
-    std::vector<void *> allocs;
+    uint8_t *memory = nullptr;  // all of the plan's buffers and tables
     unsigned long long *totals = nullptr;       // device: events, then the error word
     unsigned long long *totals_host = nullptr;  // pinned copy, written by the run
     uint32_t *record = nullptr;
@@ -967,8 +1011,8 @@ struct BatchedPlan
     {
         if (exec) cudaGraphExecDestroy(exec);
         if (stream) cudaStreamSynchronize(stream);
-        for (void *p : allocs) cudaFree(p);
-        if (totals_host) cudaFreeHost(totals_host);
+        if (memory) cudaFree(memory);
+        if (totals_host) pinned_totals().give_back(totals_host);
         if (ready) cudaEventDestroy(ready);
         if (begin) cudaEventDestroy(begin);
         if (end) cudaEventDestroy(end);
@@ -1140,20 +1184,6 @@ int batched_plan_create(
         best = -autotune;
         autotune = 0;
     }
-    auto dalloc = [&](size_t bytes) -> void *
-    {
-        void *q = nullptr;
-        if (cudaMalloc(&q, bytes ? bytes : 16) != cudaSuccess) return nullptr;
-        p.allocs.push_back(q);
-        return q;
-    };
-    auto upload = [&](const void *src, size_t bytes) -> void *
-    {
-        void *q = dalloc(bytes);
-        if (q && cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
-        return q;
-    };
-    bool ok = true;
     const uint32_t t_max = *std::max_element(steps, steps + batch);
     // Rows of layer l have wp[l] words: whole 128-neuron tiles, 16-byte aligned.
     uint32_t wp[kMaxLayers + 1], words[kMaxLayers + 1], tiles[kMaxLayers + 1], wp_most = 4;
@@ -1172,6 +1202,17 @@ int batched_plan_create(
     if (segment_steps) seg_steps = std::min(seg_steps, segment_steps);
     const uint32_t n_segs = (t_max + seg_steps - 1) / seg_steps;
 
+    // One device allocation and one copy for all of the plan's buffers and tables (one each cost 10 us and
+    // more: 11 ms instead of 3 for a plan of 300 segments). Below, what
+    // will be device pointers are offsets from its start until it is there.
+    std::vector<uint8_t> tables;
+    auto table = [&](const void *src, size_t bytes) -> size_t
+    {
+        tables.resize((tables.size() + 15) / 16 * 16);
+        const size_t at = tables.size();
+        tables.insert(tables.end(), static_cast<const uint8_t *>(src), static_cast<const uint8_t *>(src) + bytes);
+        return at;
+    };
     // Packed weights.
     p.pack.n_layers = n_layers;
     for (int l = 0; l < n_layers; ++l)
@@ -1182,16 +1223,10 @@ int batched_plan_create(
         p.pack.k[l] = sizes[l];
         p.pack.chunks[l] = chunks;
         p.pack.first[l + 1] = p.pack.first[l] + static_cast<unsigned long long>(tiles[l + 1]) * chunks * kTileN * 8;
-        ok = ok && (p.pack.out[l] = static_cast<uint8_t *>(dalloc(static_cast<size_t>(tiles[l + 1]) * chunks * kAChunk)));
     }
-    const uint32_t *d_size[kMaxLayers + 1] = {};
-    if (sample_sizes)
-        for (int l = 0; l <= n_layers && ok; ++l)
-            ok = (d_size[l] = static_cast<const uint32_t *>(
-                      upload(sample_sizes + static_cast<size_t>(l) * batch, batch * 4ull))) != nullptr;
-    ok = ok && (p.totals = static_cast<unsigned long long *>(dalloc(16))) != nullptr;
-    ok = ok && cudaHostAlloc(reinterpret_cast<void **>(&p.totals_host), 16, cudaHostAllocDefault) == cudaSuccess;
-    auto *d_err = reinterpret_cast<unsigned int *>(p.totals + 1);
+    size_t size_at[kMaxLayers + 1] = {};
+    for (int l = 0; sample_sizes && l <= n_layers; ++l)
+        size_at[l] = table(sample_sizes + static_cast<size_t>(l) * batch, batch * 4ull);
 
     // Segments: every sample's columns and rows; per layer the streams, samples dealt longest first to
     // the shortest stream so far.
@@ -1199,8 +1234,13 @@ int batched_plan_create(
     std::vector<uint32_t> order(batch);
     for (uint32_t b = 0; b < batch; ++b) order[b] = b;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return steps[x] > steps[y]; });
+    struct SegmentTables
+    {
+        size_t rows, tab[kMaxLayers], info[kMaxLayers];
+    };
+    std::vector<SegmentTables> seg_at(n_segs);
     p.segs.resize(n_segs);
-    for (uint32_t sg = 0; sg < n_segs && ok; ++sg)
+    for (uint32_t sg = 0; sg < n_segs; ++sg)
     {
         BatchedPlan::Segment &seg = p.segs[sg];
         const uint32_t t0 = sg * seg_steps, t1 = std::min(t_max, t0 + seg_steps);
@@ -1213,14 +1253,12 @@ int batched_plan_create(
             at += cols ? cols + 1 : 0;
         }
         rows_most = std::max(rows_most, at);
-        seg.draw.rows = static_cast<const uint4 *>(upload(rows.data(), batch * sizeof(uint4)));
-        ok = ok && seg.draw.rows;
+        seg_at[sg].rows = table(rows.data(), batch * sizeof(uint4));
         seg.draw.t0 = t0;
         seg.draw.blocks = (t1 - t0 + 1 + 31) / 32;
-        const uint32_t *tab = nullptr;
-        const uint4 *info_d = nullptr;
+        size_t tab = 0, info_at = 0;
         uint32_t groups = 0;
-        for (int l = 0; l < n_layers && ok; ++l)
+        for (int l = 0; l < n_layers; ++l)
         {
             const uint32_t n_pairs = (tiles[l + 1] + 1) / 2;
             const uint32_t want = std::max(1u, std::min((batch + 1) / 2, static_cast<uint32_t>(sms) / 2 / n_pairs));
@@ -1259,52 +1297,66 @@ int batched_plan_create(
                 }
                 t[2 * groups] = static_cast<uint32_t>(start.size());
                 t.insert(t.end(), start.begin(), start.end());
-                tab = static_cast<const uint32_t *>(upload(t.data(), t.size() * 4));
-                info_d = static_cast<const uint4 *>(upload(info.data(), info.size() * sizeof(uint4)));
-                ok = tab && info_d;
+                tab = table(t.data(), t.size() * 4);
+                info_at = table(info.data(), info.size() * sizeof(uint4));
             }
             LayerArgs &a = seg.layer[l];
-            a.st_off = tab;
-            a.st_len = tab + 2 * groups + 1;
-            a.st_start = tab + 4 * groups + 1;
-            a.st_info = info_d;
+            seg_at[sg].tab[l] = tab;
+            seg_at[sg].info[l] = info_at;
             a.n_groups = groups;
             a.t0 = t0;
             a.t1 = t1;
             seg.grid[l] = 2 * n_pairs * groups;
         }
     }
-    uint32_t *bits[kMaxLayers] = {}, *state[kMaxLayers] = {}, *carry[kMaxLayers] = {};
-    for (int l = 0; l < n_layers && ok; ++l)
+    size_t total = 0;
+    auto carve = [&](size_t bytes)
     {
-        ok = (bits[l] = static_cast<uint32_t *>(dalloc(rows_most * wp[l] * 4))) != nullptr;
-        if (ok && n_segs > 1)
-        {
-            state[l] = static_cast<uint32_t *>(dalloc(static_cast<size_t>(batch) * sizes[l + 1] * 12));
-            carry[l] = static_cast<uint32_t *>(dalloc(static_cast<size_t>(batch) * wp[l + 1] * 4));
-            ok = state[l] && carry[l];
-        }
+        const size_t at = total;
+        total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+        return at;
+    };
+    const size_t totals_at = carve(16), tables_at = carve(tables.size());
+    size_t pack_at[kMaxLayers], bits_at[kMaxLayers], state_at[kMaxLayers] = {}, carry_at[kMaxLayers] = {};
+    for (int l = 0; l < n_layers; ++l)
+    {
+        pack_at[l] = carve(static_cast<size_t>(tiles[l + 1]) * p.pack.chunks[l] * kAChunk);
+        bits_at[l] = carve(rows_most * wp[l] * 4);
+        if (n_segs == 1) continue;
+        state_at[l] = carve(static_cast<size_t>(batch) * sizes[l + 1] * 12);
+        carry_at[l] = carve(static_cast<size_t>(batch) * wp[l + 1] * 4);
     }
-    if (!ok)
+    if (cudaMalloc(reinterpret_cast<void **>(&p.memory), total) != cudaSuccess ||
+        cudaMemcpyAsync(p.memory + tables_at, tables.data(), tables.size(), cudaMemcpyHostToDevice, p.stream) != cudaSuccess ||
+        cudaStreamSynchronize(p.stream) != cudaSuccess ||
+        !(p.totals_host = pinned_totals().take()))
     {
         *why = "device allocation failed";
         return -5;
     }
+    p.totals = reinterpret_cast<unsigned long long *>(p.memory + totals_at);
+    auto *d_err = reinterpret_cast<unsigned int *>(p.totals + 1);
+    auto words_at = [&](size_t at) { return reinterpret_cast<uint32_t *>(p.memory + at); };
+    auto table_at = [&](size_t at) { return reinterpret_cast<const uint32_t *>(p.memory + tables_at + at); };
+    for (int l = 0; l < n_layers; ++l) p.pack.out[l] = p.memory + pack_at[l];
     p.record = record;
     p.record_bytes = static_cast<size_t>(t_max) * rec_stride * 4;
-    for (auto &seg : p.segs)
+    for (uint32_t sg = 0; sg < n_segs; ++sg)
     {
+        BatchedPlan::Segment &seg = p.segs[sg];
+        const SegmentTables &at = seg_at[sg];
         DrawArgs &d = seg.draw;
+        d.rows = reinterpret_cast<const uint4 *>(table_at(at.rows));
         d.rates = rates;
         d.n_in = sizes[0];
         d.wp = wp[0];
         d.words = words[0];
         d.batch = batch;
-        d.size0 = d_size[0];
-        d.size1 = d_size[1];
+        d.size0 = sample_sizes ? table_at(size_at[0]) : nullptr;
+        d.size1 = sample_sizes ? table_at(size_at[1]) : nullptr;
         d.n1 = sizes[1];
         d.key = key;
-        d.bits = bits[0];
+        d.bits = words_at(bits_at[0]);
         d.record = record;
         d.rec_stride = rec_stride;
         d.events = p.totals;
@@ -1318,9 +1370,13 @@ int batched_plan_create(
                 *why = "could not describe the packed weights to the TMA unit";
                 return -3;
             }
-            a.bits_in = bits[l];
+            a.st_off = table_at(at.tab[l]);
+            a.st_len = a.st_off + 2 * a.n_groups + 1;
+            a.st_start = a.st_off + 4 * a.n_groups + 1;
+            a.st_info = reinterpret_cast<const uint4 *>(table_at(at.info[l]));
+            a.bits_in = words_at(bits_at[l]);
             a.wp_in = wp[l];
-            a.bits_out = last ? nullptr : bits[l + 1];
+            a.bits_out = last ? nullptr : words_at(bits_at[l + 1]);
             a.wp_out = wp[l + 1];
             a.n = sizes[l + 1];
             a.kp = (sizes[l] + 15) / 16 * 16;
@@ -1329,11 +1385,11 @@ int batched_plan_create(
             a.thr = threshold ? threshold[l] : 1.0f;
             a.reset = reset ? reset[l] : 0.0f;
             a.refract = refract ? refract[l] : 0u;
-            a.own_size = d_size[l + 1];
-            a.next_size = last ? nullptr : d_size[l + 2];
+            a.own_size = sample_sizes ? table_at(size_at[l + 1]) : nullptr;
+            a.next_size = last || !sample_sizes ? nullptr : table_at(size_at[l + 2]);
             a.next_n = last ? 0u : sizes[l + 2];
-            a.carry = carry[l];
-            a.state = state[l];
+            a.carry = n_segs > 1 ? words_at(carry_at[l]) : nullptr;
+            a.state = n_segs > 1 ? words_at(state_at[l]) : nullptr;
             a.counts = last ? counts : nullptr;
             a.record = record;
             a.rec_off = rec_off[l + 1];

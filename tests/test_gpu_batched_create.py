@@ -1,0 +1,66 @@
+"""Making a batched plan: the time does not grow by an allocation and a copy for every segment, and plans of many
+segments, uneven sizes and recorded spikes are as they were."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_many_segments_do_not_multiply_the_time_to_make_a_plan():
+    """300 one-step segments (900 kernels to capture) within 10 times one segment's 0.45 ms (7 times; 15 with an allocation
+    and a copy for each table)."""
+    from knp_gb300 import batched
+
+    cfg = batched.dense_config(batch=32, sizes=(100, 50, 10), t_lo=300, t_hi=300)
+    took = []
+    for segment_steps in (0, 1):
+        times = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            plan = batched.BatchedPlan(cfg, segment_steps=segment_steps)
+            times.append(time.perf_counter() - t0)
+            plan.close()
+        took.append(min(times))
+    assert took[1] < 10 * took[0], took
+
+
+@pytest.mark.parametrize("uneven", [False, True])
+@pytest.mark.parametrize("segment_steps", [1, 7])
+def test_segments_with_uneven_sizes_and_record(uneven, segment_steps):
+    from knp_gb300 import batched
+
+    cfg = batched.uneven_config(batch=13) if uneven else batched.dense_config(batch=13, sizes=(130, 257, 140, 5), t_lo=3, t_hi=30)
+    out = []
+    for seg in (0, segment_steps):
+        plan = batched.BatchedPlan(cfg, record=True, segment_steps=seg)
+        events, _ = plan.run()
+        out.append((events, plan.counts(), plan.record()))
+        assert plan.run()[0] == events
+        plan.close()
+    assert out[0][0] == out[1][0] > 0
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    for layer in out[0][2]:
+        np.testing.assert_array_equal(out[0][2][layer], out[1][2][layer])
+
+
+def test_more_plans_alive_than_pinned_totals_are_shared_by():
+    """300 plans made by 4 threads, run in turn, given up in another order and made again: every run has its own totals."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from knp_gb300 import batched
+
+    cfgs = [batched.dense_config(seed=s, batch=2, sizes=(20, 10, 4), t_lo=2, t_hi=6) for s in range(5)]
+    with ThreadPoolExecutor(4) as ex:
+        plans = list(ex.map(lambda i: batched.BatchedPlan(cfgs[i % 5]), range(300)))
+        ref = [plans[i].run()[0] for i in range(5)]
+        assert len(set(ref)) > 1
+        assert [p.run()[0] for p in plans] == ref * 60
+        for p in plans[::2]:
+            p.close()
+        again = list(ex.map(lambda i: batched.BatchedPlan(cfgs[i % 5]), range(40)))
+    assert [p.run()[0] for p in again] == ref * 8
+    assert [p.run()[0] for p in plans[1::2]] == [ref[i % 5] for i in range(1, 300, 2)]
+    for p in plans[1::2] + again:
+        p.close()
