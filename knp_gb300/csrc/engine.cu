@@ -1590,6 +1590,16 @@ void Backend::build_small_net()
             spikes_alt_.emplace_back(list, arena_.make<uint32_t>(std::max<uint32_t>(q->n_pad, 4), false));
         }
     }
+    // Both sets' descriptors go to the device in one copy.
+    std::vector<uint8_t> host;
+    size_t at[2][4];
+    auto put = [&](const void *src, size_t bytes)
+    {
+        const size_t where = (host.size() + 15) / 16 * 16;
+        host.resize(where + std::max<size_t>(bytes, 16));
+        if (bytes) std::memcpy(host.data() + where, src, bytes);
+        return where;
+    };
     for (int set = 0; set < 2; ++set)
     {
         uint32_t *base = set ? counters_alt_ : counters_;
@@ -1650,37 +1660,31 @@ void Backend::build_small_net()
             }
             rules.push_back(r);
         }
-        if (!small_.pops[0])
-        {
-            small_.n_pops = static_cast<uint32_t>(pops.size());
-            small_.n_projs = static_cast<uint32_t>(projs.size());
-            small_.n_stdp = static_cast<uint32_t>(rules.size());
-            small_.n_sources = static_cast<uint32_t>(sources.size());
-            uint64_t words = 0;
-            for (auto &q : pops_) words += (static_cast<uint64_t>(q->n) + 3) / 4 * 4;
-            small_.list_words = static_cast<uint32_t>(std::min<uint64_t>(words, 0xFFFFFFFFu));
-            SmallPop *dp = arena_.make<SmallPop>(2 * std::max<size_t>(pops.size(), 1));
-            ProjectionDev *dj = arena_.make<ProjectionDev>(2 * std::max<size_t>(projs.size(), 1));
-            SmallStdp *ds = arena_.make<SmallStdp>(2 * std::max<size_t>(rules.size(), 1));
-            SmallSource *dq = arena_.make<SmallSource>(2 * std::max<size_t>(sources.size(), 1));
-            for (int k = 0; k < 2; ++k)
-            {
-                small_.pops[k] = dp + k * std::max<size_t>(pops.size(), 1);
-                small_.projs[k] = dj + k * std::max<size_t>(projs.size(), 1);
-                small_.stdp[k] = ds + k * std::max<size_t>(rules.size(), 1);
-                small_.sources[k] = dq + k * std::max<size_t>(sources.size(), 1);
-            }
-        }
+        small_.n_pops = static_cast<uint32_t>(pops.size());
+        small_.n_projs = static_cast<uint32_t>(projs.size());
+        small_.n_stdp = static_cast<uint32_t>(rules.size());
+        small_.n_sources = static_cast<uint32_t>(sources.size());
         small_.end[set] = StepEnd{base, n_counters_, n_spike_counters_};
-        KNP_CUDA(cudaMemcpy(const_cast<SmallPop *>(small_.pops[set]), pops.data(), pops.size() * sizeof(SmallPop),
-                            cudaMemcpyHostToDevice));
-        KNP_CUDA(cudaMemcpy(const_cast<ProjectionDev *>(small_.projs[set]), projs.data(),
-                            projs.size() * sizeof(ProjectionDev), cudaMemcpyHostToDevice));
-        KNP_CUDA(cudaMemcpy(const_cast<SmallStdp *>(small_.stdp[set]), rules.data(), rules.size() * sizeof(SmallStdp),
-                            cudaMemcpyHostToDevice));
-        KNP_CUDA(cudaMemcpy(const_cast<SmallSource *>(small_.sources[set]), sources.data(),
-                            sources.size() * sizeof(SmallSource), cudaMemcpyHostToDevice));
+        at[set][0] = put(pops.data(), pops.size() * sizeof(SmallPop));
+        at[set][1] = put(projs.data(), projs.size() * sizeof(ProjectionDev));
+        at[set][2] = put(rules.data(), rules.size() * sizeof(SmallStdp));
+        at[set][3] = put(sources.data(), sources.size() * sizeof(SmallSource));
     }
+    if (!small_desc_)
+    {
+        small_desc_ = static_cast<uint8_t *>(arena_.alloc(host.size(), false));
+        for (int set = 0; set < 2; ++set)
+        {
+            small_.pops[set] = reinterpret_cast<const SmallPop *>(small_desc_ + at[set][0]);
+            small_.projs[set] = reinterpret_cast<const ProjectionDev *>(small_desc_ + at[set][1]);
+            small_.stdp[set] = reinterpret_cast<const SmallStdp *>(small_desc_ + at[set][2]);
+            small_.sources[set] = reinterpret_cast<const SmallSource *>(small_desc_ + at[set][3]);
+        }
+        uint64_t words = 0;
+        for (auto &q : pops_) words += (static_cast<uint64_t>(q->n) + 3) / 4 * 4;
+        small_.list_words = static_cast<uint32_t>(std::min<uint64_t>(words, 0xFFFFFFFFu));
+    }
+    KNP_CUDA(cudaMemcpy(small_desc_, host.data(), host.size(), cudaMemcpyHostToDevice));
     if (fused_) small_cluster_ = small_net_cluster(small_);
 }
 

@@ -358,6 +358,7 @@ private:
     int step_mode_ = 0;  // knp_gb300_step_mode
     bool fused_ = false;
     SmallNet small_{};
+    uint8_t *small_desc_ = nullptr;  // device: both descriptor sets
     int small_cluster_ = 1;  // CTAs of the fused kernel's cluster
     uint32_t *counters_alt_ = nullptr;  // the fused kernel's second set of per-step counters
     std::vector<std::pair<const uint32_t *, uint32_t *>> spikes_alt_;  // spike list -> its second copy
