@@ -978,7 +978,8 @@ void Backend::build_projection(ProjectionSlot &p)
             KNP_CUDA(cudaMemcpyAsync(d_type, p.type.data(), S, cudaMemcpyHostToDevice, stream_));
         }
     }
-    p.row_ptr = arena_.make<long long>(static_cast<size_t>(p.n_rows) + 1);
+    // (One word more than the CSR's: see find_short_rows.)
+    p.row_ptr = arena_.make<long long>(static_cast<size_t>(p.n_rows) + 2);
     uint32_t *perm = arena_.make<uint32_t>(S, false);
     size_t temp_need = 0;
     KNP_CUDA(build_csr(S, p.n_rows, d_key, perm, p.row_ptr, nullptr, 0, &temp_need, stream_));
@@ -1013,9 +1014,6 @@ void Backend::build_projection(ProjectionSlot &p)
     ProjectionDev &d = p.dev;
     d.row_ptr = p.row_ptr;
     d.n_rows = p.n_rows;
-    uint32_t longest = 0;
-    if (p.n_syn <= 2 * static_cast<uint64_t>(p.n_rows)) KNP_CUDA(longest_row(p.row_ptr, p.n_rows, &longest, stream_));
-    d.short_rows = p.n_syn <= 2 * static_cast<uint64_t>(p.n_rows) && longest <= kShortRow ? 1 : 0;
     d.col = p.col;
     d.w = p.w;
     d.delay = p.delay_d;
@@ -1801,6 +1799,33 @@ void Backend::enqueue_step()
     launch_step_end(e, ctl_, stream_);
 }
 
+// Which projections the per-phase scatter takes a lane per row; looked up when that scatter is first needed.
+void Backend::find_short_rows()
+{
+    if (short_rows_known_) return;
+    short_rows_known_ = true;
+    std::vector<ProjectionSlot *> few;
+    for (auto &p : projs_)
+        if (p->n_syn && p->n_syn <= 2 * static_cast<uint64_t>(p->n_rows)) few.push_back(p.get());
+    // Through the pinned copy of the control block, a few at a time, from the word behind the CSR's row bounds.
+    auto *host = reinterpret_cast<volatile uint32_t *>(ctl_host_);
+    constexpr size_t kAtATime = sizeof(Control) / sizeof(uint32_t);
+    for (size_t k0 = 0; k0 < few.size(); k0 += kAtATime)
+    {
+        const size_t n = std::min(kAtATime, few.size() - k0);
+        for (size_t k = 0; k < n; ++k)
+        {
+            const ProjectionSlot &p = *few[k0 + k];
+            auto *out = reinterpret_cast<uint32_t *>(p.row_ptr + p.n_rows + 1);
+            KNP_CUDA(launch_longest_row(p.row_ptr, p.n_rows, out, stream_));
+            KNP_CUDA(cudaMemcpyAsync(reinterpret_cast<uint32_t *>(ctl_host_) + k, out, sizeof(uint32_t),
+                                     cudaMemcpyDeviceToHost, stream_));
+        }
+        KNP_CUDA(cudaStreamSynchronize(stream_));
+        for (size_t k = 0; k < n; ++k) few[k0 + k]->dev.short_rows = host[k] <= kShortRow ? 1 : 0;
+    }
+}
+
 void Backend::capture_graphs()
 {
     KNP_CUDA(cudaStreamSynchronize(stream_));
@@ -1819,6 +1844,7 @@ void Backend::capture_graphs()
         }
         return;
     }
+    find_short_rows();
     for (int which = 0; which < 2; ++which)
     {
         cudaGraph_t g = nullptr;
@@ -2075,6 +2101,7 @@ void Backend::profile_phases(uint64_t n, float *ms)
     bool host_inputs = !pending_impacts_.empty();
     for (auto &c : channels_) host_inputs = host_inputs || c->has_pending;
     if (host_inputs) throw Error(KNP_GB300_E_STATE, "profile_phases does not stage host messages");
+    find_short_rows();
     cudaEvent_t ev[5];
     for (auto &e : ev) KNP_CUDA(cudaEventCreate(&e));
     double acc[4] = {0, 0, 0, 0};

@@ -321,6 +321,8 @@ private:
     void build_small_net();
     void setup_ring_window();
     void capture_graphs();
+    void find_short_rows();
+    bool short_rows_known_ = false;
     void stage_host_inputs();
     void drain_recordings() { drain_recordings(step_); }
     void drain_recordings(uint64_t upto);

@@ -442,11 +442,11 @@ uint32_t blifat_batch_blocks(uint32_t n);  // blocks of a population of n in a b
 void launch_blifat_batch(const BlifatBatch &b, Control *ctl, cudaStream_t s);
 void launch_train_batch(const TrainBatch &b, Control *ctl, cudaStream_t s);
 void launch_projection_batch(const ProjectionBatch &b, Control *ctl, cudaStream_t s);
-// Synapses of a CSR's longest row (waits for the stream). A lane walks a row of kShortRow at most by itself; with
+// Synapses of a CSR's longest row, to *longest on the device (zero before). A lane walks a row of kShortRow at most by itself; with
 // longer ones among them, walked by the warp one after another, ten rows of 20000 took 238 us a step where parts
 // dealt to the warps take 120, and 2000 of 100 took 23.9 against 20.3.
 constexpr uint32_t kShortRow = 8;
-cudaError_t longest_row(const long long *row_ptr, uint32_t n_rows, uint32_t *longest, cudaStream_t s);
+cudaError_t launch_longest_row(const long long *row_ptr, uint32_t n_rows, uint32_t *longest, cudaStream_t s);
 void launch_resource_train(const TrainView &p, int blocks, Control *ctl, cudaStream_t s);
 void launch_altai(const AltaiDev &p, Control *ctl, cudaStream_t s);
 void launch_altai_blocking(const AltaiDev &p, Control *ctl, cudaStream_t s);

@@ -227,22 +227,11 @@ void launch_projection_batch(const ProjectionBatch &b, Control *ctl, cudaStream_
     launch_pdl(projection_batch_kernel, dim3(b.blocks()), dim3(256), 0, s, b, ctl);
 }
 
-cudaError_t longest_row(const long long *row_ptr, uint32_t n_rows, uint32_t *longest, cudaStream_t s)
+cudaError_t launch_longest_row(const long long *row_ptr, uint32_t n_rows, uint32_t *longest, cudaStream_t s)
 {
-    unsigned int *d = nullptr;
-    cudaError_t err = cudaMallocAsync(reinterpret_cast<void **>(&d), sizeof(*d), s);
-    if (err != cudaSuccess) return err;
-    err = cudaMemsetAsync(d, 0, sizeof(*d), s);
-    if (err == cudaSuccess)
-    {
-        const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((n_rows + 255ull) / 256, 1024));
-        longest_row_kernel<<<std::max(blocks, 1u), 256, 0, s>>>(row_ptr, n_rows, d);
-        err = cudaGetLastError();
-    }
-    if (err == cudaSuccess) err = cudaMemcpyAsync(longest, d, sizeof(*d), cudaMemcpyDeviceToHost, s);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-    cudaFreeAsync(d, s);
-    return err;
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((n_rows + 255ull) / 256, 1024));
+    longest_row_kernel<<<std::max(blocks, 1u), 256, 0, s>>>(row_ptr, n_rows, longest);
+    return cudaGetLastError();
 }
 
 }  // namespace knp_gb300
