@@ -8,22 +8,33 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def test_many_segments_do_not_multiply_the_time_to_make_a_plan():
-    """300 one-step segments (900 kernels to capture) within 10 times one segment's 0.45 ms (7 times; 15 with an allocation
-    and a copy for each table)."""
+def test_many_segments_take_less_than_capturing_as_many_kernels_elsewhere():
+    """A plan of 300 one-step segments, 900 kernels, is made in less time than torch takes to capture 900 element-wise
+    ones (0.45 times; 1.3 times with an allocation and a copy for every segment's tables)."""
+    import torch
+
     from knp_gb300 import batched
 
     cfg = batched.dense_config(batch=32, sizes=(100, 50, 10), t_lo=300, t_hi=300)
+    x = torch.zeros(8, device="cuda")
+
+    def capture():
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            for _ in range(900):
+                x.add_(1)
+
+    def plan():
+        batched.BatchedPlan(cfg, segment_steps=1).close()
+
     took = []
-    for segment_steps in (0, 1):
+    for f in (plan, capture):
         times = []
         for _ in range(6):
             t0 = time.perf_counter()
-            plan = batched.BatchedPlan(cfg, segment_steps=segment_steps)
+            f()
             times.append(time.perf_counter() - t0)
-            plan.close()
         took.append(min(times))
-    assert took[1] < 10 * took[0], took
+    assert took[0] < took[1], took
 
 
 @pytest.mark.parametrize("uneven", [False, True])
