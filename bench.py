@@ -445,7 +445,7 @@ def bptt_measure(device: int, iters: int = 10, warmup: int = 3):
         return e0.elapsed_time(e1) / iters, float(out.item())
 
     ms_eager, _ = timed(it)
-    # The same iteration captured as one CUDA graph (the eager loop is bound by ~70 launches from Python).
+    # The same iteration captured as one CUDA graph (the eager loop is bound by its launches from Python).
     graphed = bptt.GraphedTrainStep(model, opt, x, labels)
     ms, loss = timed(graphed)
     layers = [(784, 512), (512, 512), (512, 10)]

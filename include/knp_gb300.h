@@ -481,7 +481,9 @@ KNP_GB300_API int knp_gb300_bf16_gemm_tn(
  * generator of knp_gb300/network.py; a rate below 0 or NaN never fires, 1 or above always). Outputs: d_counts[batch][sizes[n_layers]] (device, int32) output
  * spike counts; optional d_record (device, uint32) with every layer's spike bitmap of every step,
  * laid out [max(steps)][layer 0..n_layers][batch][ceil(sizes[l] / 32)]; *events (host) synaptic events
- * (spikes x fan-out of their layer); *ms (host) device time of the run. Synchronous.
+ * (spikes x fan-out of their layer); *ms (host) device time of the run. Synchronous. Size limit:
+ * 2 sum over l >= 1 of ceil(batch / 128) ceil(sizes[l] / 64) is at most the device's SMs (256 samples of
+ * 784-1000-1000-10: 132 of 152); larger batches are refused and run as several.
  */
 KNP_GB300_API int knp_gb300_batched_lif_run(
     int n_layers, const uint32_t *sizes, const void *const *d_weights, const float *leak, const float *threshold,

@@ -4,8 +4,9 @@ A feed-forward LIF network (all-to-all layers, membrane decay beta, threshold th
 subtraction) is trained on spike counts. Per layer the synaptic input of all T steps is one GEMM of
 the previous layer's spikes with the layer's weights (BF16 values of the FP32 master weights,
 products exact in FP32, FP32 accumulation), with the LIF recurrence over T, and its backward, in the
-same kernel (knp_gb300/csrc/lif_gemm.cu) behind ``LIFLayerFn`` (torch.autograd.Function); the relaxed
-forward and long checkpoint intervals take product and scan apart (knp_gb300/csrc/bptt.cu).
+same kernel (knp_gb300/csrc/lif_gemm.cu) behind ``LIFLayerFn`` (torch.autograd.Function). Layers of many
+inputs whose product fills few tiles, and the relaxed forward, take product and scan apart
+(knp_gb300/csrc/bptt.cu). Checkpoint intervals are 1 to 16 steps.
 The forward keeps the membrane state only every ``checkpoint`` steps; the backward recomputes each
 segment. The reference has no gradient-based training; this form has no counterpart there.
 
@@ -229,8 +230,8 @@ def loss_fn(counts, labels):
 
 class GraphedTrainStep:
     """One training iteration (forward, loss, backward, optimizer step) on the static tensors ``x`` and
-    ``labels``, captured once as a CUDA graph and replayed by ``__call__``; the iteration's ~70
-    kernels then cost one launch. New data is copied into ``x`` / ``labels`` in place. The optimizer
+    ``labels``, captured once as a CUDA graph and replayed by ``__call__``; the iteration's
+    kernels (29 for three layers) then cost one launch. New data is copied into ``x`` / ``labels`` in place. The optimizer
     must be graph-safe (SGD; Adam with ``capturable=True``). Warm-up iterations run on a side stream
     first, as torch's graph capture asks."""
 

@@ -161,7 +161,7 @@ int bf16_gemm_tn_simple(const void *A, const void *B, float *D, int M, int N, in
 // the recurrence down its row with the membrane state in registers, and no step waits for another
 // CTA. (Stepping all layers together, one step at a time, costs a chain of expansion, product,
 // exchange and hand-over per step: 0.95 ms for 256 samples of 784-1000-1000-10 and 50-200 steps, the
-// tensor cores idle for most of it; this form takes 0.24 ms.)
+// tensor cores idle for most of it; this form takes 0.218 ms.)
 //
 // Spikes travel between layers as bitmaps: per layer one row of wpad words (bit j of word w = neuron
 // 32 w + j) for every (sample, step) of a segment of steps, a sample's rows consecutive:
@@ -200,7 +200,7 @@ constexpr uint32_t kNoRow = 0xFFFFFFFFu;
 constexpr uint32_t kMaxFanIn = 2048;
 constexpr size_t kMinDynSmem = size_t(120) << 10;  // one CTA per SM (a second would wait for tensor memory)
 constexpr size_t kRowBudget = size_t(256) << 20;   // bytes of a layer's rows per segment
-constexpr uint32_t kMaxTiles = 512;  // (layer, 128-sample tile, 64-neuron tile, half) units a plan may have
+constexpr uint32_t kMaxTiles = 512;  // see the size limit in batched_plan_create
 
 // What one launch of a layer needs. A stream is a list of samples whose columns follow one another;
 // CTA pair (pair of n tiles, g) runs streams 2 g and 2 g + 1 side by side, one per half of its columns:
@@ -1159,7 +1159,8 @@ int batched_plan_create(
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    // The batch size a plan takes: (layer, 128-sample tile, 64-neuron tile, half) units, one SM each.
+    // The size limit of the interface (knp_gb300.h), kept as it was: pairs of 128-sample and 64-neuron tiles, two a
+    // layer, at most one per SM. The kernel itself takes any number of columns.
     unsigned long long units = 0;
     for (int l = 1; l <= n_layers; ++l) units += 2ull * ((batch + 127) / 128) * ((sizes[l] + 63) / 64);
     if (units > kMaxTiles)

@@ -418,8 +418,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) gemm_tma_kernel(
 // tile each CTA stages 128 rows of A and 128 of B and the tensor cores of both read B's two halves: 64 KB
 // and 512 cycles per CTA. Persistent (one pair per two SMs) with two accumulators, so the read-back of a
 // tile overlaps the next tile's product; tiles are taken in bands of kPairBand rows of tiles, so that
-// the pairs at work share A and B in L2. 8192^3: 634 us, 1.73 PFLOP/s; 2048 x 2048 x 32768: 325 -> 169
-// us; 16384 x 2048 x 2048: 133 -> 90 us. Both CTAs' copies are counted on the even CTA's barriers, whose
+// the pairs at work share A and B in L2. Calls in a row: 8192^3 629-640 us, 1.72-1.75 PFLOP/s (among other work, under
+// the power cap, 720 against 840); 2048 x 2048 x 32768: 325 -> 172 us; 16384 x 2048 x 2048: 133 -> 90 us. Both CTAs' copies are counted on the even CTA's barriers, whose
 // issuer waits with CTA-scope acquire: a relay of the odd CTA's copies by a cluster-scope wait and arrival
 // cost 2.2 ms at 8192^3.
 constexpr int kPairM = 256, kPairN = 256, kPairStages = 6, kPairBand = 8;

@@ -106,33 +106,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
         : "memory");
 }
 
-// As mma_bf16 with the A operand in tensor memory: rows of A in lanes 0..M-1, K along columns, two
-// 16-bit elements per 32-bit column (element 2c in the low half of column c).
-__device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// Thread t of warp w (w = warp index within its warpgroup) writes tensor-memory lane 32 w + t,
-// 16 consecutive 32-bit columns starting at `taddr`'s column.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *v)
-{
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
-            taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
-}
-
-// This thread's earlier tcgen05.st have completed.
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // The mbarrier at `mbar` receives one arrival when every previously issued tcgen05.mma of this
 // thread has completed.
 __device__ __forceinline__ void commit(uint64_t *mbar)
@@ -183,49 +156,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *mbar, uint32_t parity)
     return done != 0;
 }
 
-// One poll of mbar_wait_cluster.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *mbar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(smem_u32(mbar)), "r"(parity), "r"(kSuspendNs)
-        : "memory");
-    return done != 0;
-}
-
 // 32-bit store into the shared memory of another CTA of the cluster (address from mapa).
 __device__ __forceinline__ void st_cluster_u32(uint32_t remote_addr, uint32_t v)
 {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote_addr), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_nctarank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-
-// As mbar_wait, with cluster-scope acquire: for phases completed by another CTA of the cluster
-// (st.async with complete_tx into this CTA's shared memory).
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *mbar, uint32_t parity, uint32_t limit)
-{
-    const uint32_t a = smem_u32(mbar);
-    for (uint32_t i = 0; i < limit; ++i)
-    {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(a), "r"(parity), "r"(kSuspendNs)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // Address of the same shared-memory location in CTA `rank` of this cluster.
@@ -234,16 +168,6 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank)
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
-}
-
-// 16-byte store into another CTA's shared memory; its mbarrier `remote_mbar` counts the bytes.
-__device__ __forceinline__ void st_async_v4(uint32_t remote_addr, float a, float b, float c, float d,
-                                            uint32_t remote_mbar)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
-                     remote_addr),
-                 "f"(a), "f"(b), "f"(c), "f"(d), "r"(remote_mbar)
-                 : "memory");
 }
 
 // One arrival (release, CTA scope) on a shared-memory mbarrier.
@@ -393,7 +317,7 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
         : "memory");
 }
 
-// As tmem_ld16, 8 columns, and one column without the wait (tmem_wait_ld).
+// As tmem_ld16, 8 columns, and one column.
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v)
 {
     uint32_t r[8];
